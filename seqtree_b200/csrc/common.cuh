@@ -94,6 +94,7 @@ struct Context {
     DevBuf tq[3], tr[3];  // bytes, offsets, lengths
     // plans reused by transient sets (rebuilt in place for every call)
     std::shared_ptr<void> tmp_query_plan, tmp_ref_plan, tmp_wave_plan[2];
+    std::shared_ptr<void> tmp_strip_query_plan, tmp_strip_ref_plan;
     // query plan of a row block (sparse calls whose hits are taken in several blocks)
     std::shared_ptr<void> tmp_block_plan;
     // sparse result of the host-buffer sparse call (an st_hits_s)
@@ -163,7 +164,7 @@ struct st_seqset_s {
     bool owns = true;           // false: storage borrowed from the context (transient set)
     uint64_t uid = 0;           // unique per set; plans record the uid they were built for
     // plan caches (opaque; transient sets share the context's)
-    std::shared_ptr<void> gb_query_plan, gb_ref_plan, wave_plan;
+    std::shared_ptr<void> gb_query_plan, gb_ref_plan, wave_plan, strip_query_plan, strip_ref_plan;
     ~st_seqset_s();
 };
 

@@ -21,16 +21,19 @@
 
 namespace stb {
 
+// The strip kernel's path (gotoh_strip.cu).
+bool strip_eligible(const st_seqset_s& qs, const st_seqset_s& rs, const int32_t* sim, int A,
+                    int32_t go, int32_t ge);
+void align_strip(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int A, int32_t mode,
+                 int32_t go, int32_t ge, int32_t dist, const int64_t* q_self, const int64_t* r_self,
+                 int32_t* out_d, unsigned int* ovf, cudaStream_t stream);
+
 namespace {
 
 constexpr int64_t kNegInf = INT64_MIN / 4;  // src/pairwise.cpp:37
-// Pairs a first-time tuning of per-thread against the wavefront (32- or 64-row buckets) runs
-// each variant on.
+// Pairs a first-time tuning runs each alignment kernel on.  A slice much smaller than this does
+// not fill the GPU, and so favours the kernel with the finest tasks.
 constexpr int64_t kAlignTunePairs = int64_t(20) * 1000 * 1000;
-// Pairs a first-time tuning of the wavefront's row-bucket width runs each variant on.
-// A slice much smaller than this holds too few rows per bucket to fill the GPU, and so favours
-// the wider buckets (fewer launches) where the whole matrix favours the narrower ones.
-constexpr int64_t kWaveTunePairs = int64_t(20) * 1000 * 1000;
 
 __device__ __forceinline__ int64_t gap_run(int64_t L, int32_t open, int32_t extend) {
     return L <= 0 ? 0 : int64_t(open) + (L - 1) * int64_t(extend);
@@ -172,8 +175,6 @@ struct ThreadArgs {
     const int32_t* sim;
     int A;
     int32_t go, ge;
-    int self;            // 1: self scores of the query set into self_out
-    int64_t* self_out;
     int dist;
     const int64_t* q_self;
     const int64_t* r_self;
@@ -190,15 +191,15 @@ __global__ void __launch_bounds__(128) gotoh_thread_kernel(const ThreadArgs a) {
     extern __shared__ int32_t s_sim[];
     for (int i = threadIdx.x; i < a.A * a.A; i += blockDim.x) s_sim[i] = a.sim[i];
     __syncthreads();
-    const int64_t total = a.self ? a.N : a.N * a.K;
+    const int64_t total = a.N * a.K;
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < total; idx += stride) {
-        const int64_t i = a.self ? idx : idx / a.K;
-        const int64_t k = a.self ? idx : idx - i * a.K;
+        const int64_t i = idx / a.K;
+        const int64_t k = idx - i * a.K;
         const uint8_t* q = a.qc + a.qoff[i];
         const int m = int(a.qoff[i + 1] - a.qoff[i]);
-        const uint8_t* r = a.self ? q : a.rc + a.roff[k];
-        const int n = a.self ? m : int(a.roff[k + 1] - a.roff[k]);
+        const uint8_t* r = a.rc + a.roff[k];
+        const int n = int(a.roff[k + 1] - a.roff[k]);
         int32_t score;
         if (m == 0 || n == 0) {
             score = LOCAL ? 0 : -gap_run32(m ? m : n, a.go, a.ge);
@@ -294,10 +295,6 @@ __global__ void __launch_bounds__(128) gotoh_thread_kernel(const ThreadArgs a) {
             }
             score = LOCAL ? best : __vimax3_s32(lm, lx, ly);
         }
-        if (a.self) {
-            a.self_out[idx] = score;
-            continue;
-        }
         const int64_t v = a.dist ? a.q_self[i] + a.r_self[k] - 2 * int64_t(score) : int64_t(score);
         if (v < INT32_MIN || v > INT32_MAX) {
             atomicOr(a.overflow, 1u);
@@ -338,14 +335,123 @@ void launch_thread(Context& ctx, ThreadArgs a, int nmax, bool local, int64_t wor
     note_launch("gotoh_thread_kernel");
 }
 
+// -------------------------------------------------------------------------- self scores ---
+// Score of each sequence against itself, for the distance form: one warp per sequence, both sets
+// in one launch.  A residue is plain when its own score is not negative and no other residue's score
+// against it (in either order) exceeds that.  When every residue of a sequence is plain, no
+// alignment with itself beats the identity: a pair (i, j) scores at most s(i, i), each i is
+// paired once, residues left out would have added s(i, i) >= 0, and gaps cost at least 0.  The
+// answer is then the sum of s(i, i) (all of BLOSUM62 but X).  Other sequences (up to 512
+// residues) run the three-state recurrence as a wavefront over the warp: lane t owns rows 16 t + 1
+// .. 16 t + 16 and is at column s - t + 1 at step s.
+// Measured, B200, 4,096 + 4,096 junctions: 3 us, against 75 us for two launches of one thread per
+// sequence; proteins (median 180): 5 us, against about 120 us for a wavefront launch per row bucket.
+struct SelfArgs {
+    const uint8_t* codes[2];
+    const int64_t* off[2];
+    int64_t count[2];
+    const int32_t* sim;
+    int A;
+    uint32_t plain;      // bit c: residue c is plain
+    int local;
+    int32_t go, ge;
+    int64_t* out;        // count[0] + count[1]
+};
+
+constexpr int kSelfRows = 16;
+
+__global__ void __launch_bounds__(256) self_score_kernel(const SelfArgs a) {
+    extern __shared__ int32_t s_sim[];
+    for (int i = threadIdx.x; i < a.A * a.A; i += blockDim.x) s_sim[i] = a.sim[i];
+    __syncthreads();
+    const unsigned full = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
+    for (int64_t t = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; t < a.count[0] + a.count[1];
+         t += nw) {
+        const int side = t >= a.count[0];
+        const int64_t i = side ? t - a.count[0] : t;
+        const uint8_t* q = a.codes[side] + a.off[side][i];
+        const int m = int(a.off[side][i + 1] - a.off[side][i]);
+        long long sum = 0;
+        bool plain = true;
+        for (int j = lane; j < m; j += 32) {
+            const int c = q[j];
+            plain &= ((a.plain >> c) & 1u) != 0;
+            sum += s_sim[c * a.A + c];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(full, sum, o);
+        if (__all_sync(full, plain)) {
+            if (lane == 0) a.out[t] = sum;
+            continue;
+        }
+        int32_t M[kSelfRows], X[kSelfRows], Y[kSelfRows];  // column j - 1 of this lane's rows
+        const int row0 = lane * kSelfRows;
+#pragma unroll
+        for (int r = 0; r < kSelfRows; ++r) {
+            M[r] = a.local ? 0 : kNeg32;
+            X[r] = a.local ? kNeg32 : -gap_run32(row0 + r + 1, a.go, a.ge);
+            Y[r] = kNeg32;
+        }
+        // the row above this lane's first row, at column j - 1
+        int32_t dm = lane == 0 || a.local ? 0 : kNeg32;
+        int32_t dx = lane == 0 || a.local ? kNeg32 : -gap_run32(row0, a.go, a.ge);
+        int32_t dy = kNeg32, best = a.local ? 0 : kNeg32, end = kNeg32;
+        int32_t lm = 0, lx = 0, ly = 0;  // this lane's last row at the column it did last
+        for (int s = 0; s < m + 31; ++s) {
+            int32_t um = __shfl_up_sync(full, lm, 1), ux = __shfl_up_sync(full, lx, 1),
+                    uy = __shfl_up_sync(full, ly, 1);
+            const int j = s - lane + 1;
+            if (lane == 0) {
+                um = a.local ? 0 : kNeg32;
+                ux = kNeg32;
+                uy = a.local ? kNeg32 : -gap_run32(j, a.go, a.ge);
+            }
+            if (j < 1 || j > m || row0 >= m) continue;
+            const int cj = q[j - 1];
+            const int32_t tm = um, tx = ux, ty = uy;
+#pragma unroll
+            for (int r = 0; r < kSelfRows; ++r) {
+                const int row = row0 + r;
+                const int32_t sc = s_sim[int(q[row < m ? row : m - 1]) * a.A + cj];
+                int32_t mv = max(max(dm, dx), dy) + sc;
+                if (a.local) mv = max(mv, 0);
+                const int32_t xv = max(max(um, uy) - a.go, ux - a.ge);
+                const int32_t yv = max(max(M[r], X[r]) - a.go, Y[r] - a.ge);
+                dm = M[r];
+                dx = X[r];
+                dy = Y[r];
+                M[r] = um = mv;
+                X[r] = ux = xv;
+                Y[r] = uy = yv;
+                if (row < m) {
+                    best = max(best, mv);
+                    if (row == m - 1 && j == m) end = max(max(mv, xv), yv);
+                }
+            }
+            lm = um;
+            lx = ux;
+            ly = uy;
+            dm = tm;
+            dx = tx;
+            dy = ty;
+        }
+        int32_t v = a.local ? best : end;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(full, v, o));
+        if (lane == 0) a.out[t] = v;
+    }
+}
+
 // ------------------------------------------------------------------------- wavefront path ---
-// Warp-cooperative anti-diagonal wavefront.  A warp scores one query against two refs at once
-// (int16x2 halves).  Lane t owns query rows t*R+1 .. t*R+R and at step s processes column
-// j = s - t + 1, so the row above its first row (lane t-1's last row, same column) was finished
-// one step earlier and arrives by one shuffle, together with the column's two ref residues.
-// Cells are updated with DPX max-plus ops on both halves; the substitution scores of a cell pair
-// come from one shared-memory word T[q][r1][r2] = s(q,r1) | s(q,r2) << 16, where the extra code
-// A pads rows past the query and columns past the shorter ref with NEG.
+// Warp-cooperative anti-diagonal wavefront (gotoh_qpair_kernel): a warp scores two queries against
+// one ref at once (int16x2 halves).  Lane t owns query rows t*R+1 .. t*R+R and at step s processes
+// column j = s - t + 1, so the row above its first row (lane t-1's last row, same column) was
+// finished one step earlier and arrives by one shuffle.  Cells are updated with DPX max-plus ops on
+// both halves.  The strip kernel (gotoh_strip.cu) is faster wherever its warps (two queries
+// against 32 refs) fill the GPU; this one has 32 times as many and finer tasks, and takes
+// gap_extend > gap_open.
 //
 // With gap_extend <= gap_open the vertical gap is max(H_up - open, X_up - extend): H includes X,
 // and X_up - open <= X_up - extend, so adding it to the opening term never changes the maximum --
@@ -366,181 +472,11 @@ void launch_thread(Context& ctx, ThreadArgs a, int nmax, bool local, int64_t wor
 // offset is non-negative and at most extend * (rows + cols), which the admission bound above
 // already counts, so the raised states stay within +-14000; the gap states only take maxima, so
 // NEG never drifts downwards.
-constexpr int kWaveThreads = 256;
 constexpr uint32_t kNeg2 = 0xC000C000u;  // -16384 in both halves
-
-struct WaveArgs {
-    const uint8_t* qc;
-    const int64_t* qoff;
-    const uint8_t* rc;
-    const int64_t* roff;
-    const int32_t* qlist;   // queries of this launch (all of one row bucket)
-    int64_t nq;
-    const int2* rpairs;     // ref pairs of similar length (x == y for an odd one out)
-    int64_t nrp;
-    const uint32_t* table;  // A1^3 words
-    int A1;                 // alphabet size + 1 (the last code pads)
-    int32_t go, ge;
-    int self;               // 1: each query against itself, int64 result to self_out
-    int64_t* self_out;
-    int dist;
-    const int64_t* q_self;
-    const int64_t* r_self;
-    int32_t* out;
-    int64_t K;
-    unsigned int* overflow;
-};
 
 __device__ __forceinline__ uint32_t dup2(int v) { return (uint32_t(uint16_t(int16_t(v))) * 0x10001u); }
 __device__ __forceinline__ int lo16(uint32_t v) { return int(int16_t(uint16_t(v & 0xFFFFu))); }
 __device__ __forceinline__ int hi16(uint32_t v) { return int(int16_t(uint16_t(v >> 16))); }
-
-template <int R, bool LOCAL, bool EXACT>
-__global__ void __launch_bounds__(kWaveThreads) gotoh_wave_kernel(const WaveArgs a) {
-    extern __shared__ uint32_t s_tab[];
-    const int A1 = a.A1, pad = A1 - 1;
-    for (int i = threadIdx.x; i < A1 * A1 * A1; i += blockDim.x) s_tab[i] = a.table[i];
-    __syncthreads();
-    const unsigned full = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31;
-    const int64_t gwarp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-    const int64_t ntasks = a.self ? a.nq : a.nq * a.nrp;
-    const uint32_t mgo2 = dup2(-a.go), mge2 = dup2(-a.ge);
-    constexpr bool OFFSET = !LOCAL && !EXACT;
-    const uint32_t eo2 = dup2(a.ge - a.go);  // the raised border value, and the gap-open step
-
-    for (int64_t task = gwarp; task < ntasks; task += nwarps) {
-        const int64_t qi_idx = a.self ? task : task / a.nrp;
-        const int qi = a.qlist[qi_idx];
-        int k1 = qi, k2 = qi;
-        if (!a.self) {
-            const int2 rp = a.rpairs[task - qi_idx * a.nrp];
-            k1 = rp.x;
-            k2 = rp.y;
-        }
-        const uint8_t* q = a.qc + a.qoff[qi];
-        const int m = int(a.qoff[qi + 1] - a.qoff[qi]);
-        const uint8_t* rbase = a.self ? a.qc : a.rc;
-        const int64_t* roff = a.self ? a.qoff : a.roff;
-        const uint8_t* r1 = rbase + roff[k1];
-        const uint8_t* r2 = rbase + roff[k2];
-        const int n1 = int(roff[k1 + 1] - roff[k1]);
-        const int n2 = int(roff[k2 + 1] - roff[k2]);
-        const int nmax = max(n1, n2);
-
-        // Rows of this lane: 1-indexed i = lane*R + r + 1; column 0 state per row.
-        uint32_t qb[R], Hl[R], Yl[R], MXl[EXACT ? R : 1];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int row = lane * R + r;  // 0-indexed query position
-            qb[r] = uint32_t((row < m ? q[row] : pad) * A1 * A1);
-            const int gr = a.go + row * a.ge;  // gap_run(row + 1)
-            Hl[r] = LOCAL ? 0u : (OFFSET ? eo2 : dup2(-gr));
-            Yl[r] = kNeg2;
-            if constexpr (EXACT) MXl[r] = Hl[r];
-        }
-        // H[lane*R][0]: the row above this lane's first row, at column 0.
-        uint32_t diag = (lane == 0 || LOCAL) ? 0u
-                        : (OFFSET ? eo2 : dup2(-(a.go + (lane * R - 1) * a.ge)));
-        uint32_t best = 0u, cap = 0u;
-        uint32_t outH = 0u, outX = kNeg2, outMY = 0u;
-        int outRes = 0;
-        const int cap_lane = (m - 1) / R, cap_r = (m - 1) - cap_lane * R;
-        const int steps = nmax + 31;
-        for (int s = 0; s < steps; ++s) {
-            uint32_t upH = __shfl_up_sync(full, outH, 1);
-            uint32_t upX = __shfl_up_sync(full, outX, 1);
-            uint32_t upMY = EXACT ? __shfl_up_sync(full, outMY, 1) : 0u;
-            int res = __shfl_up_sync(full, outRes, 1);
-            const int j = s - lane + 1;
-            if (lane == 0) {  // the virtual row 0 at column j
-                const uint32_t h0 = LOCAL ? 0u : (OFFSET ? eo2 : dup2(-(a.go + (j - 1) * a.ge)));
-                upH = h0;
-                upX = kNeg2;
-                upMY = h0;
-                res = (j <= n1 ? int(r1[j - 1]) : pad) | ((j <= n2 ? int(r2[j - 1]) : pad) << 8);
-            }
-            if (j >= 1 && j <= nmax) {
-                const uint32_t col = uint32_t((res & 0xFF) * A1 + (res >> 8));
-                const uint32_t top = upH;
-                uint32_t d = diag;
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const uint32_t sc = s_tab[qb[r] + col];
-                    const uint32_t M = LOCAL ? __viaddmax_s16x2_relu(d, sc, kNeg2)
-                                             : __viaddmax_s16x2(d, sc, kNeg2);
-                    uint32_t X, Y;
-                    if constexpr (EXACT) {
-                        X = __viaddmax_s16x2(upMY, mgo2, __viaddmax_s16x2(upX, mge2, kNeg2));
-                        Y = __viaddmax_s16x2(MXl[r], mgo2, __viaddmax_s16x2(Yl[r], mge2, kNeg2));
-                    } else if constexpr (OFFSET) {
-                        X = __viaddmax_s16x2(upH, eo2, upX);
-                        Y = __viaddmax_s16x2(Hl[r], eo2, Yl[r]);
-                    } else {
-                        X = __viaddmax_s16x2(upH, mgo2, __viaddmax_s16x2(upX, mge2, kNeg2));
-                        Y = __viaddmax_s16x2(Hl[r], mgo2, __viaddmax_s16x2(Yl[r], mge2, kNeg2));
-                    }
-                    const uint32_t H = __vimax3_s16x2(M, X, Y);
-                    if constexpr (LOCAL) best = __vimax3_s16x2(best, M, kNeg2);
-                    d = Hl[r];
-                    Hl[r] = H;
-                    Yl[r] = Y;
-                    upH = H;
-                    upX = X;
-                    if constexpr (EXACT) {
-                        MXl[r] = __vimax3_s16x2(M, X, kNeg2);
-                        upMY = __vimax3_s16x2(M, Y, kNeg2);
-                    }
-                }
-                diag = top;
-                outH = upH;
-                outX = upX;
-                outMY = upMY;
-                outRes = res;
-                if (!LOCAL && lane == cap_lane && (j == n1 || j == n2)) {
-                    uint32_t h = 0u;
-#pragma unroll
-                    for (int r = 0; r < R; ++r)
-                        if (r == cap_r) h = Hl[r];
-                    if (j == n1) cap = (cap & 0xFFFF0000u) | (h & 0xFFFFu);
-                    if (j == n2) cap = (cap & 0xFFFFu) | (h & 0xFFFF0000u);
-                }
-            }
-        }
-        int v1, v2;
-        if constexpr (LOCAL) {
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1)
-                best = __vimax3_s16x2(best, __shfl_xor_sync(full, best, off), kNeg2);
-            v1 = lo16(best);
-            v2 = hi16(best);
-        } else {
-            cap = __shfl_sync(full, cap, cap_lane);
-            v1 = lo16(cap);
-            v2 = hi16(cap);
-            if constexpr (OFFSET) {
-                v1 -= (m + n1) * a.ge;
-                v2 -= (m + n2) * a.ge;
-            }
-        }
-        if (lane == 0) {
-            if (a.self) {
-                a.self_out[qi] = v1;
-            } else {
-                for (int t = 0; t < (k2 != k1 ? 2 : 1); ++t) {
-                    const int k = t ? k2 : k1;
-                    const int64_t sv = t ? v2 : v1;
-                    const int64_t v = a.dist ? a.q_self[qi] + a.r_self[k] - 2 * sv : sv;
-                    if (v < INT32_MIN || v > INT32_MAX)
-                        atomicOr(a.overflow, 1u);
-                    else
-                        a.out[int64_t(qi) * a.K + k] = int32_t(v);
-                }
-            }
-        }
-    }
-}
 
 // Query-pair form of the wavefront, used for the N x K pass.  A CTA holds two queries of one row
 // bucket (neighbours in length order) and a chunk of refs taken in length order.  Its shared
@@ -551,9 +487,8 @@ __global__ void __launch_bounds__(kWaveThreads) gotoh_wave_kernel(const WaveArgs
 // one per-column base.  A warp takes one ref at a time; the ref's codes, pre-multiplied into
 // profile offsets, are staged in the warp's slice of shared memory, so every lane reads its own
 // column's code without a shuffle.  The recurrence, the int16 safety argument and the raised
-// global form are those of gotoh_wave_kernel above.  Only the packing differs: the two halves
-// are two queries against one ref, so both end at the ref's last column, and the global score
-// of each query is read at its own last row.
+// global form are those above.  Both halves end at the ref's last column, and the global score of
+// each query is read at its own last row.
 constexpr int kQpWarps = 8;
 constexpr int kQpMaxRef = 512;  // wave_eligible admits lengths up to 512
 
@@ -768,50 +703,13 @@ const void* qpair_kernel(int R, bool local, bool exact) {
     }
 }
 
-// Rows per lane of the query-pair kernel: the smallest R with 32 * R >= m, rounded up to a
-// multiple of `step` (step 1: 32-row buckets, a query carries fewer than 32 padded rows; step 2:
-// 64-row buckets, fewer and larger launches).
-int qpair_rows_per_lane(int m, int step = 1) {
-    const int r = std::max(1, int((m + 31) / 32));
-    return std::min(16, (r + step - 1) / step * step);
-}
+// Rows per lane of the query-pair kernel: the smallest R with 32 * R >= m.
+int qpair_rows_per_lane(int m) { return std::min(16, std::max(1, int((m + 31) / 32))); }
 
-constexpr int kRowBuckets[] = {2, 4, 6, 8, 10, 12, 14, 16};
-
-int rows_per_lane(int m) {
-    for (int r : kRowBuckets)
-        if (m <= 32 * r) return r;
-    return 0;
-}
-
-template <int R>
-const void* wave_kernel_ptr(bool local, bool exact) {
-    if (local)
-        return exact ? reinterpret_cast<const void*>(gotoh_wave_kernel<R, true, true>)
-                     : reinterpret_cast<const void*>(gotoh_wave_kernel<R, true, false>);
-    return exact ? reinterpret_cast<const void*>(gotoh_wave_kernel<R, false, true>)
-                 : reinterpret_cast<const void*>(gotoh_wave_kernel<R, false, false>);
-}
-
-const void* wave_kernel(int R, bool local, bool exact) {
-    switch (R) {
-        case 2: return wave_kernel_ptr<2>(local, exact);
-        case 4: return wave_kernel_ptr<4>(local, exact);
-        case 6: return wave_kernel_ptr<6>(local, exact);
-        case 8: return wave_kernel_ptr<8>(local, exact);
-        case 10: return wave_kernel_ptr<10>(local, exact);
-        case 12: return wave_kernel_ptr<12>(local, exact);
-        case 14: return wave_kernel_ptr<14>(local, exact);
-        default: return wave_kernel_ptr<16>(local, exact);
-    }
-}
-
-// Substitution tables of the wavefront path, per device, and the grid they were built from:
-// the packed T[q][r1][r2] words of gotoh_wave_kernel and the A x A s(a, b) + add grid the
-// query-pair kernel builds its profiles from.
+// The A x A s(a, b) + add grid the query-pair kernel builds its profiles from, per device.
 struct WaveState {
     std::vector<uint8_t> key;
-    DevBuf table, simadd;
+    DevBuf simadd;
     // Side streams and events that run the row buckets' launches concurrently (fork / join on
     // the caller's stream), so that one bucket's tail of idle SMs is filled by the next bucket.
     static constexpr int kSide = 4;
@@ -827,14 +725,13 @@ struct WaveState {
     }
 };
 
-// Per-set launch plan (depends only on the lengths): the set's indices grouped by rows per
-// lane, with the (R, offset, count) of each group; inside each group the sequences sorted by
-// length and paired with their neighbour (the query side of the query-pair kernel), with the
-// (R, offset, count) of each group's pairs; and every index sorted by length (the ref side).
+// Per-set launch plan (depends only on the lengths): the sequences of each 32-row bucket sorted by
+// length and paired with their neighbour (the query side), with the (R, offset, count) of each
+// bucket's pairs; and every index sorted by length (the ref side).
 struct WavePlan {
     uint64_t uid = 0;
-    std::vector<std::tuple<int, int64_t, int64_t>> groups, pair_groups[2];
-    DevBuf list, qpairs[2], sorted;
+    std::vector<std::tuple<int, int64_t, int64_t>> pair_groups;
+    DevBuf qpairs, sorted;
 };
 
 WavePlan& wave_plan(st_seqset_s& s, Context& ctx, int slot, cudaStream_t stream) {
@@ -842,46 +739,30 @@ WavePlan& wave_plan(st_seqset_s& s, Context& ctx, int slot, cudaStream_t stream)
     if (!holder) holder = std::make_shared<WavePlan>();
     WavePlan& p = *static_cast<WavePlan*>(holder.get());
     if (p.uid == s.uid) return p;
-    std::vector<std::vector<int32_t>> b(17);
-    for (int64_t i = 0; i < s.count; ++i)
-        b[size_t(rows_per_lane(s.h_len[size_t(i)]))].push_back(int32_t(i));
-    std::vector<int32_t> all;
-    all.reserve(size_t(s.count));
-    p.groups.clear();
-    for (int R = 1; R <= 16; ++R)
-        if (!b[size_t(R)].empty()) {
-            p.groups.emplace_back(R, int64_t(all.size()), int64_t(b[size_t(R)].size()));
-            all.insert(all.end(), b[size_t(R)].begin(), b[size_t(R)].end());
-        }
     auto by_len = [&](int32_t x, int32_t y) { return s.h_len[size_t(x)] < s.h_len[size_t(y)]; };
     std::vector<int32_t> order(static_cast<size_t>(s.count));
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), by_len);
-    // Query pairs per bucket, for both bucket widths (32 and 64 rows; the tuner picks one).
-    std::vector<int32_t> qpairs[2];
-    for (int w = 0; w < 2; ++w) {
-        qpairs[w].reserve(size_t(s.count) + 34);
-        p.pair_groups[w].clear();
-        std::vector<std::vector<int32_t>> fine(17);
-        for (int64_t i = 0; i < s.count; ++i)
-            fine[size_t(qpair_rows_per_lane(s.h_len[size_t(i)], w + 1))].push_back(int32_t(i));
-        for (int R = 1; R <= 16; ++R) {
-            std::vector<int32_t>& g = fine[size_t(R)];
-            if (g.empty()) continue;
-            std::stable_sort(g.begin(), g.end(), by_len);
-            const int64_t first = int64_t(qpairs[w].size() / 2);
-            for (size_t i = 0; i < g.size(); i += 2) {
-                qpairs[w].push_back(g[i]);
-                qpairs[w].push_back(i + 1 < g.size() ? g[i + 1] : g[i]);
-            }
-            p.pair_groups[w].emplace_back(R, first, int64_t(qpairs[w].size() / 2) - first);
+    // Query pairs per bucket of 32 rows.
+    std::vector<int32_t> qpairs;
+    qpairs.reserve(size_t(s.count) + 17);
+    p.pair_groups.clear();
+    std::vector<std::vector<int32_t>> fine(17);
+    for (int64_t i = 0; i < s.count; ++i)
+        fine[size_t(qpair_rows_per_lane(s.h_len[size_t(i)]))].push_back(int32_t(i));
+    for (int R = 1; R <= 16; ++R) {
+        std::vector<int32_t>& g = fine[size_t(R)];
+        if (g.empty()) continue;
+        std::stable_sort(g.begin(), g.end(), by_len);
+        const int64_t first = int64_t(qpairs.size() / 2);
+        for (size_t i = 0; i < g.size(); i += 2) {
+            qpairs.push_back(g[i]);
+            qpairs.push_back(i + 1 < g.size() ? g[i + 1] : g[i]);
         }
+        p.pair_groups.emplace_back(R, first, int64_t(qpairs.size() / 2) - first);
     }
     // (a pageable-source copy has consumed the host vectors by the time it returns)
-    h2d(p.list.as<int32_t>(all.size()), all.data(), all.size() * 4, stream);
-    for (int w = 0; w < 2; ++w)
-        h2d(p.qpairs[w].as<int32_t>(qpairs[w].size()), qpairs[w].data(), qpairs[w].size() * 4,
-            stream);
+    h2d(p.qpairs.as<int32_t>(qpairs.size()), qpairs.data(), qpairs.size() * 4, stream);
     h2d(p.sorted.as<int32_t>(order.size()), order.data(), order.size() * 4, stream);
     p.uid = s.uid;
     return p;
@@ -911,22 +792,6 @@ bool wave_eligible(const st_seqset_s& qs, const st_seqset_s& rs, const int32_t* 
     return bound <= 14000;
 }
 
-// Launches one wavefront pass: `list` queries (one row bucket) against `pairs` (or themselves).
-void launch_wave(Context& ctx, WaveArgs wa, int R, bool local, bool exact, cudaStream_t stream) {
-    const void* kern = wave_kernel(R, local, exact);
-    const size_t smem = size_t(wa.A1) * wa.A1 * wa.A1 * 4;
-    STB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    int per_sm = 0;
-    STB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWaveThreads, smem));
-    const int64_t ntasks = wa.self ? wa.nq : wa.nq * wa.nrp;
-    const int64_t warps_per_block = kWaveThreads / 32;
-    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(
-        ceil_div(ntasks, warps_per_block), int64_t(ctx.num_sms) * std::max(per_sm, 1)));
-    void* args[] = {&wa};
-    STB_CUDA(cudaLaunchKernel(kern, dim3(unsigned(blocks)), dim3(kWaveThreads), args, smem, stream));
-    note_launch("gotoh_wave_kernel");
-}
-
 // Launches one query-pair pass: the pairs of one row bucket against every ref, `chunk` refs per
 // CTA column.
 void launch_qpair(QpArgs qa, int R, bool local, bool exact, cudaStream_t stream) {
@@ -941,80 +806,97 @@ void launch_qpair(QpArgs qa, int R, bool local, bool exact, cudaStream_t stream)
     note_launch("gotoh_qpair_kernel");
 }
 
+
+// A similarity grid on the device, uploaded only when it changes (so warmed-up calls capture).
+struct SimTable {
+    std::vector<uint8_t> key;
+    DevBuf sim;
+};
+
+const int32_t* sim_table(Context& ctx, const int32_t* similarity, int A, cudaStream_t stream) {
+    static std::mutex mu;
+    static std::map<int, std::unique_ptr<SimTable>> all;
+    SimTable* t;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        auto& slot = all[ctx.device];
+        if (!slot) slot = std::make_unique<SimTable>();
+        t = slot.get();
+    }
+    int32_t* d_sim = t->sim.as<int32_t>(size_t(A) * A);
+    if (!same_as_last(t->key, similarity, size_t(A) * A * 4)) {
+        try {
+            h2d(d_sim, similarity, size_t(A) * A * 4, stream);
+        } catch (...) {
+            t->key.clear();
+            throw;
+        }
+    }
+    return d_sim;
+}
+
+// Self scores of both sets (N words, then K) into the context's scratch.
+const int64_t* self_scores(const st_seqset_s& qs, const st_seqset_s& rs, const int32_t* similarity, int A,
+                           int32_t mode, int32_t go, int32_t ge, cudaStream_t stream) {
+    Context& ctx = context();
+    SelfArgs a{};
+    const st_seqset_s* sets[2] = {&qs, &rs};
+    for (int t = 0; t < 2; ++t) {
+        a.codes[t] = sets[t]->d_bytes;
+        a.off[t] = sets[t]->d_off;
+        a.count[t] = sets[t]->count;
+    }
+    a.sim = sim_table(ctx, similarity, A, stream);
+    a.A = A;
+    for (int c = 0; c < A; ++c) {
+        const int32_t own = similarity[c * A + c];
+        bool ok = own >= 0;
+        for (int x = 0; x < A; ++x) ok &= similarity[c * A + x] <= own && similarity[x * A + c] <= own;
+        if (ok) a.plain |= 1u << c;
+    }
+    a.local = mode == ST_MODE_LOCAL;
+    a.go = go;
+    a.ge = ge;
+    const int64_t total = qs.count + rs.count;
+    a.out = ctx.work_b.as<int64_t>(size_t(total));
+    const int64_t blocks = std::min<int64_t>(ceil_div(total, 8), int64_t(ctx.num_sms) * 16);
+    self_score_kernel<<<unsigned(blocks), 256, size_t(A) * A * 4, stream>>>(a);
+    STB_CUDA(cudaGetLastError());
+    note_launch("self_score_kernel");
+    return a.out;
+}
+
 }  // namespace
 
 // The warp-wavefront path for every pair (int16x2 cells; the caller checked wave_eligible).
 void align_wave(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int A, int32_t mode,
                 int32_t go, int32_t ge, int32_t dist, int32_t* out_d, unsigned int* ovf,
-                cudaStream_t stream, int bucket = 0) {
+                cudaStream_t stream) {
     Context& ctx = context();
     const int64_t N = qs.count, K = rs.count;
     WaveState& ws = wave_state(ctx.device);
-    const int A1 = A + 1;
-    {
-        // T[(q*A1 + r1)*A1 + r2] = s(q,r1) | s(q,r2) << 16, the pad code scoring NEG; the
-        // offset form (global, gap_extend <= gap_open) adds 2 * gap_extend to every finite score.
-        const int32_t add = (mode != ST_MODE_LOCAL && ge <= go) ? 2 * ge : 0;
-        std::vector<uint8_t> key(size_t(A) * A * 4 + 4);
-        std::memcpy(key.data(), similarity, size_t(A) * A * 4);
-        std::memcpy(key.data() + size_t(A) * A * 4, &add, 4);
-        if (!same_as_last(ws.key, key.data(), key.size())) {
-            std::vector<uint32_t> tab(size_t(A1) * A1 * A1);
-            auto sv = [&](int x, int y) -> int32_t {
-                return (x == A || y == A) ? -16384 : similarity[x * A + y] + add;
-            };
-            for (int x = 0; x < A1; ++x)
-                for (int y1 = 0; y1 < A1; ++y1)
-                    for (int y2 = 0; y2 < A1; ++y2)
-                        tab[(size_t(x) * A1 + y1) * A1 + y2] =
-                            uint32_t(uint16_t(int16_t(sv(x, y1)))) |
-                            (uint32_t(uint16_t(int16_t(sv(x, y2)))) << 16);
-            std::vector<int32_t> sa(size_t(A) * A);
-            for (int x = 0; x < A * A; ++x) sa[size_t(x)] = similarity[x] + add;
-            try {
-                h2d(ws.table.as<uint32_t>(tab.size()), tab.data(), tab.size() * 4, stream);
-                h2d(ws.simadd.as<int32_t>(sa.size()), sa.data(), sa.size() * 4, stream);
-            } catch (...) {
-                ws.key.clear();  // not uploaded: the next call builds it again
-                throw;
-            }
+    // s(a, b), plus 2 * gap_extend in the raised form (global, gap_extend <= gap_open)
+    const int32_t add = (mode != ST_MODE_LOCAL && ge <= go) ? 2 * ge : 0;
+    std::vector<int32_t> sa(size_t(A) * A);
+    for (int x = 0; x < A * A; ++x) sa[size_t(x)] = similarity[x] + add;
+    if (!same_as_last(ws.key, sa.data(), sa.size() * 4)) {
+        try {
+            h2d(ws.simadd.as<int32_t>(sa.size()), sa.data(), sa.size() * 4, stream);
+        } catch (...) {
+            ws.key.clear();  // not uploaded: the next call builds it again
+            throw;
         }
     }
     WavePlan& qp = wave_plan(qs, ctx, 0, stream);
     WavePlan& rp = wave_plan(rs, ctx, 1, stream);
+    const int64_t* q_self = dist ? self_scores(qs, rs, similarity, A, mode, go, ge, stream) : nullptr;
+    const int64_t* r_self = dist ? q_self + N : nullptr;
     const bool local = mode == ST_MODE_LOCAL;
     const bool exact = ge > go;
-    WaveArgs wa{};
-    wa.table = static_cast<uint32_t*>(ws.table.ptr);
-    wa.A1 = A1;
-    wa.go = go;
-    wa.ge = ge;
-    wa.overflow = ovf;
-    wa.K = K;
-    int64_t* q_self = nullptr;
-    int64_t* r_self = nullptr;
-    if (dist) {
-        q_self = ctx.work_b.as<int64_t>(size_t(N + K));
-        r_self = q_self + N;
-        for (int t = 0; t < 2; ++t) {
-            const st_seqset_s& s = t == 0 ? qs : rs;
-            const WavePlan& p = t == 0 ? qp : rp;
-            for (auto& [R, off, cnt] : p.groups) {
-                WaveArgs sa = wa;
-                sa.qc = s.d_bytes;
-                sa.qoff = s.d_off;
-                sa.qlist = static_cast<int32_t*>(p.list.ptr) + off;
-                sa.nq = cnt;
-                sa.self = 1;
-                sa.self_out = t == 0 ? q_self : r_self;
-                launch_wave(ctx, sa, R, local, exact, stream);
-            }
-        }
-    }
     // The buckets' launches run on side streams forked from (and joined back into) the caller's
     // stream; the longest rows first, so the short buckets fill the long ones' tails.
     ws.ensure_streams();
-    const auto& pgroups = qp.pair_groups[bucket];
+    const auto& pgroups = qp.pair_groups;
     const int nside = std::min<int>(WaveState::kSide, int(pgroups.size()));
     STB_CUDA(cudaEventRecord(ws.fork, stream));
     for (int i = 0; i < nside; ++i) STB_CUDA(cudaStreamWaitEvent(ws.side[i], ws.fork, 0));
@@ -1026,7 +908,7 @@ void align_wave(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
         ma.qoff = qs.d_off;
         ma.rc = rs.d_bytes;
         ma.roff = rs.d_off;
-        ma.qpairs = static_cast<int2*>(qp.qpairs[bucket].ptr) + off;
+        ma.qpairs = static_cast<int2*>(qp.qpairs.ptr) + off;
         ma.nqp = cnt;
         ma.rorder = static_cast<int32_t*>(rp.sorted.ptr);
         ma.K = K;
@@ -1069,80 +951,63 @@ void align_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
 
     const int tn = thread_nmax(qs, rs, similarity, A, go, ge, dist != 0, dist != 0);
     const bool wave_ok = wave_eligible(qs, rs, similarity, A, go, ge);
-    if (tn > 0) {
-        // Short sequences: one thread per pair (registers only) or the warp wavefront, whichever
-        // the autotuner measured faster for this shape.
-        // the similarity table, uploaded only when it changes (so warmed-up calls capture)
-        struct ThreadTable {
-            std::vector<uint8_t> key;
-            DevBuf sim;
-        };
-        static std::mutex tmu;
-        static std::map<int, std::unique_ptr<ThreadTable>> tables;
-        ThreadTable* tt;
-        {
-            std::lock_guard<std::mutex> lk(tmu);
-            auto& slot = tables[ctx.device];
-            if (!slot) slot = std::make_unique<ThreadTable>();
-            tt = slot.get();
-        }
-        int32_t* d_sim = tt->sim.as<int32_t>(size_t(A) * A);
-        if (!same_as_last(tt->key, similarity, size_t(A) * A * 4)) {
-            try {
-                h2d(d_sim, similarity, size_t(A) * A * 4, stream);
-            } catch (...) {
-                tt->key.clear();
-                throw;
+    const bool strip_ok = strip_eligible(qs, rs, similarity, A, go, ge);
+
+    auto run_thread = [&](st_seqset_s& q) {  // registers only; sequences of at most 32
+        const int64_t* self = dist ? self_scores(q, rs, similarity, A, mode, go, ge, stream) : nullptr;
+        ThreadArgs t{};
+        t.sim = sim_table(ctx, similarity, A, stream);
+        t.A = A;
+        t.go = go;
+        t.ge = ge;
+        t.overflow = ovf;
+        t.qc = q.d_bytes;
+        t.qoff = q.d_off;
+        t.rc = rs.d_bytes;
+        t.roff = rs.d_off;
+        t.N = q.count;
+        t.K = K;
+        t.dist = dist;
+        t.q_self = self;
+        t.r_self = dist ? self + q.count : nullptr;
+        t.out = out_d;
+        launch_thread(ctx, t, tn, mode == ST_MODE_LOCAL, q.count * K, stream);
+    };
+    auto run_strip = [&](st_seqset_s& q) {
+        const int64_t* self = dist ? self_scores(q, rs, similarity, A, mode, go, ge, stream) : nullptr;
+        align_strip(q, rs, similarity, A, mode, go, ge, dist, self, dist ? self + q.count : nullptr, out_d,
+                    ovf, stream);
+    };
+
+    // The kernels that can take the call; where there are several, the autotuner measures them
+    // once per shape.  The strip kernel wins wherever the pairs fill the GPU's warps; a
+    // small matrix of long sequences leaves them idle, and there a warp per (query pair, ref) wins.
+    enum Kind { kThread, kWave, kStrip };
+    std::vector<Kind> kinds;
+    if (tn > 0) kinds.push_back(kThread);
+    if (wave_ok) kinds.push_back(kWave);
+    if (strip_ok) kinds.push_back(kStrip);
+    if (!kinds.empty()) {
+        auto variant = [&](int c, st_seqset_s& q) {
+            switch (kinds[size_t(c)]) {
+                case kThread: run_thread(q); break;
+                case kWave: align_wave(q, rs, similarity, A, mode, go, ge, dist, out_d, ovf, stream); break;
+                case kStrip: run_strip(q); break;
             }
-        }
-        auto run_thread = [&](st_seqset_s& q) {
-            const int64_t Nq = q.count;
-            ThreadArgs t{};
-            t.sim = d_sim;
-            t.A = A;
-            t.go = go;
-            t.ge = ge;
-            t.overflow = ovf;
-            int64_t* q_self = nullptr;
-            int64_t* r_self = nullptr;
-            if (dist) {
-                q_self = ctx.work_b.as<int64_t>(size_t(Nq + K));
-                r_self = q_self + Nq;
-                for (int side = 0; side < 2; ++side) {
-                    const st_seqset_s& s = side == 0 ? q : rs;
-                    ThreadArgs b = t;
-                    b.qc = s.d_bytes;
-                    b.qoff = s.d_off;
-                    b.N = s.count;
-                    b.self = 1;
-                    b.self_out = side == 0 ? q_self : r_self;
-                    launch_thread(ctx, b, tn, mode == ST_MODE_LOCAL, s.count, stream);
-                }
-            }
-            t.qc = q.d_bytes;
-            t.qoff = q.d_off;
-            t.rc = rs.d_bytes;
-            t.roff = rs.d_off;
-            t.N = Nq;
-            t.K = K;
-            t.dist = dist;
-            t.q_self = q_self;
-            t.r_self = r_self;
-            t.out = out_d;
-            launch_thread(ctx, t, tn, mode == ST_MODE_LOCAL, Nq * K, stream);
         };
-        if (!wave_ok) {
-            run_thread(qs);
+        if (kinds.size() == 1) {
+            variant(0, qs);
             return;
         }
-        const std::string key = "align|" + std::to_string(mode) + "|" + std::to_string(dist) + "|" +
-                                std::to_string(A) + "|" + std::to_string(qs.max_len) + "|" +
-                                std::to_string(rs.max_len) + "|" + std::to_string(size_bucket(N)) +
-                                "|" + std::to_string(size_bucket(K));
-        auto variant = [&](int c, st_seqset_s& q) {
-            if (c == 0) run_thread(q);
-            else align_wave(q, rs, similarity, A, mode, go, ge, dist, out_d, ovf, stream, c - 1);
-        };
+        std::string key = (tn > 0 ? "align|" : "wave|") + std::to_string(mode) + "|" + std::to_string(dist) +
+                          "|" + std::to_string(A) + "|" + std::to_string(qs.max_len) + "|" +
+                          std::to_string(rs.max_len) + "|" + std::to_string(size_bucket(N)) + "|" +
+                          std::to_string(size_bucket(K)) + "|";
+        for (Kind k : kinds) key += "tws"[k];
+        // Without a measurement (tuning off, or a stream being captured): the strip kernel when
+        // its warps fill the GPU, else the first kind.
+        const bool fills = N / 2 * (K / 32) >= int64_t(ctx.num_sms) * 16;
+        const int fallback = strip_ok && (fills || !wave_ok) ? int(kinds.size()) - 1 : 0;
         // A shape seen for the first time is tuned on its first query rows only (about
         // kAlignTunePairs pairs, written into their own rows of the result); the choice then
         // computes the whole matrix.
@@ -1150,34 +1015,11 @@ void align_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
             N, std::max<int64_t>(64, kAlignTunePairs / std::max<int64_t>(K, 1)));
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         STB_CUDA(cudaStreamIsCapturing(stream, &cs));
-        if (slice < N && tuning_enabled() && cs == cudaStreamCaptureStatusNone &&
-            tuned_lookup(key) < 0) {
+        if (slice < N && tuning_enabled() && cs == cudaStreamCaptureStatusNone && tuned_lookup(key) < 0) {
             std::unique_ptr<st_seqset_s> view = row_view(qs, slice);
-            tuned_run(key, 3, 0, [&](int c) { variant(c, *view); }, stream);
+            tuned_run(key, int(kinds.size()), fallback, [&](int c) { variant(c, *view); }, stream);
         }
-        tuned_run(key, 3, 0, [&](int c) { variant(c, qs); }, stream);
-        return;
-    }
-    if (wave_ok) {
-        // The row-bucket width (32 or 64 rows) is tuned once per shape, on the first query rows
-        // (about kWaveTunePairs pairs, written into their own rows of the result).
-        const std::string key = "wave|" + std::to_string(mode) + "|" + std::to_string(dist) + "|" +
-                                std::to_string(A) + "|" + std::to_string(qs.max_len) + "|" +
-                                std::to_string(rs.max_len) + "|" + std::to_string(size_bucket(N)) +
-                                "|" + std::to_string(size_bucket(K));
-        auto bucketed = [&](int c, st_seqset_s& q) {
-            align_wave(q, rs, similarity, A, mode, go, ge, dist, out_d, ovf, stream, c);
-        };
-        const int64_t slice = std::min<int64_t>(
-            N, std::max<int64_t>(64, kWaveTunePairs / std::max<int64_t>(K, 1)));
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        STB_CUDA(cudaStreamIsCapturing(stream, &cs));
-        if (slice < N && tuning_enabled() && cs == cudaStreamCaptureStatusNone &&
-            tuned_lookup(key) < 0) {
-            std::unique_ptr<st_seqset_s> view = row_view(qs, slice);
-            tuned_run(key, 2, 0, [&](int c) { bucketed(c, *view); }, stream);
-        }
-        tuned_run(key, 2, 0, [&](int c) { bucketed(c, qs); }, stream);
+        tuned_run(key, int(kinds.size()), fallback, [&](int c) { variant(c, qs); }, stream);
         return;
     }
 
