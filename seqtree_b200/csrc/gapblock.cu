@@ -10,33 +10,41 @@
 // result is the same integer as the reference's (integer sums, no reassociation hazard while
 // the reference itself does not overflow int32).
 //
-// Fast path (every length <= 64, min(m,n) <= 32, L*max_pen <= 8191):
-//   * Queries are sorted by length and paired; the penalties of a pair against one ref residue
-//     travel as int16x2.  A query profile QP[pair][j][b] = pen(q1[j], b) | pen(q2[j], b) << 16
-//     (32 words per row: one pass over the banks) is built once per call in global memory.
-//   * Refs are cut into chunks of RC columns (original order); inside a chunk they are grouped
-//     by length into warp tasks of <= 32 refs, so d, L and the prior row are warp-uniform.  The
-//     refs' codes are laid out per task as [j][lane] bytes holding 4*code (a byte offset into a
-//     profile row), also once per call.
-//   * A CTA owns (chunk, 4 query pairs).  Two bulk (TMA) copies stage its 4-pair profile slab
-//     and the chunk's code slab into shared memory, completing on one mbarrier.  A warp unit is
-//     (task, slice of 4 pairs of one length); the 4 pairs are swept together, and every lookup
-//     is LDS [lane register + compile-time immediate]: the register is the residue's byte offset
-//     and the immediate ((slice*4 + pair)*LQ + j)*128.  Both penalties of two pairs arrive in
-//     one LDS, the running sums are plain 32-bit adds on halves kept in [0, 2^15), and one DPX
-//     __viaddmin_s16x2 updates both running minima.
-//   * Results go through a shared tile so that global stores are coalesced 16-byte vectors in
-//     the original column order; the per-(m,n) term (prior minimum + gap cost) is added there.
+// Fast path (every length <= 64, min(m,n) * max_pen <= 8191, no negative penalty):
+//   * The minimum runs along the sweep: A[i] = pre[i] + prior[i] and B[i] = the best layout whose
+//     block has opened at or before i, charged up to column i:
+//         A += P0[j] + (prior[j+1] - prior[j]);   B = min(B + Pd[j], A)
+//     -- one three-input add and one DPX __viaddmin_s16x2 for two queries packed int16x2.
+//   * Queries of one length travel in quads: a profile word holds the four queries' penalties
+//     against one residue, 8 bits each (one LDS.32 = four pair-cells per lane), split into two
+//     int16x2 words by a PRMT (odd bytes) and an IMAD (w - 256 * odd) on the otherwise idle FMA
+//     pipe.  Penalties above 255 use two 16-bit words instead (WIDE).  A CTA's four quads form a
+//     slice; its profile is [row][quad][32 words], one pass over the banks per quad.
+//   * Refs are cut into chunks of RC columns (original order); inside a chunk they are sorted by
+//     length and taken 32 at a time, one per lane, whatever their lengths: each lane has its own
+//     diagonal, a ref's code rows past its end hold a code whose penalties are 0, and the prior's
+//     steps past a layout's last position are 0, so the positions past a lane's own end change
+//     nothing.  (Warps of one length only were 82 % full.)  The codes are laid out per warp task
+//     as [j][lane] bytes holding 4 * code, a byte offset into a profile row.
+//   * A CTA owns (chunk, slice).  Two bulk (TMA) copies stage the slice's profile and the chunk's
+//     code slab, completing on one mbarrier.  Every lookup is LDS [lane register + immediate].
+//   * Dense results go through a shared tile so that the global stores are coalesced in the
+//     original column order; the per-(m,n) term (prior minimum + gap cost) is added there.
+//   Measured, B200 at 1965 MHz, against the form with 16-bit pair words, three ALU operations per
+//   pair-cell and warps of one length: 9,973 x 50,021 junctions of 8-25, BLOSUM62, dense 2.10 ->
+//   0.91 ms; 100,000 x 1,000,000 thresholded at 24 366 -> 139 ms.  The sweep is bound by issue
+//   slots (78-82 % issue active; ALU 57-63 %, FMA 53-60 %, shared wavefronts 75 % of a cycle).
 // General path: one thread per pair in int32 for any lengths and penalty magnitudes.
 //
 // Thresholded sparse form (for matrices too large to hold densely): the same kernels keep only
-// the cells with score <= max_penalty.  Hits are appended as (query << shift | ref, score) with one
-// atomic per warp, then radix-sorted by key and turned into CSR rows (indptr, ref ids, scores):
-// exactly the entries of the dense matrix's rows that pass the threshold, in ref order.
+// the cells with score <= max_penalty and turn them into CSR rows (indptr, ref ids, scores):
+// exactly the entries of the dense matrix's rows that pass the threshold, in ref order.  The fast
+// kernel tests its results in registers, marks hits in a bitmap of the tile and writes them in
+// column order; the general kernel appends (query << shift | ref, score) with one atomic per warp
+// and the hits are radix-sorted.
 #include <algorithm>
 #include <cstdlib>
 #include <map>
-#include <numeric>
 #include <type_traits>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -49,12 +57,15 @@ namespace stb {
 
 namespace {
 
-constexpr int kGP = 4;          // query pairs per CTA (tile rows = 8 queries; 8 pairs measured slower)
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kRow = 32;        // words per profile row
-constexpr int kPairsPerSlice = 4;
-static_assert(kWarps == 2 * kGP, "the ordered sparse epilogue gives each tile row one warp");
+constexpr int kRow = 32;        // words of one quad in a profile row
+constexpr int kQuads = 4;       // quads per slice
+constexpr int kSliceQ = 4 * kQuads;
+constexpr int kNullCode = 31;   // a residue past a ref's end: its profile column is 0
+constexpr int kMaxSpread = 8;   // lengths of one warp task differ by at most this
+constexpr int kTileW = 2 * kQuads + 1;  // tile words per column: 8 results and the (m, n) term
+static_assert(kWarps == 2 * kQuads, "the dense write-out gives each result word one warp");
 
 // ---------------------------------------------------------------------------- plans ---------
 // Plans depend only on the lengths (and codes) of a set, so a device-resident set builds them
@@ -63,12 +74,12 @@ static_assert(kWarps == 2 * kGP, "the ordered sparse epilogue gives each tile ro
 struct QueryPlan {
     uint64_t uid = 0;                    // set the plan was built for
     int64_t r0 = 0, r1 = -1;             // its rows [r0, r1) (r1 = -1: the whole set)
-    int64_t P = 0;                       // query pairs, a multiple of 4
-    std::vector<int2> pairs;             // original indices (-1 marks an empty slot)
-    std::vector<int32_t> plen;           // m of each pair
-    DevBuf d_pairs, d_plen;
-    std::vector<uint8_t> prof_key;       // (A, LQ, penalty grid) the profile was built for
-    DevBuf d_prof;                       // [P][LQ][32] uint32
+    std::vector<int4> quads;             // original indices (-1 marks an empty slot)
+    std::vector<int4> slices;            // (first quad, quads, length, profile row offset)
+    int64_t prof_rows = 0;               // profile rows of all slices
+    DevBuf d_plan;                       // quads, then slices
+    std::vector<uint8_t> prof_key;       // (A, word width, penalty grid) the profile was built for
+    DevBuf d_prof;                       // [row][quad][32] uint32 (twice the words when WIDE)
 };
 
 struct RefPlan {
@@ -78,97 +89,110 @@ struct RefPlan {
     int64_t ntasks = 0;
     int64_t max_slab = 0;                // largest per-chunk code slab (bytes)
     int max_tasks = 0;                   // most warp tasks in one chunk
-    int64_t slab_bytes = 0;              // whole slab
-    std::vector<int32_t> sorted;
-    std::vector<int4> tasks;             // (n, start in sorted, count <= 32, slab byte offset)
-    std::vector<int32_t> task_off;       // nchunks + 1
-    DevBuf d_sorted, d_tasks, d_task_off;
-    DevBuf d_slab;                       // per task: n rows of 32 bytes (4*code per lane)
+    int max_spread = 0;                  // largest length difference inside one task
+    std::vector<int4> tasks;             // (longest, start in meta, count <= 32, slab byte offset);
+                                         // longest | 0x100 when all are that long
+    std::vector<int4> chunks;            // (first task, tasks, slab byte offset, slab bytes)
+    int64_t slab_bytes = 0;
+    DevBuf d_plan;                       // chunks, then tasks
+    DevBuf d_meta;                       // per slot: column in the chunk | length << 16
+    DevBuf d_slab;                       // per task: longest rows of 32 bytes (4*code per lane)
 };
 
-// Queries (rows [r0, r1) of the set; r1 = -1 for all) sorted by length (stable) and paired
-// within each length; an odd one out is paired with -1.  Each length's pairs are padded with
-// (-1, -1) to a multiple of 4, so that every slice of 4 consecutive pairs has one length.  Empty
-// slots are computed and never stored.
+// Queries (rows [r0, r1) of the set; r1 = -1 for all) sorted by length (stable); each length's
+// queries fill quads and its quads fill slices.  Empty slots are computed and never stored.
 void build_query_plan(QueryPlan& plan, const st_seqset_s& q, cudaStream_t stream, int64_t r0 = 0,
                       int64_t r1 = -1) {
     const int64_t N = (r1 < 0 ? q.count : r1) - r0;
     std::vector<int32_t> order(static_cast<size_t>(N));
-    std::iota(order.begin(), order.end(), int32_t(r0));
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int32_t a, int32_t b) { return q.h_len[size_t(a)] < q.h_len[size_t(b)]; });
-    plan.pairs.clear();
-    plan.plen.clear();
+    std::vector<int64_t> at(size_t(q.max_len) + 2, 0);
+    for (int64_t i = 0; i < N; ++i) at[size_t(q.h_len[size_t(r0 + i)]) + 1]++;
+    for (size_t l = 1; l < at.size(); ++l) at[l] += at[l - 1];
+    for (int64_t i = 0; i < N; ++i) order[size_t(at[size_t(q.h_len[size_t(r0 + i)])]++)] = int32_t(r0 + i);
+    plan.quads.clear();
+    plan.slices.clear();
+    plan.prof_rows = 0;
     for (int64_t i = 0; i < N;) {
         const int32_t m = q.h_len[size_t(order[size_t(i)])];
         int64_t e = i;
         while (e < N && q.h_len[size_t(order[size_t(e)])] == m) ++e;
-        const size_t first = plan.pairs.size();
-        for (int64_t t = i; t < e; t += 2)
-            plan.pairs.push_back(make_int2(order[size_t(t)], t + 1 < e ? order[size_t(t + 1)] : -1));
-        while ((plan.pairs.size() - first) % kPairsPerSlice) plan.pairs.push_back(make_int2(-1, -1));
-        plan.plen.resize(plan.pairs.size(), m);
+        for (int64_t t = i; t < e; t += kSliceQ) {
+            const int first = int(plan.quads.size());
+            for (int64_t u = t; u < std::min<int64_t>(e, t + kSliceQ); u += 4) {
+                int v[4];
+                for (int x = 0; x < 4; ++x) v[x] = u + x < e ? order[size_t(u + x)] : -1;
+                plan.quads.push_back(make_int4(v[0], v[1], v[2], v[3]));
+            }
+            plan.slices.push_back(
+                make_int4(first, int(plan.quads.size()) - first, m, int(plan.prof_rows)));
+            plan.prof_rows += m;
+        }
         i = e;
     }
-    plan.P = int64_t(plan.pairs.size());
-    h2d(plan.d_pairs.as<int2>(size_t(plan.P)), plan.pairs.data(),
-                             sizeof(int2) * size_t(plan.P), stream);
-    h2d(plan.d_plen.as<int32_t>(size_t(plan.P)), plan.plen.data(),
-                             sizeof(int32_t) * size_t(plan.P), stream);
+    if (plan.prof_rows > INT32_MAX) fail(ST_EINVAL, "seqtree_b200: query set too large for one call");
+    std::vector<int4> up(plan.quads);
+    up.insert(up.end(), plan.slices.begin(), plan.slices.end());
+    h2d(plan.d_plan.as<int4>(up.size()), up.data(), sizeof(int4) * up.size(), stream);
     plan.prof_key.clear();
     plan.uid = q.uid;
     plan.r0 = r0;
     plan.r1 = r1;
 }
 
-// Refs in chunks of rc columns (original order); inside a chunk a counting sort by length
-// yields warp tasks of <= 32 refs of one length.  Each task's code rows occupy n*32 bytes of
-// the slab, so a chunk's slab is one contiguous range.
-void build_ref_plan(RefPlan& plan, const st_seqset_s& r, int rc, cudaStream_t stream,
-                    bool upload = true) {
+// Refs in chunks of rc columns (original order), sorted by length inside a chunk and taken 32 at a
+// time (fewer at the end of the chunk, and where lengths would differ by more than kMaxSpread): the
+// warp tasks, which follow from the chunk's length histogram alone.  The order inside a length is
+// chunk_order_kernel's.  Each task's code rows occupy longest * 32 bytes of the slab, so a chunk's
+// slab is one contiguous range.
+void build_ref_plan(RefPlan& plan, const st_seqset_s& r, int rc) {
     const int64_t K = r.count;
     plan.rc = rc;
     plan.nchunks = ceil_div(K, rc);
-    plan.sorted.resize(size_t(K));
     plan.tasks.clear();
-    plan.task_off.assign(size_t(plan.nchunks + 1), 0);
+    plan.chunks.clear();
     plan.max_slab = 0;
     plan.max_tasks = 0;
-    std::vector<int32_t> cnt(size_t(r.max_len) + 2);
-    std::vector<int32_t> start(cnt.size());
+    plan.max_spread = 0;
+    std::vector<int32_t> hist(size_t(r.max_len) + 1);
     int64_t slab = 0;
     for (int64_t c = 0; c < plan.nchunks; ++c) {
         const int64_t k0 = c * rc, k1 = std::min<int64_t>(K, k0 + rc);
-        std::fill(cnt.begin(), cnt.end(), 0);
-        for (int64_t k = k0; k < k1; ++k) cnt[size_t(r.h_len[size_t(k)]) + 1]++;
-        for (size_t l = 1; l < cnt.size(); ++l) cnt[l] += cnt[l - 1];
-        std::copy(cnt.begin(), cnt.end(), start.begin());
-        for (int64_t k = k0; k < k1; ++k)
-            plan.sorted[size_t(k0 + start[size_t(r.h_len[size_t(k)])]++)] = int32_t(k);
+        std::fill(hist.begin(), hist.end(), 0);
+        for (int64_t k = k0; k < k1; ++k) hist[size_t(r.h_len[size_t(k)])]++;
         const int64_t slab0 = slab;
-        for (int32_t l = 0; l <= r.max_len; ++l) {
-            const int32_t b = cnt[size_t(l)], e = cnt[size_t(l) + 1];
-            for (int32_t s = b; s < e; s += 32) {
-                plan.tasks.push_back(make_int4(l, int32_t(k0) + s, std::min(32, e - s), int32_t(slab)));
-                slab += int64_t(l) * 32;
+        const int first_task = int(plan.tasks.size());
+        int shortest = 0, longest = 0, count = 0;
+        int64_t start = k0;
+        auto close = [&] {
+            if (!count) return;
+            plan.max_spread = std::max(plan.max_spread, longest - shortest);
+            plan.tasks.push_back(make_int4(longest | (longest == shortest ? 0x100 : 0), int32_t(start),
+                                           count, int32_t(slab)));
+            slab += int64_t(longest) * 32;
+            start += count;
+            count = 0;
+        };
+        for (int l = 0; l <= r.max_len; ++l) {
+            int left = hist[size_t(l)];
+            if (left && count && l - shortest > kMaxSpread) close();
+            while (left) {
+                if (!count) shortest = l;
+                longest = l;
+                const int take = std::min(left, 32 - count);
+                count += take;
+                left -= take;
+                if (count == 32) close();
             }
         }
+        close();
         plan.max_slab = std::max(plan.max_slab, slab - slab0);
-        plan.max_tasks = std::max(plan.max_tasks, int(plan.tasks.size()) - plan.task_off[size_t(c)]);
-        plan.task_off[size_t(c + 1)] = int32_t(plan.tasks.size());
+        const int ntasks = int(plan.tasks.size()) - first_task;
+        plan.max_tasks = std::max(plan.max_tasks, ntasks);
+        plan.chunks.push_back(make_int4(first_task, ntasks, int(slab0), int(slab - slab0)));
+        if (slab > INT32_MAX) fail(ST_EINVAL, "seqtree_b200: reference set too large for one call");
     }
-    if (slab > INT32_MAX) fail(ST_EINVAL, "seqtree_b200: reference set too large for one call");
     plan.ntasks = int64_t(plan.tasks.size());
     plan.slab_bytes = slab;
-    if (!upload) return;
-    h2d(plan.d_sorted.as<int32_t>(size_t(K)), plan.sorted.data(),
-                             sizeof(int32_t) * size_t(K), stream);
-    h2d(plan.d_tasks.as<int4>(plan.tasks.size()), plan.tasks.data(),
-                             sizeof(int4) * plan.tasks.size(), stream);
-    h2d(plan.d_task_off.as<int32_t>(plan.task_off.size()),
-                             plan.task_off.data(), sizeof(int32_t) * plan.task_off.size(), stream);
-    plan.d_slab.as<uint8_t>(size_t(slab) + 16);
-    plan.uid = r.uid;
 }
 
 template <class Plan>
@@ -178,68 +202,130 @@ Plan& plan_slot(std::shared_ptr<void>& own, std::shared_ptr<void>& shared, bool 
     return *static_cast<Plan*>(slot.get());
 }
 
-// QP[p][j][b] for b < 32 (zero beyond A, beyond the pair's length and for empty slots).
+// The slices' profiles, one block per slice: word (row j, quad, b) holds pen(q[j], b) of the
+// quad's four queries, 8 bits each; WIDE rows hold two words per quad and residue, [quad][half][32]
+// with queries 0 | 2 << 16 in half 0 and 1 | 3 << 16 in half 1.  Zero beyond A; empty slots hold the
+// largest penalty, so that the sparse sweep's early end does not wait for them.
+template <bool WIDE>
 __global__ void profile_kernel(const uint8_t* __restrict__ codes, const int64_t* __restrict__ off,
-                               const int2* __restrict__ pairs, const int32_t* __restrict__ plen,
-                               const int32_t* __restrict__ pen, int A, int LQ, int64_t total,
+                               const int4* __restrict__ quads, const int4* __restrict__ slices,
+                               const int32_t* __restrict__ pen, int A, uint32_t maxpen,
                                uint32_t* __restrict__ prof) {
-    const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (idx >= total) return;
-    const int64_t p = idx / (int64_t(LQ) * kRow);
-    const int j = int((idx / kRow) % LQ);
-    const int b = int(idx % kRow);
-    const int2 pr = pairs[p];
-    uint32_t v = 0;
-    if (b < A && j < plen[p] && pr.x >= 0) {
-        const int c1 = codes[off[pr.x] + j];
-        const int c2 = codes[off[pr.y >= 0 ? pr.y : pr.x] + j];
-        v = uint32_t(pen[c1 * A + b]) | (uint32_t(pen[c2 * A + b]) << 16);
+    const int4 sl = slices[blockIdx.x];
+    constexpr int kWords = kQuads * kRow * (WIDE ? 2 : 1);
+    uint32_t* dst = prof + int64_t(sl.w) * kWords;
+    for (int i = threadIdx.x; i < sl.z * kWords; i += blockDim.x) {
+        const int j = i / kWords, w = i - j * kWords;
+        const int quad = w / (kWords / kQuads), half = (w / kRow) & 1, b = w & (kRow - 1);
+        uint32_t v = 0;
+        if (b < A) {
+            const int4 q = quad < sl.y ? quads[sl.x + quad] : make_int4(-1, -1, -1, -1);
+            const int qs[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                if (WIDE && (x & 1) != half) continue;
+                const uint32_t p =
+                    qs[x] < 0 ? maxpen : uint32_t(pen[int(codes[off[qs[x]] + j]) * A + b]);
+                v |= p << (WIDE ? 16 * (x >> 1) : 8 * x);
+            }
+        }
+        dst[i] = v;
     }
-    prof[idx] = v;
 }
 
-// Per task: n rows of 32 lane bytes, each 4*code (lanes past the task's count repeat lane 0).
+// Slots of one chunk (one block): its columns sorted by length, and inside a length so that
+// neighbours have different columns modulo 32 -- each round takes one ref of every residue -- which
+// puts the dense tile's words of a task into different banks.  (Which of several refs of one
+// length and residue comes first does not matter.)
+constexpr int kMaxRounds = 40;  // rc / 32 of the widest chunk
+
+__global__ void __launch_bounds__(256) chunk_order_kernel(const int32_t* __restrict__ rlen, int64_t K, int rc,
+                                                          int max_len, uint32_t* __restrict__ meta) {
+    __shared__ uint32_t occ[65 * 32];
+    __shared__ uint32_t at[65 * kMaxRounds];
+    const int64_t k0 = int64_t(blockIdx.x) * rc;
+    const int kcount = int(K - k0 < rc ? K - k0 : rc);
+    const int rounds = rc / 32, buckets = (max_len + 1) * rounds;
+    for (int i = threadIdx.x; i < (max_len + 1) * 32; i += 256) occ[i] = 0u;
+    for (int i = threadIdx.x; i < buckets; i += 256) at[i] = 0u;
+    __syncthreads();
+    uint32_t bucket[kMaxRounds * 32 / 256];
+#pragma unroll
+    for (int t = 0; t < kMaxRounds * 32 / 256; ++t) {
+        const int c = t * 256 + threadIdx.x;
+        if (c < kcount) {
+            const int l = rlen[k0 + c];
+            bucket[t] = uint32_t(l) * rounds + atomicAdd(&occ[l * 32 + (c & 31)], 1u);
+            atomicAdd(&at[bucket[t]], 1u);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {  // exclusive prefix of the buckets by one warp
+        uint32_t base = 0;
+        for (int b0 = 0; b0 < buckets; b0 += 32) {
+            const int b = b0 + int(threadIdx.x);
+            const uint32_t v = b < buckets ? at[b] : 0u;
+            uint32_t incl = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+                if (int(threadIdx.x) >= o) incl += u;
+            }
+            if (b < buckets) at[b] = base + incl - v;
+            base += __shfl_sync(0xffffffffu, incl, 31);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kMaxRounds * 32 / 256; ++t) {
+        const int c = t * 256 + threadIdx.x;
+        if (c < kcount)
+            meta[k0 + atomicAdd(&at[bucket[t]], 1u)] = uint32_t(c) | (bucket[t] / rounds) << 16;
+    }
+}
+
+// Per task: its longest ref's rows of 32 lane bytes, each 4*code (the null code past a ref's end
+// and past the task's count).
 __global__ void ref_slab_kernel(const uint8_t* __restrict__ codes, const int64_t* __restrict__ off,
-                                const int32_t* __restrict__ sorted, const int4* __restrict__ tasks,
+                                const uint32_t* __restrict__ meta, const int4* __restrict__ tasks, int rc,
                                 uint8_t* __restrict__ slab) {
     const int4 t = tasks[blockIdx.x];
-    for (int idx = threadIdx.x; idx < t.x * 32; idx += blockDim.x) {
-        const int j = idx >> 5, l = idx & 31;
-        const int k = sorted[t.y + (l < t.z ? l : 0)];
-        slab[int64_t(t.w) + idx] = uint8_t(codes[off[k] + j] * 4);
-    }
+    const int rows = t.x & 0xFF, l = threadIdx.x & 31;
+    const uint32_t mt = l < t.z ? meta[t.y + l] : 0u;
+    const int n = int(mt >> 16);
+    const uint8_t* src = codes + (l < t.z ? off[int64_t(t.y) / rc * rc + (mt & 0xFFFFu)] : 0);
+    for (int j = threadIdx.x >> 5; j < rows; j += blockDim.x >> 5)
+        slab[int64_t(t.w) + j * 32 + l] = uint8_t((j < n ? int(src[j]) : kNullCode) * 4);
 }
 
 // ---------------------------------------------------------------------------- fast kernel ---
+// Shared memory of one CTA: byte offsets, in this order.
+struct FastSmem {
+    int codes, tile, bits, frow, task, meta, bar, total;
+};
+
 struct FastArgs {
-    const uint32_t* prof;    // [P][LQ][32]
+    const uint32_t* prof;
     const uint8_t* slab;     // ref code slab
     const int32_t* rlen;
     int64_t K;
     int rc;                  // columns per chunk
-    const int2* pairs;       // (q1, q2); -1 marks an empty slot
-    const int32_t* plen;
-    int64_t P;
-    const int32_t* ref_sorted;
+    const int4* quads;       // original query indices; -1 marks an empty slot
+    const int4* slices;      // (first quad, quads, length, profile row offset)
+    int64_t nslices;
+    const uint32_t* ref_meta;  // per sorted slot: column in the chunk | length << 16
     const int4* tasks;
-    const int32_t* task_off;
-    int slab_cap;            // shared bytes reserved for a chunk's slab
-    int max_tasks;           // shared task slots (the most tasks of one chunk)
-    const uint32_t* prior2;  // rows (M*W1 + d) of pstride words, value i at i + 3; or null
+    const int4* chunks;      // (first task, tasks, slab byte offset, slab bytes)
+    FastSmem sm;
+    int score16;             // sparse scores of 16 bits (else 8: the threshold is at most 255)
+    int spread;              // rows past the query that a mixed task's diagonal may read
+    const uint32_t* prior2;  // rows (M*W1 + d) of pstride words: [3] the first value, [4 + j] steps
     int pstride;
     const int32_t* ftab;     // [m*W1 + n]: per-(m,n) additive term (prior minimum + gap cost)
     int W1;
-    uint32_t bias2;          // BIAS in both halves
     int32_t* out;            // dense output (unused by the sparse form)
     unsigned long long* err; // set when the bounded wait for the staging copies gives up
     SparseSink sink;         // sparse output (unused by the dense form)
-    // Persistent form: a grid of about one wave of CTAs takes tiles (chunk, pair group) from a
-    // global counter, longest query pairs first (the pairs are sorted by length), so the
-    // expensive tiles start early and the wave drains evenly.  0: one CTA per tile.
-    int persistent;
-    int nchunks;
-    int ntiles;
-    unsigned int* queue;     // zeroed before every launch
 };
 
 // One non-blocking probe of an mbarrier phase (callers bound the number of probes).
@@ -262,350 +348,344 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
         : "memory");
 }
 
-// One warp unit: the 4 pairs of one slice of the CTA against the 32 refs of one task.  The
-// sweep reads each residue offset straight from the staged code slab; the slice base and the
-// row offset j*128 are folded into two per-position addresses, so the 8 lookups of a position
-// are LDS [address + compile-time immediate (pair * LQ * 128)].  Query-longer pairs shift the
-// diagonal-d address by d rows; ref-longer pairs read the residue d positions further on.
-template <int LQ, bool PRIOR>
-__device__ __forceinline__ void run_unit(const FastArgs& a, const uint8_t* smem,
-                                         const uint8_t* s_codes, uint32_t* s_tile,
-                                         const int32_t* s_plen, const int16_t* s_col, int slice,
-                                         const int4 task, int tb, int64_t k0, int lane) {
-    constexpr int kRowB = kRow * 4;
-    constexpr int kPairB = LQ * kRowB;
-    const int n = task.x;
-    const int m = s_plen[slice * kPairsPerSlice];
-    const int L = min(m, n);
-    const int d = abs(m - n);
-    const int dq = m > n ? d : 0;   // query longer: diagonal d is d profile rows further down
-    const int dr = n > m ? d : 0;   // ref longer: diagonal d reads residue j + d
-    const uint8_t* rows0 = s_codes + tb + lane;
-    const uint8_t* rowsd = rows0 + dr * 32;
-    const uint32_t base0 = uint32_t(slice * kPairsPerSlice * kPairB);
-    const uint32_t based = base0 + uint32_t(dq * kRowB);
-    uint32_t res[kPairsPerSlice];
-    if (d == 0) {
-        uint32_t S[kPairsPerSlice] = {0u, 0u, 0u, 0u};
-#pragma unroll 4
-        for (int j = 0; j < L; ++j) {
-            const uint32_t a0 = base0 + uint32_t(j * kRowB) + rows0[j * 32];
-#pragma unroll
-            for (int q = 0; q < kPairsPerSlice; ++q)
-                S[q] += *reinterpret_cast<const uint32_t*>(smem + a0 + q * kPairB);
-        }
-#pragma unroll
-        for (int q = 0; q < kPairsPerSlice; ++q) res[q] = S[q];
+inline FastSmem fast_smem(int prof_cap, int slab_cap, int rc, int W1, int max_tasks, int score_bytes) {
+    FastSmem m;
+    auto up = [](int v) { return (v + 15) & ~15; };
+    m.codes = prof_cap;
+    m.tile = m.codes + up(slab_cap);
+    // prof_cap: a slice's profile and its zero rows; slab_cap: a chunk's code slab; the tile is rc
+    // columns of kTileW words (dense, score_bytes 0), or scores [query][column] and the hit bitmap
+    m.bits = m.tile + up(score_bytes ? kSliceQ * rc * score_bytes : rc * kTileW * 4);
+    m.frow = m.bits + up(score_bytes ? kSliceQ * (rc / 32) * 4 : 0);
+    m.task = m.frow + up(W1 * 4);
+    m.meta = m.task + up(max_tasks * 16);
+    m.bar = m.meta + up(rc * 4);
+    m.total = m.bar + 16;
+    return m;
+}
+
+// The (even, odd) int16x2 words of a quad at one profile address.
+template <bool WIDE>
+__device__ __forceinline__ void quad_words(const uint8_t* p, uint32_t& e, uint32_t& o) {
+    if constexpr (WIDE) {
+        e = *reinterpret_cast<const uint32_t*>(p);
+        o = *reinterpret_cast<const uint32_t*>(p + kRow * 4);
     } else {
-        // Prior row of (max(m,n), d): value i at prow[i + 3], so values j+1..j+4 of an aligned
-        // group of four positions are one 16-byte load.
-        const uint32_t* prow = PRIOR ? a.prior2 + (size_t(max(m, n)) * a.W1 + d) * a.pstride : nullptr;
-        uint32_t S[kPairsPerSlice], Cb[kPairsPerSlice], best[kPairsPerSlice];
-        const uint32_t first = PRIOR ? a.bias2 + __ldg(prow + 3) : a.bias2;
-#pragma unroll
-        for (int q = 0; q < kPairsPerSlice; ++q) {
-            S[q] = 0u;
-            Cb[q] = a.bias2;
-            best[q] = first;
-        }
-        // The sweep, in two versions: when the query is the longer one (dr == 0) both diagonals
-        // read residue j of the ref, so one byte load serves both addresses.
-        auto sweep = [&](auto same_residue) {
-            constexpr bool kSame = decltype(same_residue)::value;
-            auto step = [&](int j, uint32_t pr) {
-                const uint32_t c0 = rows0[j * 32];
-                const uint32_t a0 = base0 + uint32_t(j * kRowB) + c0;
-                const uint32_t ad = based + uint32_t(j * kRowB) + (kSame ? c0 : uint32_t(rowsd[j * 32]));
-#pragma unroll
-                for (int q = 0; q < kPairsPerSlice; ++q) {
-                    const uint32_t p0v = *reinterpret_cast<const uint32_t*>(smem + a0 + q * kPairB);
-                    const uint32_t pdv = *reinterpret_cast<const uint32_t*>(smem + ad + q * kPairB);
-                    S[q] += pdv;
-                    Cb[q] = Cb[q] + p0v - pdv;  // per-half exact: halves stay in [0, 2^15)
-                    best[q] = __viaddmin_s16x2(Cb[q], pr, best[q]);
-                }
-            };
-            // The prior values of the next group of four positions are requested one group
-            // ahead, so their load latency hides behind the current group's lookups.
-            int j = 0;
-            uint4 pnext = make_uint4(0u, 0u, 0u, 0u);
-            if constexpr (PRIOR)
-                if (L >= 4) pnext = __ldg(reinterpret_cast<const uint4*>(prow + 4));
-            for (; j + 4 <= L; j += 4) {
-                const uint4 pv = pnext;
-                if constexpr (PRIOR)
-                    if (j + 8 <= L) pnext = __ldg(reinterpret_cast<const uint4*>(prow + j + 8));
-                step(j, pv.x);
-                step(j + 1, pv.y);
-                step(j + 2, pv.z);
-                step(j + 3, pv.w);
-            }
-            for (; j < L; ++j) step(j, PRIOR ? __ldg(prow + j + 4) : 0u);
-        };
-        if (dr == 0)
-            sweep(std::true_type{});
-        else
-            sweep(std::false_type{});
-#pragma unroll
-        for (int q = 0; q < kPairsPerSlice; ++q) res[q] = S[q] + best[q] - a.bias2;
-    }
-    if (lane < task.z) {
-        const int col = s_col[int(task.y - k0) + lane];
-#pragma unroll
-        for (int q = 0; q < kPairsPerSlice; ++q)
-            s_tile[(slice * kPairsPerSlice + q) * a.rc + col] = res[q];
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(p);
+        o = __byte_perm(w, 0u, 0x4341);  // bytes 1 and 3
+        e = w - o * 256u;                // bytes 0 and 2, an IMAD
     }
 }
 
-template <int LQ, bool PRIOR, bool SPARSE>
-__global__ void __launch_bounds__(kThreads, 3) gapblock_fast_kernel(const FastArgs a) {
-    extern __shared__ __align__(128) uint8_t smem[];
-    constexpr int kProfB = kGP * LQ * kRow * 4;
-    const int prof_area = kProfB > (kGP / kPairsPerSlice) * a.rc * 4 ? kProfB
-                                                                    : (kGP / kPairsPerSlice) * a.rc * 4;
-    uint8_t* s_codes = smem + prof_area;
-    uint32_t* s_tile = reinterpret_cast<uint32_t*>(s_codes + a.slab_cap);
-    int32_t* s_ftab = reinterpret_cast<int32_t*>(s_tile + kGP * a.rc);
-    uint8_t* s_len = reinterpret_cast<uint8_t*>(s_ftab + ((a.W1 * a.W1 + 3) & ~3));
-    int4* s_task = reinterpret_cast<int4*>(s_len + ((a.rc + 15) & ~15));
-    int16_t* s_col = reinterpret_cast<int16_t*>(s_task + a.max_tasks);
-    int32_t* s_plen = reinterpret_cast<int32_t*>(s_col + ((a.rc + 7) & ~7));
-    uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_plen + kGP);
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    volatile int* s_next = reinterpret_cast<volatile int*>(s_bar + 1);  // in the barrier's 16 bytes
-    const uint32_t bar = uint32_t(__cvta_generic_to_shared(s_bar));
-    if (tid == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
-    const int npg = int((a.P + kGP - 1) / kGP);
-    for (int iter = 0;; ++iter) {
-    int chunk, pg;
-    if (a.persistent) {
-        if (tid == 0) *s_next = int(atomicAdd(a.queue, 1u));
-        __syncthreads();
-        const int t = *s_next;
-        if (t >= a.ntiles) break;
-        pg = npg - 1 - t / a.nchunks;
-        chunk = t - (t / a.nchunks) * a.nchunks;
-    } else {
-        if (iter > 0) break;
-        chunk = blockIdx.x;
-        pg = int(blockIdx.y + blockIdx.z * gridDim.y);  // pair groups past 65,535 use z
-        if (pg >= npg) break;
+// One warp unit: NQ quads of the slice against the 32 refs of one task.  Per position: one or two
+// code bytes, 2 * NQ lookups at immediates from two addresses, and per quad two splits, two adds and
+// two DPX minima.  What bounds it: issue slots (10 per quad and position, 2.5 cycles of an SM's
+// four schedulers), with the LDS pipe (2 cycles), the ALU (2 to 3) and the FMA pipe just below.
+// SPARSE without a prior: both states only grow, so once every A and B of the warp is above its
+// lane's threshold no cell can pass and the unit ends (false).  Looked at every four positions from
+// the eighth on: 13 instructions, against 44 a position; on junctions with BLOSUM62 at 24 the
+// sweep ends after 9.8 of 13.2 positions on average.
+template <int NQ, bool PRIOR, bool WIDE, bool SPARSE>
+__device__ __forceinline__ bool run_unit(const FastArgs& a, const uint8_t* s_prof, const uint8_t* rows0,
+                                         int m, int n, int nmax, bool same_len, uint32_t lim,
+                                         uint32_t (&res)[2 * NQ]) {
+    constexpr bool kStop = SPARSE && !PRIOR;
+    constexpr int kQuadB = kRow * 4 * (WIDE ? 2 : 1);
+    constexpr int kRowB = kQuadB * kQuads;
+    const int L = min(m, nmax);
+    if (same_len && nmax == m) {  // no block: the plain sum
+#pragma unroll
+        for (int q = 0; q < 2 * NQ; ++q) res[q] = 0u;
+        auto step = [&](int j) {
+            const uint8_t* p = s_prof + j * kRowB + rows0[j * 32];
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                uint32_t e, o;
+                quad_words<WIDE>(p + q * kQuadB, e, o);
+                res[2 * q] += e;
+                res[2 * q + 1] += o;
+            }
+        };
+        int j = 0;
+        for (; j + 4 <= L; j += 4) {
+            if (kStop && j >= 8) {
+                uint32_t low = res[0];
+#pragma unroll
+                for (int q = 1; q < 2 * NQ; q += 2)
+                    low = __vimin3_s16x2(low, res[q], q + 1 < 2 * NQ ? res[q + 1] : res[q]);
+                if (!__any_sync(0xffffffffu, (lim - low) & 0x80008000u)) return false;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) step(j + u);
+        }
+        for (; j < L; ++j) step(j);
+        return true;
     }
-    const uint32_t parity = uint32_t(iter & 1);
+    // Diagonal d: a longer query reads d profile rows further down, a longer ref reads the residue d
+    // positions further on.
+    const uint8_t* pd = s_prof + max(m - n, 0) * kRowB;
+    const uint8_t* rowsd = rows0 + max(n - m, 0) * 32;
+    const uint32_t* prow =
+        PRIOR ? a.prior2 + (size_t(max(m, n)) * a.W1 + abs(m - n)) * a.pstride : nullptr;
+    uint32_t A[2 * NQ];
+    const uint32_t first = PRIOR ? __ldg(prow + 3) : 0u;
+#pragma unroll
+    for (int q = 0; q < 2 * NQ; ++q) A[q] = res[q] = first;
+    // The sweep, in two versions: when no ref is longer than the query both diagonals read
+    // residue j of the ref, so one byte load serves both addresses.
+    auto sweep = [&](auto same_residue) {
+        constexpr bool kSame = decltype(same_residue)::value;
+        auto step = [&](int j, uint32_t dp) {
+            const uint32_t c0 = rows0[j * 32];
+            const uint8_t* p0 = s_prof + j * kRowB + c0;
+            const uint8_t* p1 = pd + j * kRowB + (kSame ? c0 : uint32_t(rowsd[j * 32]));
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                uint32_t e0, o0, e1, o1;
+                quad_words<WIDE>(p0 + q * kQuadB, e0, o0);
+                quad_words<WIDE>(p1 + q * kQuadB, e1, o1);
+                A[2 * q] += PRIOR ? e0 + dp : e0;
+                A[2 * q + 1] += PRIOR ? o0 + dp : o0;
+                res[2 * q] = __viaddmin_s16x2(res[2 * q], e1, A[2 * q]);
+                res[2 * q + 1] = __viaddmin_s16x2(res[2 * q + 1], o1, A[2 * q + 1]);
+            }
+        };
+        // The prior's steps of the next group of four positions are requested one group ahead,
+        // so their load latency hides behind the current group's lookups.
+        int j = 0;
+        uint4 pnext = make_uint4(0u, 0u, 0u, 0u);
+        if constexpr (PRIOR)
+            if (L >= 4) pnext = __ldg(reinterpret_cast<const uint4*>(prow + 4));
+        for (; j + 4 <= L; j += 4) {
+            if (kStop && j >= 8) {
+                uint32_t low = __vimin3_s16x2(A[0], res[0], res[1]);
+#pragma unroll
+                for (int q = 1; q < 2 * NQ; ++q)
+                    low = __vimin3_s16x2(low, A[q], q + 1 < 2 * NQ ? res[q + 1] : A[q]);
+                if (!__any_sync(0xffffffffu, (lim - low) & 0x80008000u)) return false;
+            }
+            const uint4 pv = pnext;
+            if constexpr (PRIOR)
+                if (j + 8 <= L) pnext = __ldg(reinterpret_cast<const uint4*>(prow + j + 8));
+            step(j, pv.x);
+            step(j + 1, pv.y);
+            step(j + 2, pv.z);
+            step(j + 3, pv.w);
+        }
+        for (; j < L; ++j) step(j, PRIOR ? __ldg(prow + j + 4) : 0u);
+        return true;
+    };
+    return nmax <= m ? sweep(std::true_type{}) : sweep(std::false_type{});
+}
+
+// One CTA per (chunk, slice).  CTAs per SM: three of 80 registers, or in the sparse form four of 64,
+// which with 8-bit scores fit at the 1,024-column width: 148 -> 139 ms on 100,000 x 1,000,000 (a
+// tile's staging and its barriers are then covered by three others).  Narrower chunks
+// cost more tiles: 3.0 (1,024) / 3.3 (768) / 3.8 (512) / 5.1 ms (256) per 2e9 pairs.
+template <bool PRIOR, bool WIDE, bool SPARSE>
+__global__ void __launch_bounds__(kThreads, SPARSE ? 4 : 3) gapblock_fast_kernel(const FastArgs a) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    const FastSmem& sm = a.sm;
+    constexpr int kRowB = kRow * 4 * kQuads * (WIDE ? 2 : 1);
+    uint8_t* s_codes = smem + sm.codes;
+    uint32_t* s_tile = reinterpret_cast<uint32_t*>(smem + sm.tile);
+    uint8_t* s_score = smem + sm.tile;
+    uint32_t* s_bits = reinterpret_cast<uint32_t*>(smem + sm.bits);
+    int32_t* s_frow = reinterpret_cast<int32_t*>(smem + sm.frow);
+    int4* s_task = reinterpret_cast<int4*>(smem + sm.task);
+    uint32_t* s_meta = reinterpret_cast<uint32_t*>(smem + sm.meta);
+    uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + sm.bar);
+
+    const int64_t slice = blockIdx.y + int64_t(blockIdx.z) * gridDim.y;  // slices past 65,535 use z
+    if (slice >= a.nslices) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t bar = uint32_t(__cvta_generic_to_shared(s_bar));
+    const int chunk = blockIdx.x;
     const int64_t k0 = int64_t(chunk) * a.rc;
     const int kcount = int(a.K - k0 < a.rc ? a.K - k0 : a.rc);
-    const int p0 = pg * kGP;
-    const int np = int(a.P - p0 < kGP ? a.P - p0 : kGP);
-    const int t0 = a.task_off[chunk], t1 = a.task_off[chunk + 1];
-    const int tw0 = a.tasks[t0].w;
-    const int slab_bytes = (t1 > t0 ? a.tasks[t1 - 1].w + a.tasks[t1 - 1].x * 32 : tw0) - tw0;
+    const int4 sl = a.slices[slice];
+    const int nq = sl.y, m = sl.z;
+    const int4 ch = a.chunks[chunk];
+    const int t0 = ch.x, nt = ch.y, slab0 = ch.z, slab_bytes = ch.w;
 
-    // Stage the CTA's profile slab and the chunk's code slab with two bulk (TMA) copies that
-    // complete on one mbarrier, while the other threads load the (m, n) terms and lengths.
-    // (In the persistent form every tile is one phase of the barrier; the previous tile's
-    // generic-proxy writes to the same shared memory are ordered before these copies by the
-    // barrier that ended it and the proxy fence.)
+    // Stage the slice's profile and the chunk's code slab with two bulk (TMA) copies that complete
+    // on one mbarrier, while the threads load the rest.
     if (tid == 0) {
-        const uint32_t prof_bytes = uint32_t(np) * LQ * kRow * 4;
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                     "r"(prof_bytes + uint32_t(slab_bytes))
+                     "r"(uint32_t(m * kRowB + slab_bytes))
                      : "memory");
-        bulk_g2s(uint32_t(__cvta_generic_to_shared(smem)),
-                 a.prof + size_t(p0) * LQ * kRow, prof_bytes, bar);
+        if (m > 0)
+            bulk_g2s(uint32_t(__cvta_generic_to_shared(smem)),
+                     reinterpret_cast<const uint8_t*>(a.prof) + int64_t(sl.w) * kRowB,
+                     uint32_t(m * kRowB), bar);
         if (slab_bytes > 0)
-            bulk_g2s(uint32_t(__cvta_generic_to_shared(s_codes)), a.slab + tw0,
+            bulk_g2s(uint32_t(__cvta_generic_to_shared(s_codes)), a.slab + slab0,
                      uint32_t(slab_bytes), bar);
     }
-    // Per-tile metadata in shared memory, so that a warp unit starts without a chain of global
-    // loads: the chunk's tasks, each sorted slot's column, the pairs' query lengths.
-    for (int i = tid; i < a.W1 * a.W1; i += kThreads) s_ftab[i] = a.ftab[i];
-    for (int c = tid; c < kcount; c += kThreads) {
-        s_len[c] = uint8_t(a.rlen[k0 + c]);
-        s_col[c] = int16_t(a.ref_sorted[k0 + c] - k0);
+    // Per-tile metadata: the (m, n) terms, the chunk's tasks, each sorted slot's column and length.
+    // Rows past the query keep the null column at 0 for lanes past their ref's end.
+    // The sparse form keeps the test word instead of the term: 0x8000 + T in both halves, T =
+    // threshold - term; a half is a hit when it is at most T, bit 15 of the difference.
+    for (int i = tid; i < a.W1; i += kThreads) {
+        const int32_t f = a.ftab[m * a.W1 + i];
+        const int64_t room = int64_t(a.sink.thresh) - f;
+        s_frow[i] = !SPARSE ? f
+                    : room >= 0 ? int32_t(0x80008000u + uint32_t(room < 32767 ? room : 32767) * 0x10001u)
+                                : 0x7FFF7FFF;
     }
-    for (int i = tid; i < t1 - t0; i += kThreads) s_task[i] = a.tasks[t0 + i];
-    if (tid < np) s_plen[tid] = a.plen[p0 + tid];
+    for (int i = tid; i < a.spread * kQuads * (WIDE ? 2 : 1); i += kThreads)
+        reinterpret_cast<uint32_t*>(smem + m * kRowB)[i * kRow + kNullCode] = 0u;
+#pragma unroll 4
+    for (int c = tid; c < kcount; c += kThreads) s_meta[c] = a.ref_meta[k0 + c];
+    if (SPARSE)
+        for (int i = tid; i < kSliceQ * (a.rc / 32) / 4; i += kThreads)
+            reinterpret_cast<uint4*>(s_bits)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = tid; i < nt; i += kThreads) s_task[i] = a.tasks[t0 + i];
     __syncthreads();
     {
         // Bounded wait on phase 0 by every thread.  If any thread runs out, the CTA records
         // the failure, waits once more (bounded) for its copies in flight, and leaves as a
         // whole -- the host then reports ST_ETIMEOUT and no tile is stored.
         uint32_t done = 0;
-        for (int it = 0; it < (1 << 20) && !done; ++it) done = mbar_try_wait(bar, parity);
+        for (int it = 0; it < (1 << 20) && !done; ++it) done = mbar_try_wait(bar, 0);
         if (__syncthreads_or(!done)) {
             if (tid == 0) atomicExch(a.err, 1ull);
-            for (int it = 0; it < (1 << 20) && !done; ++it) done = mbar_try_wait(bar, parity);
+            for (int it = 0; it < (1 << 20) && !done; ++it) done = mbar_try_wait(bar, 0);
             __syncthreads();
             return;
         }
     }
 
-    const int nslices = np / kPairsPerSlice;
-    const int units = (t1 - t0) * nslices;
-    for (int u = warp; u < units; u += kWarps) {
-        const int ti = u / nslices;
-        const int4 task = s_task[ti];
-        const int tb = task.w - tw0;
-        run_unit<LQ, PRIOR>(a, smem, s_codes, s_tile, s_plen, s_col, u - ti * nslices, task, tb,
-                            k0, lane);
+    for (int t = warp; t < nt; t += kWarps) {
+        const int4 task = s_task[t];
+        const int nmax = task.x & 0xFF;
+        const bool same_len = (task.x & 0x100) != 0;
+        const bool live = lane < task.z;
+        const uint32_t meta = s_meta[int(task.y - k0) + (live ? lane : 0)];
+        const int n = live ? int(meta >> 16) : nmax;
+        const int col = int(meta & 0xFFFFu);
+        const uint8_t* rows0 = s_codes + (task.w - slab0) + lane;
+        const int32_t f = s_frow[n];
+        const uint32_t lim = live ? uint32_t(f) : 0x7FFF7FFFu;
+        auto unit = [&](auto quads) {
+            constexpr int NQ = decltype(quads)::value;
+            uint32_t res[2 * NQ];
+            const bool done =
+                run_unit<NQ, PRIOR, WIDE, SPARSE>(a, smem, rows0, m, n, nmax, same_len, lim, res);
+            if constexpr (!SPARSE) {
+                if (live) {
+                    uint32_t* dst = s_tile + col * kTileW;
+#pragma unroll
+                    for (int q = 0; q < 2 * NQ; ++q) dst[q] = res[q];
+                    dst[2 * kQuads] = uint32_t(f);
+                }
+            } else {
+                if (!done) return;
+                uint32_t any = 0u;
+#pragma unroll
+                for (int q = 0; q < 2 * NQ; ++q) any |= lim - res[q];
+                if (any & 0x80008000u) {
+#pragma unroll
+                    for (int q = 0; q < 2 * NQ; ++q) {
+                        const uint32_t hit = lim - res[q];
+                        // word q of quad q / 2: queries (q & 1) and (q & 1) + 2
+                        const int row = (q >> 1) * 4 + (q & 1);
+                        auto keep = [&](int at, uint32_t v) {
+                            atomicOr(s_bits + at * (a.rc / 32) + (col >> 5), 1u << (col & 31));
+                            if (a.score16)
+                                reinterpret_cast<uint16_t*>(s_score)[at * a.rc + col] = uint16_t(v);
+                            else
+                                s_score[at * a.rc + col] = uint8_t(v);
+                        };
+                        if (hit & 0x8000u) keep(row, res[q]);
+                        if (hit & 0x80000000u) keep(row + 2, res[q] >> 16);
+                    }
+                }
+            }
+        };
+        if (nq > 2)
+            unit(std::integral_constant<int, 4>{});
+        else if (nq == 2)
+            unit(std::integral_constant<int, 2>{});
+        else
+            unit(std::integral_constant<int, 1>{});
     }
     __syncthreads();
 
-    // Per-slice column terms fcol[slice][c] = ftab[m_slice][len(c)], written over the profile
-    // (no longer read), then the coalesced write-out: each thread takes one pair and four
-    // columns, reads the packed tile and the terms once and stores both queries' rows as
-    // 16-byte vectors.
-    int32_t* s_fcol = reinterpret_cast<int32_t*>(smem);
-    for (int i = tid; i < nslices * a.rc; i += kThreads) {
-        const int sl = i / a.rc, c = i - sl * a.rc;
-        s_fcol[i] = c < kcount ? s_ftab[s_plen[sl * kPairsPerSlice] * a.W1 + s_len[c]] : 0;
-    }
-    __syncthreads();
-    const int cols4 = (kcount + 3) >> 2;
-    if (SPARSE && a.sink.ordered) {
-        // Ordered form: warp w owns tile row (pair w / 2, half w % 2).  It counts its hits, the
-        // CTA reserves one segment for all of them, and the warp writes its row's hits there in
-        // ascending column order, recording the piece (row, chunk) it wrote.
-        __shared__ unsigned long long s_rowcnt[kWarps + 1];  // row counts, then the base
-        __shared__ int s_fits;
-        const unsigned full = 0xffffffffu;
-        const int pl = warp >> 1, hf = warp & 1;
-        int qrow = -1;
-        if (pl < np) {
-            const int2 pr = a.pairs[p0 + pl];
-            qrow = hf ? pr.y : pr.x;
-        }
-        const uint32_t* src = s_tile + pl * a.rc;
-        const int32_t* fc = s_fcol + (pl / kPairsPerSlice) * a.rc;
-        // Lane l takes columns 4l..4l+3 of each 128-column group (16-byte loads of the packed
-        // tile and of the column terms); bit u of the result marks a hit in column 4l + u.
-        auto group = [&](int g, int32_t (&v)[4]) {
-            const int c = g * 128 + lane * 4;
-            uint32_t hits = 0;
-            if (c < kcount) {
-                const uint4 t = *reinterpret_cast<const uint4*>(src + c);
-                const int4 f = *reinterpret_cast<const int4*>(fc + c);
-                const uint32_t tw[4] = {t.x, t.y, t.z, t.w};
-                const int32_t fw[4] = {f.x, f.y, f.z, f.w};
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    v[u] = int32_t((hf ? (tw[u] >> 16) : (tw[u] & 0xFFFFu)) + uint32_t(fw[u]));
-                    if (c + u < kcount && v[u] <= a.sink.thresh) hits |= 1u << u;
-                }
+    if constexpr (!SPARSE) {
+        // Warp w writes the two rows of result word w: 128 contiguous bytes per store.
+        const int quad = warp >> 1;
+        if (quad < nq) {
+            const int4 q = a.quads[sl.x + quad];
+            const int q1 = (warp & 1) ? q.y : q.x, q2 = (warp & 1) ? q.w : q.z;
+            int32_t* d1 = a.out + int64_t(q1) * a.K + k0;
+            int32_t* d2 = a.out + int64_t(q2) * a.K + k0;
+#pragma unroll 4
+            for (int c = lane; c < kcount; c += 32) {
+                const uint32_t v = s_tile[c * kTileW + warp], f = s_tile[c * kTileW + 2 * kQuads];
+                if (q1 >= 0) d1[c] = int32_t((v & 0xFFFFu) + f);
+                if (q2 >= 0) d2[c] = int32_t((v >> 16) + f);
             }
-            return hits;
-        };
-        const int groups = (kcount + 127) >> 7;
-        int n = 0;
-        if (qrow >= 0)
-            for (int g = 0; g < groups; ++g) {
-                int32_t v[4];
-                n += __popc(group(g, v));
-            }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(full, n, o);
-        if (lane == 0) s_rowcnt[warp] = (unsigned long long)n;
-        __syncthreads();
-        if (tid == 0) {
-            unsigned long long tot = 0;
-            for (int w = 0; w < kWarps; ++w) tot += s_rowcnt[w];
-            const unsigned long long base = tot ? atomicAdd(a.sink.count, tot) : 0ull;
-            s_rowcnt[kWarps] = base;
-            s_fits = base + tot <= a.sink.cap ? 1 : 0;  // else counted only; the host re-runs
-        }
-        __syncthreads();
-        if (qrow >= 0) {
-            unsigned long long off = s_rowcnt[kWarps];
-            for (int w = 0; w < warp; ++w) off += s_rowcnt[w];
-            const int64_t piece = (int64_t(qrow) - a.sink.row0) * a.sink.nchunks + chunk;
-            if (lane == 0) {
-                a.sink.piece_off[piece] = int64_t(off);
-                a.sink.piece_cnt[piece] = n;
-            }
-            if (s_fits && n > 0) {
-                for (int g = 0; g < groups; ++g) {
-                    int32_t v[4];
-                    uint32_t hits = group(g, v);
-                    const int cnt = __popc(hits);
-                    int incl = cnt;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int t = __shfl_up_sync(full, incl, o);
-                        if (lane >= o) incl += t;
-                    }
-                    unsigned long long pos = off + (unsigned long long)(incl - cnt);
-                    const int c = g * 128 + lane * 4;
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (hits & (1u << u)) a.sink.seg[pos++] = make_int2(int(k0 + c + u), v[u]);
-                    off += (unsigned long long)__shfl_sync(full, incl, 31);
-                }
-            }
-        }
-    } else if constexpr (SPARSE) {
-        // Every lane runs the same number of rounds (sink_append is warp-collective).
-        const int total = np * cols4;
-        for (int i0 = 0; i0 < total; i0 += kThreads) {
-            const int i = i0 + tid;
-            uint32_t hits = 0;
-            int pl = 0, c = 0;
-            int2 pr = make_int2(-1, -1);
-            if (i < total) {
-                pl = i / cols4;
-                c = (i - pl * cols4) * 4;
-                pr = a.pairs[p0 + pl];
-            }
-            const uint32_t* src = s_tile + pl * a.rc + c;
-            const int32_t* fc = s_fcol + (pl / kPairsPerSlice) * a.rc + c;
-            if (pr.x >= 0) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (c + u >= kcount) break;
-                    const uint32_t t = src[u];
-                    const uint32_t f = uint32_t(fc[u]);
-                    if (int32_t((t & 0xFFFFu) + f) <= a.sink.thresh) hits |= 1u << u;
-                    if (pr.y >= 0 && int32_t((t >> 16) + f) <= a.sink.thresh) hits |= 16u << u;
-                }
-            }
-            sink_append(a.sink, hits, lane, [&](int b, unsigned long long& key, int32_t& val) {
-                const int u = b & 3;
-                const uint32_t t = src[u];
-                val = int32_t((b < 4 ? (t & 0xFFFFu) : (t >> 16)) + uint32_t(fc[u]));
-                key = sink_key(a.sink, b < 4 ? pr.x : pr.y, k0 + c + u);
-            });
         }
     } else {
-    const bool vec = (a.K & 3) == 0;
-    for (int i = tid; i < np * cols4; i += kThreads) {
-        const int pl = i / cols4;
-        const int c = (i - pl * cols4) * 4;
-        const int2 pr = a.pairs[p0 + pl];
-        if (pr.x < 0) continue;
-        const uint32_t* src = s_tile + pl * a.rc + c;
-        const int32_t* fc = s_fcol + (pl / kPairsPerSlice) * a.rc + c;
-        int32_t* d1 = a.out + int64_t(pr.x) * a.K + k0 + c;
-        int32_t* d2 = pr.y >= 0 ? a.out + int64_t(pr.y) * a.K + k0 + c : nullptr;
-        if (vec && c + 4 <= kcount) {
-            const uint4 t = *reinterpret_cast<const uint4*>(src);
-            const int4 f = *reinterpret_cast<const int4*>(fc);
-            *reinterpret_cast<int4*>(d1) =
-                make_int4(int32_t((t.x & 0xFFFFu) + uint32_t(f.x)), int32_t((t.y & 0xFFFFu) + uint32_t(f.y)),
-                          int32_t((t.z & 0xFFFFu) + uint32_t(f.z)), int32_t((t.w & 0xFFFFu) + uint32_t(f.w)));
-            if (d2)
-                *reinterpret_cast<int4*>(d2) =
-                    make_int4(int32_t((t.x >> 16) + uint32_t(f.x)), int32_t((t.y >> 16) + uint32_t(f.y)),
-                              int32_t((t.z >> 16) + uint32_t(f.z)), int32_t((t.w >> 16) + uint32_t(f.w)));
-        } else {
-            for (int u = 0; u < 4 && c + u < kcount; ++u) {
-                d1[u] = int32_t((src[u] & 0xFFFFu) + uint32_t(fc[u]));
-                if (d2) d2[u] = int32_t((src[u] >> 16) + uint32_t(fc[u]));
+        // Warp w owns queries 2w and 2w + 1 of the slice: it counts their hits, reserves a segment
+        // for them and writes each row's hits there in ascending column order, recording the piece
+        // (row, chunk) it wrote.  (One reservation per CTA made every warp wait for the atomic's
+        // round trip on each tile.)
+        const unsigned full = 0xffffffffu;
+        const int words = (kcount + 31) >> 5, pitch = a.rc / 32;
+        if ((warp >> 1) >= nq) return;
+        const int4 q = a.quads[sl.x + (warp >> 1)];
+        const int qrow[2] = {(warp & 1) ? q.z : q.x, (warp & 1) ? q.w : q.y};
+        int cnt[2] = {0, 0};
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            if (qrow[r] < 0) continue;
+            int n = 0;
+            for (int w = lane; w < words; w += 32) n += __popc(s_bits[(warp * 2 + r) * pitch + w]);
+            cnt[r] = int(__reduce_add_sync(full, unsigned(n)));
+        }
+        const int tot = cnt[0] + cnt[1];
+        unsigned long long off = 0;
+        if (tot > 0) {
+            if (lane == 0) off = atomicAdd(a.sink.count, (unsigned long long)tot);
+            off = __shfl_sync(full, off, 0);
+        }
+        const bool fits = off + tot <= a.sink.cap;  // else counted only; the host re-runs
+        const int row_of = lane ? qrow[1] : qrow[0];
+        if (lane < 2 && row_of >= 0) {
+            const int64_t piece = (int64_t(row_of) - a.sink.row0) * a.sink.nchunks + chunk;
+            a.sink.piece_cnt[piece] = lane ? cnt[1] : cnt[0];
+            if (tot > 0) a.sink.piece_off[piece] = int64_t(off + (lane ? cnt[0] : 0));
+        }
+        if (tot == 0 || !fits) return;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            if (cnt[r] == 0) continue;
+            const int row = warp * 2 + r;
+            for (int w0 = 0; w0 < words; w0 += 32) {
+                uint32_t word = w0 + lane < words ? s_bits[row * pitch + w0 + lane] : 0u;
+                const int c0 = __popc(word);
+                int incl = c0;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(full, incl, o);
+                    if (lane >= o) incl += t;
+                }
+                unsigned long long pos = off + (unsigned long long)(incl - c0);
+                while (word) {
+                    const int c = (w0 + lane) * 32 + __ffs(int(word)) - 1;
+                    word &= word - 1;
+                    const int at = row * a.rc + c;
+                    const int v = a.score16 ? reinterpret_cast<const uint16_t*>(s_score)[at] : s_score[at];
+                    a.sink.seg[pos++] =
+                        make_int2(int(k0 + c), v + __ldg(a.ftab + m * a.W1 + a.rlen[k0 + c]));
+                }
+                off += (unsigned long long)__shfl_sync(full, incl, 31);
             }
         }
-    }
-    }
-    __syncthreads();  // this tile's shared memory is free for the next one
     }
 }
 
@@ -714,44 +794,18 @@ __global__ void __launch_bounds__(256) gapblock_general_kernel(const GeneralArgs
     }
 }
 
-template <int LQ, bool PRIOR>
-const char* launch_fast(const FastArgs& args, dim3 grid, size_t smem, cudaStream_t stream) {
-    const bool sparse = args.sink.keys != nullptr || args.sink.ordered;  // either sparse form
-    auto kern = sparse ? gapblock_fast_kernel<LQ, PRIOR, true>
-                       : gapblock_fast_kernel<LQ, PRIOR, false>;
-    STB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    kern<<<grid, kThreads, smem, stream>>>(args);
-    STB_CUDA(cudaGetLastError());
-    return sparse ? "gapblock_fast_kernel<sparse>" : "gapblock_fast_kernel";
+using FastKernel = void (*)(FastArgs);
+
+FastKernel fast_kernel(bool prior, bool wide, bool sparse) {
+    if (sparse)
+        return prior ? (wide ? gapblock_fast_kernel<true, true, true> : gapblock_fast_kernel<true, false, true>)
+                     : (wide ? gapblock_fast_kernel<false, true, true> : gapblock_fast_kernel<false, false, true>);
+    return prior ? (wide ? gapblock_fast_kernel<true, true, false> : gapblock_fast_kernel<true, false, false>)
+                 : (wide ? gapblock_fast_kernel<false, true, false> : gapblock_fast_kernel<false, false, false>);
 }
 
-// Profile height LQ >= longest query: rows per pair in shared memory.
-int profile_height(int longest_query) {
-    for (int h : {16, 24, 32, 48})
-        if (longest_query <= h) return h;
-    return 64;
-}
-
-template <int LQ>
-const char* dispatch_prior(bool prior, const FastArgs& args, dim3 grid, size_t smem,
-                           cudaStream_t stream) {
-    return prior ? launch_fast<LQ, true>(args, grid, smem, stream)
-                 : launch_fast<LQ, false>(args, grid, smem, stream);
-}
-
-const char* dispatch_fast(int lq, bool prior, const FastArgs& args, dim3 grid, size_t smem,
-                          cudaStream_t stream) {
-    switch (lq) {
-        case 16: return dispatch_prior<16>(prior, args, grid, smem, stream);
-        case 24: return dispatch_prior<24>(prior, args, grid, smem, stream);
-        case 32: return dispatch_prior<32>(prior, args, grid, smem, stream);
-        case 48: return dispatch_prior<48>(prior, args, grid, smem, stream);
-        default: return dispatch_prior<64>(prior, args, grid, smem, stream);
-    }
-}
-
-// Words per prior row: value i at i + 3, rounded up so that every row is 16-byte aligned and
-// the last aligned group of four stays inside the row.
+// Words per prior row: the first value at 3, step j at 4 + j, rounded up so that every row is
+// 16-byte aligned and the last aligned group of four stays inside the row.
 int prior_stride(int W1) { return (W1 + 3 + 4 + 3) & ~3; }
 
 // Device-side tables of the fast path and the arguments they were built from.
@@ -771,7 +825,9 @@ GbTables& gb_tables(int device) {
 
 // Penalty grid; per-(M,d) prior rows shifted by their minimum (added back through ftab) and
 // clamped at CAP = 2*BIAS + 1 -- a clamped position can never win, because the position holding
-// the row's minimum scores at most BIAS while a clamped one scores above it;
+// the row's minimum scores at most BIAS while a clamped one scores above it; a row keeps its first
+// value and the steps between values (0 past the last position; A and B stay at most BIAS + CAP <
+// 2^15, and each packed sum of non-negative halves is exact whatever the step's sign);
 // ftab[m][n] = prior minimum + gap_open + (d-1)*gap_extend (int32 wrap, as the reference's
 // int32 arithmetic).
 void build_tables(GbTables& tb, const std::vector<int32_t>& pen, int32_t go, int32_t ge, int W,
@@ -793,8 +849,13 @@ void build_tables(GbTables& tb, const std::vector<int32_t>& pen, int32_t go, int
                 for (int i = 1; i <= L; ++i) pmin = std::min(pmin, row[i]);
                 if (m >= n) {  // fill each (M, d) row once
                     uint32_t* dst = prior2.data() + (size_t(M) * W1 + d) * pstride + 3;
-                    for (int i = 0; i <= L; ++i)
-                        dst[i] = uint32_t(std::min<int64_t>(int64_t(row[i]) - pmin, cap)) * 0x10001u;
+                    uint32_t last = 0;
+                    for (int i = 0; i <= L; ++i) {
+                        const uint32_t v =
+                            uint32_t(std::min<int64_t>(int64_t(row[i]) - pmin, cap)) * 0x10001u;
+                        dst[i] = v - last;
+                        last = v;
+                    }
                 }
             }
             ftab[size_t(m) * W1 + n] = int32_t(uint32_t(pmin) + uint32_t(go) +
@@ -807,43 +868,26 @@ void build_tables(GbTables& tb, const std::vector<int32_t>& pen, int32_t go, int
                                  prior2.size() * 4, stream);
 }
 
-// Shared memory of one CTA for a given chunk width.
-// CTAs per SM the fast kernel's registers allow (256 threads x <= 80 registers).
-constexpr int kTargetBlocks = 3;
+// CTAs per SM the fast kernel's registers allow (256 threads of 80 registers, 64 in the sparse form).
+constexpr int kTargetBlocks[2] = {3, 4};
 
-// The dense variant stands in for both forms when sizing (same registers and shared memory,
-// apart from the epilogue).
-const void* fast_kernel_ptr(int lq, bool prior) {
-#define STB_K(LQ)                                                                             \
-    if (lq == LQ)                                                                             \
-        return prior ? reinterpret_cast<const void*>(gapblock_fast_kernel<LQ, true, false>)   \
-                     : reinterpret_cast<const void*>(gapblock_fast_kernel<LQ, false, false>);
-    STB_K(16) STB_K(24) STB_K(32) STB_K(48)
-#undef STB_K
-    return prior ? reinterpret_cast<const void*>(gapblock_fast_kernel<64, true, false>)
-                 : reinterpret_cast<const void*>(gapblock_fast_kernel<64, false, false>);
-}
-
-// The profile area is reused for the per-slice column terms at write-out time.
-size_t fast_smem(int lq, int64_t slab_cap, int rc, int W1, int max_tasks) {
-    const size_t prof = std::max(size_t(kGP) * lq * kRow * 4, size_t(kGP / kPairsPerSlice) * rc * 4);
-    return prof + size_t(slab_cap) + size_t(kGP) * rc * 4 + size_t((W1 * W1 + 3) & ~3) * 4 +
-           size_t((rc + 15) & ~15) + size_t(max_tasks) * 16 + size_t((rc + 7) & ~7) * 2 +
-           size_t(kGP) * 4 + 16;
+int prof_bytes(int max_qlen, int spread, bool wide) {
+    return (max_qlen + spread) * kRow * 4 * kQuads * (wide ? 2 : 1);
 }
 
 }  // namespace
 
 namespace {
 
-// Chunk widths the fast kernel may use.  The widest that reaches the best CTA residency is the
-// static choice; the autotuner (dense calls) measures all of them once per shape.
-constexpr int kRcCandidates[] = {1536, 1280, 1024, 896, 768, 640, 512, 384, 256};
+// Chunk widths the fast kernel may use (multiples of 32).  The widest of 1,024 or less that
+// reaches the best CTA residency is the static choice; the autotuner measures all of them once per
+// shape.
+constexpr int kRcCandidates[] = {1280, 1024, 768, 640, 512, 384, 256};
 constexpr int kNumRc = int(sizeof(kRcCandidates) / sizeof(kRcCandidates[0]));
+static_assert(kRcCandidates[0] <= kMaxRounds * 32, "chunk_order_kernel's buckets");
 // Pairs a dense call's first-time tuning runs each variant on (its first query rows).
 constexpr int64_t kTuneSlicePairs = int64_t(100) * 1000 * 1000;
-thread_local int t_force_rc = 0;           // set while the autotuner times one chunk width
-thread_local int t_force_persistent = -1;  // and the launch form (-1: the tuned or static one)
+thread_local int t_force_rc = 0;  // set while the autotuner times one chunk width
 
 // The conditions under which gapblock_run takes the fast kernel (non-negative penalties, every
 // length <= 64, halves that cannot carry), the form whose sparse output is ordered.
@@ -864,7 +908,7 @@ bool fast_form_possible(const st_seqset_s& qs, const st_seqset_s& rs, const int3
 }
 
 std::string gb_shape_key(const st_seqset_s& qs, const st_seqset_s& rs, bool has_prior) {
-    return "gapblock|" + std::to_string(profile_height(qs.max_len)) + "|" +
+    return "gapblock|" + std::to_string(qs.max_len) + "|" +
            std::to_string(int(has_prior)) + "|" + std::to_string(std::max(qs.max_len, rs.max_len)) +
            "|" + std::to_string(size_bucket(qs.count)) + "|" + std::to_string(size_bucket(rs.count));
 }
@@ -910,57 +954,68 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
     bool fast = nonneg && longest <= 64 && lmaxpen <= 8191;
 
     const int W = longest, W1 = W + 1;
-    const int lq = profile_height(qs.max_len);
+    const bool wide = maxpen > 255;  // the penalties of four queries do not fit one word
+    const FastKernel kern = fast_kernel(has_prior, wide, sink != nullptr);
     const int tuned_choice =
         t_force_rc ? -1
                    : tuned_lookup(sink ? "sparse|" + gb_shape_key(qs, rs, has_prior)
                                        : gb_shape_key(qs, rs, has_prior));
     RefPlan* rpp = nullptr;
-    size_t smem = 0;
+    FastSmem sm{};
+    auto layout = [&](const RefPlan& rp) {
+        return fast_smem(prof_bytes(qs.max_len, rp.max_spread, wide), int(rp.max_slab), rp.rc, W1,
+                         rp.max_tasks, sink ? (sink->thresh > 255 ? 2 : 1) : 0);
+    };
     if (fast) {
         RefPlan& rp = plan_slot<RefPlan>(rs.gb_ref_plan, ctx.tmp_ref_plan, rs.owns);
-        const int want_rc = t_force_rc ? t_force_rc : (tuned_choice >= 0 ? kRcCandidates[tuned_choice % kNumRc] : 0);
+        const int want_rc = t_force_rc ? t_force_rc : (tuned_choice >= 0 ? kRcCandidates[tuned_choice] : 0);
         if (rp.uid != rs.uid || (want_rc && rp.rc != want_rc)) {
             Phase ph("ref_plan");
             // Chunk width: the autotuner's measured choice when there is one; otherwise the
             // widest (best warp fill) that still reaches the highest CTA residency the
             // kernel's registers allow, checked with the occupancy calculator.
-            const void* kern = fast_kernel_ptr(lq, has_prior);
             int best_rc = 0, best_blocks = -1;
-            const std::vector<int> widths =
-                want_rc ? std::vector<int>{want_rc} : std::vector<int>{1024, 896, 768, 640, 512, 384, 256};
+            std::vector<int> widths(kRcCandidates + 1, kRcCandidates + kNumRc);
+            if (want_rc) widths.insert(widths.begin(), want_rc);
             for (int rc : widths) {
-                build_ref_plan(rp, rs, rc, stream, /*upload=*/false);
-                const size_t sm = fast_smem(lq, (rp.max_slab + 15) & ~int64_t(15), rc, W1,
-                                            rp.max_tasks);
-                if (sm > size_t(ctx.max_smem_optin)) continue;
+                build_ref_plan(rp, rs, rc);
+                const int bytes = layout(rp).total;
+                if (bytes > ctx.max_smem_optin) continue;
+                if (rc == want_rc) {
+                    best_rc = rc;
+                    break;
+                }
                 int blocks = 0;
-                STB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              ctx.max_smem_optin));
-                STB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, kThreads, sm));
+                ensure_smem_limit(reinterpret_cast<const void*>(kern), size_t(bytes));
+                STB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, kThreads,
+                                                                       size_t(bytes)));
                 if (blocks > best_blocks) {
                     best_blocks = blocks;
                     best_rc = rc;
                 }
-                if (blocks >= kTargetBlocks) break;
+                if (blocks >= kTargetBlocks[sink != nullptr]) break;
             }
+            rp.uid = 0;  // stays so when no width fits shared memory: the general kernel runs
             if (best_rc) {
-                build_ref_plan(rp, rs, best_rc, stream);
-            } else {
-                rp.uid = 0;  // no width fits shared memory: the plan is not used (general kernel)
-                rp.ntasks = 0;
-            }
-            const unsigned blocks = unsigned(rp.ntasks);
-            if (blocks) {
-                ref_slab_kernel<<<blocks, 128, 0, stream>>>(
-                    rs.d_bytes, rs.d_off, static_cast<int32_t*>(rp.d_sorted.ptr),
-                    static_cast<int4*>(rp.d_tasks.ptr), static_cast<uint8_t*>(rp.d_slab.ptr));
+                if (rp.rc != best_rc) build_ref_plan(rp, rs, best_rc);
+                std::vector<int4> up(rp.chunks);
+                up.insert(up.end(), rp.tasks.begin(), rp.tasks.end());
+                int4* d_plan = rp.d_plan.as<int4>(up.size());
+                h2d(d_plan, up.data(), sizeof(int4) * up.size(), stream);
+                uint32_t* meta = rp.d_meta.as<uint32_t>(size_t(K));
+                chunk_order_kernel<<<unsigned(rp.nchunks), 256, 0, stream>>>(rs.d_len, K, rp.rc, rs.max_len,
+                                                                             meta);
                 STB_CUDA(cudaGetLastError());
-                note_launch(nullptr);
+                ref_slab_kernel<<<unsigned(rp.ntasks), 128, 0, stream>>>(
+                    rs.d_bytes, rs.d_off, meta, d_plan + rp.nchunks, rp.rc,
+                    rp.d_slab.as<uint8_t>(size_t(rp.slab_bytes) + 16));
+                STB_CUDA(cudaGetLastError());
+                note_launch(nullptr, 2);
+                rp.uid = rs.uid;
             }
         }
-        smem = fast_smem(lq, (rp.max_slab + 15) & ~int64_t(15), rp.rc, W1, rp.max_tasks);
-        fast = rp.uid == rs.uid && smem <= size_t(ctx.max_smem_optin);
+        sm = layout(rp);
+        fast = rp.uid == rs.uid && sm.total <= ctx.max_smem_optin;
         rpp = &rp;
     }
 
@@ -1024,17 +1079,19 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
     }
     {
         std::vector<uint8_t> key(sizeof(int) * 2 + pen.size() * 4);
-        const int hdr[2] = {A, lq};
+        const int hdr[2] = {A, int(wide)};
         std::memcpy(key.data(), hdr, sizeof hdr);
         std::memcpy(key.data() + sizeof hdr, pen.data(), pen.size() * 4);
         if (!same_as_last(qp.prof_key, key.data(), key.size())) {
             qp.prof_key.clear();  // set again once the profile kernel is enqueued
-            const int64_t total = qp.P * lq * kRow;
-            uint32_t* prof = qp.d_prof.as<uint32_t>(size_t(total));
-            profile_kernel<<<unsigned(ceil_div(total, 256)), 256, 0, stream>>>(
-                qs.d_bytes, qs.d_off, static_cast<int2*>(qp.d_pairs.ptr),
-                static_cast<int32_t*>(qp.d_plen.ptr), static_cast<int32_t*>(tb.pen.ptr), A, lq,
-                total, prof);
+            const size_t words = size_t(qp.prof_rows) * kQuads * kRow * (wide ? 2 : 1);
+            uint32_t* prof = qp.d_prof.as<uint32_t>(words);
+            const int4* quads = static_cast<const int4*>(qp.d_plan.ptr);
+            const int4* slices = quads + qp.quads.size();
+            auto fill = wide ? profile_kernel<true> : profile_kernel<false>;
+            fill<<<unsigned(qp.slices.size()), 256, 0, stream>>>(
+                qs.d_bytes, qs.d_off, quads, slices, static_cast<int32_t*>(tb.pen.ptr), A,
+                uint32_t(maxpen), prof);
             STB_CUDA(cudaGetLastError());
             note_launch(nullptr);
             qp.prof_key = key;
@@ -1050,19 +1107,19 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
     fa.rlen = rs.d_len;
     fa.K = K;
     fa.rc = rp.rc;
-    fa.pairs = static_cast<int2*>(qp.d_pairs.ptr);
-    fa.plen = static_cast<int32_t*>(qp.d_plen.ptr);
-    fa.P = qp.P;
-    fa.ref_sorted = static_cast<int32_t*>(rp.d_sorted.ptr);
-    fa.tasks = static_cast<int4*>(rp.d_tasks.ptr);
-    fa.task_off = static_cast<int32_t*>(rp.d_task_off.ptr);
-    fa.slab_cap = int((rp.max_slab + 15) & ~int64_t(15));
-    fa.max_tasks = rp.max_tasks;
+    fa.quads = static_cast<int4*>(qp.d_plan.ptr);
+    fa.slices = fa.quads + qp.quads.size();
+    fa.nslices = int64_t(qp.slices.size());
+    fa.ref_meta = static_cast<uint32_t*>(rp.d_meta.ptr);
+    fa.chunks = static_cast<int4*>(rp.d_plan.ptr);
+    fa.tasks = fa.chunks + rp.nchunks;
+    fa.sm = sm;
+    fa.score16 = sink && sink->thresh > 255;
+    fa.spread = rp.max_spread;
     fa.prior2 = has_prior ? static_cast<uint32_t*>(tb.prior2.ptr) : nullptr;
     fa.ftab = static_cast<int32_t*>(tb.ftab.ptr);
     fa.W1 = W1;
     fa.pstride = prior_stride(W1);
-    fa.bias2 = uint32_t(bias) * 0x10001u;
     fa.out = out_d;
     fa.err = err;
     if (sink && sink->ordered) {
@@ -1074,30 +1131,17 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
     }
     if (sink) fa.sink = *sink;
 
-    const int64_t npg = ceil_div(qp.P, kGP);
-    const int64_t ntiles = int64_t(rp.nchunks) * npg;
-    const int tuned_mode = t_force_persistent >= 0 ? t_force_persistent
-                           : (tuned_choice >= 0 ? tuned_choice / kNumRc : 0);
-    dim3 grid(unsigned(rp.nchunks), unsigned(npg));
-    if (tuned_mode == 1 && ntiles < (int64_t(1) << 31)) {
-        const void* kern = fast_kernel_ptr(lq, has_prior);
-        int per_sm = 0;
-        STB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        STB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem));
-        fa.persistent = 1;
-        fa.nchunks = rp.nchunks;
-        fa.ntiles = int(ntiles);
-        fa.queue = reinterpret_cast<unsigned int*>(ctx.flags_d + 13);
-        STB_CUDA(cudaMemsetAsync(fa.queue, 0, sizeof(unsigned int), stream));
-        grid = dim3(unsigned(std::min<int64_t>(ntiles, int64_t(std::max(per_sm, 1)) * ctx.num_sms)), 1);
-    } else if (npg > 65535) {
-        // pair groups split over y and z (the kernel skips the padding of the last z slice)
+    dim3 grid(unsigned(rp.nchunks), unsigned(fa.nslices));
+    if (fa.nslices > 65535) {
+        // slices split over y and z (the kernel skips the padding of the last z layer)
         grid.y = 65535;
-        grid.z = unsigned(ceil_div(npg, 65535));
-        if (grid.z > 65535) fail(ST_EINVAL, "seqtree_b200: too many query pairs for one launch");
+        grid.z = unsigned(ceil_div(fa.nslices, 65535));
+        if (grid.z > 65535) fail(ST_EINVAL, "seqtree_b200: too many queries for one launch");
     }
-    const char* name = dispatch_fast(lq, has_prior, fa, grid, smem, stream);
-    note_launch(name);
+    ensure_smem_limit(reinterpret_cast<const void*>(kern), size_t(sm.total));
+    kern<<<grid, kThreads, size_t(sm.total), stream>>>(fa);
+    STB_CUDA(cudaGetLastError());
+    note_launch(sink ? "gapblock_fast_kernel<sparse>" : "gapblock_fast_kernel");
     // The timeout flag is read by the caller after its synchronisation point.
 }
 
@@ -1123,10 +1167,9 @@ void gapblock_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int
     }
     const bool has_prior = prior && prior_len > 0;
     const std::string key = gb_shape_key(qs, rs, has_prior);
-    // Candidates: every chunk width, each with one CTA per tile and in the persistent form.
+    // Candidates: every chunk width.
     auto variant = [&](int c, int64_t rows) {
-        t_force_rc = c >= 0 ? kRcCandidates[c % kNumRc] : 0;  // -1: the static choice
-        t_force_persistent = c >= 0 ? c / kNumRc : -1;
+        t_force_rc = c >= 0 ? kRcCandidates[c] : 0;  // -1: the static choice
         try {
             if (rows < 0)
                 run();
@@ -1135,24 +1178,22 @@ void gapblock_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int
                              out_d, nullptr, stream, 0, rows);
         } catch (...) {
             t_force_rc = 0;
-            t_force_persistent = -1;
             throw;
         }
         t_force_rc = 0;
-        t_force_persistent = -1;
     };
     // A shape seen for the first time is tuned on its first query rows only (about
     // kTuneSlicePairs pairs, written into their own rows of the result), so the first call costs
     // the variants' runs on that slice rather than on the whole matrix; the chosen variant then
     // computes the whole matrix.
     const int64_t slice = std::min<int64_t>(
-        qs.count, std::max<int64_t>(4 * kGP * 2, kTuneSlicePairs / std::max<int64_t>(rs.count, 1)));
+        qs.count, std::max<int64_t>(2 * kSliceQ, kTuneSlicePairs / std::max<int64_t>(rs.count, 1)));
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     STB_CUDA(cudaStreamIsCapturing(stream, &cs));
     if (slice < qs.count && tuning_enabled() && cs == cudaStreamCaptureStatusNone &&
         tuned_lookup(key) < 0)
-        tuned_run(key, 2 * kNumRc, -1, [&](int c) { variant(c, slice); }, stream);
-    tuned_run(key, 2 * kNumRc, -1, [&](int c) { variant(c, -1); }, stream);
+        tuned_run(key, kNumRc, -1, [&](int c) { variant(c, slice); }, stream);
+    tuned_run(key, kNumRc, -1, [&](int c) { variant(c, -1); }, stream);
 }
 
 // Scores of listed pairs (device index arrays) into out_d; the general int32 kernel's
@@ -1401,20 +1442,17 @@ void gapblock_sparse_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penal
                 ts.keys = ctx.sp_keys.as<unsigned long long>(size_t(tcap));
                 ts.vals = ctx.sp_vals.as<int32_t>(size_t(tcap));
             }
-            tuned_run(skey, 2 * kNumRc, -1, [&](int c) {
-                t_force_rc = c >= 0 ? kRcCandidates[c % kNumRc] : 0;
-                t_force_persistent = c >= 0 ? c / kNumRc : -1;
+            tuned_run(skey, kNumRc, -1, [&](int c) {
+                t_force_rc = c >= 0 ? kRcCandidates[c] : 0;
                 try {
                     STB_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned long long), stream));
                     gapblock_run(qs, rs, penalty, matrix_size, go, ge, prior, prior_len,
                                  prior_width, nullptr, &ts, stream, 0, tr1 == N ? -1 : tr1);
                 } catch (...) {
                     t_force_rc = 0;
-                    t_force_persistent = -1;
                     throw;
                 }
                 t_force_rc = 0;
-                t_force_persistent = -1;
             }, stream);
         }
     }
