@@ -66,6 +66,15 @@ struct DevBuf {
     ~DevBuf();
 };
 
+// A DevBuf that frees its memory with its owner: the buffers of a set's plans (the set's destructor
+// frees device memory, which waits for the kernels that still read it).
+struct OwnedBuf : DevBuf {
+    OwnedBuf() = default;
+    OwnedBuf(const OwnedBuf&) = delete;
+    OwnedBuf& operator=(const OwnedBuf&) = delete;
+    ~OwnedBuf() { release(); }
+};
+
 struct Context {
     int device = 0;
     std::mutex mu;              // serialises calls on this device
@@ -74,7 +83,7 @@ struct Context {
     int max_smem_optin = 0;
     // Small device word area for error reporting, with a pinned host mirror.  Word 0: first
     // invalid symbol of an encode; word 8: a bounded wait gave up; word 9: an int32 overflow;
-    // words 16-19: byte-presence bitmap.  Words 8-15 are cleared before and read after each
+    // words 16-23: byte-presence bitmaps of two sets.  Words 8-15 are cleared before and read after each
     // host call.
     int64_t* flags_d = nullptr;
     int64_t* flags_h = nullptr;
@@ -94,7 +103,7 @@ struct Context {
     DevBuf tq[3], tr[3];  // bytes, offsets, lengths
     // plans reused by transient sets (rebuilt in place for every call)
     std::shared_ptr<void> tmp_query_plan, tmp_ref_plan, tmp_wave_plan[2];
-    std::shared_ptr<void> tmp_strip_query_plan, tmp_strip_ref_plan;
+    std::shared_ptr<void> tmp_strip_query_plan, tmp_strip_ref_plan, tmp_dist_plan[2];
     // query plan of a row block (sparse calls whose hits are taken in several blocks)
     std::shared_ptr<void> tmp_block_plan;
     // sparse result of the host-buffer sparse call (an st_hits_s)
@@ -159,12 +168,15 @@ struct st_seqset_s {
     std::vector<int64_t> h_off; // count + 1
     std::vector<int32_t> h_len; // count
     uint8_t* d_bytes = nullptr; // encoded codes (alphabet >= 0) or raw bytes, +64 B padding
+    uint8_t* d_codes = nullptr;   // raw sets: room for total + 64 dense codes,
+    uint32_t* d_packed = nullptr; // and for total + 4 * count bytes of packed words (in d_bytes' block)
     int64_t* d_off = nullptr;
     int32_t* d_len = nullptr;
     bool owns = true;           // false: storage borrowed from the context (transient set)
     uint64_t uid = 0;           // unique per set; plans record the uid they were built for
     // plan caches (opaque; transient sets share the context's)
     std::shared_ptr<void> gb_query_plan, gb_ref_plan, wave_plan, strip_query_plan, strip_ref_plan;
+    std::shared_ptr<void> dist_plan;
     ~st_seqset_s();
 };
 

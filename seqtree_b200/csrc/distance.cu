@@ -10,12 +10,12 @@
 //   warp writes 512 contiguous bytes of a row per query.
 //
 //   Levenshtein (integer-ALU bound): Myers' bit-vector algorithm in Hyyro's formulation for
-//   whole-string edit distance.  The ref is the bit pattern (one 64-bit word per lane, n <= 64)
-//   and the query is the text, warp-uniform, so the per-character loop never diverges; the
-//   pattern-match masks Peq[c] of the 32 lanes live in shared memory as [c][lane].  Lanes own
-//   32 consecutive refs, so stores stay coalesced in the original column order.  Longer refs,
-//   or more than 64 distinct symbols, take a one-thread-per-pair DP with its row in global
-//   scratch (any length).
+//   whole-string edit distance.  The ref is the bit pattern (one integer of 1 to 16 32-bit words per
+//   lane, as many as the longest ref needs) and the query is the text, warp-uniform, so the
+//   per-character loop never diverges; the pattern-match masks Peq[c] of the 32 lanes live in
+//   shared memory as [c][word][lane].  Lanes own 32 consecutive refs, so stores stay coalesced in
+//   the original column order.  Longer refs, or more than 64 distinct symbols, take a
+//   one-thread-per-pair DP with its row in global scratch (any length).
 #include <algorithm>
 #include <map>
 
@@ -30,97 +30,150 @@ struct ByteLut {
     uint8_t v[256];
 };
 
-__global__ void remap_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, int64_t n,
-                             ByteLut lut) {
+// Up to two sets' buffers in one launch, a set per blockIdx.y.
+struct TwoSets {
+    const uint8_t* in[2];
+    uint8_t* out[2];
+    int64_t bytes[2];
+};
+
+// Dense codes of each set's bytes, and 64 zero bytes past them.
+__global__ void remap_kernel(const TwoSets t, ByteLut lut) {
     __shared__ uint8_t s[256];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) s[i] = lut.v[i];
     __syncthreads();
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+    const uint8_t* in = t.in[blockIdx.y];
+    uint8_t* out = t.out[blockIdx.y];
+    const int64_t n = t.bytes[blockIdx.y];
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n + 64;
          i += int64_t(gridDim.x) * blockDim.x)
-        out[i] = s[in[i]];
+        out[i] = i < n ? s[in[i]] : 0;
 }
 
-// Byte-presence bitmap of a set, computed on the device (distinct bytes -> dense codes).
-__global__ void presence_kernel(const uint8_t* __restrict__ bytes, int64_t n,
-                                unsigned int* __restrict__ present) {
+// Byte-presence bitmap of each set (distinct bytes -> dense codes).
+__global__ void presence_kernel(const TwoSets t, unsigned int* __restrict__ present) {
     __shared__ unsigned int s[8];
     if (threadIdx.x < 8) s[threadIdx.x] = 0;
     __syncthreads();
+    const uint8_t* bytes = t.in[blockIdx.y];
+    const int64_t n = t.bytes[blockIdx.y];
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
          i += int64_t(gridDim.x) * blockDim.x) {
         const uint8_t c = bytes[i];
         atomicOr(&s[c >> 5], 1u << (c & 31));
     }
     __syncthreads();
-    if (threadIdx.x < 8 && s[threadIdx.x]) atomicOr(&present[threadIdx.x], s[threadIdx.x]);
+    if (threadIdx.x < 8 && s[threadIdx.x]) atomicOr(&present[blockIdx.y * 8 + threadIdx.x], s[threadIdx.x]);
 }
 
-// Dense codes of a (set, set) pair, cached by the sets' uids so that repeated calls on
-// device-resident sets enqueue no host round trip (and can be captured in a CUDA graph).
-struct DistCache {
-    uint64_t a_uid = 0, b_uid = 0;
-    int sigma = 0;
-    DevBuf ac, bc;             // codes of a and b
-    int packB = 0, packW = 0;  // Hamming packing built for (bits, words); 0 = none
-    DevBuf qp, rp;             // packed words
+// What a set keeps for the distances: the bytes it holds, and whether its dense codes (and Hamming
+// packing) are there, under which alphabet.  The alphabet of a call is the union of both sets'
+// bytes, so sets over the same symbols keep their codes from call to call whatever they are
+// paired with, and such calls enqueue no host round trip (and can be captured in a CUDA graph).
+struct DistPlan {
+    uint64_t uid = 0;               // set the plan was built for
+    uint32_t present[8] = {};       // bytes of the set
+    uint32_t symbols[8] = {};       // bytes the codes were built for
+    bool coded = false;
+    int packB = 0, packW = 0;       // Hamming packing built for (bits, words); 0 = none
 };
 
-DistCache& dist_cache(int device) {
-    static std::mutex mu;
-    static std::map<int, std::unique_ptr<DistCache>> all;
-    std::lock_guard<std::mutex> lk(mu);
-    auto& p = all[device];
-    if (!p) p = std::make_unique<DistCache>();
-    return *p;
+struct DistCodes {
+    DistPlan *a, *b;
+    int sigma;
+    bool fresh;  // codes were enqueued on the call's stream just now
+};
+
+// A set's codes may next be read from another stream: waits for them once they are made.
+void settle(const st_seqset_s& a, const st_seqset_s& b, cudaStream_t stream) {
+    if (a.owns || b.owns) STB_CUDA(cudaStreamSynchronize(stream));
 }
 
-DistCache& compute_codes(st_seqset_s& a, st_seqset_s& b, cudaStream_t stream, Context& ctx) {
-    DistCache& dc = dist_cache(ctx.device);
-    if (dc.a_uid == a.uid && dc.b_uid == b.uid && a.uid != 0) return dc;
+DistPlan& dist_plan(st_seqset_s& s, Context& ctx, int slot) {
+    std::shared_ptr<void>& holder = s.owns ? s.dist_plan : ctx.tmp_dist_plan[slot];
+    if (!holder) holder = std::make_shared<DistPlan>();
+    return *static_cast<DistPlan*>(holder.get());
+}
+
+DistCodes compute_codes(st_seqset_s& a, st_seqset_s& b, cudaStream_t stream, Context& ctx) {
+    st_seqset_s* sets[2] = {&a, &b};
+    DistPlan* plans[2] = {&dist_plan(a, ctx, 0), &dist_plan(b, ctx, 1)};
+    auto blocks_of = [&ctx](const TwoSets& t) {
+        const int64_t most = std::max<int64_t>({t.bytes[0], t.bytes[1], 1});
+        return dim3(unsigned(std::min<int64_t>(ceil_div(most, 256), ctx.num_sms * 4)), 2);
+    };
     auto* present = reinterpret_cast<unsigned int*>(ctx.flags_d + 16);
-    STB_CUDA(cudaMemsetAsync(present, 0, 32, stream));
-    for (st_seqset_s* s : {&a, &b}) {
-        if (s->total == 0) continue;
-        const unsigned grid = unsigned(std::min<int64_t>(ceil_div(s->total, 256), ctx.num_sms * 4));
-        presence_kernel<<<grid, 256, 0, stream>>>(s->d_bytes, s->total, present);
+    const auto* bits = reinterpret_cast<const unsigned int*>(ctx.flags_h + 16);
+    if (plans[0]->uid != a.uid || plans[1]->uid != b.uid) {
+        STB_CUDA(cudaMemsetAsync(present, 0, 64, stream));
+        TwoSets args{};
+        for (int t = 0; t < 2; ++t) {
+            args.in[t] = sets[t]->d_bytes;
+            args.bytes[t] = plans[t]->uid == sets[t]->uid ? 0 : sets[t]->total;
+        }
+        presence_kernel<<<blocks_of(args), 256, 0, stream>>>(args, present);
         STB_CUDA(cudaGetLastError());
         note_launch(nullptr);
+        STB_CUDA(cudaMemcpyAsync(ctx.flags_h + 16, present, 64, cudaMemcpyDeviceToHost, stream));
+        STB_CUDA(cudaStreamSynchronize(stream));
+        for (int t = 0; t < 2; ++t) {
+            if (plans[t]->uid == sets[t]->uid) continue;
+            std::memcpy(plans[t]->present, bits + 8 * t, 32);
+            plans[t]->coded = false;
+            plans[t]->uid = sets[t]->uid;
+        }
     }
-    STB_CUDA(cudaMemcpyAsync(ctx.flags_h + 16, present, 32, cudaMemcpyDeviceToHost, stream));
-    STB_CUDA(cudaStreamSynchronize(stream));
-    const auto* bits = reinterpret_cast<const unsigned int*>(ctx.flags_h + 16);
+    uint32_t symbols[8];
+    for (int w = 0; w < 8; ++w) symbols[w] = plans[0]->present[w] | plans[1]->present[w];
     ByteLut lut;
     std::memset(lut.v, 0, sizeof lut.v);
     int sigma = 0;
     for (int c = 0; c < 256; ++c)
-        if (bits[c >> 5] & (1u << (c & 31))) lut.v[c] = uint8_t(sigma++);
-    DevBuf* bufs[2] = {&dc.ac, &dc.bc};
-    st_seqset_s* sets[2] = {&a, &b};
+        if (symbols[c >> 5] & (1u << (c & 31))) lut.v[c] = uint8_t(sigma++);
+    TwoSets args{};
+    int todo = 0;
     for (int t = 0; t < 2; ++t) {
         st_seqset_s* s = sets[t];
-        uint8_t* dst = bufs[t]->as<uint8_t>(size_t(s->total) + 64);
-        STB_CUDA(cudaMemsetAsync(dst + s->total, 0, 64, stream));
-        if (s->total > 0) {
-            const unsigned grid = unsigned(std::min<int64_t>(ceil_div(s->total, 256), ctx.num_sms * 4));
-            remap_kernel<<<grid, 256, 0, stream>>>(s->d_bytes, dst, s->total, lut);
-            STB_CUDA(cudaGetLastError());
-            note_launch(nullptr);
+        DistPlan& p = *plans[t];
+        if (p.coded && std::memcmp(p.symbols, symbols, 32) == 0) continue;
+        // kernels on other streams may still read the codes of the last alphabet
+        if (p.coded && s->owns) STB_CUDA(cudaDeviceSynchronize());
+        p.coded = false;
+        p.packB = p.packW = 0;
+        args.in[todo] = s->d_bytes;
+        args.out[todo] = s->d_codes;
+        args.bytes[todo++] = s->total;
+        if (sets[0] == sets[1]) break;
+    }
+    if (todo) {
+        dim3 grid = blocks_of(args);
+        grid.y = unsigned(todo);
+        remap_kernel<<<grid, 256, 0, stream>>>(args, lut);
+        STB_CUDA(cudaGetLastError());
+        note_launch(nullptr);
+        for (DistPlan* p : plans) {
+            std::memcpy(p->symbols, symbols, 32);
+            p->coded = true;
         }
     }
-    dc.sigma = sigma;
-    dc.a_uid = a.uid;
-    dc.b_uid = b.uid;
-    dc.packB = dc.packW = 0;
-    return dc;
+    const bool fresh = todo > 0;
+    return DistCodes{plans[0], plans[1], sigma, fresh};
 }
 
 // ---------------------------------------------------------------------------- Hamming -------
-// Pack each string's codes at B bits per symbol into W words (low symbol in low bits).
-__global__ void pack_kernel(const uint8_t* __restrict__ codes, const int64_t* __restrict__ off,
-                            int64_t count, int L, int B, int W, uint32_t* __restrict__ packed) {
+// Pack each string's codes at B bits per symbol into W words (low symbol in low bits); up to two
+// sets in one launch, a set per blockIdx.y.
+struct PackArgs {
+    const uint8_t* codes[2];
+    const int64_t* off[2];
+    int64_t count[2];
+    uint32_t* packed[2];
+};
+
+__global__ void pack_kernel(const PackArgs a, int L, int B, int W) {
     const int64_t s = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (s >= count) return;
-    const uint8_t* c = codes + off[s];
+    if (s >= a.count[blockIdx.y]) return;
+    const uint8_t* c = a.codes[blockIdx.y] + a.off[blockIdx.y][s];
     const int per = 32 / B;
     for (int w = 0; w < W; ++w) {
         uint32_t v = 0;
@@ -128,7 +181,7 @@ __global__ void pack_kernel(const uint8_t* __restrict__ codes, const int64_t* __
             const int j = w * per + t;
             if (j < L) v |= uint32_t(c[j]) << (t * B);
         }
-        packed[s * W + w] = v;
+        a.packed[blockIdx.y][s * W + w] = v;
     }
 }
 
@@ -225,34 +278,77 @@ const char* launch_hamming(const uint32_t* qp, const uint32_t* rp, int64_t N, in
 
 // ---------------------------------------------------------------------------- Levenshtein ---
 constexpr int kLevWarps = 8;
-constexpr int kLevRows = 16;  // query rows per CTA
 
-// Pattern = ref (lane), text = query (warp-uniform).  Peq in shared memory as [c][word][lane].
-// W = 64-bit words per pattern: one word takes refs up to 64 symbols; longer refs (W = 2, 4, 8)
-// run the blocked form, where each word passes its bottom horizontal step (-1, 0 or +1) to the
-// next word as the carry into its first row (Myers 1999, "advance_block"): a -1 carry sets the
-// match bit of row 0 for the add and shifts a 1 into Mh, a +1 carry shifts a 1 into Ph.  Rows
-// past a lane's own ref length act as unmatched rows below the pattern and never reach rows above
-// them, so every lane runs all W words and masks its own length at the end.
-template <int W>
+// s = a + b + carry over N = 2 or 4 words as one carry chain; `carry` (0 or 1) becomes the carry out.
+template <int N>
+__device__ __forceinline__ void add_words(uint32_t* s, const uint32_t* a, const uint32_t* b, uint32_t& carry) {
+    static_assert(N == 2 || N == 4, "chains of two or four words");
+    if constexpr (N == 2)
+        asm("{ .reg .u32 x; add.cc.u32 x, %2, 0xffffffff; addc.cc.u32 %0, %3, %5; addc.cc.u32 %1, %4, %6;"
+            " addc.u32 %2, 0, 0; }"
+            : "=&r"(s[0]), "=&r"(s[1]), "+r"(carry)
+            : "r"(a[0]), "r"(a[1]), "r"(b[0]), "r"(b[1]));
+    else
+        asm("{ .reg .u32 x; add.cc.u32 x, %4, 0xffffffff; addc.cc.u32 %0, %5, %9; addc.cc.u32 %1, %6, %10;"
+            " addc.cc.u32 %2, %7, %11; addc.cc.u32 %3, %8, %12; addc.u32 %4, 0, 0; }"
+            : "=&r"(s[0]), "=&r"(s[1]), "=&r"(s[2]), "=&r"(s[3]), "+r"(carry)
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]));
+}
+
+// s = a + b over NW words (the carry out of the last word is dropped).
+template <int NW>
+__device__ __forceinline__ void add_all(uint32_t* s, const uint32_t* a, const uint32_t* b) {
+    if constexpr (NW == 1) {
+        s[0] = a[0] + b[0];
+    } else if constexpr (NW == 2) {
+        asm("add.cc.u32 %0, %2, %4; addc.u32 %1, %3, %5;"
+            : "=&r"(s[0]), "=r"(s[1])
+            : "r"(a[0]), "r"(a[1]), "r"(b[0]), "r"(b[1]));
+    } else if constexpr (NW == 3) {
+        asm("add.cc.u32 %0, %3, %6; addc.cc.u32 %1, %4, %7; addc.u32 %2, %5, %8;"
+            : "=&r"(s[0]), "=&r"(s[1]), "=r"(s[2])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(b[0]), "r"(b[1]), "r"(b[2]));
+    } else if constexpr (NW == 4) {
+        asm("add.cc.u32 %0, %4, %8; addc.cc.u32 %1, %5, %9; addc.cc.u32 %2, %6, %10; addc.u32 %3, %7, %11;"
+            : "=&r"(s[0]), "=&r"(s[1]), "=&r"(s[2]), "=r"(s[3])
+            : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]));
+    } else {  // chains of four words (and two), each handing its carry on through a register
+        static_assert(NW % 2 == 0, "whole chains");
+        uint32_t carry = 0;
+#pragma unroll
+        for (int w = 0; w + 4 <= NW; w += 4) add_words<4>(s + w, a + w, b + w, carry);
+        if constexpr (NW % 4 == 2) add_words<2>(s + NW - 2, a + NW - 2, b + NW - 2, carry);
+    }
+}
+
+// Pattern = ref (lane), text = query (warp-uniform).  Peq in shared memory as [c][word][lane].  The
+// pattern is one integer of NW 32-bit words: the add and the two shifts run across the words, the
+// rest word by word -- ten ALU operations a word and text character, whatever NW (a blocked form
+// that hands each word's bottom step to the next costs eight more per 64 bits).  Rows past a lane's
+// own ref length act as unmatched rows below the pattern and never reach rows above them, so every
+// lane runs all NW words and masks its own length at the end.
+// The bound is the ALU pipe.  Measured, B200: 20,000 x 20,000 ACGT 30-60 (NW 2) 21.5 -> 20.7
+// ms (64-bit words, 16 rows per CTA -> this; ALU 88 %); 5,003 x 10,007 amino acids 8-25 (NW 1) 1.13 ->
+// 0.60 ms (ALU 80 %, issue 79 %).
+template <int NW>
 __global__ void __launch_bounds__(kLevWarps * 32)
 levenshtein_kernel(const uint8_t* __restrict__ qc, const int64_t* __restrict__ qoff,
                    const uint8_t* __restrict__ rc, const int64_t* __restrict__ roff, int64_t N,
-                   int64_t K, int sigma, int32_t* __restrict__ out) {
-    extern __shared__ unsigned long long s_peq[];  // [warp][sigma][W][32]
+                   int64_t K, int sigma, int rows, int32_t* __restrict__ out) {
+    extern __shared__ uint32_t s_peq[];  // [warp][sigma][NW][32]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned long long* peq = s_peq + size_t(warp) * sigma * W * 32;
+    uint32_t* peq = s_peq + size_t(warp) * sigma * NW * 32;
     const int64_t k = (int64_t(blockIdx.x) * kLevWarps + warp) * 32 + lane;
     const bool valid = k < K;
     const int64_t kk = valid ? k : (K - 1);
     const uint8_t* r = rc + roff[kk];
     const int n = int(roff[kk + 1] - roff[kk]);
-    for (int c = 0; c < sigma * W; ++c) peq[c * 32 + lane] = 0ull;
-    for (int j = 0; j < n; ++j) peq[(r[j] * W + (j >> 6)) * 32 + lane] |= 1ull << (j & 63);
+    for (int c = 0; c < sigma * NW; ++c) peq[c * 32 + lane] = 0u;
+    for (int j = 0; j < n; ++j) peq[(r[j] * NW + (j >> 5)) * 32 + lane] |= 1u << (j & 31);
     __syncwarp();
-    const unsigned long long ones = n >= 64 ? ~0ull : ((1ull << n) - 1ull);
-    const int64_t r0 = int64_t(blockIdx.y) * kLevRows;
-    const int64_t r1 = (N < r0 + kLevRows ? N : r0 + kLevRows);
+    const uint32_t* mine = peq + lane;
+    const int64_t r0 = int64_t(blockIdx.y) * rows;
+    const int64_t r1 = (N < r0 + rows ? N : r0 + rows);
     for (int64_t i = r0; i < r1; ++i) {
         const uint8_t* q = qc + qoff[i];
         const int m = int(qoff[i + 1] - qoff[i]);
@@ -260,57 +356,76 @@ levenshtein_kernel(const uint8_t* __restrict__ qc, const int64_t* __restrict__ q
         // read once from the last column, D[n][m] = D[0][m] + sum of its steps
         // = m + popc(Pv) - popc(Mv) over the n pattern bits, instead of following the bottom
         // cell through every column (which costs about a fifth of the loop's instructions).
-        if constexpr (W > 1) {
-            unsigned long long Pv[W], Mv[W];
+        uint32_t Pv[NW], Mv[NW];
 #pragma unroll
-            for (int w = 0; w < W; ++w) {
-                Pv[w] = ~0ull;
-                Mv[w] = 0ull;
-            }
-            for (int t = 0; t < m; ++t) {
-                const unsigned long long* e = peq + q[t] * W * 32 + lane;
-                int h = 1;  // row 0 of the global distance: +1 per text character
-#pragma unroll
-                for (int w = 0; w < W; ++w) {
-                    unsigned long long Eq = e[w * 32];
-                    const unsigned long long Xv = Eq | Mv[w];
-                    Eq |= h < 0 ? 1ull : 0ull;
-                    const unsigned long long Xh = (((Eq & Pv[w]) + Pv[w]) ^ Pv[w]) | Eq;
-                    unsigned long long Ph = Mv[w] | ~(Xh | Pv[w]);
-                    unsigned long long Mh = Pv[w] & Xh;
-                    const int hout = int(Ph >> 63) - int(Mh >> 63);
-                    Ph = (Ph << 1) | (h > 0 ? 1ull : 0ull);
-                    Mh = (Mh << 1) | (h < 0 ? 1ull : 0ull);
-                    Pv[w] = Mh | ~(Xv | Ph);
-                    Mv[w] = Ph & Xv;
-                    h = hout;
-                }
-            }
-            int score = m;
-#pragma unroll
-            for (int w = 0; w < W; ++w) {
-                const int bits = min(64, max(0, n - 64 * w));
-                const unsigned long long mask = bits >= 64 ? ~0ull : ((1ull << bits) - 1ull);
-                score += __popcll(Pv[w] & mask) - __popcll(Mv[w] & mask);
-            }
-            if (valid) out[i * K + k] = score;
-            continue;
+        for (int w = 0; w < NW; ++w) {
+            Pv[w] = ~0u;
+            Mv[w] = 0u;
         }
-        unsigned long long Pv = ones, Mv = 0ull;
-        for (int t = 0; t < m; ++t) {
-            const unsigned long long Eq = peq[q[t] * 32 + lane];
-            const unsigned long long Xv = Eq | Mv;
-            const unsigned long long Xh = (((Eq & Pv) + Pv) ^ Pv) | Eq;
-            unsigned long long Ph = Mv | ~(Xh | Pv);
-            unsigned long long Mh = Pv & Xh;
-            Ph = (Ph << 1) | 1ull;
-            Mh <<= 1;
-            Pv = Mh | ~(Xv | Ph);
-            Mv = Ph & Xv;
+        auto step = [&](int c) {
+            const uint32_t* e = mine + c * (NW * 32);
+            uint32_t Eq[NW], t[NW], Ph[NW], Mh[NW];
+#pragma unroll
+            for (int w = 0; w < NW; ++w) {
+                Eq[w] = e[w * 32];
+                t[w] = Eq[w] & Pv[w];
+            }
+            add_all<NW>(t, t, Pv);
+#pragma unroll
+            for (int w = 0; w < NW; ++w) {
+                const uint32_t Xh = (t[w] ^ Pv[w]) | Eq[w];
+                Ph[w] = Mv[w] | ~(Xh | Pv[w]);
+                Mh[w] = Pv[w] & Xh;
+            }
+#pragma unroll
+            for (int w = NW - 1; w >= 0; --w) {  // row 0 of the global distance: +1 per character
+                const uint32_t Xv = Eq[w] | Mv[w];
+                const uint32_t ph = w ? __funnelshift_l(Ph[w ? w - 1 : 0], Ph[w], 1) : Ph[0] * 2u + 1u;
+                const uint32_t mh = w ? __funnelshift_l(Mh[w ? w - 1 : 0], Mh[w], 1) : Mh[0] * 2u;
+                Pv[w] = mh | ~(Xv | ph);
+                Mv[w] = ph & Xv;
+            }
+        };
+        int t = 0;
+        for (; t + 4 <= m; t += 4) {
+            int c[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) c[u] = q[t + u];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) step(c[u]);
         }
-        const int score = m + __popcll(Pv & ones) - __popcll(Mv & ones);
+        for (; t < m; ++t) step(q[t]);
+        int score = m;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            const int bits = min(32, max(0, n - 32 * w));
+            const uint32_t mask = bits >= 32 ? ~0u : (1u << bits) - 1u;
+            score += __popc(Pv[w] & mask) - __popc(Mv[w] & mask);
+        }
         if (valid) out[i * K + k] = score;
     }
+}
+
+using LevKernel = void (*)(const uint8_t*, const int64_t*, const uint8_t*, const int64_t*, int64_t, int64_t, int,
+                           int, int32_t*);
+
+// The kernel for refs of up to `longest` symbols and its words per pattern; null past 512 symbols.
+LevKernel lev_kernel(int longest, int& words) {
+    struct Form {
+        int words;
+        LevKernel kernel;
+    };
+    static const Form forms[] = {{1, levenshtein_kernel<1>},   {2, levenshtein_kernel<2>},
+                                 {3, levenshtein_kernel<3>},   {4, levenshtein_kernel<4>},
+                                 {6, levenshtein_kernel<6>},   {8, levenshtein_kernel<8>},
+                                 {12, levenshtein_kernel<12>}, {16, levenshtein_kernel<16>}};
+    for (const Form& f : forms)
+        if (longest <= 32 * f.words) {
+            words = f.words;
+            return f.kernel;
+        }
+    words = 0;
+    return nullptr;
 }
 
 // Any lengths / alphabets: classic single-row DP per (i, k), row kept in global scratch laid
@@ -380,24 +495,38 @@ void hamming_sets(st_seqset_s& a, st_seqset_s& b, int32_t* out_d, cudaStream_t s
                             std::to_string(a.h_len[size_t(bi)]) + " and " +
                             std::to_string(b.h_len[size_t(bk)]) + ")");
     Context& ctx = context();
-    DistCache& dc = compute_codes(a, b, stream, ctx);
+    const DistCodes dc = compute_codes(a, b, stream, ctx);
     const int sigma = dc.sigma;
     const int B = sigma <= 2 ? 1 : sigma <= 4 ? 2 : sigma <= 16 ? 4 : 8;
     const int per = 32 / B;
     const int W = std::max(1, int(ceil_div(L, per)));
-    uint32_t* qp = dc.qp.as<uint32_t>(size_t(N) * W);
-    uint32_t* rp = dc.rp.as<uint32_t>(size_t(K) * W);
-    if (dc.packB != B || dc.packW != W) {
-        const uint8_t* ac = static_cast<uint8_t*>(dc.ac.ptr);
-        const uint8_t* bc = static_cast<uint8_t*>(dc.bc.ptr);
-        pack_kernel<<<unsigned(ceil_div(N, 256)), 256, 0, stream>>>(ac, a.d_off, N, L, B, W, qp);
-        STB_CUDA(cudaGetLastError());
-        pack_kernel<<<unsigned(ceil_div(K, 256)), 256, 0, stream>>>(bc, b.d_off, K, L, B, W, rp);
-        STB_CUDA(cudaGetLastError());
-        note_launch(nullptr, 2);
-        dc.packB = B;
-        dc.packW = W;
+    const st_seqset_s* sets[2] = {&a, &b};
+    DistPlan* plans[2] = {dc.a, dc.b};
+    bool fresh = dc.fresh;
+    PackArgs pa{};
+    int todo = 0;
+    for (int t = 0; t < 2; ++t) {
+        DistPlan& p = *plans[t];
+        if (p.packB == B && p.packW == W) continue;
+        pa.codes[todo] = sets[t]->d_codes;
+        pa.off[todo] = sets[t]->d_off;
+        pa.count[todo] = sets[t]->count;
+        pa.packed[todo++] = sets[t]->d_packed;
+        p.packB = B;
+        p.packW = W;
     }
+    if (todo) {
+        fresh = true;
+        const int64_t most = std::max(pa.count[0], pa.count[1]);
+        pack_kernel<<<dim3(unsigned(ceil_div(most, 256)), unsigned(todo)), 256, 0, stream>>>(pa, L, B, W);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) plans[0]->packB = plans[1]->packB = 0;
+        STB_CUDA(e);
+        note_launch(nullptr);
+    }
+    if (fresh) settle(a, b, stream);
+    const uint32_t* qp = a.d_packed;
+    const uint32_t* rp = b.d_packed;
     const char* name;
     switch (B) {
         case 1: name = launch_hamming<1>(qp, rp, N, K, W, out_d, stream, ctx.num_sms); break;
@@ -417,39 +546,27 @@ void levenshtein_sets(st_seqset_s& a, st_seqset_s& b, int32_t* out_d, cudaStream
     const int64_t N = r1 - r0, K = b.count;
     if (N == 0 || K == 0) return;
     Context& ctx = context();
-    DistCache& dc = compute_codes(a, b, stream, ctx);
+    const DistCodes dc = compute_codes(a, b, stream, ctx);
+    if (dc.fresh) settle(a, b, stream);
     const int sigma = std::max(1, dc.sigma);
-    const uint8_t* ac = static_cast<uint8_t*>(dc.ac.ptr);
-    const uint8_t* bc = static_cast<uint8_t*>(dc.bc.ptr);
+    const uint8_t* ac = a.d_codes;
+    const uint8_t* bc = b.d_codes;
     // rows [r0, r1): their offsets and their block of the result
     const int64_t* aoff = a.d_off + r0;
     out_d += r0 * K;
-    const dim3 grid(unsigned(ceil_div(K, kLevWarps * 32)), unsigned(ceil_div(N, kLevRows)));
-    // Bit-vector path: refs up to 512 symbols (1, 2, 4 or 8 words) while the Peq table fits.
-    const int words = b.max_len <= 64    ? 1
-                    : b.max_len <= 128 ? 2
-                    : b.max_len <= 256 ? 4
-                    : b.max_len <= 512 ? 8
-                                       : 0;
-    const size_t smem = size_t(kLevWarps) * sigma * std::max(words, 1) * 32 * 8;
-    if (words && sigma <= 64 && smem <= size_t(200) * 1024 && grid.y <= 65535) {
-        const void* kern = words == 1 ? reinterpret_cast<const void*>(levenshtein_kernel<1>)
-                         : words == 2 ? reinterpret_cast<const void*>(levenshtein_kernel<2>)
-                         : words == 4 ? reinterpret_cast<const void*>(levenshtein_kernel<4>)
-                                      : reinterpret_cast<const void*>(levenshtein_kernel<8>);
-        ensure_smem_limit(kern, smem);
-        if (words == 1)
-            levenshtein_kernel<1><<<grid, kLevWarps * 32, smem, stream>>>(ac, aoff, bc, b.d_off,
-                                                                         N, K, sigma, out_d);
-        else if (words == 2)
-            levenshtein_kernel<2><<<grid, kLevWarps * 32, smem, stream>>>(ac, aoff, bc, b.d_off,
-                                                                         N, K, sigma, out_d);
-        else if (words == 4)
-            levenshtein_kernel<4><<<grid, kLevWarps * 32, smem, stream>>>(ac, aoff, bc, b.d_off,
-                                                                         N, K, sigma, out_d);
-        else
-            levenshtein_kernel<8><<<grid, kLevWarps * 32, smem, stream>>>(ac, aoff, bc, b.d_off,
-                                                                         N, K, sigma, out_d);
+    // Bit-vector path: refs up to 512 symbols while the Peq table fits.  Rows per CTA: enough that
+    // building the table (about as long as one row) does not show, while the GPU (eight CTAs
+    // per SM) still gets six waves of CTAs.
+    int words = 0;
+    const LevKernel kern = lev_kernel(b.max_len, words);
+    const size_t smem = size_t(kLevWarps) * sigma * std::max(words, 1) * 32 * 4;
+    const int64_t colblocks = ceil_div(K, kLevWarps * 32);
+    const int rows = int(std::min<int64_t>(
+        128, std::max<int64_t>(16, N * colblocks / (int64_t(ctx.num_sms) * 8 * 6))));
+    const dim3 grid(unsigned(colblocks), unsigned(std::min<int64_t>(ceil_div(N, rows), 65536)));
+    if (kern && sigma <= 64 && smem <= size_t(200) * 1024 && grid.y <= 65535) {
+        ensure_smem_limit(reinterpret_cast<const void*>(kern), smem);
+        kern<<<grid, kLevWarps * 32, smem, stream>>>(ac, aoff, bc, b.d_off, N, K, sigma, rows, out_d);
         STB_CUDA(cudaGetLastError());
         note_launch("levenshtein_kernel");
         return;

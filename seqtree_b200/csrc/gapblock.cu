@@ -77,9 +77,9 @@ struct QueryPlan {
     std::vector<int4> quads;             // original indices (-1 marks an empty slot)
     std::vector<int4> slices;            // (first quad, quads, length, profile row offset)
     int64_t prof_rows = 0;               // profile rows of all slices
-    DevBuf d_plan;                       // quads, then slices
+    OwnedBuf d_plan;                     // quads, then slices
     std::vector<uint8_t> prof_key;       // (A, word width, penalty grid) the profile was built for
-    DevBuf d_prof;                       // [row][quad][32] uint32 (twice the words when WIDE)
+    OwnedBuf d_prof;                     // [row][quad][32] uint32 (twice the words when WIDE)
 };
 
 struct RefPlan {
@@ -94,9 +94,9 @@ struct RefPlan {
                                          // longest | 0x100 when all are that long
     std::vector<int4> chunks;            // (first task, tasks, slab byte offset, slab bytes)
     int64_t slab_bytes = 0;
-    DevBuf d_plan;                       // chunks, then tasks
-    DevBuf d_meta;                       // per slot: column in the chunk | length << 16
-    DevBuf d_slab;                       // per task: longest rows of 32 bytes (4*code per lane)
+    OwnedBuf d_plan;                     // chunks, then tasks
+    OwnedBuf d_meta;                     // per slot: column in the chunk | length << 16
+    OwnedBuf d_slab;                     // per task: longest rows of 32 bytes (4*code per lane)
 };
 
 // Queries (rows [r0, r1) of the set; r1 = -1 for all) sorted by length (stable); each length's

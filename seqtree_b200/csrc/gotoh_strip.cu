@@ -295,13 +295,13 @@ __global__ void strip_slab_kernel(const uint8_t* __restrict__ codes, const int64
 struct StripQueryPlan {
     uint64_t uid = 0;
     int64_t nqp = 0;
-    DevBuf pairs;
+    OwnedBuf pairs;
 };
 
 struct StripRefPlan {
     uint64_t uid = 0;
     int ngroups = 0;
-    DevBuf sorted, groups, slab;
+    OwnedBuf sorted, groups, slab;
 };
 
 std::vector<int32_t> longest_first(const st_seqset_s& s) {

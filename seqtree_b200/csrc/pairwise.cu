@@ -731,7 +731,7 @@ struct WaveState {
 struct WavePlan {
     uint64_t uid = 0;
     std::vector<std::tuple<int, int64_t, int64_t>> pair_groups;
-    DevBuf qpairs, sorted;
+    OwnedBuf qpairs, sorted;
 };
 
 WavePlan& wave_plan(st_seqset_s& s, Context& ctx, int slot, cudaStream_t stream) {
