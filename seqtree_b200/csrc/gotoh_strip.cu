@@ -2,7 +2,7 @@
 //
 // A warp scores two queries (neighbours in length order, packed int16x2) against 32 refs
 // (neighbours in length order), one ref per lane.  The query's rows are cut into strips of R rows
-// (R <= 48, a multiple of 4, chosen so that at most 3 rows per strip are padding); a lane keeps H
+// (R <= 48, even up to 24 and a multiple of 4 beyond, so at most 3 rows per strip are padding); a lane keeps H
 // and Y of the strip's rows in registers and walks the columns of its ref, so there are no
 // shuffles, no ramp and no idle lanes, which is where the query-pair wavefront (pairwise.cu) loses
 // its time: 31 of n + 31 steps, up to 31 padded rows and the per-step exchange.  Between strips the
@@ -53,9 +53,9 @@ struct StripArgs {
     const int2* qpairs;       // longest first; x == y for a single
     int64_t nqp;
     const uint32_t* slab;     // per group of 32 refs: ceil(longest / 4) x 32 words, 4 codes * 4 each
-    const int2* groups;       // per group: slab offset (in 32-word rows), rows of 4 columns
-    const int32_t* rsorted;   // refs, longest first
-    const int32_t* rlen;
+    const int2* groups;       // per group: slab offset (in 32-word rows), its longest ref | 1 << 16
+                              // when it has 32 refs of that length
+    const int2* rmeta;        // refs (index, length), longest first
     int64_t K;
     int ngroups;
     int gpw;                  // groups a warp takes per unit
@@ -77,11 +77,13 @@ struct StripArgs {
 
 __device__ __forceinline__ uint32_t dup16(int v) { return uint32_t(uint16_t(int16_t(v))) * 0x10001u; }
 
-// Strips of at most `most` rows for m rows: how many, and rows per strip (a multiple of 4).
+// Strips of at most `most` rows for m rows: how many, and rows per strip (even up to 24, then a
+// multiple of 4).
 __host__ __device__ inline void strip_shape(int m, int most, int& strips, int& rows) {
     strips = (m + most - 1) / most;
     if (strips < 1) strips = 1;
-    rows = ((m + strips - 1) / strips + 3) / 4 * 4;
+    rows = (m + strips - 1) / strips;
+    rows = rows <= 24 ? (rows + 1) / 2 * 2 : (rows + 3) / 4 * 4;
     if (rows < 4) rows = 4;
 }
 
@@ -94,13 +96,24 @@ __device__ __forceinline__ void strip_unit(const StripArgs& a, const uint32_t* s
     const uint32_t eo2 = dup16(a.ge - a.go), mge2 = dup16(-a.ge);
     const uint32_t mgo_add = 0u - uint32_t(a.go) * 0x10001u;  // subtracts go from both halves
     const uint32_t e2 = uint32_t(a.ge) * 0x10001u;
-    for (int g = g0; g < g1; g += kStripWarps) {
-        const int2 grp = a.groups[g];
+    auto ref_of = [&](int g) {
         const int64_t t = int64_t(g) * 32 + lane;
-        const bool live = t < a.K;
-        const int k = live ? a.rsorted[t] : 0;
-        const int n = live ? a.rlen[k] : 0;
+        return t < a.K ? a.rmeta[t] : make_int2(-1, 0);
+    };
+    if (g0 >= g1) return;
+    int2 grp = a.groups[g0], ref = ref_of(g0);
+    uint32_t head = a.slab[int64_t(grp.x) * 32 + lane];
+    for (int g = g0; g < g1; g += kStripWarps) {
         const uint32_t* codes = a.slab + int64_t(grp.x) * 32 + lane;
+        const int k = ref.x, n = ref.y, cols = grp.y & 0xFFFF;
+        const bool one_length = (grp.y >> 16) != 0;
+        const uint32_t first_codes = head;
+        // the next group's head is on its way while this one runs
+        if (g + kStripWarps < g1) {
+            grp = a.groups[g + kStripWarps];
+            ref = ref_of(g + kStripWarps);
+            head = a.slab[int64_t(grp.x) * 32 + lane];
+        }
         uint32_t c1 = 0u, c2 = 0u, best = 0u;
         for (int s = 0; s < strips; ++s) {
             const uint8_t* prof = reinterpret_cast<const uint8_t*>(s_prof + s * R * kProfW);
@@ -120,75 +133,82 @@ __device__ __forceinline__ void strip_unit(const StripArgs& a, const uint32_t* s
             uint2 nxt = make_uint2(0u, 0u), nx2 = make_uint2(0u, 0u);
             if (!first) {
                 nxt = scr[lane];
-                nx2 = scr[32 + lane];
+                if (cols > 1) nx2 = scr[32 + lane];
             }
             // rows of the two queries' last residues in this strip, or -1
             const int cr1 = (!LOCAL && (m1 - 1) / R == s) ? (m1 - 1) - s * R : -1;
             const int cr2 = (!LOCAL && (m2 - 1) / R == s) ? (m2 - 1) - s * R : -1;
-            const bool capture = !LOCAL && (cr1 >= 0 || cr2 >= 0);
-            const int cols = grp.y * 4;
-            uint32_t w = 0u, wn = codes[0];
+            const bool capture = !LOCAL && (cr1 >= 0 || cr2 >= 0), mixed = capture && !one_length;
+            uint32_t w = 0u, wn = first_codes;
             uint32_t nfl = 0u;  // local: -(j * extend) in both halves
             int je = 0;
-            // Four columns per code word; short strips take them unrolled (a tall strip's column is
-            // long enough to hide the loop, and four of them would outgrow the instruction cache).
-#pragma unroll 1
-            for (int j0 = 0; j0 < cols; j0 += 4) {
-                w = wn;
-                if (j0 + 4 < cols) wn = codes[j0 * 8 + 32];
-#pragma unroll(R <= 24 ? 4 : 1)
-                for (int j = j0; j < j0 + 4; ++j) {
-                    const uint8_t* pc = prof + (w & 0xFFu);
-                    w >>= 8;
-                    if constexpr (LOCAL) {
-                        floor2 += e2;
-                        je += a.ge;
-                        nfl = dup16(-je);
-                    }
-                    if (!first) {
-                        top = nxt;
-                        nxt = nx2;
-                        if (j + 2 < cols) nx2 = scr[(j + 2) * 32 + lane];
-                    } else if constexpr (LOCAL) {
-                        top.x = floor2;
-                        top.y = floor2 + mgo_add;
-                    }
-                    uint32_t x = top.y;
-                    uint32_t my = __viaddmax_s16x2(diag, *reinterpret_cast<const uint32_t*>(pc), Y[0]);
-                    uint32_t colmax = floor2, hprev = 0u;
-                    diag = top.x;
+            auto keep = [&] {  // the scores' halves, once column n is done
 #pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        uint32_t myn = 0u;
-                        if (r + 1 < R)
-                            myn = __viaddmax_s16x2(
-                                H[r], *reinterpret_cast<const uint32_t*>(pc + (r + 1) * kProfW * 4),
-                                Y[r + 1]);
-                        uint32_t h;
-                        if constexpr (LOCAL) {
-                            h = __vimax3_s16x2(my, x, floor2);
-                            x = __viaddmax_s16x2(x, mge2, my * a.one + mgo_add);
-                            if (r & 1) colmax = __vimax3_s16x2(colmax, hprev, h);
-                            hprev = h;
-                        } else {
-                            h = __vmaxs2(my, x);
-                            x = __viaddmax_s16x2(my, eo2, x);
-                        }
-                        Y[r] = __viaddmax_s16x2(h, eo2, Y[r]);
-                        H[r] = h;
-                        my = myn;
-                    }
-                    if constexpr (LOCAL) best = __viaddmax_s16x2(colmax, nfl, best);
-                    if (!last) scr[j * 32 + lane] = make_uint2(H[R - 1], x);
-                    if (!LOCAL && capture && j + 1 == n) {
-#pragma unroll
-                        for (int r = 0; r < R; ++r) {
-                            if (r == cr1) c1 = H[r];
-                            if (r == cr2) c2 = H[r];
-                        }
-                    }
+                for (int r = 0; r < R; ++r) {
+                    if (r == cr1) c1 = H[r];
+                    if (r == cr2) c2 = H[r];
                 }
+            };
+            auto column = [&](int j) {
+                const uint8_t* pc = prof + (w & 0xFFu);
+                w >>= 8;
+                if constexpr (LOCAL) {
+                    floor2 += e2;
+                    je += a.ge;
+                    nfl = dup16(-je);
+                }
+                if (!first) {
+                    top = nxt;
+                    nxt = nx2;
+                    if (j + 2 < cols) nx2 = scr[(j + 2) * 32 + lane];
+                } else if constexpr (LOCAL) {
+                    top.x = floor2;
+                    top.y = floor2 + mgo_add;
+                }
+                uint32_t x = top.y;
+                uint32_t my = __viaddmax_s16x2(diag, *reinterpret_cast<const uint32_t*>(pc), Y[0]);
+                uint32_t colmax = floor2, hprev = 0u;
+                diag = top.x;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    uint32_t myn = 0u;
+                    if (r + 1 < R)
+                        myn = __viaddmax_s16x2(
+                            H[r], *reinterpret_cast<const uint32_t*>(pc + (r + 1) * kProfW * 4),
+                            Y[r + 1]);
+                    uint32_t h;
+                    if constexpr (LOCAL) {
+                        h = __vimax3_s16x2(my, x, floor2);
+                        x = __viaddmax_s16x2(x, mge2, my * a.one + mgo_add);
+                        if (r & 1) colmax = __vimax3_s16x2(colmax, hprev, h);
+                        hprev = h;
+                    } else {
+                        h = __vmaxs2(my, x);
+                        x = __viaddmax_s16x2(my, eo2, x);
+                    }
+                    Y[r] = __viaddmax_s16x2(h, eo2, Y[r]);
+                    H[r] = h;
+                    my = myn;
+                }
+                if constexpr (LOCAL) best = __viaddmax_s16x2(colmax, nfl, best);
+                if (!last) scr[j * 32 + lane] = make_uint2(H[R - 1], x);
+                if (mixed && j + 1 == n) keep();
+            };
+            // Four columns per code word, not unrolled: a column is long enough to hide its loop, and
+            // with a body per strip height the instruction cache holds single columns at best
+            // (two at a time 0.71 against 0.69 ms on 4,096 x 4,096 junctions, four 0.74).
+            int j = 0;
+#pragma unroll 1
+            for (; j + 4 <= cols; j += 4) {
+                w = wn;
+                if (j + 4 < cols) wn = codes[j * 8 + 32];
+#pragma unroll 1
+                for (int u = 0; u < 4; ++u) column(j + u);
             }
+            w = wn;
+#pragma unroll 1
+            for (; j < cols; ++j) column(j);
+            if (capture && !mixed) keep();
         }
         int v1, v2;
         if constexpr (LOCAL) {
@@ -198,7 +218,7 @@ __device__ __forceinline__ void strip_unit(const StripArgs& a, const uint32_t* s
             v1 = int(int16_t(uint16_t(c1 & 0xFFFFu))) - (m1 + n) * a.ge;
             v2 = int(int16_t(uint16_t(c2 >> 16))) - (m2 + n) * a.ge;
         }
-        if (live) {
+        if (k >= 0) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 if (h == 1 && qp.y == qp.x) break;
@@ -260,8 +280,9 @@ gotoh_strip_kernel(const StripArgs a) {
         strip_unit<RR, LOCAL>(a, s_prof, strips, qp, m1, m2, g0, g1, scr);                     \
         break;
         switch (R) {
-            STB_STRIP(4) STB_STRIP(8) STB_STRIP(12) STB_STRIP(16) STB_STRIP(20) STB_STRIP(24)
-            STB_STRIP(28) STB_STRIP(32)
+            STB_STRIP(4) STB_STRIP(6) STB_STRIP(8) STB_STRIP(10) STB_STRIP(12) STB_STRIP(14)
+            STB_STRIP(16) STB_STRIP(18) STB_STRIP(20) STB_STRIP(22) STB_STRIP(24) STB_STRIP(28)
+            STB_STRIP(32)
         }
         if constexpr (MAXR == 48)
             switch (R) { STB_STRIP(36) STB_STRIP(40) STB_STRIP(44) STB_STRIP(48) }
@@ -272,16 +293,16 @@ gotoh_strip_kernel(const StripArgs a) {
 // Ref codes of every group: word [g][j / 4][lane] holds four columns' 4 * code (the padding code
 // past a ref's end and past the last ref).
 __global__ void strip_slab_kernel(const uint8_t* __restrict__ codes, const int64_t* __restrict__ off,
-                                  const int32_t* __restrict__ sorted, int64_t K,
+                                  const int2* __restrict__ meta, int64_t K,
                                   const int2* __restrict__ groups, uint32_t* __restrict__ slab) {
     const int g = blockIdx.x;
     const int2 grp = groups[g];
-    for (int i = threadIdx.x; i < grp.y * 32; i += blockDim.x) {
+    for (int i = threadIdx.x; i < ((grp.y & 0xFFFF) + 3) / 4 * 32; i += blockDim.x) {
         const int lane = i & 31, j = (i >> 5) * 4;
         const int64_t t = int64_t(g) * 32 + lane;
         uint32_t w = 0u;
-        const int k = t < K ? sorted[t] : 0;
-        const int n = t < K ? int(off[k + 1] - off[k]) : 0;
+        const int2 ref = t < K ? meta[t] : make_int2(0, 0);
+        const int k = ref.x, n = ref.y;
         for (int b = 0; b < 4; ++b) {
             const uint32_t c = j + b < n ? uint32_t(codes[off[k] + j + b]) : uint32_t(kPadCode);
             w |= (c * 4u) << (8 * b);
@@ -301,7 +322,7 @@ struct StripQueryPlan {
 struct StripRefPlan {
     uint64_t uid = 0;
     int ngroups = 0;
-    OwnedBuf sorted, groups, slab;
+    OwnedBuf meta, groups, slab;
 };
 
 std::vector<int32_t> longest_first(const st_seqset_s& s) {
@@ -340,15 +361,19 @@ StripRefPlan& ref_plan(st_seqset_s& s, Context& ctx, cudaStream_t stream) {
     int64_t rows = 0;
     for (size_t g = 0; g < groups.size(); ++g) {
         const int longest = s.h_len[size_t(order[g * 32])];
-        groups[g] = make_int2(int(rows), (longest + 3) / 4);
-        rows += groups[g].y;
+        const bool one_length = g * 32 + 32 <= order.size() &&
+                                s.h_len[size_t(order[g * 32 + 31])] == longest;
+        groups[g] = make_int2(int(rows), longest | (one_length ? 1 << 16 : 0));
+        rows += (longest + 3) / 4;
     }
     if (rows > INT32_MAX) fail(ST_EINVAL, "seqtree_b200: reference set too large for one call");
     p.uid = 0;
-    h2d(p.sorted.as<int32_t>(order.size()), order.data(), order.size() * 4, stream);
+    std::vector<int2> meta(order.size());
+    for (size_t t = 0; t < order.size(); ++t) meta[t] = make_int2(order[t], s.h_len[size_t(order[t])]);
+    h2d(p.meta.as<int2>(meta.size()), meta.data(), meta.size() * sizeof(int2), stream);
     h2d(p.groups.as<int2>(groups.size()), groups.data(), groups.size() * sizeof(int2), stream);
     strip_slab_kernel<<<unsigned(groups.size()), 256, 0, stream>>>(
-        s.d_bytes, s.d_off, static_cast<int32_t*>(p.sorted.ptr), s.count,
+        s.d_bytes, s.d_off, static_cast<int2*>(p.meta.ptr), s.count,
         static_cast<int2*>(p.groups.ptr), p.slab.as<uint32_t>(size_t(rows) * 32));
     STB_CUDA(cudaGetLastError());
     note_launch(nullptr);
@@ -469,8 +494,7 @@ void align_strip(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, in
     a.nqp = qp.nqp;
     a.slab = static_cast<const uint32_t*>(rp.slab.ptr);
     a.groups = static_cast<const int2*>(rp.groups.ptr);
-    a.rsorted = static_cast<const int32_t*>(rp.sorted.ptr);
-    a.rlen = rs.d_len;
+    a.rmeta = static_cast<const int2*>(rp.meta.ptr);
     a.K = rs.count;
     a.ngroups = rp.ngroups;
     a.dist = dist;
