@@ -123,7 +123,7 @@ struct Transient {
 void finish(Context& ctx, int32_t* out, int64_t N, int64_t K, int32_t* out_d) {
     const size_t bytes = size_t(N) * size_t(K) * sizeof(int32_t);
     STB_CUDA(cudaMemcpyAsync(out, out_d, bytes, cudaMemcpyDeviceToHost, ctx.stream));
-    STB_CUDA(cudaMemcpyAsync(ctx.flags_h + 8, ctx.flags_d + 8, 8 * sizeof(int64_t),
+    STB_CUDA(cudaMemcpyAsync(ctx.flags_h + 6, ctx.flags_d + 6, 10 * sizeof(int64_t),
                              cudaMemcpyDeviceToHost, ctx.stream));
     STB_CUDA(cudaStreamSynchronize(ctx.stream));
 }
@@ -161,7 +161,7 @@ void check_timeout(Context& ctx) {
 }
 
 void clear_flags(Context& ctx) {
-    STB_CUDA(cudaMemsetAsync(ctx.flags_d + 8, 0, 8 * sizeof(int64_t), ctx.stream));
+    STB_CUDA(cudaMemsetAsync(ctx.flags_d + 6, 0, 10 * sizeof(int64_t), ctx.stream));
 }
 
 }  // namespace
@@ -259,24 +259,22 @@ int32_t st_gapblock_matrix(const st_strings* queries, const st_strings* refs, in
         std::lock_guard<std::mutex> lk(ctx.mu);
         clear_flags(ctx);
         // src/gapblock.cpp:85-94: queries are encoded before refs.  The symbol check is
-        // deferred to the call's one synchronisation (words 0 and 1 of the flag area: the first
-        // invalid byte of the queries, of the refs); invalid symbols compute as code 0 meanwhile
-        // and the call then fails with the reference's message, queries first, as the reference
-        // does.  `out` is unspecified after a failed call.
-        Transient t;
+        // deferred to the call's one synchronisation (words 6 and 7 of the flag area); invalid
+        // symbols compute as code 0 meanwhile and the call then fails with the reference's
+        // message, queries first, as the reference does.  `out` is unspecified after a failed call.
+        std::unique_ptr<st_seqset_s> sets[2];
         {
             Phase ph("upload+encode");
-            STB_CUDA(cudaMemsetAsync(ctx.flags_d, 0xFF, 2 * sizeof(int64_t), ctx.stream));
-            t.q.reset(make_seqset(queries, alphabet, ctx.stream, nullptr, nullptr, ctx.tq, 0));
-            t.r.reset(make_seqset(refs, alphabet, ctx.stream, nullptr, nullptr, ctx.tr, 1));
+            const st_strings* const in[2] = {queries, refs};
+            make_pair(in, alphabet, ctx.stream, reinterpret_cast<unsigned long long*>(ctx.flags_d + 6), sets);
         }
         auto check_symbols = [&] {
             for (int w = 0; w < 2; ++w) {
-                const uint64_t bad = static_cast<uint64_t>(ctx.flags_h[w]);
-                if (bad != ~uint64_t(0)) {
+                const uint64_t bad = static_cast<uint64_t>(ctx.flags_h[6 + w]);
+                if (bad != 0) {
                     const st_strings* s = w == 0 ? queries : refs;
                     const char c =
-                        reinterpret_cast<const char*>(s->bytes)[s->offsets[0] + int64_t(bad)];
+                        reinterpret_cast<const char*>(s->bytes)[s->offsets[0] + int64_t(~bad)];
                     fail(ST_EINVAL, std::string("symbol '") + c + "' is not in the alphabet");
                 }
             }
@@ -285,12 +283,12 @@ int32_t st_gapblock_matrix(const st_strings* queries, const st_strings* refs, in
         {
             Phase ph("plan+launch");
             try {
-                gapblock_sets(*t.q, *t.r, penalty, matrix_size, gap_open, gap_extend, prior,
+                gapblock_sets(*sets[0], *sets[1], penalty, matrix_size, gap_open, gap_extend, prior,
                               prior_len, prior_width, out_d, ctx.stream);
             } catch (...) {
                 // the reference reports an invalid symbol before the prior-table errors that
                 // planning finds (src/gapblock.cpp:85-102)
-                STB_CUDA(cudaMemcpyAsync(ctx.flags_h, ctx.flags_d, 2 * sizeof(int64_t),
+                STB_CUDA(cudaMemcpyAsync(ctx.flags_h + 6, ctx.flags_d + 6, 2 * sizeof(int64_t),
                                          cudaMemcpyDeviceToHost, ctx.stream));
                 STB_CUDA(cudaStreamSynchronize(ctx.stream));
                 check_symbols();
@@ -299,8 +297,6 @@ int32_t st_gapblock_matrix(const st_strings* queries, const st_strings* refs, in
         }
         {
             Phase ph("kernel+d2h");
-            STB_CUDA(cudaMemcpyAsync(ctx.flags_h, ctx.flags_d, 2 * sizeof(int64_t),
-                                     cudaMemcpyDeviceToHost, ctx.stream));
             finish(ctx, out, N, K, out_d);
         }
         check_symbols();

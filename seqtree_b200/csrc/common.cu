@@ -330,7 +330,7 @@ Lut make_lut(int32_t alphabet) {
 // recorded with atomicMin so the error names the same symbol the reference's sequential
 // encoder stops at.
 __global__ void encode_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ out,
-                              int64_t n, Lut lut, unsigned long long* first_bad, uint8_t bad_code) {
+                              int64_t n, Lut lut, unsigned long long* first_bad) {
     __shared__ uint8_t s_lut[256];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) s_lut[i] = lut.v[i];
     __syncthreads();
@@ -347,7 +347,6 @@ __global__ void encode_kernel(const uint8_t* __restrict__ in, uint8_t* __restric
                 if (c == 0xFF) {
                     if (!bad) atomicMin(first_bad, (unsigned long long)(base + b));
                     bad = true;
-                    c = bad_code;
                 }
                 o |= uint32_t(c) << (8 * b);
             }
@@ -357,7 +356,6 @@ __global__ void encode_kernel(const uint8_t* __restrict__ in, uint8_t* __restric
                 uint8_t c = s_lut[in[i]];
                 if (c == 0xFF) {
                     atomicMin(first_bad, (unsigned long long)i);
-                    c = bad_code;
                 }
                 out[i] = c;
             }
@@ -395,16 +393,13 @@ std::unique_ptr<st_seqset_s> row_view(const st_seqset_s& s, int64_t rows) {
     return v;
 }
 
-st_seqset_s* make_seqset(const st_strings* s, int32_t alphabet, cudaStream_t stream,
-                         int64_t* bad_index, char* bad_char, DevBuf* storage, int defer_word) {
-    std::atomic<uint64_t>& next_uid = g_next_uid;
-    if (!s || (s->count > 0 && !s->offsets)) fail(ST_EINVAL, "seqtree_b200: null sequence set");
-    if (alphabet != -1 && alphabet_size(alphabet) == 0)
-        fail(ST_EINVAL, "unknown alphabet code " + std::to_string(alphabet));
-    Context& ctx = context();
+namespace {
+
+// A set's host side: counts, offsets from 0, lengths.
+std::unique_ptr<st_seqset_s> describe(const st_strings* s, int32_t alphabet, const Context& ctx) {
     auto set = std::make_unique<st_seqset_s>();
     set->device = ctx.device;
-    set->uid = next_uid.fetch_add(1);
+    set->uid = g_next_uid.fetch_add(1);
     set->alphabet = alphabet;
     set->count = s->count;
     set->h_off.assign(s->offsets, s->offsets + (s->count + 1));
@@ -421,6 +416,110 @@ st_seqset_s* make_seqset(const st_strings* s, int32_t alphabet, cudaStream_t str
         mx = std::max<int32_t>(mx, int32_t(l));
     }
     set->max_len = mx;
+    return set;
+}
+
+// Both sets of a host call on the device: codes, 64 zero bytes past them, lengths, in one launch
+// (a set per blockIdx.y).  bad[set] keeps the complement of the first invalid byte's index (0: none).
+struct PairPrep {
+    const uint8_t* raw[2];
+    const int64_t* off[2];
+    uint8_t* codes[2];
+    int32_t* len[2];
+    int64_t total[2], count[2];
+    unsigned long long* bad;
+    Lut lut;
+};
+
+__global__ void __launch_bounds__(256) pair_prep_kernel(const PairPrep p) {
+    __shared__ uint8_t s_lut[256];
+    s_lut[threadIdx.x] = p.lut.v[threadIdx.x];
+    __syncthreads();
+    const int t = blockIdx.y;
+    const int64_t stride = int64_t(gridDim.x) * 256, first = int64_t(blockIdx.x) * 256 + threadIdx.x;
+    for (int64_t i = first; i < p.count[t]; i += stride) p.len[t][i] = int32_t(p.off[t][i + 1] - p.off[t][i]);
+    for (int64_t base = first * 4; base < p.total[t] + 64; base += stride * 4) {
+        uint32_t o = 0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            if (base + b >= p.total[t]) break;
+            uint8_t c = s_lut[p.raw[t][base + b]];
+            if (c == 0xFF) {  // stored as code 0, so every later kernel indexes its tables in range
+                atomicMax(p.bad + t, ~(unsigned long long)(base + b));
+                c = 0;
+            }
+            o |= uint32_t(c) << (8 * b);
+        }
+        *reinterpret_cast<uint32_t*>(p.codes[t] + base) = o;
+    }
+}
+
+}  // namespace
+
+void make_pair(const st_strings* const in[2], int32_t alphabet, cudaStream_t stream, unsigned long long* bad,
+               std::unique_ptr<st_seqset_s> sets[2]) {
+    Context& ctx = context();
+    auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
+    // one block: what is uploaded (offsets and letters of both sets), then what is made of it
+    size_t off_at[2], raw_at[2], codes_at[2], len_at[2], at = 0;
+    for (int t = 0; t < 2; ++t) {
+        sets[t] = describe(in[t], alphabet, ctx);
+        sets[t]->owns = false;
+        off_at[t] = at;
+        at = up(at + sizeof(int64_t) * size_t(sets[t]->count + 1));
+        raw_at[t] = at;
+        at = up(at + size_t(sets[t]->total));
+    }
+    const size_t upload = at;
+    for (int t = 0; t < 2; ++t) {
+        codes_at[t] = at;
+        at = up(at + size_t(sets[t]->total) + 64);
+        len_at[t] = at;
+        at = up(at + sizeof(int32_t) * size_t(sets[t]->count));
+    }
+    uint8_t* d = ctx.pair_buf.as<uint8_t>(at);
+    PairPrep p{};
+    p.bad = bad;
+    p.lut = make_lut(alphabet);
+    // Small uploads go through a pinned block as one copy; larger ones are copied part by part (the
+    // driver stages pageable memory itself, at the same rate).
+    constexpr size_t kStage = size_t(1) << 20;
+    if (upload <= kStage && !ctx.stage_h) STB_CUDA(cudaHostAlloc(&ctx.stage_h, kStage, cudaHostAllocDefault));
+    for (int t = 0; t < 2; ++t) {
+        const uint8_t* letters = reinterpret_cast<const uint8_t*>(in[t]->bytes) + in[t]->offsets[0];
+        const size_t off_bytes = sizeof(int64_t) * size_t(sets[t]->count + 1), total = size_t(sets[t]->total);
+        if (upload <= kStage) {
+            std::memcpy(ctx.stage_h + off_at[t], sets[t]->h_off.data(), off_bytes);
+            if (total) std::memcpy(ctx.stage_h + raw_at[t], letters, total);
+        } else {
+            STB_CUDA(cudaMemcpyAsync(d + off_at[t], sets[t]->h_off.data(), off_bytes, cudaMemcpyHostToDevice,
+                                     stream));
+            if (total) STB_CUDA(cudaMemcpyAsync(d + raw_at[t], letters, total, cudaMemcpyHostToDevice, stream));
+        }
+        sets[t]->d_bytes = p.codes[t] = d + codes_at[t];
+        sets[t]->d_off = reinterpret_cast<int64_t*>(d + off_at[t]);
+        sets[t]->d_len = p.len[t] = reinterpret_cast<int32_t*>(d + len_at[t]);
+        p.off[t] = sets[t]->d_off;
+        p.raw[t] = d + raw_at[t];
+        p.total[t] = sets[t]->total;
+        p.count[t] = sets[t]->count;
+    }
+    if (upload <= kStage) STB_CUDA(cudaMemcpyAsync(d, ctx.stage_h, upload, cudaMemcpyHostToDevice, stream));
+    const int64_t work = std::max({ceil_div(p.total[0] + 64, 4), ceil_div(p.total[1] + 64, 4), p.count[0],
+                                   p.count[1]});
+    const unsigned grid = unsigned(std::min<int64_t>(ceil_div(work, 256), int64_t(ctx.num_sms) * 8));
+    pair_prep_kernel<<<dim3(grid, 2), 256, 0, stream>>>(p);
+    STB_CUDA(cudaGetLastError());
+    note_launch(nullptr);
+}
+
+st_seqset_s* make_seqset(const st_strings* s, int32_t alphabet, cudaStream_t stream,
+                         int64_t* bad_index, char* bad_char, DevBuf* storage) {
+    if (!s || (s->count > 0 && !s->offsets)) fail(ST_EINVAL, "seqtree_b200: null sequence set");
+    if (alphabet != -1 && alphabet_size(alphabet) == 0)
+        fail(ST_EINVAL, "unknown alphabet code " + std::to_string(alphabet));
+    Context& ctx = context();
+    std::unique_ptr<st_seqset_s> set = describe(s, alphabet, ctx);
     const size_t padded = size_t(set->total) + 64;
     // Raw sets have room for the distances' dense codes and packed words behind their bytes, so that
     // a first distance call allocates nothing.
@@ -451,7 +550,7 @@ st_seqset_s* make_seqset(const st_strings* s, int32_t alphabet, cudaStream_t str
         note_launch(nullptr);
     }
     if (set->total > 0) {
-        const uint8_t* src = reinterpret_cast<const uint8_t*>(s->bytes) + base;
+        const uint8_t* src = reinterpret_cast<const uint8_t*>(s->bytes) + s->offsets[0];
         if (alphabet < 0) {
             STB_CUDA(cudaMemcpyAsync(set->d_bytes, src, size_t(set->total), cudaMemcpyHostToDevice,
                                      stream));
@@ -460,16 +559,14 @@ st_seqset_s* make_seqset(const st_strings* s, int32_t alphabet, cudaStream_t str
             uint8_t* d_raw = raw.as<uint8_t>(padded);
             STB_CUDA(cudaMemsetAsync(d_raw + set->total, 0, 64, stream));
             STB_CUDA(cudaMemcpyAsync(d_raw, src, size_t(set->total), cudaMemcpyHostToDevice, stream));
-            auto* flag = reinterpret_cast<unsigned long long*>(ctx.flags_d + (defer_word > 0 ? defer_word : 0));
+            auto* flag = reinterpret_cast<unsigned long long*>(ctx.flags_d);
             STB_CUDA(cudaMemsetAsync(flag, 0xFF, sizeof(unsigned long long), stream));
             const Lut lut = make_lut(alphabet);
             const int64_t words = ceil_div(set->total, 4);
             const unsigned grid = unsigned(std::min<int64_t>(ceil_div(words, 256), ctx.num_sms * 8));
-            encode_kernel<<<grid, 256, 0, stream>>>(d_raw, set->d_bytes, set->total, lut, flag,
-                                                    uint8_t(defer_word >= 0 ? 0 : 0xFF));
+            encode_kernel<<<grid, 256, 0, stream>>>(d_raw, set->d_bytes, set->total, lut, flag);
             STB_CUDA(cudaGetLastError());
             note_launch(nullptr);
-            if (defer_word >= 0) return set.release();
             const unsigned long long none = ~0ull;
             STB_CUDA(cudaMemcpyAsync(ctx.flags_h, flag, sizeof none, cudaMemcpyDeviceToHost, stream));
             STB_CUDA(cudaStreamSynchronize(stream));

@@ -82,8 +82,8 @@ struct Context {
     int num_sms = 148;
     int max_smem_optin = 0;
     // Small device word area for error reporting, with a pinned host mirror.  Word 0: first
-    // invalid symbol of an encode; word 8: a bounded wait gave up; word 9: an int32 overflow;
-    // words 16-23: byte-presence bitmaps of two sets.  Words 8-15 are cleared before and read after each
+    // invalid symbol of an encode; words 6-7: make_pair's invalid symbols; word 8: a bounded wait gave up; word 9: an int32 overflow;
+    // words 16-23: byte-presence bitmaps of two sets.  Words 6-15 are cleared before and read after each
     // host call.
     int64_t* flags_d = nullptr;
     int64_t* flags_h = nullptr;
@@ -99,6 +99,9 @@ struct Context {
     std::vector<uint8_t> prop_thr_key;
     // bf16 operands of the training GEMM, packed in the tensor-core layout
     DevBuf gemm_a, gemm_b;
+    // block of make_pair's sets and its pinned upload block (1 MiB, made on first use)
+    DevBuf pair_buf;
+    uint8_t* stage_h = nullptr;
     // storage of the transient sets made by the host-buffer entry points
     DevBuf tq[3], tr[3];  // bytes, offsets, lengths
     // plans reused by transient sets (rebuilt in place for every call)
@@ -203,13 +206,15 @@ namespace stb {
 // order errors across two sets exactly as the reference does.
 // `storage` (three buffers: bytes, offsets, lengths) makes a transient set that borrows
 // context memory instead of allocating.
-// `defer_word` >= 0 defers the symbol check: nothing waits for the encode, an invalid symbol is
-// stored as code 0 (so every later kernel indexes its tables in range) and the first invalid
-// byte index is left in device word `defer_word` of the context's flag area (all ones when
-// there is none) for the caller to read after its own final synchronisation.
 st_seqset_s* make_seqset(const st_strings* s, int32_t alphabet, cudaStream_t stream,
-                         int64_t* bad_index, char* bad_char, DevBuf* storage = nullptr,
-                         int defer_word = -1);
+                         int64_t* bad_index, char* bad_char, DevBuf* storage = nullptr);
+
+// Both sets of a host-buffer call as transient sets, in one upload (of up to 1 MiB) and one launch.
+// Nothing waits for the symbol check: an invalid symbol is stored as code 0 (so every later kernel
+// indexes its tables in range) and bad[t], two device words that hold 0 before, gets the complement
+// of set t's first invalid byte index for the caller to read after its final synchronisation.
+void make_pair(const st_strings* const in[2], int32_t alphabet, cudaStream_t stream, unsigned long long* bad,
+               std::unique_ptr<st_seqset_s> sets[2]);
 
 int32_t alphabet_size(int32_t alphabet);
 

@@ -233,14 +233,34 @@ __global__ void profile_kernel(const uint8_t* __restrict__ codes, const int64_t*
     }
 }
 
+// A task's code rows j0, j0 + step, ...: 32 lane bytes each, 4*code of the lane's ref (the null code
+// past a ref's end and past the task's count).
+__device__ __forceinline__ void fill_task(const uint8_t* codes, const int64_t* off, const uint32_t* meta, int4 t,
+                                          int rc, int lane, int j0, int step, uint8_t* slab) {
+    const int rows = t.x & 0xFF;
+    const uint32_t mt = lane < t.z ? meta[t.y + lane] : 0u;
+    const int n = int(mt >> 16);
+    const uint8_t* src = codes + (lane < t.z ? off[int64_t(t.y) / rc * rc + (mt & 0xFFFFu)] : 0);
+#pragma unroll 4
+    for (int j = j0; j < rows; j += step)
+        slab[int64_t(t.w) + j * 32 + lane] = uint8_t((j < n ? int(src[j]) : kNullCode) * 4);
+}
+
 // Slots of one chunk (one block): its columns sorted by length, and inside a length so that
 // neighbours have different columns modulo 32 -- each round takes one ref of every residue -- which
 // puts the dense tile's words of a task into different banks.  (Which of several refs of one
 // length and residue comes first does not matter.)
 constexpr int kMaxRounds = 40;  // rc / 32 of the widest chunk
 
+// With SLAB the block goes on to write its chunk's code slab (a launch less, for few chunks).
+template <bool SLAB>
 __global__ void __launch_bounds__(256) chunk_order_kernel(const int32_t* __restrict__ rlen, int64_t K, int rc,
-                                                          int max_len, uint32_t* __restrict__ meta) {
+                                                          int max_len, uint32_t* __restrict__ meta,
+                                                          const uint8_t* __restrict__ codes,
+                                                          const int64_t* __restrict__ off,
+                                                          const int4* __restrict__ chunks,
+                                                          const int4* __restrict__ tasks,
+                                                          uint8_t* __restrict__ slab) {
     __shared__ uint32_t occ[65 * 32];
     __shared__ uint32_t at[65 * kMaxRounds];
     const int64_t k0 = int64_t(blockIdx.x) * rc;
@@ -282,20 +302,19 @@ __global__ void __launch_bounds__(256) chunk_order_kernel(const int32_t* __restr
         if (c < kcount)
             meta[k0 + atomicAdd(&at[bucket[t]], 1u)] = uint32_t(c) | (bucket[t] / rounds) << 16;
     }
+    if constexpr (SLAB) {
+        __syncthreads();  // also makes the block's global writes visible to the block
+        const int4 ch = chunks[blockIdx.x];
+        for (int u = threadIdx.x >> 5; u < ch.y; u += 8)
+            fill_task(codes, off, meta, tasks[ch.x + u], rc, threadIdx.x & 31, 0, 1, slab);
+    }
 }
 
-// Per task: its longest ref's rows of 32 lane bytes, each 4*code (the null code past a ref's end
-// and past the task's count).
 __global__ void ref_slab_kernel(const uint8_t* __restrict__ codes, const int64_t* __restrict__ off,
                                 const uint32_t* __restrict__ meta, const int4* __restrict__ tasks, int rc,
                                 uint8_t* __restrict__ slab) {
-    const int4 t = tasks[blockIdx.x];
-    const int rows = t.x & 0xFF, l = threadIdx.x & 31;
-    const uint32_t mt = l < t.z ? meta[t.y + l] : 0u;
-    const int n = int(mt >> 16);
-    const uint8_t* src = codes + (l < t.z ? off[int64_t(t.y) / rc * rc + (mt & 0xFFFFu)] : 0);
-    for (int j = threadIdx.x >> 5; j < rows; j += blockDim.x >> 5)
-        slab[int64_t(t.w) + j * 32 + l] = uint8_t((j < n ? int(src[j]) : kNullCode) * 4);
+    fill_task(codes, off, meta, tasks[blockIdx.x], rc, threadIdx.x & 31, threadIdx.x >> 5, blockDim.x >> 5,
+              slab);
 }
 
 // ---------------------------------------------------------------------------- fast kernel ---
@@ -1003,14 +1022,18 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
                 int4* d_plan = rp.d_plan.as<int4>(up.size());
                 h2d(d_plan, up.data(), sizeof(int4) * up.size(), stream);
                 uint32_t* meta = rp.d_meta.as<uint32_t>(size_t(K));
-                chunk_order_kernel<<<unsigned(rp.nchunks), 256, 0, stream>>>(rs.d_len, K, rp.rc, rs.max_len,
-                                                                             meta);
+                uint8_t* slab = rp.d_slab.as<uint8_t>(size_t(rp.slab_bytes) + 16);
+                const int4* tasks = d_plan + rp.nchunks;
+                const bool few = rp.nchunks <= 4;  // beyond, a block per task fills more of the GPU
+                (few ? chunk_order_kernel<true> : chunk_order_kernel<false>)<<<unsigned(rp.nchunks), 256, 0, stream>>>(
+                    rs.d_len, K, rp.rc, rs.max_len, meta, rs.d_bytes, rs.d_off, d_plan, tasks, slab);
                 STB_CUDA(cudaGetLastError());
-                ref_slab_kernel<<<unsigned(rp.ntasks), 128, 0, stream>>>(
-                    rs.d_bytes, rs.d_off, meta, d_plan + rp.nchunks, rp.rc,
-                    rp.d_slab.as<uint8_t>(size_t(rp.slab_bytes) + 16));
-                STB_CUDA(cudaGetLastError());
-                note_launch(nullptr, 2);
+                if (!few) {
+                    ref_slab_kernel<<<unsigned(rp.ntasks), 128, 0, stream>>>(rs.d_bytes, rs.d_off, meta, tasks,
+                                                                             rp.rc, slab);
+                    STB_CUDA(cudaGetLastError());
+                }
+                note_launch(nullptr, few ? 1 : 2);
                 rp.uid = rs.uid;
             }
         }
@@ -1099,7 +1122,7 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
     }
 
     auto* err = reinterpret_cast<unsigned long long*>(ctx.flags_d + 8);
-    STB_CUDA(cudaMemsetAsync(err, 0, 8, stream));
+    if (qs.owns || rs.owns) STB_CUDA(cudaMemsetAsync(err, 0, 8, stream));  // host calls cleared it
 
     FastArgs fa{};
     fa.prof = static_cast<uint32_t*>(qp.d_prof.ptr);
