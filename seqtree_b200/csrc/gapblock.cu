@@ -63,6 +63,7 @@ constexpr int kRow = 32;        // words of one quad in a profile row
 constexpr int kQuads = 4;       // quads per slice
 constexpr int kSliceQ = 4 * kQuads;
 constexpr int kNullCode = 31;   // a residue past a ref's end: its profile column is 0
+constexpr int kMaxSum = 8191;   // largest sum of penalties along a pair that the fast form takes
 constexpr int kMaxSpread = 8;   // lengths of one warp task differ by at most this
 constexpr int kTileW = 2 * kQuads + 1;  // tile words per column: 8 results and the (m, n) term
 static_assert(kWarps == 2 * kQuads, "the dense write-out gives each result word one warp");
@@ -830,7 +831,9 @@ int prior_stride(int W1) { return (W1 + 3 + 4 + 3) & ~3; }
 // Device-side tables of the fast path and the arguments they were built from.
 struct GbTables {
     std::vector<uint8_t> key;
-    DevBuf pen, ftab, prior2;
+    DevBuf buf;
+    const uint32_t* prior2 = nullptr;
+    const int32_t *pen = nullptr, *ftab = nullptr;
 };
 
 GbTables& gb_tables(int device) {
@@ -843,16 +846,18 @@ GbTables& gb_tables(int device) {
 }
 
 // Penalty grid; per-(M,d) prior rows shifted by their minimum (added back through ftab) and
-// clamped at CAP = 2*BIAS + 1 -- a clamped position can never win, because the position holding
-// the row's minimum scores at most BIAS while a clamped one scores above it; a row keeps its first
-// value and the steps between values (0 past the last position; A and B stay at most BIAS + CAP <
-// 2^15, and each packed sum of non-negative halves is exact whatever the step's sign);
+// clamped at CAP = 2 * kMaxSum + 1 -- a clamped position can never win, because the position
+// holding the row's minimum scores at most kMaxSum while a clamped one scores above it; a row keeps
+// its first value and the steps between values (0 past the last position; A and B stay at most
+// kMaxSum + CAP < 2^15, and each packed sum of non-negative halves is exact whatever the step's
+// sign).  Nothing here depends on the sets beyond their longest sequence, so calls with new
+// queries against the same panel keep the tables;
 // ftab[m][n] = prior minimum + gap_open + (d-1)*gap_extend (int32 wrap, as the reference's
 // int32 arithmetic).
 void build_tables(GbTables& tb, const std::vector<int32_t>& pen, int32_t go, int32_t ge, int W,
-                  int32_t bias, const int32_t* prior, int64_t W1p, cudaStream_t stream) {
+                  const int32_t* prior, int64_t W1p, cudaStream_t stream) {
     const int W1 = W + 1;
-    const int32_t cap = 2 * bias + 1;
+    constexpr int32_t cap = 2 * kMaxSum + 1;
     std::vector<int32_t> ftab(size_t(W1) * W1, 0);
     const int pstride = prior_stride(W1);
     std::vector<uint32_t> prior2;
@@ -880,11 +885,16 @@ void build_tables(GbTables& tb, const std::vector<int32_t>& pen, int32_t go, int
             ftab[size_t(m) * W1 + n] = int32_t(uint32_t(pmin) + uint32_t(go) +
                                                uint32_t(d - 1) * uint32_t(ge));
         }
-    h2d(tb.pen.as<int32_t>(pen.size()), pen.data(), pen.size() * 4, stream);
-    h2d(tb.ftab.as<int32_t>(ftab.size()), ftab.data(), ftab.size() * 4, stream);
-    if (prior)
-        h2d(tb.prior2.as<uint32_t>(prior2.size()), prior2.data(),
-                                 prior2.size() * 4, stream);
+    // one upload: prior steps (16-byte rows), penalties, terms
+    std::vector<uint32_t> up(std::move(prior2));
+    const size_t pen_at = up.size(), ftab_at = pen_at + pen.size();
+    up.insert(up.end(), pen.begin(), pen.end());
+    up.insert(up.end(), ftab.begin(), ftab.end());
+    uint32_t* d = tb.buf.as<uint32_t>(up.size());
+    h2d(d, up.data(), up.size() * 4, stream);
+    tb.prior2 = d;
+    tb.pen = reinterpret_cast<int32_t*>(d + pen_at);
+    tb.ftab = reinterpret_cast<int32_t*>(d + ftab_at);
 }
 
 // CTAs per SM the fast kernel's registers allow (256 threads of 80 registers, 64 in the sparse form).
@@ -923,7 +933,7 @@ bool fast_form_possible(const st_seqset_s& qs, const st_seqset_s& rs, const int3
             maxpen = std::max(maxpen, v);
         }
     const int32_t longest = std::max(qs.max_len, rs.max_len);
-    return longest <= 64 && int64_t(std::min(qs.max_len, rs.max_len)) * maxpen <= 8191;
+    return longest <= 64 && int64_t(std::min(qs.max_len, rs.max_len)) * maxpen <= kMaxSum;
 }
 
 std::string gb_shape_key(const st_seqset_s& qs, const st_seqset_s& rs, bool has_prior) {
@@ -970,7 +980,7 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
     }
     const int32_t Lmax = std::min(qs.max_len, rs.max_len);
     const int64_t lmaxpen = int64_t(Lmax) * maxpen;
-    bool fast = nonneg && longest <= 64 && lmaxpen <= 8191;
+    bool fast = nonneg && longest <= 64 && lmaxpen <= kMaxSum;
 
     const int W = longest, W1 = W + 1;
     const bool wide = maxpen > 255;  // the penalties of four queries do not fit one word
@@ -1070,24 +1080,26 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
     // Tables for this (matrix, gaps, prior, lengths): rebuilt only when they change, so repeated
     // calls with the same arguments enqueue nothing but the kernel.
     GbTables& tb = gb_tables(ctx.device);
-    const int32_t bias = int32_t(std::max<int64_t>(lmaxpen, 1));
     {
-        std::vector<uint8_t> key;
-        auto put = [&key](const void* p, size_t n) {
-            const auto* b = static_cast<const uint8_t*>(p);
-            key.insert(key.end(), b, b + n);
-        };
-        const int64_t hdr[8] = {A, go, ge, W, bias, int64_t(prior_width), has_prior, 0};
-        put(hdr, sizeof hdr);
-        put(pen.data(), pen.size() * 4);
-        if (has_prior) put(prior, size_t(prior_len) * 4);
+        const int64_t hdr[8] = {A, go, ge, W, int64_t(prior_width), has_prior, 0, 0};
+        const struct {
+            const void* p;
+            size_t n;
+        } parts[3] = {{hdr, sizeof hdr}, {pen.data(), pen.size() * 4},
+                      {prior, has_prior ? size_t(prior_len) * 4 : 0}};
         Phase ph("tables");
-        if (!same_as_last(tb.key, key.data(), key.size())) {
-            try {
-                build_tables(tb, pen, go, ge, W, bias, has_prior ? prior : nullptr, W1p, stream);
-            } catch (...) {
-                tb.key.clear();  // not uploaded: the next call builds them again
-                throw;
+        bool same = tb.key.size() == parts[0].n + parts[1].n + parts[2].n;
+        size_t at = 0;
+        for (const auto& part : parts) {
+            same = same && (part.n == 0 || std::memcmp(tb.key.data() + at, part.p, part.n) == 0);
+            at += part.n;
+        }
+        if (!same) {
+            tb.key.clear();  // set again once everything is uploaded
+            build_tables(tb, pen, go, ge, W, has_prior ? prior : nullptr, W1p, stream);
+            for (const auto& part : parts) {
+                const auto* bytes = static_cast<const uint8_t*>(part.p);
+                if (part.n) tb.key.insert(tb.key.end(), bytes, bytes + part.n);
             }
         }
     }
@@ -1113,7 +1125,7 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
             const int4* slices = quads + qp.quads.size();
             auto fill = wide ? profile_kernel<true> : profile_kernel<false>;
             fill<<<unsigned(qp.slices.size()), 256, 0, stream>>>(
-                qs.d_bytes, qs.d_off, quads, slices, static_cast<int32_t*>(tb.pen.ptr), A,
+                qs.d_bytes, qs.d_off, quads, slices, tb.pen, A,
                 uint32_t(maxpen), prof);
             STB_CUDA(cudaGetLastError());
             note_launch(nullptr);
@@ -1139,8 +1151,8 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
     fa.sm = sm;
     fa.score16 = sink && sink->thresh > 255;
     fa.spread = rp.max_spread;
-    fa.prior2 = has_prior ? static_cast<uint32_t*>(tb.prior2.ptr) : nullptr;
-    fa.ftab = static_cast<int32_t*>(tb.ftab.ptr);
+    fa.prior2 = has_prior ? tb.prior2 : nullptr;
+    fa.ftab = tb.ftab;
     fa.W1 = W1;
     fa.pstride = prior_stride(W1);
     fa.out = out_d;
