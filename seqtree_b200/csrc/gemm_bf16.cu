@@ -7,7 +7,8 @@
 // 128-byte swizzle), zero outside the matrix.  Packing absorbs the transposes (op(A) is A or
 // A^T, the same for B), so the GEMM kernel only ever sees "rows x K" tiles.  One CTA computes
 // one 128 x 128 output tile over a range of K chunks: warp 0 bulk-copies A and B chunks through a
-// 3-stage shared-memory ring, one thread of warp 1 issues M=128 N=128 K=16 tcgen05.mma into a
+// 2-stage shared-memory ring (64 KB, so that three CTAs share an SM and one's epilogue overlaps
+// another's loads: the layers are thin), one thread of warp 1 issues M=128 N=128 K=16 tcgen05.mma into a
 // 128-column TMEM accumulator, and warps 2-5 (one TMEM lane quarter each) stage the tile in
 // shared memory, from where all six warps store, add or atomically add (split K) it into C with
 // coalesced writes.
@@ -18,6 +19,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "gemm_bf16.cuh"
 #include "tc.cuh"
 
 namespace stb {
@@ -26,17 +28,64 @@ namespace {
 
 constexpr int kGT = 128;                 // tile rows (M) and columns (N)
 constexpr int kGK = 64;                  // K per chunk: one 128-byte swizzled row
-constexpr int kGStages = 3;
+constexpr int kGStages = 2;
 constexpr int kGThreads = 192;
 constexpr int kBlockB = kGT * kGK * 2;   // 16 KB
 constexpr int kGSmBar = kGStages * 2 * kBlockB;
 constexpr size_t kGSmem = size_t(kGSmBar) + 128 + 1024;
 
-// Packed operand: op[(tile * kchunks + chunk)][row][unit], value(i, k) = X[i * ld + k] (rows of
-// X are the operand's rows).  One thread per 16-byte output unit, in output order: a warp reads
-// four 256-byte row pieces and writes 512 contiguous bytes.
-__global__ void pack_rows_kernel(const float* __restrict__ X, int ld, int rows, int K, int kchunks,
-                                 int64_t units, uint8_t* __restrict__ op) {
+// One value of an operand's matrix, (row r, column c); callers check the ranges.
+template <int KIND>
+__device__ __forceinline__ float src_value(const PackSrc& s, int64_t r, int c) {
+    if constexpr (KIND == PackSrc::kConv) {
+        const int t = int(r & 31) + (c >> 7) - 1, L = s.lens[r >> 5];
+        return (int(r & 31) < L && t >= 0 && t < L) ? s.x[(r + (c >> 7) - 1) * s.ld + (c & 127)] : 0.f;
+    }
+    const int64_t at = r * s.ld + c;
+    if constexpr (KIND == PackSrc::kRelu) return s.y[at] > 0.f ? s.x[at] : 0.f;
+    return s.x[at];
+}
+
+// Eight consecutive values (row r, columns c..c+7, c a multiple of 8) as two 16-byte loads.
+template <int KIND>
+__device__ __forceinline__ void src_eight(const PackSrc& s, int64_t r, int c, float (&v)[8]) {
+    int64_t at = r * s.ld + c;
+    if constexpr (KIND == PackSrc::kConv) {
+        const int t = int(r & 31) + (c >> 7) - 1, L = s.lens[r >> 5];
+        if (int(r & 31) >= L || t < 0 || t >= L) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = 0.f;
+            return;
+        }
+        at = (r + (c >> 7) - 1) * s.ld + (c & 127);
+    }
+    const float4 a = *reinterpret_cast<const float4*>(s.x + at), b = *reinterpret_cast<const float4*>(s.x + at + 4);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+    if constexpr (KIND == PackSrc::kRelu) {
+        const float4 p = *reinterpret_cast<const float4*>(s.y + at), q = *reinterpret_cast<const float4*>(s.y + at + 4);
+        const float y[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = y[e] > 0.f ? v[e] : 0.f;
+    }
+}
+
+__device__ __forceinline__ uint4 bf16_unit(const float (&v)[8]) {
+    union {
+        uint4 q;
+        __nv_bfloat162 h[4];
+    } pk;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) pk.h[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+    return pk.q;
+}
+
+// Packed operand: op[(tile * kchunks + chunk)][row][unit], value(i, k) = matrix(i, k) (rows of the
+// matrix are the operand's rows).  One thread per 16-byte output unit, in output order: a warp
+// reads four 256-byte row pieces and writes 512 contiguous bytes.  VEC: 16-byte loads (base and leading
+// dimension aligned, K a multiple of 8).
+template <int KIND, bool VEC>
+__global__ void pack_rows_kernel(const PackSrc s, int rows, int K, int kchunks, int64_t units,
+                                 uint8_t* __restrict__ op) {
     const int64_t pos = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (pos >= units) return;
     const int pu = int(pos & 7);
@@ -47,44 +96,48 @@ __global__ void pack_rows_kernel(const float* __restrict__ X, int ld, int rows, 
     const int64_t i = (blk / kchunks) * kGT + row;
     const int k0 = chunk * kGK + (pu ^ (row & 7)) * 8;
     float v[8];
+    if (VEC && i < rows && k0 < K) {
+        src_eight<KIND>(s, i, k0, v);
+    } else {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = (i < rows && k0 + e < K) ? X[i * ld + k0 + e] : 0.f;
-    union {
-        uint4 q;
-        __nv_bfloat162 h[4];
-    } pk;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) pk.h[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
-    *reinterpret_cast<uint4*>(op + pos * 16) = pk.q;
+        for (int e = 0; e < 8; ++e) v[e] = (!VEC && i < rows && k0 + e < K) ? src_value<KIND>(s, i, k0 + e) : 0.f;
+    }
+    *reinterpret_cast<uint4*>(op + pos * 16) = bf16_unit(v);
 }
 
-// The same packed operand from the transpose: value(i, k) = X[k * ld + i].  One 256-thread
-// block per (tile, chunk) block: it reads the 64 x 128 fp32 piece of X row by row (coalesced)
-// into shared memory and writes the 16 KB block in output order.
-__global__ void __launch_bounds__(256) pack_cols_kernel(const float* __restrict__ X, int ld, int rows,
-                                                        int K, int kchunks,
+// The same packed operand from the transpose: value(i, k) = matrix(k, i).  One 256-thread
+// block per (tile, chunk) block: it reads the 64 x 128 fp32 piece row by row (coalesced)
+// into shared memory and writes the 16 KB block in output order; with colsum it adds the piece's
+// column sums first.
+template <int KIND>
+__global__ void __launch_bounds__(256) pack_cols_kernel(const PackSrc s, int rows, int K, int kchunks,
                                                         uint8_t* __restrict__ op) {
     __shared__ float t[kGK][kGT + 1];
     const int chunk = int(blockIdx.x % unsigned(kchunks));
     const int64_t i0 = int64_t(blockIdx.x / unsigned(kchunks)) * kGT;
     const int k0 = chunk * kGK;
+#pragma unroll 8
     for (int idx = threadIdx.x; idx < kGK * kGT; idx += 256) {
         const int kk = idx >> 7, ii = idx & 127;
         const int64_t i = i0 + ii;
-        t[kk][ii] = (i < rows && k0 + kk < K) ? X[int64_t(k0 + kk) * ld + i] : 0.f;
+        t[kk][ii] = (i < rows && k0 + kk < K) ? src_value<KIND>(s, k0 + kk, int(i)) : 0.f;
     }
     __syncthreads();
     uint8_t* dst = op + int64_t(blockIdx.x) * kBlockB;
+#pragma unroll
     for (int pos = threadIdx.x; pos < kGT * 8; pos += 256) {
         const int row = pos >> 3, u = (pos & 7) ^ (row & 7);
-        union {
-            uint4 q;
-            __nv_bfloat162 h[4];
-        } pk;
+        float v[8];
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-            pk.h[e] = __floats2bfloat162_rn(t[u * 8 + 2 * e][row], t[u * 8 + 2 * e + 1][row]);
-        *reinterpret_cast<uint4*>(dst + pos * 16) = pk.q;
+        for (int e = 0; e < 8; ++e) v[e] = t[u * 8 + e][row];
+        *reinterpret_cast<uint4*>(dst + pos * 16) = bf16_unit(v);
+    }
+    if (s.colsum) {  // two threads per column, 32 rows each
+        const int ii = threadIdx.x & 127, h = threadIdx.x >> 7;
+        float sum = 0.f;
+#pragma unroll 8
+        for (int kk = 0; kk < kGK / 2; ++kk) sum += t[h * (kGK / 2) + kk][ii];
+        if (i0 + ii < rows) atomicAdd(s.colsum + i0 + ii, sum);
     }
 }
 
@@ -95,13 +148,14 @@ struct GemmBf16Args {
     float* C;
     int ldc, M, N;
     int mode;           // 0 store, 1 add, 2 atomic add
+    GemmEpi epi;        // (mode 0 or 1)
     unsigned long long* err;
 };
 
 __global__ void __launch_bounds__(kGThreads) gemm_bf16_kernel(GemmBf16Args g) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((uintptr_t(smem_raw) + 1023) & ~uintptr_t(1023));
-    // barriers: 0-2 full, 3-5 empty, 6 accumulator ready, 7 MMA drain
+    // barriers: 0-1 full, 2-3 empty, 6 accumulator ready, 7 MMA drain
     const uint32_t bar0 = smem_u32(smem + kGSmBar);
     auto BAR = [&](int i) { return bar0 + 8u * uint32_t(i); };
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + kGSmBar + 64);
@@ -212,50 +266,81 @@ __global__ void __launch_bounds__(kGThreads) gemm_bf16_kernel(GemmBf16Args g) {
                 x[b][q] = r < kGT ? stage[r * kGT + (((c >> 2) ^ (r & 7)) << 2) + (c & 3)] : 0.f;
             }
         }
-        if (g.mode == 1) {
-            float y[4][4];
+        const GemmEpi& ep = g.epi;
+        const float* addend = ep.kind == GemmEpi::kResidual || ep.kind == GemmEpi::kConv ? ep.res
+                              : g.mode == 1                                              ? g.C
+                                                                                         : nullptr;
+        float y[4][4];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const int r = r0 + b * kWarps, row = tm * kGT + r;
+        for (int b = 0; b < 4; ++b) {
+            const int r = r0 + b * kWarps, row = tm * kGT + r;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int col = tn * kGT + lane + 32 * q;
-                    y[b][q] = (r < kGT && row < g.M && col < g.N) ? g.C[int64_t(row) * g.ldc + col] : 0.f;
-                }
+            for (int q = 0; q < 4; ++q) {
+                const int col = tn * kGT + lane + 32 * q;
+                y[b][q] = (addend && r < kGT && row < g.M && col < g.N) ? addend[int64_t(row) * g.ldc + col] : 0.f;
             }
+        }
+        float bias[4];
 #pragma unroll
-            for (int b = 0; b < 4; ++b)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) x[b][q] += y[b][q];
+        for (int q = 0; q < 4; ++q) {
+            const int col = tn * kGT + lane + 32 * q;
+            bias[q] = ep.bias && col < g.N ? ep.bias[col] : 0.f;
         }
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             const int r = r0 + b * kWarps, row = tm * kGT + r;
             if (r >= kGT || row >= g.M) continue;
+            const bool valid = !ep.lens || (row & 31) < ep.lens[row >> 5];
             float* crow = g.C + int64_t(row) * g.ldc;
+            float* orow = ep.out + int64_t(row) * g.ldc;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int col = tn * kGT + lane + 32 * q;
-                if (col < g.N) {
-                    if (g.mode == 2) atomicAdd(crow + col, x[b][q]);
-                    else crow[col] = x[b][q];
+                if (col >= g.N) continue;
+                // (the sums in the order of the separate passes they replace)
+                switch (ep.kind) {
+                    case GemmEpi::kBias: crow[col] = x[b][q] + bias[q]; break;
+                    case GemmEpi::kResidual: orow[col] = valid ? y[b][q] + x[b][q] + bias[q] : 0.f; break;
+                    case GemmEpi::kConv: {
+                        const float p = x[b][q] + bias[q];
+                        crow[col] = p;
+                        orow[col] = valid ? y[b][q] + fmaxf(p, 0.f) : 0.f;
+                        break;
+                    }
+                    case GemmEpi::kMaskAdd: crow[col] = valid ? x[b][q] + y[b][q] : 0.f; break;
+                    default:
+                        if (g.mode == 2) atomicAdd(crow + col, x[b][q]);
+                        else crow[col] = g.mode == 1 ? x[b][q] + y[b][q] : x[b][q];
                 }
             }
         }
     }
 }
 
-void pack(const float* X, int ld, bool trans, int rows, int K, DevBuf& buf, cudaStream_t st,
-          int& tiles, int& kchunks) {
+template <int KIND>
+void launch_pack(const PackSrc& s, bool trans, int rows, int K, int tiles, int kchunks, uint8_t* op,
+                 cudaStream_t st) {
+    const int64_t units = int64_t(tiles) * kchunks * kGT * 8;
+    if (trans) {
+        pack_cols_kernel<KIND><<<unsigned(tiles * kchunks), 256, 0, st>>>(s, rows, K, kchunks, op);
+        return;
+    }
+    const uintptr_t bases = uintptr_t(s.x) | uintptr_t(s.y);
+    const bool vec = (bases & 15) == 0 && s.ld % 4 == 0 && K % 8 == 0;
+    (vec ? pack_rows_kernel<KIND, true> : pack_rows_kernel<KIND, false>)<<<unsigned(ceil_div(units, 256)), 256, 0, st>>>(
+        s, rows, K, kchunks, units, op);
+}
+
+void pack(const PackSrc& s, bool trans, int rows, int K, DevBuf& buf, cudaStream_t st, int& tiles,
+          int& kchunks) {
     tiles = int(ceil_div(rows, kGT));
     kchunks = int(ceil_div(K, kGK));
-    const int64_t units = int64_t(tiles) * kchunks * kGT * 8;
-    uint8_t* op = buf.as<uint8_t>(size_t(units) * 16);
-    if (trans)
-        pack_cols_kernel<<<unsigned(tiles * kchunks), 256, 0, st>>>(X, ld, rows, K, kchunks, op);
-    else
-        pack_rows_kernel<<<unsigned(ceil_div(units, 256)), 256, 0, st>>>(X, ld, rows, K, kchunks,
-                                                                         units, op);
+    uint8_t* op = buf.as<uint8_t>(size_t(tiles) * kchunks * kBlockB);
+    switch (s.kind) {
+        case PackSrc::kConv: launch_pack<PackSrc::kConv>(s, trans, rows, K, tiles, kchunks, op, st); break;
+        case PackSrc::kRelu: launch_pack<PackSrc::kRelu>(s, trans, rows, K, tiles, kchunks, op, st); break;
+        default: launch_pack<PackSrc::kPlain>(s, trans, rows, K, tiles, kchunks, op, st);
+    }
     STB_CUDA(cudaGetLastError());
 }
 
@@ -265,8 +350,9 @@ void pack(const float* X, int ld, bool trans, int rows, int K, DevBuf& buf, cuda
 // [K x M]), op(B) is [K x N] (B^T when tb, B being [N x K]); row-major with leading dimensions.
 // Products with a long K and few output tiles are split over K and added atomically, in which
 // case C must already hold the value to add to (it is cleared first when !accumulate).
-void gemm_bf16(bool ta, bool tb, int M, int N, int K, const float* A, int lda, const float* B,
-               int ldb, float* C, int ldc, bool accumulate, cudaStream_t st, int sms) {
+// An epilogue other than kNone takes the product unsplit.
+void gemm_bf16(bool ta, bool tb, int M, int N, int K, const PackSrc& A, const PackSrc& B, float* C, int ldc,
+               bool accumulate, const GemmEpi& epi, cudaStream_t st, int sms) {
     if (M <= 0 || N <= 0) return;
     if (K <= 0) {
         if (!accumulate)
@@ -278,11 +364,12 @@ void gemm_bf16(bool ta, bool tb, int M, int N, int K, const float* A, int lda, c
     ensure_smem_limit(reinterpret_cast<const void*>(gemm_bf16_kernel), kGSmem);
     int mtiles, ntiles, kchunks, kb;
     // op(A)[i][k] = ta ? A[k][i] : A[i][k];  op(B)^T[n][k] = tb ? B[n][k] : B[k][n]
-    pack(A, lda, ta, M, K, ctx.gemm_a, st, mtiles, kchunks);
-    pack(B, ldb, !tb, N, K, ctx.gemm_b, st, ntiles, kb);
+    pack(A, ta, M, K, ctx.gemm_a, st, mtiles, kchunks);
+    pack(B, !tb, N, K, ctx.gemm_b, st, ntiles, kb);
     const int tiles = mtiles * ntiles;
     int splits = 1;
-    if (tiles < sms && kchunks >= 16) splits = std::min(int(ceil_div(2 * sms, tiles)), kchunks / 4);
+    if (epi.kind == GemmEpi::kNone && tiles < sms && kchunks >= 16)
+        splits = std::min(int(ceil_div(2 * sms, tiles)), kchunks / 4);
     const int cps = int(ceil_div(kchunks, splits));
     splits = int(ceil_div(kchunks, cps));
     const int mode = splits > 1 ? 2 : (accumulate ? 1 : 0);
@@ -298,11 +385,22 @@ void gemm_bf16(bool ta, bool tb, int M, int N, int K, const float* A, int lda, c
     g.M = M;
     g.N = N;
     g.mode = mode;
+    g.epi = epi;
     g.err = reinterpret_cast<unsigned long long*>(ctx.flags_d + 8);
     gemm_bf16_kernel<<<dim3(unsigned(ntiles), unsigned(mtiles), unsigned(splits)), kGThreads, kGSmem,
                        st>>>(g);
     STB_CUDA(cudaGetLastError());
     note_launch("gemm_bf16_kernel", 3);
+}
+
+void gemm_bf16(bool ta, bool tb, int M, int N, int K, const float* A, int lda, const float* B, int ldb,
+               float* C, int ldc, bool accumulate, cudaStream_t st, int sms) {
+    PackSrc a{}, b{};
+    a.x = A;
+    a.ld = lda;
+    b.x = B;
+    b.ld = ldb;
+    gemm_bf16(ta, tb, M, N, K, a, b, C, ldc, accumulate, GemmEpi{}, st, sms);
 }
 
 }  // namespace stb

@@ -1,0 +1,46 @@
+// The encoder's training GEMM with what surrounds each product folded into it: how an operand's
+// values are formed while it is packed, and what happens to a result before it is stored.  The layers
+// are bound by memory; folding the im2col gather, the ReLU gradient, the biases, the residuals, the
+// masks and the bias gradients took their passes over 67 to 201 MB out of a 2,048-pair step: 3.57 ->
+// 2.77 ms with the attention kernels' wider reads (B200; sums keep the separate passes' order except
+// the bias gradients').
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+namespace stb {
+
+// Values of a row-major fp32 operand, formed as they are packed to bf16.
+struct PackSrc {
+    enum Kind { kPlain, kConv, kRelu };
+    const float* x = nullptr;
+    int ld = 0;
+    int kind = kPlain;
+    // kConv: x holds rows of 128 columns; value (r, c) of the 384-column im2col matrix is row r - 1, r or
+    // r + 1 (c / 128) of x inside the 32-row sequence's first lens[r / 32] rows, 0 outside.
+    const int32_t* lens = nullptr;
+    // kRelu: x where y > 0 (y as x), else 0.
+    const float* y = nullptr;
+    // When set: the column sums of the matrix are added to it (only where the operand is packed
+    // from its transpose, i.e. the matrix' rows run along K).
+    float* colsum = nullptr;
+};
+
+// What becomes of the product before it is stored.  Rows are positions of 32-row sequences; kinds
+// with lens give 0 past a sequence's end.
+struct GemmEpi {
+    enum Kind { kNone, kBias, kResidual, kConv, kMaskAdd };
+    int kind = kNone;
+    const float* bias = nullptr;   // kBias, kResidual, kConv: per column
+    const float* res = nullptr;    // kResidual, kConv: added, laid out as C
+    float* out = nullptr;          // kResidual: res + C + bias here and C untouched;
+                                   // kConv: C + bias to C, res + relu(C + bias) here
+    const int32_t* lens = nullptr; // kResidual, kConv, kMaskAdd (C += product, 0 past the end)
+};
+
+void gemm_bf16(bool ta, bool tb, int M, int N, int K, const PackSrc& A, const PackSrc& B, float* C, int ldc,
+               bool accumulate, const GemmEpi& epi, cudaStream_t st, int sms);
+
+}  // namespace stb
