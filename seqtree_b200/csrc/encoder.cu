@@ -1002,7 +1002,7 @@ float encoder_train_step(Encoder& m, const uint8_t* codes, const int32_t* lens, 
 }
 
 void encoder_embed_bf16(const float* prm, int64_t version, std::shared_ptr<void>& state,
-                        const st_seqset_s& set, void* out, int layout, cudaStream_t st);
+                        const st_seqset_s& set, __nv_bfloat16* out, cudaStream_t st);
 
 // Embeddings of every sequence of a device set (amino-acid codes, lengths 1..32) into `out`.
 void encoder_embed(Encoder& m, const st_seqset_s& set, void* out, int layout, cudaStream_t st) {
@@ -1011,7 +1011,7 @@ void encoder_embed(Encoder& m, const st_seqset_s& set, void* out, int layout, cu
     for (int32_t L : set.h_len)
         if (L < 1 || L > kP) fail(ST_EINVAL, "seqtree_b200: encoder inputs must have 1..32 residues");
     if (layout == 1) {
-        encoder_embed_bf16(P(m), m.step, m.bf16, set, out, layout, st);
+        encoder_embed_bf16(P(m), m.step, m.bf16, set, static_cast<__nv_bfloat16*>(out), st);
         return;
     }
     Context& ctx = context();

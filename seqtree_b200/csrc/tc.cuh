@@ -26,16 +26,26 @@ __device__ __forceinline__ bool bar_test(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// As bar_test, but returns at once.
+__device__ __forceinline__ bool bar_poll(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // Bounded wait for the phase of `parity` to complete.  Gives up (returns false) when the CTA's
 // abort word is set or after kWaitNs, setting the abort word and the host-visible error word.
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* abort,
                                          unsigned long long* err) {
-    if (bar_test(bar, parity)) return true;
-    const uint64_t t0 = now_ns();
+    uint64_t t0 = 0;  // the clock is read only in waits that last
     for (uint32_t it = 1;; ++it) {
         if (bar_test(bar, parity)) return true;
         if ((it & 255) == 0) {
             if (*abort) return false;
+            if (t0 == 0) t0 = now_ns();
             if (now_ns() - t0 > kWaitNs) {
                 *abort = 1;
                 atomicExch(err, 1ull);
@@ -48,13 +58,15 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile
 // sees it complete, so a group of warps waiting on one phase either all pass or all time out
 // (after kWaitNs) -- none is left behind at a later rendezvous.
 __device__ __forceinline__ bool bar_wait_own(uint32_t bar, uint32_t parity, unsigned long long* err) {
-    if (bar_test(bar, parity)) return true;
-    const uint64_t t0 = now_ns();
+    uint64_t t0 = 0;
     for (uint32_t it = 1;; ++it) {
         if (bar_test(bar, parity)) return true;
-        if ((it & 255) == 0 && now_ns() - t0 > kWaitNs) {
-            atomicExch(err, 1ull);
-            return false;
+        if ((it & 255) == 0) {
+            if (t0 == 0) t0 = now_ns();
+            if (now_ns() - t0 > kWaitNs) {
+                atomicExch(err, 1ull);
+                return false;
+            }
         }
     }
 }
@@ -148,6 +160,43 @@ __device__ __forceinline__ void tmem_ld32_wait(uint32_t (&v)[32]) {
                    "+r"(v[30]), "+r"(v[31])
                  :
                  : "memory");
+}
+__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+        "%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+          "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+          "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld4_issue(uint32_t taddr, uint32_t (&v)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld4_wait(uint32_t (&v)[4]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3])
+                 :
+                 : "memory");
+}
+// One column of the warp's 32 lanes.
+__device__ __forceinline__ void tmem_st1(uint32_t taddr, uint32_t v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(v) : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ld16_wait(uint32_t (&v)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]),
+                   "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]),
+                   "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
+                 :
+                 : "memory");
+}
+// Asks for a later bulk load's bytes in L2 (16-byte aligned, a multiple of 16 bytes).
+__device__ __forceinline__ void bulk_prefetch(const void* src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t bytes) {
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src),
