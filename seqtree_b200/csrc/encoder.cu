@@ -702,16 +702,25 @@ struct Encoder {
         e, z, nrm;
     // backward
     DevBuf dz, de, dpool, dh, dO, dqkv, dx2, dpre;
+    // bf16 operands of the training products, each packed once for its two products (x2, h and o from
+    // forward to backward), in one block of which a unit is R x 128 values
+    DevBuf packed;
+    enum Slot { kX2 = 0, kH = 3, kO = 5, kDh = 7, kDqkv = 8, kSlots = 11 };
+    uint8_t* slot(int which, int S) {
+        return static_cast<uint8_t*>(packed.ptr) + size_t(which) * packed_bytes(int64_t(S) * kP, kW);
+    }
 
-    void reserve(int S) {
-        if (S <= S_cap) return;
+    void reserve(int S, bool bf) {  // bf: as the passes over S sequences that follow
         const size_t R = size_t(S) * kP;
+        if (bf) packed.as<uint8_t>(kSlots * packed_bytes(int64_t(R), kW));
+        else x2.as<float>(R * 3 * kW);
+        if (S <= S_cap) return;
         codes.as<uint8_t>(R);
         lens.as<int32_t>(size_t(S));
         scores.as<int32_t>(size_t(S));
         for (DevBuf* b : {&pre1, &h1, &pre2, &hA, &hB, &hC, &o0, &o1, &y, &dh, &dO, &dpre})
             b->as<float>(R * kW);
-        for (DevBuf* b : {&x2, &qkv0, &qkv1, &dqkv, &dx2}) b->as<float>(R * 3 * kW);
+        for (DevBuf* b : {&qkv0, &qkv1, &dqkv, &dx2}) b->as<float>(R * 3 * kW);
         a0.as<float>(size_t(S) * kP * kP);
         a1.as<float>(size_t(S) * kP * kP);
         for (DevBuf* b : {&pool, &dpool}) b->as<float>(size_t(S) * kW);
@@ -770,8 +779,8 @@ void forward(Encoder& m, int S, cudaStream_t st, int sms, bool bf) {
         epi.res = F(m.h1);
         epi.out = F(m.hA);
         epi.lens = lens;
-        gemm_bf16(false, false, int(R), kW, 3 * kW, conv_rows(m), plain(prm + oW2, kW), F(m.pre2), kW, false,
-                  epi, st, sms);
+        gemm_packed(pack_matrix(conv_rows(m), int(R), 3 * kW, m.slot(m.kX2, S), st), false, kW, plain(prm + oW2, kW),
+                    F(m.pre2), kW, false, epi, st, sms);
     } else {
         im2col_kernel<<<R / kRowsPerCta, dim3(kW, kRowsPerCta), 0, st>>>(F(m.h1), lens, F(m.x2));
         sgemm<false, false>(int(R), kW, 3 * kW, F(m.x2), 3 * kW, prm + oW2, kW, F(m.pre2), kW, false, st, sms);
@@ -789,8 +798,8 @@ void forward(Encoder& m, int S, cudaStream_t st, int sms, bool bf) {
             GemmEpi epi{};
             epi.kind = GemmEpi::kBias;
             epi.bias = L + lbqkv;
-            gemm_bf16(false, false, int(R), 3 * kW, kW, plain(hin[l], kW), plain(L + lWqkv, 3 * kW), qkv[l],
-                      3 * kW, false, epi, st, sms);
+            gemm_packed(pack_matrix(plain(hin[l], kW), int(R), kW, m.slot(m.kH + l, S), st), false, 3 * kW,
+                        plain(L + lWqkv, 3 * kW), qkv[l], 3 * kW, false, epi, st, sms);
         } else {
             sgemm<false, false>(int(R), 3 * kW, kW, hin[l], kW, L + lWqkv, 3 * kW, qkv[l], 3 * kW, false, st, sms);
             add_bias_kernel<<<R / kRowsPerCta, dim3(128, kRowsPerCta), 0, st>>>(qkv[l], L + lbqkv, 3 * kW);
@@ -803,8 +812,8 @@ void forward(Encoder& m, int S, cudaStream_t st, int sms, bool bf) {
             epi.res = hin[l];
             epi.out = hout[l];
             epi.lens = lens;
-            gemm_bf16(false, false, int(R), kW, kW, plain(ob[l], kW), plain(L + lWo, kW), F(m.y), kW, false, epi,
-                      st, sms);
+            gemm_packed(pack_matrix(plain(ob[l], kW), int(R), kW, m.slot(m.kO + l, S), st), false, kW, plain(L + lWo, kW),
+                        F(m.y), kW, false, epi, st, sms);
         } else {
             sgemm<false, false>(int(R), kW, kW, ob[l], kW, L + lWo, kW, F(m.y), kW, false, st, sms);
             residual_kernel<<<R / kRowsPerCta, dim3(kW, kRowsPerCta), 0, st>>>(hin[l], F(m.y), L + lbo, lens,
@@ -845,22 +854,23 @@ void loss_backward(Encoder& m, int S, cudaStream_t st, int sms, bool bf) {
         float* G = g + oL0 + l * kLayer;
         // h_next = (h + o Wo + bo) * mask; dh is already masked.  dh_prev = (dh + dqkv Wqkv^T) * mask.
         if (bf) {  // the bias gradients are summed while dh and dqkv are packed
-            gemm_bf16(true, false, kW, kW, int(R), plain(ob[l], kW), plain(F(m.dh), kW, G + lbo), G + lWo, kW,
-                      true, GemmEpi{}, st, sms);
+            const Packed dh = pack_matrix(plain(F(m.dh), kW, G + lbo), int(R), kW, m.slot(m.kDh, S), st);
+            gemm_packed_tn(Packed{m.slot(m.kO + l, S), int(R), kW}, dh, G + lWo, kW, st, sms);
+            gemm_packed(dh, true, kW, plain(L + lWo, kW), F(m.dO), kW, false, GemmEpi{}, st, sms);
         } else {
             sgemm<true, false>(kW, kW, int(R), ob[l], kW, F(m.dh), kW, G + lWo, kW, true, st, sms);
             colsum(F(m.dh), R, kW, G + lbo, st);
+            sgemm<false, true>(int(R), kW, kW, F(m.dh), kW, L + lWo, kW, F(m.dO), kW, false, st, sms);
         }
-        mm<false, true>(bf, int(R), kW, kW, F(m.dh), kW, L + lWo, kW, F(m.dO), kW, false, st, sms);
         attn_bwd_kernel<<<unsigned(S), 256, attn_bwd_smem(), st>>>(qkv[l], att[l], F(m.dO), lens, F(m.dqkv));
         if (bf) {
-            gemm_bf16(true, false, kW, 3 * kW, int(R), plain(hin[l], kW), plain(F(m.dqkv), 3 * kW, G + lbqkv),
-                      G + lWqkv, 3 * kW, true, GemmEpi{}, st, sms);
+            const Packed dqkv = pack_matrix(plain(F(m.dqkv), 3 * kW, G + lbqkv), int(R), 3 * kW,
+                                            m.slot(m.kDqkv, S), st);
+            gemm_packed_tn(Packed{m.slot(m.kH + l, S), int(R), kW}, dqkv, G + lWqkv, 3 * kW, st, sms);
             GemmEpi epi{};
             epi.kind = GemmEpi::kMaskAdd;
             epi.lens = lens;
-            gemm_bf16(false, true, int(R), kW, 3 * kW, plain(F(m.dqkv), 3 * kW), plain(L + lWqkv, 3 * kW),
-                      F(m.dh), kW, true, epi, st, sms);
+            gemm_packed(dqkv, true, kW, plain(L + lWqkv, 3 * kW), F(m.dh), kW, true, epi, st, sms);
         } else {
             sgemm<true, false>(kW, 3 * kW, int(R), hin[l], kW, F(m.dqkv), 3 * kW, G + lWqkv, 3 * kW, true, st,
                                sms);
@@ -872,10 +882,9 @@ void loss_backward(Encoder& m, int S, cudaStream_t st, int sms, bool bf) {
     }
     // hA = (h1 + relu(pre2)) * mask
     if (bf) {
-        gemm_bf16(true, false, 3 * kW, kW, int(R), conv_rows(m), relu_grad(m, g + ob2), g + oW2, kW, true,
-                  GemmEpi{}, st, sms);
-        gemm_bf16(false, true, int(R), 3 * kW, kW, relu_grad(m), plain(prm + oW2, kW), F(m.dx2), 3 * kW, false,
-                  GemmEpi{}, st, sms);
+        const Packed dpre = pack_matrix(relu_grad(m, g + ob2), int(R), kW, m.slot(m.kDh, S), st);
+        gemm_packed_tn(Packed{m.slot(m.kX2, S), int(R), 3 * kW}, dpre, g + oW2, kW, st, sms);
+        gemm_packed(dpre, true, 3 * kW, plain(prm + oW2, kW), F(m.dx2), 3 * kW, false, GemmEpi{}, st, sms);
     } else {
         relu_bwd_kernel<<<R / kRowsPerCta, dim3(kW, kRowsPerCta), 0, st>>>(F(m.dh), F(m.pre2), F(m.dpre));
         sgemm<true, false>(3 * kW, kW, int(R), F(m.x2), 3 * kW, F(m.dpre), kW, g + oW2, kW, true, st, sms);
@@ -909,7 +918,7 @@ void upload_batch(Encoder& m, const uint8_t* codes, const int32_t* lens, const i
             fail(ST_EINVAL, "seqtree_b200: encoder inputs must have 1..32 residues");
     for (int64_t i = 0; i < int64_t(S) * kP; ++i)
         if (codes[i] >= kA) fail(ST_EINVAL, "seqtree_b200: encoder codes must be < 24");
-    m.reserve(S);
+    m.reserve(S, m.precision == 1);
     h2d(m.codes.ptr, codes, size_t(S) * kP, st);
     h2d(m.lens.ptr, lens, sizeof(int32_t) * size_t(S), st);
     if (scores) h2d(m.scores.ptr, scores, sizeof(int32_t) * size_t(S / 2), st);
@@ -942,7 +951,7 @@ void encoder_destroy(Encoder* m) {
                       &m->scores, &m->pre1, &m->h1, &m->x2, &m->pre2, &m->hA, &m->hB, &m->hC,
                       &m->qkv0, &m->qkv1, &m->a0, &m->a1, &m->o0, &m->o1, &m->y, &m->pool, &m->e,
                       &m->z, &m->nrm, &m->dz, &m->de, &m->dpool, &m->dh, &m->dO, &m->dqkv, &m->dx2,
-                      &m->dpre})
+                      &m->dpre, &m->packed})
         b->release();
     delete m;
 }
@@ -1016,7 +1025,7 @@ void encoder_embed(Encoder& m, const st_seqset_s& set, void* out, int layout, cu
     }
     Context& ctx = context();
     constexpr int kChunk = 16384;
-    m.reserve(kChunk);
+    m.reserve(kChunk, false);
     for (int64_t first = 0; first < set.count; first += kChunk) {
         const int S = int(std::min<int64_t>(kChunk, set.count - first));
         gather_codes_kernel<<<unsigned(S), kP, 0, st>>>(set.d_bytes, set.d_off, set.d_len, first, S,

@@ -5,7 +5,8 @@
 // Both operands are first packed into the tcgen05 K-major operand layout in bf16: blocks of 128
 // rows x 64 k (16 KB), row r at r*128 bytes, the 16-byte unit u of a row at u ^ (r & 7) (the
 // 128-byte swizzle), zero outside the matrix.  Packing absorbs the transposes (op(A) is A or
-// A^T, the same for B), so the GEMM kernel only ever sees "rows x K" tiles.  One CTA computes
+// A^T, the same for B); a matrix that takes part in two products, along its rows and along its columns,
+// is packed once and read MN-major for the second (pack_matrix).  One CTA computes
 // one 128 x 128 output tile over a range of K chunks: warp 0 bulk-copies A and B chunks through a
 // 2-stage shared-memory ring (64 KB, so that three CTAs share an SM and one's epilogue overlaps
 // another's loads: the layers are thin), one thread of warp 1 issues M=128 N=128 K=16 tcgen05.mma into a
@@ -105,11 +106,45 @@ __global__ void pack_rows_kernel(const PackSrc s, int rows, int K, int kchunks, 
     *reinterpret_cast<uint4*>(op + pos * 16) = bf16_unit(v);
 }
 
+// The same, four passes of 32 rows over one 128 x 64 block after another (kSumTiles of them), with the
+// matrix' column sums: a thread meets the same eight columns in each of its rows (row & 7 is fixed), so
+// the sums stay in registers until the end.  Aligned as VEC.
+constexpr int kSumTiles = 4;
+
+template <int KIND>
+__global__ void __launch_bounds__(256) pack_rows_sum_kernel(const PackSrc s, int rows, int cols, int tiles,
+                                                            uint8_t* __restrict__ op) {
+    __shared__ float part[32][kGK + 1];
+    const int kchunks = cols / kGK, chunk = blockIdx.x % kchunks, t0 = blockIdx.x / kchunks * kSumTiles;
+    const int pu = threadIdx.x & 7, r0 = threadIdx.x >> 3;
+    const int u = pu ^ (r0 & 7);
+    float sum[8] = {};
+    for (int t = t0; t < min(t0 + kSumTiles, tiles); ++t) {
+#pragma unroll
+        for (int p = 0; p < kGT / 32; ++p) {
+            const int row = p * 32 + r0;
+            const int64_t i = int64_t(t) * kGT + row;
+            float v[8] = {};
+            if (i < rows) src_eight<KIND>(s, i, chunk * kGK + u * 8, v);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sum[e] += v[e];
+            *reinterpret_cast<uint4*>(op + (int64_t(t) * kchunks + chunk) * kBlockB + row * 128 + pu * 16) = bf16_unit(v);
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) part[r0][u * 8 + e] = sum[e];
+    __syncthreads();
+    if (threadIdx.x < kGK) {
+        float total = 0.f;
+#pragma unroll 8
+        for (int r = 0; r < 32; ++r) total += part[r][threadIdx.x];
+        atomicAdd(s.colsum + chunk * kGK + threadIdx.x, total);
+    }
+}
+
 // The same packed operand from the transpose: value(i, k) = matrix(k, i).  One 256-thread
 // block per (tile, chunk) block: it reads the 64 x 128 fp32 piece row by row (coalesced)
-// into shared memory and writes the 16 KB block in output order; with colsum it adds the piece's
-// column sums first.
-template <int KIND>
+// into shared memory and writes the 16 KB block in output order.
 __global__ void __launch_bounds__(256) pack_cols_kernel(const PackSrc s, int rows, int K, int kchunks,
                                                         uint8_t* __restrict__ op) {
     __shared__ float t[kGK][kGT + 1];
@@ -120,7 +155,7 @@ __global__ void __launch_bounds__(256) pack_cols_kernel(const PackSrc s, int row
     for (int idx = threadIdx.x; idx < kGK * kGT; idx += 256) {
         const int kk = idx >> 7, ii = idx & 127;
         const int64_t i = i0 + ii;
-        t[kk][ii] = (i < rows && k0 + kk < K) ? src_value<KIND>(s, k0 + kk, int(i)) : 0.f;
+        t[kk][ii] = (i < rows && k0 + kk < K) ? src_value<PackSrc::kPlain>(s, k0 + kk, int(i)) : 0.f;
     }
     __syncthreads();
     uint8_t* dst = op + int64_t(blockIdx.x) * kBlockB;
@@ -132,19 +167,13 @@ __global__ void __launch_bounds__(256) pack_cols_kernel(const PackSrc s, int row
         for (int e = 0; e < 8; ++e) v[e] = t[u * 8 + e][row];
         *reinterpret_cast<uint4*>(dst + pos * 16) = bf16_unit(v);
     }
-    if (s.colsum) {  // two threads per column, 32 rows each
-        const int ii = threadIdx.x & 127, h = threadIdx.x >> 7;
-        float sum = 0.f;
-#pragma unroll 8
-        for (int kk = 0; kk < kGK / 2; ++kk) sum += t[h * (kGK / 2) + kk][ii];
-        if (i0 + ii < rows) atomicAdd(s.colsum + i0 + ii, sum);
-    }
 }
 
 struct GemmBf16Args {
     const uint8_t* a;   // packed op(A): mtiles x kchunks blocks
     const uint8_t* b;   // packed op(B): ntiles x kchunks blocks
     int kchunks, chunks_per_split;
+    int acols, bcols;   // TN: 64-column blocks of a row of A and of B
     float* C;
     int ldc, M, N;
     int mode;           // 0 store, 1 add, 2 atomic add
@@ -152,6 +181,16 @@ struct GemmBf16Args {
     unsigned long long* err;
 };
 
+// MN-major operand in the 128-byte swizzle: 64 columns x 8 k to an atom of 1024 B, the next 8 k 1024 B on
+// and the next 64 columns kBlockB / 2 on.
+__device__ __forceinline__ uint64_t sw128_desc_mn(uint32_t addr) {
+    return uint64_t((addr >> 4) & 0x3FFFu) | (uint64_t(kBlockB / 2 >> 4) << 16) | (uint64_t(1024 >> 4) << 32) |
+           (uint64_t(1) << 46) | (uint64_t(2) << 61);
+}
+
+// TN: C = A^T B of two matrices packed as rows: a chunk is 64 of their rows, two half blocks (64 columns each)
+// of either, read MN-major.  Packing both transposes instead took 503 us of a 2,048-pair step.
+template <bool TN>
 __global__ void __launch_bounds__(kGThreads) gemm_bf16_kernel(GemmBf16Args g) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((uintptr_t(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -188,8 +227,18 @@ __global__ void __launch_bounds__(kGThreads) gemm_bf16_kernel(GemmBf16Args g) {
             if (!bar_wait(BAR(kGStages + stage), phase ^ 1u, s_abort, g.err)) break;
             bar_expect_tx(BAR(stage), 2 * kBlockB);
             const uint32_t dst = sbase + stage * 2 * kBlockB;
-            bulk_load(dst, g.a + (int64_t(tm) * g.kchunks + c) * kBlockB, kBlockB, BAR(stage));
-            bulk_load(dst + kBlockB, g.b + (int64_t(tn) * g.kchunks + c) * kBlockB, kBlockB, BAR(stage));
+            if (TN) {
+                const int64_t half = int64_t(c & 1) * (kBlockB / 2);
+                for (int j = 0; j < 2; ++j) {
+                    bulk_load(dst + j * (kBlockB / 2), g.a + (int64_t(c >> 1) * g.acols + 2 * tm + j) * kBlockB + half,
+                              kBlockB / 2, BAR(stage));
+                    bulk_load(dst + kBlockB + j * (kBlockB / 2),
+                              g.b + (int64_t(c >> 1) * g.bcols + 2 * tn + j) * kBlockB + half, kBlockB / 2, BAR(stage));
+                }
+            } else {
+                bulk_load(dst, g.a + (int64_t(tm) * g.kchunks + c) * kBlockB, kBlockB, BAR(stage));
+                bulk_load(dst + kBlockB, g.b + (int64_t(tn) * g.kchunks + c) * kBlockB, kBlockB, BAR(stage));
+            }
             issued |= 1u << stage;
             par = phase ? (par | (1u << stage)) : (par & ~(1u << stage));
             if (++stage == kGStages) {
@@ -200,7 +249,7 @@ __global__ void __launch_bounds__(kGThreads) gemm_bf16_kernel(GemmBf16Args g) {
         for (int s = 0; s < kGStages; ++s)
             if (issued & (1u << s)) bar_drain(BAR(s), (par >> s) & 1u);
     } else if (warp == 1 && lane == 0) {
-        constexpr uint32_t idesc = idesc_bf16(128, 128);
+        constexpr uint32_t idesc = idesc_bf16(128, 128) | (TN ? 3u << 15 : 0u);  // A and B MN-major
         uint32_t stage = 0, phase = 0;
         for (int c = c0; c < c1; ++c) {
             if (!bar_wait(BAR(stage), phase, s_abort, g.err)) break;
@@ -208,7 +257,8 @@ __global__ void __launch_bounds__(kGThreads) gemm_bf16_kernel(GemmBf16Args g) {
             const uint32_t a = sbase + stage * 2 * kBlockB, b = a + kBlockB;
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-                tc_mma(tmem, sw128_desc(a + kk * 32), sw128_desc(b + kk * 32), idesc,
+                tc_mma(tmem, TN ? sw128_desc_mn(a + kk * 2048) : sw128_desc(a + kk * 32),
+                       TN ? sw128_desc_mn(b + kk * 2048) : sw128_desc(b + kk * 32), idesc,
                        (c > c0 || kk > 0) ? 1u : 0u);
             tc_commit(BAR(kGStages + stage));
             if (++stage == kGStages) {
@@ -317,42 +367,104 @@ __global__ void __launch_bounds__(kGThreads) gemm_bf16_kernel(GemmBf16Args g) {
     }
 }
 
-template <int KIND>
-void launch_pack(const PackSrc& s, bool trans, int rows, int K, int tiles, int kchunks, uint8_t* op,
-                 cudaStream_t st) {
-    const int64_t units = int64_t(tiles) * kchunks * kGT * 8;
-    if (trans) {
-        pack_cols_kernel<KIND><<<unsigned(tiles * kchunks), 256, 0, st>>>(s, rows, K, kchunks, op);
-        return;
-    }
-    const uintptr_t bases = uintptr_t(s.x) | uintptr_t(s.y);
-    const bool vec = (bases & 15) == 0 && s.ld % 4 == 0 && K % 8 == 0;
-    (vec ? pack_rows_kernel<KIND, true> : pack_rows_kernel<KIND, false>)<<<unsigned(ceil_div(units, 256)), 256, 0, st>>>(
-        s, rows, K, kchunks, units, op);
+bool vec_ok(const PackSrc& s, int K) {
+    return ((uintptr_t(s.x) | uintptr_t(s.y)) & 15) == 0 && s.ld % 4 == 0 && K % 8 == 0;
 }
 
-void pack(const PackSrc& s, bool trans, int rows, int K, DevBuf& buf, cudaStream_t st, int& tiles,
-          int& kchunks) {
-    tiles = int(ceil_div(rows, kGT));
-    kchunks = int(ceil_div(K, kGK));
+// op[i][k] = trans ? s[k][i] : s[i][k]
+const uint8_t* pack(const PackSrc& s, bool trans, int rows, int K, DevBuf& buf, cudaStream_t st) {
+    const int tiles = int(ceil_div(rows, kGT)), kchunks = int(ceil_div(K, kGK));
     uint8_t* op = buf.as<uint8_t>(size_t(tiles) * kchunks * kBlockB);
-    switch (s.kind) {
-        case PackSrc::kConv: launch_pack<PackSrc::kConv>(s, trans, rows, K, tiles, kchunks, op, st); break;
-        case PackSrc::kRelu: launch_pack<PackSrc::kRelu>(s, trans, rows, K, tiles, kchunks, op, st); break;
-        default: launch_pack<PackSrc::kPlain>(s, trans, rows, K, tiles, kchunks, op, st);
-    }
+    const int64_t units = int64_t(tiles) * kchunks * kGT * 8;
+    if (trans)
+        pack_cols_kernel<<<unsigned(tiles * kchunks), 256, 0, st>>>(s, rows, K, kchunks, op);
+    else
+        (vec_ok(s, K) ? pack_rows_kernel<PackSrc::kPlain, true> : pack_rows_kernel<PackSrc::kPlain, false>)
+            <<<unsigned(ceil_div(units, 256)), 256, 0, st>>>(s, rows, K, kchunks, units, op);
+    STB_CUDA(cudaGetLastError());
+    return op;
+}
+
+template <int KIND>
+void launch_matrix(const PackSrc& s, int rows, int cols, int tiles, uint8_t* op, cudaStream_t st) {
+    const int kchunks = cols / kGK;
+    const int64_t units = int64_t(tiles) * kchunks * kGT * 8;
+    if (s.colsum)
+        pack_rows_sum_kernel<KIND><<<unsigned(ceil_div(tiles, kSumTiles)) * kchunks, 256, 0, st>>>(s, rows, cols, tiles, op);
+    else
+        pack_rows_kernel<KIND, true><<<unsigned(ceil_div(units, 256)), 256, 0, st>>>(s, rows, cols, kchunks, units, op);
+}
+
+// The product of packed operands.  Products with a long K and few output tiles are split over K and added
+// atomically, in which case C must already hold the value to add to (it is cleared first when
+// !accumulate).  An epilogue other than kNone takes the product unsplit.
+void run_gemm(GemmBf16Args g, bool tn, bool accumulate, cudaStream_t st, int sms) {
+    Context& ctx = context();
+    const int mtiles = int(ceil_div(g.M, kGT)), ntiles = int(ceil_div(g.N, kGT)), tiles = mtiles * ntiles;
+    int splits = 1;
+    if (g.epi.kind == GemmEpi::kNone && tiles < sms && g.kchunks >= 16)
+        splits = std::min(int(ceil_div(2 * sms, tiles)), g.kchunks / 4);
+    g.chunks_per_split = int(ceil_div(g.kchunks, splits));
+    splits = int(ceil_div(g.kchunks, g.chunks_per_split));
+    g.mode = splits > 1 ? 2 : (accumulate ? 1 : 0);
+    if (splits > 1 && !accumulate)
+        STB_CUDA(cudaMemsetAsync(g.C, 0, sizeof(float) * size_t(g.M) * size_t(g.ldc), st));
+    g.err = reinterpret_cast<unsigned long long*>(ctx.flags_d + 8);
+    auto kernel = tn ? gemm_bf16_kernel<true> : gemm_bf16_kernel<false>;
+    ensure_smem_limit(reinterpret_cast<const void*>(kernel), kGSmem);
+    kernel<<<dim3(unsigned(ntiles), unsigned(mtiles), unsigned(splits)), kGThreads, kGSmem, st>>>(g);
     STB_CUDA(cudaGetLastError());
 }
 
 }  // namespace
 
+Packed pack_matrix(const PackSrc& s, int rows, int cols, uint8_t* op, cudaStream_t st) {
+    if (cols % kGT || !vec_ok(s, cols)) fail(ST_EINVAL, "seqtree_b200: pack_matrix takes aligned rows of 128 columns");
+    const int tiles = int(ceil_div(rows, kGT));
+    switch (s.kind) {
+        case PackSrc::kConv: launch_matrix<PackSrc::kConv>(s, rows, cols, tiles, op, st); break;
+        case PackSrc::kRelu: launch_matrix<PackSrc::kRelu>(s, rows, cols, tiles, op, st); break;
+        default: launch_matrix<PackSrc::kPlain>(s, rows, cols, tiles, op, st);
+    }
+    STB_CUDA(cudaGetLastError());
+    note_launch(nullptr);
+    return Packed{op, rows, cols};
+}
+
+void gemm_packed(const Packed& A, bool tb, int N, const PackSrc& B, float* C, int ldc, bool accumulate,
+                 const GemmEpi& epi, cudaStream_t st, int sms) {
+    GemmBf16Args g{};
+    g.a = A.op;
+    g.b = pack(B, !tb, N, A.cols, context().gemm_b, st);
+    g.kchunks = A.cols / kGK;
+    g.C = C;
+    g.ldc = ldc;
+    g.M = A.rows;
+    g.N = N;
+    g.epi = epi;
+    run_gemm(g, false, accumulate, st, sms);
+    note_launch("gemm_bf16_kernel", 2);
+}
+
+void gemm_packed_tn(const Packed& A, const Packed& B, float* C, int ldc, cudaStream_t st, int sms) {
+    GemmBf16Args g{};
+    g.a = A.op;
+    g.b = B.op;
+    g.kchunks = 2 * int(ceil_div(A.rows, kGT));  // (rows past the last are packed as zeros)
+    g.acols = A.cols / kGK;
+    g.bcols = B.cols / kGK;
+    g.C = C;
+    g.ldc = ldc;
+    g.M = A.cols;
+    g.N = B.cols;
+    run_gemm(g, true, true, st, sms);
+    note_launch("gemm_bf16_kernel", 1);
+}
+
 // C (=, +=) op(A) op(B) in bf16 with fp32 accumulation.  op(A) is [M x K] (A^T when ta, A being
 // [K x M]), op(B) is [K x N] (B^T when tb, B being [N x K]); row-major with leading dimensions.
-// Products with a long K and few output tiles are split over K and added atomically, in which
-// case C must already hold the value to add to (it is cleared first when !accumulate).
-// An epilogue other than kNone takes the product unsplit.
-void gemm_bf16(bool ta, bool tb, int M, int N, int K, const PackSrc& A, const PackSrc& B, float* C, int ldc,
-               bool accumulate, const GemmEpi& epi, cudaStream_t st, int sms) {
+void gemm_bf16(bool ta, bool tb, int M, int N, int K, const float* A, int lda, const float* B, int ldb,
+               float* C, int ldc, bool accumulate, cudaStream_t st, int sms) {
     if (M <= 0 || N <= 0) return;
     if (K <= 0) {
         if (!accumulate)
@@ -361,46 +473,22 @@ void gemm_bf16(bool ta, bool tb, int M, int N, int K, const PackSrc& A, const Pa
         return;
     }
     Context& ctx = context();
-    ensure_smem_limit(reinterpret_cast<const void*>(gemm_bf16_kernel), kGSmem);
-    int mtiles, ntiles, kchunks, kb;
-    // op(A)[i][k] = ta ? A[k][i] : A[i][k];  op(B)^T[n][k] = tb ? B[n][k] : B[k][n]
-    pack(A, ta, M, K, ctx.gemm_a, st, mtiles, kchunks);
-    pack(B, !tb, N, K, ctx.gemm_b, st, ntiles, kb);
-    const int tiles = mtiles * ntiles;
-    int splits = 1;
-    if (epi.kind == GemmEpi::kNone && tiles < sms && kchunks >= 16)
-        splits = std::min(int(ceil_div(2 * sms, tiles)), kchunks / 4);
-    const int cps = int(ceil_div(kchunks, splits));
-    splits = int(ceil_div(kchunks, cps));
-    const int mode = splits > 1 ? 2 : (accumulate ? 1 : 0);
-    if (splits > 1 && !accumulate)
-        STB_CUDA(cudaMemsetAsync(C, 0, sizeof(float) * size_t(M) * size_t(ldc), st));
-    GemmBf16Args g{};
-    g.a = static_cast<const uint8_t*>(ctx.gemm_a.ptr);
-    g.b = static_cast<const uint8_t*>(ctx.gemm_b.ptr);
-    g.kchunks = kchunks;
-    g.chunks_per_split = cps;
-    g.C = C;
-    g.ldc = ldc;
-    g.M = M;
-    g.N = N;
-    g.mode = mode;
-    g.epi = epi;
-    g.err = reinterpret_cast<unsigned long long*>(ctx.flags_d + 8);
-    gemm_bf16_kernel<<<dim3(unsigned(ntiles), unsigned(mtiles), unsigned(splits)), kGThreads, kGSmem,
-                       st>>>(g);
-    STB_CUDA(cudaGetLastError());
-    note_launch("gemm_bf16_kernel", 3);
-}
-
-void gemm_bf16(bool ta, bool tb, int M, int N, int K, const float* A, int lda, const float* B, int ldb,
-               float* C, int ldc, bool accumulate, cudaStream_t st, int sms) {
     PackSrc a{}, b{};
     a.x = A;
     a.ld = lda;
     b.x = B;
     b.ld = ldb;
-    gemm_bf16(ta, tb, M, N, K, a, b, C, ldc, accumulate, GemmEpi{}, st, sms);
+    GemmBf16Args g{};
+    // op(A)[i][k] = ta ? A[k][i] : A[i][k];  op(B)^T[n][k] = tb ? B[n][k] : B[k][n]
+    g.a = pack(a, ta, M, K, ctx.gemm_a, st);
+    g.b = pack(b, !tb, N, K, ctx.gemm_b, st);
+    g.kchunks = int(ceil_div(K, kGK));
+    g.C = C;
+    g.ldc = ldc;
+    g.M = M;
+    g.N = N;
+    run_gemm(g, false, accumulate, st, sms);
+    note_launch("gemm_bf16_kernel", 3);
 }
 
 }  // namespace stb

@@ -3,12 +3,15 @@
 // are bound by memory; folding the im2col gather, the ReLU gradient, the biases, the residuals, the
 // masks and the bias gradients took their passes over 67 to 201 MB out of a 2,048-pair step: 3.57 ->
 // 2.77 ms with the attention kernels' wider reads (B200; sums keep the separate passes' order except
-// the bias gradients').
+// the bias gradients').  Packing a matrix once for its product along the rows and the one along the
+// columns, whose operands are read MN-major: 2.53 -> 2.06 ms.
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include <cstdint>
+
+#include "common.cuh"
 
 namespace stb {
 
@@ -23,8 +26,7 @@ struct PackSrc {
     const int32_t* lens = nullptr;
     // kRelu: x where y > 0 (y as x), else 0.
     const float* y = nullptr;
-    // When set: the column sums of the matrix are added to it (only where the operand is packed
-    // from its transpose, i.e. the matrix' rows run along K).
+    // When set: the column sums of the matrix are added to it (pack_matrix).
     float* colsum = nullptr;
 };
 
@@ -40,7 +42,19 @@ struct GemmEpi {
     const int32_t* lens = nullptr; // kResidual, kConv, kMaskAdd (C += product, 0 past the end)
 };
 
-void gemm_bf16(bool ta, bool tb, int M, int N, int K, const PackSrc& A, const PackSrc& B, float* C, int ldc,
-               bool accumulate, const GemmEpi& epi, cudaStream_t st, int sms);
+// A matrix packed once for both of its products: as rows (op(A) = A) it is a K-major operand, and the
+// same blocks, read along their rows, are the MN-major operand of A^T.  cols is a multiple of 128.
+struct Packed {
+    const uint8_t* op = nullptr;
+    int rows = 0, cols = 0;
+};
+constexpr size_t packed_bytes(int64_t rows, int cols) { return size_t((rows + 127) / 128 * 128) * size_t(cols) * 2; }
+Packed pack_matrix(const PackSrc& s, int rows, int cols, uint8_t* op, cudaStream_t st);  // op: packed_bytes
+
+// C (=, +=) A op(B), A [M x K] packed, op(B) = B or B^T.
+void gemm_packed(const Packed& A, bool tb, int N, const PackSrc& B, float* C, int ldc, bool accumulate,
+                 const GemmEpi& epi, cudaStream_t st, int sms);
+// C += A^T B, both packed with the same rows.
+void gemm_packed_tn(const Packed& A, const Packed& B, float* C, int ldc, cudaStream_t st, int sms);
 
 }  // namespace stb
