@@ -60,7 +60,7 @@ TRAFFIC: dict[str, float | None] = {
     "gapblock": 1.92e6,     # 1.88 MB read + 0.03 MB write (the result stays in L2)
     "hamming": 1.31e9,      # 262 MB per 4,000 rows, scaled to 20,000 rows
     "levenshtein": 1.03e9,  # 102.5 MB per 2,000 rows, scaled to 20,000 rows
-    "align": 1.05e6,        # one row-bucket launch of the wavefront kernel
+    "align": None,          # not measured for the strip kernel
 }
 
 
@@ -260,16 +260,18 @@ def kernel_roofline(w, cells: float, seconds: float, clocks, int_peaks=None) -> 
     Peaks are the instruction rates measured in this process (``int_peaks``, all SMs, at the clock
     the probe ran); without them, the nominal 148 SMs x lanes/clk x SM clock.
 
-    gap block: one conflict-free LDS.32 of a packed penalty word feeds two cells (two queries), so
-    the algorithmic shared-memory traffic is 2 B/cell; the same two cells take one
-    ``__viaddmin_s16x2``.  The bound is the LDS.32 rate (4 B per lane-load).
+    gap block: counted at two cells per conflict-free LDS.32 of a packed penalty word (2 B/cell) and
+    one ``__viaddmin_s16x2``, against the LDS.32 rate (4 B per lane-load).  The kernel packs four
+    queries' penalties as bytes of a word (two as 16-bit halves only above 255), so its lookups take half
+    of what is counted; its bound is instruction issue (profiles/gapblock_fast_kernel_quads.md).
     alignment: DPX.  A DPX instruction updates one int16x2 cell pair.  Local mode needs 6 of them
     per pair (M, X, Y, H and the two gap extends) -- 3 per cell; global mode keeps the states
     raised by (i+j)*gap_extend, which folds each gap extend into its add-max, so 4 per pair -- 2
     per cell.  The bound is the measured ``__viaddmin_s16x2`` rate.
-    levenshtein: ALU pipe.  The bit-vector step per text character is ten 64-bit logic, add and
-    shift operations (the whole pattern, <= 64 symbols, in one word): 20 32-bit ALU lane-ops per
-    (pair, query character), against the measured ALU-pipe rate (the IADD3 probe).
+    levenshtein: ALU pipe.  The bit-vector step per text character is ten logic, add and shift
+    operations per 32-bit word of the pattern, counted at two words (<= 64 symbols): 20 32-bit ALU
+    lane-ops per (pair, query character), against the measured ALU-pipe rate (the IADD3 probe).
+    Patterns of up to 32 symbols take one word, so the fraction counts them double.
     """
     mhz = (clocks or {}).get("sm_mhz") or 1965.0
     sms = 148
@@ -283,7 +285,7 @@ def kernel_roofline(w, cells: float, seconds: float, clocks, int_peaks=None) -> 
         else:
             peak, basis = sms * 128 * mhz * 1e6 / 1e9, f"148 SMs x 128 B/clk at {mhz:.0f} MHz"
         out = {"bound": "smem", "achieved": achieved, "peak": peak, "unit": "GB/s",
-               "frac": achieved / peak, "work": "2 B of penalty per cell (one LDS.32 per 2 cells)",
+               "frac": achieved / peak, "work": "2 B of penalty per cell (one LDS.32 per 2 cells; the kernel packs 4)",
                "peak_basis": basis}
         if dpx:
             a = cells / 2.0 / seconds
@@ -314,7 +316,7 @@ def kernel_roofline(w, cells: float, seconds: float, clocks, int_peaks=None) -> 
             peak, basis = sms * 64 * mhz * 1e6 / 1e9, f"148 SMs x 64 ALU lanes/clk at {mhz:.0f} MHz"
         return {"bound": "alu", "achieved": achieved, "peak": peak, "unit": "Glane-op/s",
                 "frac": achieved / peak,
-                "work": "20 ALU lane-ops per (pair, query character): one 64-bit bit-vector step",
+                "work": "20 ALU lane-ops per (pair, query character): a bit-vector step over two 32-bit words",
                 "peak_basis": basis}
     return None
 
