@@ -704,7 +704,9 @@ struct Encoder {
     DevBuf dz, de, dpool, dh, dO, dqkv, dx2, dpre;
     // bf16 operands of the training products, each packed once for its two products (x2, h and o from
     // forward to backward), in one block of which a unit is R x 128 values
-    DevBuf packed;
+    DevBuf packed, packed_w;
+    // the weights' operands, packed by forward: [0] for the product itself, [1] for the gradient's
+    Packed w2[2], wqkv[2][2], wo[2][2];
     enum Slot { kX2 = 0, kH = 3, kO = 5, kDh = 7, kDqkv = 8, kSlots = 11 };
     uint8_t* slot(int which, int S) {
         return static_cast<uint8_t*>(packed.ptr) + size_t(which) * packed_bytes(int64_t(S) * kP, kW);
@@ -712,8 +714,10 @@ struct Encoder {
 
     void reserve(int S, bool bf) {  // bf: as the passes over S sequences that follow
         const size_t R = size_t(S) * kP;
-        if (bf) packed.as<uint8_t>(kSlots * packed_bytes(int64_t(R), kW));
-        else x2.as<float>(R * 3 * kW);
+        if (bf) {
+            packed.as<uint8_t>(kSlots * packed_bytes(int64_t(R), kW));
+            packed_w.as<uint8_t>(2 * (packed_bytes(3 * kW, kW) * 3 + packed_bytes(kW, kW) * 2));
+        } else x2.as<float>(R * 3 * kW);
         if (S <= S_cap) return;
         codes.as<uint8_t>(R);
         lens.as<int32_t>(size_t(S));
@@ -764,6 +768,30 @@ PackSrc relu_grad(Encoder& m, float* colsum = nullptr) {  // dh where pre2 > 0
     return s;
 }
 
+// Every weight as the B operand of its product and of its input gradient.
+void pack_step_weights(Encoder& m, cudaStream_t st) {
+    const float* prm = P(m);
+    WeightSrc w[kMaxWeights];
+    Packed out[kMaxWeights];
+    auto both = [&](int i, const float* x, int K, int N) {  // x [K x N]: rows of x^T, then rows of x
+        w[i] = WeightSrc{x, N, N, K, true};
+        w[i + 1] = WeightSrc{x, N, K, N, false};
+    };
+    both(0, prm + oW2, 3 * kW, kW);
+    for (int l = 0; l < 2; ++l) {
+        both(2 + 4 * l, prm + oL0 + l * kLayer + lWqkv, kW, 3 * kW);
+        both(4 + 4 * l, prm + oL0 + l * kLayer + lWo, kW, kW);
+    }
+    pack_weights(w, kMaxWeights, static_cast<uint8_t*>(m.packed_w.ptr), out, st);
+    for (int b = 0; b < 2; ++b) {
+        m.w2[b] = out[b];
+        for (int l = 0; l < 2; ++l) {
+            m.wqkv[l][b] = out[2 + 4 * l + b];
+            m.wo[l][b] = out[4 + 4 * l + b];
+        }
+    }
+}
+
 // Forward of S sequences whose padded codes and lengths are in m.codes / m.lens; z in m.z.
 void forward(Encoder& m, int S, cudaStream_t st, int sms, bool bf) {
     set_attn_attrs();
@@ -773,14 +801,15 @@ void forward(Encoder& m, int S, cudaStream_t st, int sms, bool bf) {
     float* prm = P(m);
     conv1_fwd_kernel<<<R / kRowsPerCta, 32 * kRowsPerCta, 0, st>>>(codes, lens, prm, F(m.pre1), F(m.h1));
     if (bf) {  // the gather of the three rows is folded into the operand, bias / ReLU / skip into the product
+        pack_step_weights(m, st);
         GemmEpi epi{};
         epi.kind = GemmEpi::kConv;
         epi.bias = prm + ob2;
         epi.res = F(m.h1);
         epi.out = F(m.hA);
         epi.lens = lens;
-        gemm_packed(pack_matrix(conv_rows(m), int(R), 3 * kW, m.slot(m.kX2, S), st), false, kW, plain(prm + oW2, kW),
-                    F(m.pre2), kW, false, epi, st, sms);
+        gemm_packed(pack_matrix(conv_rows(m), int(R), 3 * kW, m.slot(m.kX2, S), st), m.w2[0], F(m.pre2), kW, false,
+                    epi, st, sms);
     } else {
         im2col_kernel<<<R / kRowsPerCta, dim3(kW, kRowsPerCta), 0, st>>>(F(m.h1), lens, F(m.x2));
         sgemm<false, false>(int(R), kW, 3 * kW, F(m.x2), 3 * kW, prm + oW2, kW, F(m.pre2), kW, false, st, sms);
@@ -798,8 +827,8 @@ void forward(Encoder& m, int S, cudaStream_t st, int sms, bool bf) {
             GemmEpi epi{};
             epi.kind = GemmEpi::kBias;
             epi.bias = L + lbqkv;
-            gemm_packed(pack_matrix(plain(hin[l], kW), int(R), kW, m.slot(m.kH + l, S), st), false, 3 * kW,
-                        plain(L + lWqkv, 3 * kW), qkv[l], 3 * kW, false, epi, st, sms);
+            gemm_packed(pack_matrix(plain(hin[l], kW), int(R), kW, m.slot(m.kH + l, S), st), m.wqkv[l][0], qkv[l],
+                        3 * kW, false, epi, st, sms);
         } else {
             sgemm<false, false>(int(R), 3 * kW, kW, hin[l], kW, L + lWqkv, 3 * kW, qkv[l], 3 * kW, false, st, sms);
             add_bias_kernel<<<R / kRowsPerCta, dim3(128, kRowsPerCta), 0, st>>>(qkv[l], L + lbqkv, 3 * kW);
@@ -812,8 +841,8 @@ void forward(Encoder& m, int S, cudaStream_t st, int sms, bool bf) {
             epi.res = hin[l];
             epi.out = hout[l];
             epi.lens = lens;
-            gemm_packed(pack_matrix(plain(ob[l], kW), int(R), kW, m.slot(m.kO + l, S), st), false, kW, plain(L + lWo, kW),
-                        F(m.y), kW, false, epi, st, sms);
+            gemm_packed(pack_matrix(plain(ob[l], kW), int(R), kW, m.slot(m.kO + l, S), st), m.wo[l][0], F(m.y), kW,
+                        false, epi, st, sms);
         } else {
             sgemm<false, false>(int(R), kW, kW, ob[l], kW, L + lWo, kW, F(m.y), kW, false, st, sms);
             residual_kernel<<<R / kRowsPerCta, dim3(kW, kRowsPerCta), 0, st>>>(hin[l], F(m.y), L + lbo, lens,
@@ -856,7 +885,7 @@ void loss_backward(Encoder& m, int S, cudaStream_t st, int sms, bool bf) {
         if (bf) {  // the bias gradients are summed while dh and dqkv are packed
             const Packed dh = pack_matrix(plain(F(m.dh), kW, G + lbo), int(R), kW, m.slot(m.kDh, S), st);
             gemm_packed_tn(Packed{m.slot(m.kO + l, S), int(R), kW}, dh, G + lWo, kW, st, sms);
-            gemm_packed(dh, true, kW, plain(L + lWo, kW), F(m.dO), kW, false, GemmEpi{}, st, sms);
+            gemm_packed(dh, m.wo[l][1], F(m.dO), kW, false, GemmEpi{}, st, sms);
         } else {
             sgemm<true, false>(kW, kW, int(R), ob[l], kW, F(m.dh), kW, G + lWo, kW, true, st, sms);
             colsum(F(m.dh), R, kW, G + lbo, st);
@@ -870,7 +899,7 @@ void loss_backward(Encoder& m, int S, cudaStream_t st, int sms, bool bf) {
             GemmEpi epi{};
             epi.kind = GemmEpi::kMaskAdd;
             epi.lens = lens;
-            gemm_packed(dqkv, true, kW, plain(L + lWqkv, 3 * kW), F(m.dh), kW, true, epi, st, sms);
+            gemm_packed(dqkv, m.wqkv[l][1], F(m.dh), kW, true, epi, st, sms);
         } else {
             sgemm<true, false>(kW, 3 * kW, int(R), hin[l], kW, F(m.dqkv), 3 * kW, G + lWqkv, 3 * kW, true, st,
                                sms);
@@ -884,7 +913,7 @@ void loss_backward(Encoder& m, int S, cudaStream_t st, int sms, bool bf) {
     if (bf) {
         const Packed dpre = pack_matrix(relu_grad(m, g + ob2), int(R), kW, m.slot(m.kDh, S), st);
         gemm_packed_tn(Packed{m.slot(m.kX2, S), int(R), 3 * kW}, dpre, g + oW2, kW, st, sms);
-        gemm_packed(dpre, true, 3 * kW, plain(prm + oW2, kW), F(m.dx2), 3 * kW, false, GemmEpi{}, st, sms);
+        gemm_packed(dpre, m.w2[1], F(m.dx2), 3 * kW, false, GemmEpi{}, st, sms);
     } else {
         relu_bwd_kernel<<<R / kRowsPerCta, dim3(kW, kRowsPerCta), 0, st>>>(F(m.dh), F(m.pre2), F(m.dpre));
         sgemm<true, false>(3 * kW, kW, int(R), F(m.x2), 3 * kW, F(m.dpre), kW, g + oW2, kW, true, st, sms);
@@ -951,7 +980,7 @@ void encoder_destroy(Encoder* m) {
                       &m->scores, &m->pre1, &m->h1, &m->x2, &m->pre2, &m->hA, &m->hB, &m->hC,
                       &m->qkv0, &m->qkv1, &m->a0, &m->a1, &m->o0, &m->o1, &m->y, &m->pool, &m->e,
                       &m->z, &m->nrm, &m->dz, &m->de, &m->dpool, &m->dh, &m->dO, &m->dqkv, &m->dx2,
-                      &m->dpre, &m->packed})
+                      &m->dpre, &m->packed, &m->packed_w})
         b->release();
     delete m;
 }

@@ -43,7 +43,7 @@ struct GemmEpi {
 };
 
 // A matrix packed once for both of its products: as rows (op(A) = A) it is a K-major operand, and the
-// same blocks, read along their rows, are the MN-major operand of A^T.  cols is a multiple of 128.
+// same blocks, read along their rows, are the MN-major operand of A^T (cols a multiple of 128).
 struct Packed {
     const uint8_t* op = nullptr;
     int rows = 0, cols = 0;
@@ -51,9 +51,19 @@ struct Packed {
 constexpr size_t packed_bytes(int64_t rows, int cols) { return size_t((rows + 127) / 128 * 128) * size_t(cols) * 2; }
 Packed pack_matrix(const PackSrc& s, int rows, int cols, uint8_t* op, cudaStream_t st);  // op: packed_bytes
 
-// C (=, +=) A op(B), A [M x K] packed, op(B) = B or B^T.
-void gemm_packed(const Packed& A, bool tb, int N, const PackSrc& B, float* C, int ldc, bool accumulate,
-                 const GemmEpi& epi, cudaStream_t st, int sms);
+// Weights as B operands, all of a step's in one launch: rows x cols (multiples of 128 and 64) from x[r][c], or
+// from x[c][r] when trans.  Each takes packed_bytes(rows, cols), one after another from op.
+struct WeightSrc {
+    const float* x = nullptr;
+    int ld = 0, rows = 0, cols = 0;
+    bool trans = false;
+};
+constexpr int kMaxWeights = 10;
+void pack_weights(const WeightSrc* w, int n, uint8_t* op, Packed* out, cudaStream_t st);
+
+// C (=, +=) A B^T, A [M x K] and B [N x K] packed.
+void gemm_packed(const Packed& A, const Packed& B, float* C, int ldc, bool accumulate, const GemmEpi& epi,
+                 cudaStream_t st, int sms);
 // C += A^T B, both packed with the same rows.
 void gemm_packed_tn(const Packed& A, const Packed& B, float* C, int ldc, cudaStream_t st, int sms);
 
