@@ -263,7 +263,7 @@ def kernel_roofline(w, cells: float, seconds: float, clocks, int_peaks=None) -> 
     gap block: counted at two cells per conflict-free LDS.32 of a packed penalty word (2 B/cell) and
     one ``__viaddmin_s16x2``, against the LDS.32 rate (4 B per lane-load).  The kernel packs four
     queries' penalties as bytes of a word (two as 16-bit halves only above 255), so its lookups take half
-    of what is counted; its bound is instruction issue (profiles/gapblock_fast_kernel_quads.md).
+    of what is counted; its bound is instruction issue (80 % of the slots).
     alignment: DPX.  A DPX instruction updates one int16x2 cell pair.  Local mode needs 6 of them
     per pair (M, X, Y, H and the two gap extends) -- 3 per cell; global mode keeps the states
     raised by (i+j)*gap_extend, which folds each gap extend into its add-max, so 4 per pair -- 2
