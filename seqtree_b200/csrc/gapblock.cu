@@ -337,7 +337,7 @@ struct FastArgs {
     const int4* tasks;
     const int4* chunks;      // (first task, tasks, slab byte offset, slab bytes)
     FastSmem sm;
-    int score16;             // sparse scores of 16 bits (else 8: the threshold is at most 255)
+    int score16;             // sparse sums of 16 bits (else 8: no hit's sum is above 255)
     int spread;              // rows past the query that a mixed task's diagonal may read
     const uint32_t* prior2;  // rows (M*W1 + d) of pstride words: [3] the first value, [4 + j] steps
     int pstride;
@@ -834,6 +834,7 @@ struct GbTables {
     DevBuf buf;
     const uint32_t* prior2 = nullptr;
     const int32_t *pen = nullptr, *ftab = nullptr;
+    int32_t least_term = 0;  // of ftab: below 0 where a prior's minimum outweighs the gap cost
 };
 
 GbTables& gb_tables(int device) {
@@ -885,6 +886,7 @@ void build_tables(GbTables& tb, const std::vector<int32_t>& pen, int32_t go, int
             ftab[size_t(m) * W1 + n] = int32_t(uint32_t(pmin) + uint32_t(go) +
                                                uint32_t(d - 1) * uint32_t(ge));
         }
+    tb.least_term = *std::min_element(ftab.begin(), ftab.end());
     // one upload: prior steps (16-byte rows), penalties, terms
     std::vector<uint32_t> up(std::move(prior2));
     const size_t pen_at = up.size(), ftab_at = pen_at + pen.size();
@@ -984,6 +986,36 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
 
     const int W = longest, W1 = W + 1;
     const bool wide = maxpen > 255;  // the penalties of four queries do not fit one word
+    // Tables for this (matrix, gaps, prior, lengths): rebuilt only when they change, so repeated
+    // calls with the same arguments enqueue nothing but the kernel.
+    GbTables& tb = gb_tables(ctx.device);
+    if (fast) {
+        const int64_t hdr[8] = {A, go, ge, W, int64_t(prior_width), has_prior, 0, 0};
+        const struct {
+            const void* p;
+            size_t n;
+        } parts[3] = {{hdr, sizeof hdr}, {pen.data(), pen.size() * 4},
+                      {prior, has_prior ? size_t(prior_len) * 4 : 0}};
+        Phase ph("tables");
+        bool same = tb.key.size() == parts[0].n + parts[1].n + parts[2].n;
+        size_t at = 0;
+        for (const auto& part : parts) {
+            same = same && (part.n == 0 || std::memcmp(tb.key.data() + at, part.p, part.n) == 0);
+            at += part.n;
+        }
+        if (!same) {
+            tb.key.clear();  // set again once everything is uploaded
+            build_tables(tb, pen, go, ge, W, has_prior ? prior : nullptr, W1p, stream);
+            for (const auto& part : parts) {
+                const auto* bytes = static_cast<const uint8_t*>(part.p);
+                if (part.n) tb.key.insert(tb.key.end(), bytes, bytes + part.n);
+            }
+        }
+    }
+    // A sparse tile keeps a hit's sum without its term, at most threshold - term; sums stay below
+    // 2^15, so two bytes always hold one.
+    const bool score16 = sink && int64_t(sink->thresh) - tb.least_term > 255;
+
     const FastKernel kern = fast_kernel(has_prior, wide, sink != nullptr);
     const int tuned_choice =
         t_force_rc ? -1
@@ -993,7 +1025,7 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
     FastSmem sm{};
     auto layout = [&](const RefPlan& rp) {
         return fast_smem(prof_bytes(qs.max_len, rp.max_spread, wide), int(rp.max_slab), rp.rc, W1,
-                         rp.max_tasks, sink ? (sink->thresh > 255 ? 2 : 1) : 0);
+                         rp.max_tasks, sink ? (score16 ? 2 : 1) : 0);
     };
     if (fast) {
         RefPlan& rp = plan_slot<RefPlan>(rs.gb_ref_plan, ctx.tmp_ref_plan, rs.owns);
@@ -1077,33 +1109,6 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
     }
     RefPlan& rp = *rpp;
 
-    // Tables for this (matrix, gaps, prior, lengths): rebuilt only when they change, so repeated
-    // calls with the same arguments enqueue nothing but the kernel.
-    GbTables& tb = gb_tables(ctx.device);
-    {
-        const int64_t hdr[8] = {A, go, ge, W, int64_t(prior_width), has_prior, 0, 0};
-        const struct {
-            const void* p;
-            size_t n;
-        } parts[3] = {{hdr, sizeof hdr}, {pen.data(), pen.size() * 4},
-                      {prior, has_prior ? size_t(prior_len) * 4 : 0}};
-        Phase ph("tables");
-        bool same = tb.key.size() == parts[0].n + parts[1].n + parts[2].n;
-        size_t at = 0;
-        for (const auto& part : parts) {
-            same = same && (part.n == 0 || std::memcmp(tb.key.data() + at, part.p, part.n) == 0);
-            at += part.n;
-        }
-        if (!same) {
-            tb.key.clear();  // set again once everything is uploaded
-            build_tables(tb, pen, go, ge, W, has_prior ? prior : nullptr, W1p, stream);
-            for (const auto& part : parts) {
-                const auto* bytes = static_cast<const uint8_t*>(part.p);
-                if (part.n) tb.key.insert(tb.key.end(), bytes, bytes + part.n);
-            }
-        }
-    }
-
     // Query pairs and their profile (rebuilt when the set or the penalty grid changes).
     const bool row_block = r0 != 0 || (r1 >= 0 && r1 != N);
     QueryPlan& qp = row_block ? plan_slot<QueryPlan>(ctx.tmp_block_plan, ctx.tmp_block_plan, false)
@@ -1149,7 +1154,7 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
     fa.chunks = static_cast<int4*>(rp.d_plan.ptr);
     fa.tasks = fa.chunks + rp.nchunks;
     fa.sm = sm;
-    fa.score16 = sink && sink->thresh > 255;
+    fa.score16 = score16;
     fa.spread = rp.max_spread;
     fa.prior2 = has_prior ? tb.prior2 : nullptr;
     fa.ftab = tb.ftab;
