@@ -64,6 +64,7 @@ constexpr int kQuads = 4;       // quads per slice
 constexpr int kSliceQ = 4 * kQuads;
 constexpr int kNullCode = 31;   // a residue past a ref's end: its profile column is 0
 constexpr int kMaxSum = 8191;   // largest sum of penalties along a pair that the fast form takes
+constexpr int kMaxHalf = 32767; // largest value of a packed half
 constexpr int kMaxSpread = 8;   // lengths of one warp task differ by at most this
 constexpr int kTileW = 2 * kQuads + 1;  // tile words per column: 8 results and the (m, n) term
 static_assert(kWarps == 2 * kQuads, "the dense write-out gives each result word one warp");
@@ -502,7 +503,9 @@ __device__ __forceinline__ bool run_unit(const FastArgs& a, const uint8_t* s_pro
 // which with 8-bit scores fit at the 1,024-column width: 148 -> 139 ms on 100,000 x 1,000,000 (a
 // tile's staging and its barriers are then covered by three others).  Narrower chunks
 // cost more tiles: 3.0 (1,024) / 3.3 (768) / 3.8 (512) / 5.1 ms (256) per 2e9 pairs.
-template <bool PRIOR, bool WIDE, bool SPARSE>
+// WRAPS: the sparse form where some sum + term may pass the end of int32 (a test of its own on every
+// hit costs 7 % where 2.75 % of the cells are hits, so it is a variant).
+template <bool PRIOR, bool WIDE, bool SPARSE, bool WRAPS = false>
 __global__ void __launch_bounds__(kThreads, SPARSE ? 4 : 3) gapblock_fast_kernel(const FastArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
     const FastSmem& sm = a.sm;
@@ -547,12 +550,13 @@ __global__ void __launch_bounds__(kThreads, SPARSE ? 4 : 3) gapblock_fast_kernel
     // Per-tile metadata: the (m, n) terms, the chunk's tasks, each sorted slot's column and length.
     // Rows past the query keep the null column at 0 for lanes past their ref's end.
     // The sparse form keeps the test word instead of the term: 0x8000 + T in both halves, T =
-    // threshold - term; a half is a hit when it is at most T, bit 15 of the difference.
+    // threshold - term; a half is a hit when it is at most T, bit 15 of the difference.  Beside a term
+    // so near the end of int32 that the score may wrap below 0, every half is tested again as a score.
     for (int i = tid; i < a.W1; i += kThreads) {
         const int32_t f = a.ftab[m * a.W1 + i];
-        const int64_t room = int64_t(a.sink.thresh) - f;
+        const int64_t room = WRAPS && f > INT32_MAX - kMaxHalf ? kMaxHalf : int64_t(a.sink.thresh) - f;
         s_frow[i] = !SPARSE ? f
-                    : room >= 0 ? int32_t(0x80008000u + uint32_t(room < 32767 ? room : 32767) * 0x10001u)
+                    : room >= 0 ? int32_t(0x80008000u + uint32_t(room < kMaxHalf ? room : kMaxHalf) * 0x10001u)
                                 : 0x7FFF7FFF;
     }
     for (int i = tid; i < a.spread * kQuads * (WIDE ? 2 : 1); i += kThreads)
@@ -613,6 +617,8 @@ __global__ void __launch_bounds__(kThreads, SPARSE ? 4 : 3) gapblock_fast_kernel
                         // word q of quad q / 2: queries (q & 1) and (q & 1) + 2
                         const int row = (q >> 1) * 4 + (q & 1);
                         auto keep = [&](int at, uint32_t v) {
+                            if (WRAPS && int32_t((v & 0xFFFFu) + uint32_t(__ldg(a.ftab + m * a.W1 + n))) > a.sink.thresh)
+                                return;
                             atomicOr(s_bits + at * (a.rc / 32) + (col >> 5), 1u << (col & 31));
                             if (a.score16)
                                 reinterpret_cast<uint16_t*>(s_score)[at * a.rc + col] = uint16_t(v);
@@ -699,9 +705,9 @@ __global__ void __launch_bounds__(kThreads, SPARSE ? 4 : 3) gapblock_fast_kernel
                     const int c = (w0 + lane) * 32 + __ffs(int(word)) - 1;
                     word &= word - 1;
                     const int at = row * a.rc + c;
-                    const int v = a.score16 ? reinterpret_cast<const uint16_t*>(s_score)[at] : s_score[at];
-                    a.sink.seg[pos++] =
-                        make_int2(int(k0 + c), v + __ldg(a.ftab + m * a.W1 + a.rlen[k0 + c]));
+                    const uint32_t v = a.score16 ? reinterpret_cast<const uint16_t*>(s_score)[at] : s_score[at];
+                    a.sink.seg[pos++] = make_int2(
+                        int(k0 + c), int(v + uint32_t(__ldg(a.ftab + m * a.W1 + a.rlen[k0 + c]))));
                 }
                 off += (unsigned long long)__shfl_sync(full, incl, 31);
             }
@@ -816,12 +822,10 @@ __global__ void __launch_bounds__(256) gapblock_general_kernel(const GeneralArgs
 
 using FastKernel = void (*)(FastArgs);
 
-FastKernel fast_kernel(bool prior, bool wide, bool sparse) {
-    if (sparse)
-        return prior ? (wide ? gapblock_fast_kernel<true, true, true> : gapblock_fast_kernel<true, false, true>)
-                     : (wide ? gapblock_fast_kernel<false, true, true> : gapblock_fast_kernel<false, false, true>);
-    return prior ? (wide ? gapblock_fast_kernel<true, true, false> : gapblock_fast_kernel<true, false, false>)
-                 : (wide ? gapblock_fast_kernel<false, true, false> : gapblock_fast_kernel<false, false, false>);
+template <bool SPARSE, bool WRAPS>
+FastKernel fast_kernel(bool prior, bool wide) {
+    return prior ? (wide ? gapblock_fast_kernel<true, true, SPARSE, WRAPS> : gapblock_fast_kernel<true, false, SPARSE, WRAPS>)
+                 : (wide ? gapblock_fast_kernel<false, true, SPARSE, WRAPS> : gapblock_fast_kernel<false, false, SPARSE, WRAPS>);
 }
 
 // Words per prior row: the first value at 3, step j at 4 + j, rounded up so that every row is
@@ -835,6 +839,7 @@ struct GbTables {
     const uint32_t* prior2 = nullptr;
     const int32_t *pen = nullptr, *ftab = nullptr;
     int32_t least_term = 0;  // of ftab: below 0 where a prior's minimum outweighs the gap cost
+    int32_t most_term = 0;
 };
 
 GbTables& gb_tables(int device) {
@@ -887,6 +892,7 @@ void build_tables(GbTables& tb, const std::vector<int32_t>& pen, int32_t go, int
                                                uint32_t(d - 1) * uint32_t(ge));
         }
     tb.least_term = *std::min_element(ftab.begin(), ftab.end());
+    tb.most_term = *std::max_element(ftab.begin(), ftab.end());
     // one upload: prior steps (16-byte rows), penalties, terms
     std::vector<uint32_t> up(std::move(prior2));
     const size_t pen_at = up.size(), ftab_at = pen_at + pen.size();
@@ -1013,10 +1019,13 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
         }
     }
     // A sparse tile keeps a hit's sum without its term, at most threshold - term; sums stay below
-    // 2^15, so two bytes always hold one.
-    const bool score16 = sink && int64_t(sink->thresh) - tb.least_term > 255;
+    // 2^15, so two bytes always hold one.  Where sum + term can pass the end of int32 any sum is kept.
+    const bool wraps = sink && tb.most_term > INT32_MAX - kMaxHalf;
+    const FastKernel kern = wraps  ? fast_kernel<true, true>(has_prior, wide)
+                            : sink ? fast_kernel<true, false>(has_prior, wide)
+                                   : fast_kernel<false, false>(has_prior, wide);
+    const bool score16 = sink && (wraps || int64_t(sink->thresh) - tb.least_term > 255);
 
-    const FastKernel kern = fast_kernel(has_prior, wide, sink != nullptr);
     const int tuned_choice =
         t_force_rc ? -1
                    : tuned_lookup(sink ? "sparse|" + gb_shape_key(qs, rs, has_prior)

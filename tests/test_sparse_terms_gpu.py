@@ -59,3 +59,15 @@ def test_priors_below_zero(stb, low, hi):
                                   prior_width=hi, threads=os.cpu_count() or 1)
     assert np.array_equal(dense, want)
     check_rows(dense, rows)
+
+
+@pytest.mark.parametrize("below", [0, 5, 60, 3000])
+@pytest.mark.parametrize("t", [0, 24, 300, 2 ** 31 - 1])
+def test_terms_at_the_end_of_int32(stb, below, t):
+    """A gap cost so near 2^31 that a score wraps below 0 for some sums and not for others: the rows
+    are still those of the dense matrix, which wraps as the reference's int32 arithmetic does."""
+    rng = np.random.default_rng(below)
+    q, r = rand_seqs(rng, 33, 8, 25), rand_seqs(rng, 600, 8, 25)
+    dense, rows = dense_and_rows(q, r, stb.SubstitutionMatrix.blosum62(), (t,), 2 ** 31 - 1 - below, 1, (), 0)
+    assert below == 3000 or (dense < 0).any()
+    check_rows(dense, rows)
