@@ -158,11 +158,13 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv2_gemm_kernel(GemmArgs g)
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((uintptr_t(smem_raw) + 1023) & ~uintptr_t(1023));
     // barriers: 0 weights, 1-3 tile loaded, 4-6 tile read by its store, 7-8 accumulator full, 9-10
-    // accumulator empty (an arrival per drain warp), 11 output in place (16), 12 MMA drain
+    // accumulator empty (an arrival per drain warp), 11-13 output in place (16), 14 MMA drain.  No drain
+    // warp waits for the store warp, so the output has a barrier per stage: a stage's next tile is loaded
+    // only after its store, so that barrier cannot run a phase ahead of the store warp's wait.
     const uint32_t bar0 = smem_u32(smem + S::kSmBar);
     auto BAR = [&](int i) { return bar0 + 8u * uint32_t(i); };
-    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + S::kSmBar + 104);
-    volatile int* s_abort = reinterpret_cast<volatile int*>(smem + S::kSmBar + 108);
+    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(smem + S::kSmBar + 120);
+    volatile int* s_abort = reinterpret_cast<volatile int*>(smem + S::kSmBar + 124);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -170,13 +172,13 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv2_gemm_kernel(GemmArgs g)
         for (int s = 0; s < kGemmStages; ++s) {
             bar_init(BAR(1 + s), 1);
             bar_init(BAR(4 + s), 1);
+            bar_init(BAR(11 + s), kConvDrain);
         }
         for (int h = 0; h < 2; ++h) {
             bar_init(BAR(7 + h), 1);
             bar_init(BAR(9 + h), kConvDrain);
         }
-        bar_init(BAR(11), kConvDrain);
-        bar_init(BAR(12), 1);
+        bar_init(BAR(14), 1);
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_smem();
@@ -236,19 +238,21 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv2_gemm_kernel(GemmArgs g)
                 accphase ^= 1u;
             }
         }
-        tc_commit(BAR(12));
-        bar_drain(BAR(12), 0);
+        tc_commit(BAR(14));
+        bar_drain(BAR(14), 0);
     } else if (warp == 2 + kConvDrain) {
         // ----------------------------------------------------------------- stores ---------
         if (lane == 0) {
             uint32_t ph = 0, stage = 0;
             for (int64_t tile = blockIdx.x; tile < g.tiles; tile += gridDim.x) {
-                if (!bar_wait(BAR(11), ph, s_abort, g.err)) break;
+                if (!bar_wait(BAR(11 + stage), ph, s_abort, g.err)) break;
                 bulk_store(g.out + tile * kTileBytes, sA + stage * kTileBytes, kTileBytes);
                 bulk_store_drain();
                 bar_arrive(BAR(4 + stage));
-                ph ^= 1u;
-                if (++stage == kGemmStages) stage = 0;
+                if (++stage == kGemmStages) {
+                    stage = 0;
+                    ph ^= 1u;
+                }
             }
         }
     } else if (warp >= 2) {
@@ -316,7 +320,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv2_gemm_kernel(GemmArgs g)
             if (!ok) break;
             fence_async_smem();  // all 16 warps' rows -> one bulk store
             __syncwarp();
-            if (lane == 0) bar_arrive(BAR(11));
+            if (lane == 0) bar_arrive(BAR(11 + stage));
             if (++stage == kGemmStages) stage = 0;
             accphase ^= 1u;
         }
