@@ -138,6 +138,11 @@ constexpr int kConvDrain = 16;     // drain warps: a lane quarter x 16 channels 
 constexpr int kConvThreads = 96 + kConvDrain * 32;  // warp 0 loads, 1 issues MMAs, 2-17 drain, 18 stores
 constexpr int kGemmStages = 3;
 
+// x += y where `on` is not 0, as one predicated add.
+__device__ __forceinline__ void add_if(float& x, float y, uint32_t on) {
+    asm("{ .reg .pred p; setp.ne.u32 p, %2, 0; @p add.f32 %0, %0, %1; }" : "+f"(x) : "f"(y), "r"(on));
+}
+
 struct Conv2Shape {
     static constexpr int N = 384;
     static constexpr int kW_ = N * kW * 2;                         // weight bytes
@@ -260,7 +265,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv2_gemm_kernel(GemmArgs g)
         const int quarter = warp & 3, part = (warp - 2) >> 2;  // this warp's lanes, 16 channels of a half
         const int r = quarter * 32 + lane;
         const uint32_t tl = tmem + (uint32_t(quarter * 32) << 16);
-        const float above = lane > 0 ? 1.f : 0.f, below = lane < 31 ? 1.f : 0.f;
+        const uint32_t above = lane > 0, below = lane < 31;
         uint32_t stage = 0, accphase = 0;
         for (int64_t tile = blockIdx.x; tile < g.tiles; tile += gridDim.x) {
             const int L = g.lens[tile * kSeqPerTile + quarter];
@@ -309,7 +314,11 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv2_gemm_kernel(GemmArgs g)
                             const int j = u * 8 + e * 2 + q;
                             const float up = __shfl_up_sync(0xffffffffu, __uint_as_float(y0[j]), 1);
                             const float dn = __shfl_down_sync(0xffffffffu, __uint_as_float(y2[j]), 1);
-                            const float pre = fmaf(dn, below, fmaf(up, above, __uint_as_float(y1[j]))) + bias[e * 2 + q];
+                            // (left out, not multiplied by 0: a value from outside the sequence may be infinite)
+                            float pre = __uint_as_float(y1[j]);
+                            add_if(pre, up, above);
+                            add_if(pre, dn, below);
+                            pre += bias[e * 2 + q];
                             o2[q] = valid ? (q ? x.y : x.x) + fmaxf(pre, 0.f) : 0.f;
                         }
                         pk.h[e] = __floats2bfloat162_rn(o2[0], o2[1]);
