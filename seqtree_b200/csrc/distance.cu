@@ -81,8 +81,26 @@ struct DistPlan {
 struct DistCodes {
     DistPlan *a, *b;
     int sigma;
-    bool fresh;  // codes were enqueued on the call's stream just now
+    uint32_t symbols[8];
+    bool fresh;  // codes were enqueued on the call's stream just now: valid once settle() returns
+
+    void made() {
+        for (DistPlan* p : {a, b}) {
+            std::memcpy(p->symbols, symbols, 32);
+            p->coded = true;
+        }
+    }
 };
+
+// Codes and packed words are made before the call that needs them, never as part of a captured graph
+// (a capture would only record the launches, and the wait below would end it).
+void refuse_capture(cudaStream_t stream) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    STB_CUDA(cudaStreamIsCapturing(stream, &st));
+    if (st != cudaStreamCaptureStatusNone)
+        fail(ST_EINVAL, "seqtree_b200: this call has codes or packed words of a set to make; make the same "
+                        "call once before capturing it into a CUDA graph");
+}
 
 // A set's codes may next be read from another stream: waits for them once they are made.
 void settle(const st_seqset_s& a, const st_seqset_s& b, cudaStream_t stream) {
@@ -105,6 +123,7 @@ DistCodes compute_codes(st_seqset_s& a, st_seqset_s& b, cudaStream_t stream, Con
     auto* present = reinterpret_cast<unsigned int*>(ctx.flags_d + 16);
     const auto* bits = reinterpret_cast<const unsigned int*>(ctx.flags_h + 16);
     if (plans[0]->uid != a.uid || plans[1]->uid != b.uid) {
+        refuse_capture(stream);
         STB_CUDA(cudaMemsetAsync(present, 0, 64, stream));
         TwoSets args{};
         for (int t = 0; t < 2; ++t) {
@@ -136,6 +155,7 @@ DistCodes compute_codes(st_seqset_s& a, st_seqset_s& b, cudaStream_t stream, Con
         st_seqset_s* s = sets[t];
         DistPlan& p = *plans[t];
         if (p.coded && std::memcmp(p.symbols, symbols, 32) == 0) continue;
+        refuse_capture(stream);
         // kernels on other streams may still read the codes of the last alphabet
         if (p.coded && s->owns) STB_CUDA(cudaDeviceSynchronize());
         p.coded = false;
@@ -151,13 +171,10 @@ DistCodes compute_codes(st_seqset_s& a, st_seqset_s& b, cudaStream_t stream, Con
         remap_kernel<<<grid, 256, 0, stream>>>(args, lut);
         STB_CUDA(cudaGetLastError());
         note_launch(nullptr);
-        for (DistPlan* p : plans) {
-            std::memcpy(p->symbols, symbols, 32);
-            p->coded = true;
-        }
     }
-    const bool fresh = todo > 0;
-    return DistCodes{plans[0], plans[1], sigma, fresh};
+    DistCodes dc{plans[0], plans[1], sigma, {}, todo > 0};
+    std::memcpy(dc.symbols, symbols, 32);
+    return dc;
 }
 
 // ---------------------------------------------------------------------------- Hamming -------
@@ -495,7 +512,7 @@ void hamming_sets(st_seqset_s& a, st_seqset_s& b, int32_t* out_d, cudaStream_t s
                             std::to_string(a.h_len[size_t(bi)]) + " and " +
                             std::to_string(b.h_len[size_t(bk)]) + ")");
     Context& ctx = context();
-    const DistCodes dc = compute_codes(a, b, stream, ctx);
+    DistCodes dc = compute_codes(a, b, stream, ctx);
     const int sigma = dc.sigma;
     const int B = sigma <= 2 ? 1 : sigma <= 4 ? 2 : sigma <= 16 ? 4 : 8;
     const int per = 32 / B;
@@ -512,19 +529,24 @@ void hamming_sets(st_seqset_s& a, st_seqset_s& b, int32_t* out_d, cudaStream_t s
         pa.off[todo] = sets[t]->d_off;
         pa.count[todo] = sets[t]->count;
         pa.packed[todo++] = sets[t]->d_packed;
-        p.packB = B;
-        p.packW = W;
+        p.packB = p.packW = 0;
     }
     if (todo) {
+        refuse_capture(stream);
         fresh = true;
         const int64_t most = std::max(pa.count[0], pa.count[1]);
         pack_kernel<<<dim3(unsigned(ceil_div(most, 256)), unsigned(todo)), 256, 0, stream>>>(pa, L, B, W);
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) plans[0]->packB = plans[1]->packB = 0;
-        STB_CUDA(e);
+        STB_CUDA(cudaGetLastError());
         note_launch(nullptr);
     }
-    if (fresh) settle(a, b, stream);
+    if (fresh) {  // recorded as made only now that they are
+        settle(a, b, stream);
+        dc.made();
+        for (DistPlan* p : plans) {
+            p->packB = B;
+            p->packW = W;
+        }
+    }
     const uint32_t* qp = a.d_packed;
     const uint32_t* rp = b.d_packed;
     const char* name;
@@ -546,8 +568,11 @@ void levenshtein_sets(st_seqset_s& a, st_seqset_s& b, int32_t* out_d, cudaStream
     const int64_t N = r1 - r0, K = b.count;
     if (N == 0 || K == 0) return;
     Context& ctx = context();
-    const DistCodes dc = compute_codes(a, b, stream, ctx);
-    if (dc.fresh) settle(a, b, stream);
+    DistCodes dc = compute_codes(a, b, stream, ctx);
+    if (dc.fresh) {
+        settle(a, b, stream);
+        dc.made();
+    }
     const int sigma = std::max(1, dc.sigma);
     const uint8_t* ac = a.d_codes;
     const uint8_t* bc = b.d_codes;
