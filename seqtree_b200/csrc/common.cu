@@ -238,6 +238,32 @@ DevBuf::~DevBuf() {
     // Contexts live until process exit; the driver reclaims device memory then.
 }
 
+void StreamScratch::take(int device, size_t bytes, cudaStream_t st) {
+    if (!bytes) return;
+    constexpr uint64_t kKeep = uint64_t(256) << 20;  // bytes that stay cached in the pool
+    static std::mutex mu;
+    static std::map<int, cudaMemPool_t> pools;
+    cudaMemPool_t pool;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        cudaMemPool_t& slot = pools[device];
+        if (!slot) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = device;
+            cudaMemPool_t fresh = nullptr;
+            STB_CUDA(cudaMemPoolCreate(&fresh, &props));
+            uint64_t keep_bytes = kKeep;
+            STB_CUDA(cudaMemPoolSetAttribute(fresh, cudaMemPoolAttrReleaseThreshold, &keep_bytes));
+            slot = fresh;
+        }
+        pool = slot;
+    }
+    STB_CUDA(cudaMallocFromPoolAsync(&ptr, bytes, pool, st));
+    stream = st;
+}
+
 void h2d(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
     if (bytes == 0) return;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;

@@ -75,6 +75,27 @@ struct OwnedBuf : DevBuf {
     ~OwnedBuf() { release(); }
 };
 
+// Stream-ordered memory from a pool of the library's own: calls on several streams each get theirs, a
+// captured call gets its allocation as graph nodes, and a bounded amount stays cached for the next.  Freed
+// on the stream it was taken for, unless keep() hands it to an owner.
+struct StreamScratch {
+    void* ptr = nullptr;
+    cudaStream_t stream = nullptr;
+    StreamScratch() = default;
+    StreamScratch(int device, size_t bytes, cudaStream_t st) { take(device, bytes, st); }
+    void take(int device, size_t bytes, cudaStream_t st);
+    void* keep() {
+        void* p = ptr;
+        ptr = nullptr;
+        return p;
+    }
+    ~StreamScratch() {
+        if (ptr) cudaFreeAsync(ptr, stream);
+    }
+    StreamScratch(const StreamScratch&) = delete;
+    StreamScratch& operator=(const StreamScratch&) = delete;
+};
+
 struct Context {
     int device = 0;
     std::mutex mu;              // serialises calls on this device

@@ -1,8 +1,8 @@
 // Dense Hamming and Levenshtein matrices over raw bytes (case-sensitive) on sm_100a.
 //
 // Reference: seqtree src/distance.cpp:68-109.  Both distances compare bytes for equality only,
-// so each call first maps the bytes present in either set to dense codes 0..sigma-1 (any
-// bijection preserves equality) and then:
+// so a call maps the bytes present in either set to dense codes 0..sigma-1 (any bijection preserves
+// equality; the table travels with the launch) and then:
 //
 //   Hamming (output-write bound): every string is packed at b = 1/2/4/8 bits per symbol into
 //   32-bit words; a pair costs one XOR, one fold of each symbol's b bits onto its lowest bit and
@@ -25,30 +25,16 @@ namespace stb {
 
 namespace {
 
-// ---------------------------------------------------------------------------- remap ---------
-struct ByteLut {
+// ------------------------------------------------------------------------- alphabets -------
+struct alignas(4) ByteLut {
     uint8_t v[256];
 };
 
-// Up to two sets' buffers in one launch, a set per blockIdx.y.
+// Up to two sets' bytes in one launch, a set per blockIdx.y.
 struct TwoSets {
     const uint8_t* in[2];
-    uint8_t* out[2];
     int64_t bytes[2];
 };
-
-// Dense codes of each set's bytes, and 64 zero bytes past them.
-__global__ void remap_kernel(const TwoSets t, ByteLut lut) {
-    __shared__ uint8_t s[256];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) s[i] = lut.v[i];
-    __syncthreads();
-    const uint8_t* in = t.in[blockIdx.y];
-    uint8_t* out = t.out[blockIdx.y];
-    const int64_t n = t.bytes[blockIdx.y];
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n + 64;
-         i += int64_t(gridDim.x) * blockDim.x)
-        out[i] = i < n ? s[in[i]] : 0;
-}
 
 // Byte-presence bitmap of each set (distinct bytes -> dense codes).
 __global__ void presence_kernel(const TwoSets t, unsigned int* __restrict__ present) {
@@ -66,34 +52,41 @@ __global__ void presence_kernel(const TwoSets t, unsigned int* __restrict__ pres
     if (threadIdx.x < 8 && s[threadIdx.x]) atomicOr(&present[blockIdx.y * 8 + threadIdx.x], s[threadIdx.x]);
 }
 
-// What a set keeps for the distances: the bytes it holds, and whether its dense codes (and Hamming
-// packing) are there, under which alphabet.  The alphabet of a call is the union of both sets'
-// bytes, so sets over the same symbols keep their codes from call to call whatever they are
-// paired with, and such calls enqueue no host round trip (and can be captured in a CUDA graph).
-struct DistPlan {
-    uint64_t uid = 0;               // set the plan was built for
-    uint32_t present[8] = {};       // bytes of the set
-    uint32_t symbols[8] = {};       // bytes the codes were built for
-    bool coded = false;
-    int packB = 0, packW = 0;       // Hamming packing built for (bits, words); 0 = none
+// What a set keeps for the distances: which bytes it holds, and its dense codes (Levenshtein) and
+// packed words (Hamming) under the alphabets it has met.  The alphabet of a call is the union of both
+// sets' bytes.  Nothing here is ever written again once it is made, so calls on several streams and
+// captured graphs may read it for as long as the set lives, whatever partners the set meets in
+// between; an alphabet past the last place is coded for its call alone.
+constexpr int kMaxKept = 4;  // of either kind
+
+enum Form { kCodes, kWords };
+
+struct Kept {
+    Form form;
+    uint32_t symbols[8];
+    void* ptr;
 };
 
-struct DistCodes {
-    DistPlan *a, *b;
-    int sigma;
-    uint32_t symbols[8];
-    bool fresh;  // codes were enqueued on the call's stream just now: valid once settle() returns
-
-    void made() {
-        for (DistPlan* p : {a, b}) {
-            std::memcpy(p->symbols, symbols, 32);
-            p->coded = true;
-        }
+struct DistPlan {
+    uint64_t uid = 0;               // set the plan was built for
+    bool owns = true;               // false: a transient set's, in buffers that the next one takes over
+    uint32_t present[8] = {};       // bytes of the set
+    std::vector<Kept> kept;
+    DevBuf transient[2];            // by form
+    ~DistPlan() {  // (with the set, after its bytes: freeing those waits for the kernels that read either)
+        for (const Kept& k : kept)
+            if (owns) cudaFree(k.ptr);
     }
 };
 
-// Codes and packed words are made before the call that needs them, never as part of a captured graph
-// (a capture would only record the launches, and the wait below would end it).
+struct Alphabet {
+    uint32_t symbols[8];
+    ByteLut lut;   // byte -> 0 .. sigma - 1
+    int sigma;
+};
+
+// What a set keeps is made before a capture, not as part of it (a capture would only record the
+// launches, and the wait for them would end it).
 void refuse_capture(cudaStream_t stream) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     STB_CUDA(cudaStreamIsCapturing(stream, &st));
@@ -102,24 +95,18 @@ void refuse_capture(cudaStream_t stream) {
                         "call once before capturing it into a CUDA graph");
 }
 
-// A set's codes may next be read from another stream: waits for them once they are made.
-void settle(const st_seqset_s& a, const st_seqset_s& b, cudaStream_t stream) {
-    if (a.owns || b.owns) STB_CUDA(cudaStreamSynchronize(stream));
-}
-
 DistPlan& dist_plan(st_seqset_s& s, Context& ctx, int slot) {
     std::shared_ptr<void>& holder = s.owns ? s.dist_plan : ctx.tmp_dist_plan[slot];
-    if (!holder) holder = std::make_shared<DistPlan>();
+    if (!holder) {
+        holder = std::make_shared<DistPlan>();
+        static_cast<DistPlan*>(holder.get())->owns = s.owns;
+    }
     return *static_cast<DistPlan*>(holder.get());
 }
 
-DistCodes compute_codes(st_seqset_s& a, st_seqset_s& b, cudaStream_t stream, Context& ctx) {
-    st_seqset_s* sets[2] = {&a, &b};
-    DistPlan* plans[2] = {&dist_plan(a, ctx, 0), &dist_plan(b, ctx, 1)};
-    auto blocks_of = [&ctx](const TwoSets& t) {
-        const int64_t most = std::max<int64_t>({t.bytes[0], t.bytes[1], 1});
-        return dim3(unsigned(std::min<int64_t>(ceil_div(most, 256), ctx.num_sms * 4)), 2);
-    };
+Alphabet joint_alphabet(st_seqset_s& a, st_seqset_s& b, DistPlan* const plans[2], cudaStream_t stream,
+                        Context& ctx) {
+    const st_seqset_s* sets[2] = {&a, &b};
     auto* present = reinterpret_cast<unsigned int*>(ctx.flags_d + 16);
     const auto* bits = reinterpret_cast<const unsigned int*>(ctx.flags_h + 16);
     if (plans[0]->uid != a.uid || plans[1]->uid != b.uid) {
@@ -130,7 +117,9 @@ DistCodes compute_codes(st_seqset_s& a, st_seqset_s& b, cudaStream_t stream, Con
             args.in[t] = sets[t]->d_bytes;
             args.bytes[t] = plans[t]->uid == sets[t]->uid ? 0 : sets[t]->total;
         }
-        presence_kernel<<<blocks_of(args), 256, 0, stream>>>(args, present);
+        const int64_t most = std::max<int64_t>({args.bytes[0], args.bytes[1], 1});
+        presence_kernel<<<dim3(unsigned(std::min<int64_t>(ceil_div(most, 256), ctx.num_sms * 4)), 2), 256, 0,
+                          stream>>>(args, present);
         STB_CUDA(cudaGetLastError());
         note_launch(nullptr);
         STB_CUDA(cudaMemcpyAsync(ctx.flags_h + 16, present, 64, cudaMemcpyDeviceToHost, stream));
@@ -138,65 +127,112 @@ DistCodes compute_codes(st_seqset_s& a, st_seqset_s& b, cudaStream_t stream, Con
         for (int t = 0; t < 2; ++t) {
             if (plans[t]->uid == sets[t]->uid) continue;
             std::memcpy(plans[t]->present, bits + 8 * t, 32);
-            plans[t]->coded = false;
+            plans[t]->kept.clear();  // (empty but for a transient set's plan)
             plans[t]->uid = sets[t]->uid;
         }
     }
-    uint32_t symbols[8];
-    for (int w = 0; w < 8; ++w) symbols[w] = plans[0]->present[w] | plans[1]->present[w];
-    ByteLut lut;
-    std::memset(lut.v, 0, sizeof lut.v);
-    int sigma = 0;
+    Alphabet al;
+    for (int w = 0; w < 8; ++w) al.symbols[w] = plans[0]->present[w] | plans[1]->present[w];
+    std::memset(al.lut.v, 0, sizeof al.lut.v);
+    al.sigma = 0;
     for (int c = 0; c < 256; ++c)
-        if (symbols[c >> 5] & (1u << (c & 31))) lut.v[c] = uint8_t(sigma++);
-    TwoSets args{};
-    int todo = 0;
-    for (int t = 0; t < 2; ++t) {
-        st_seqset_s* s = sets[t];
-        DistPlan& p = *plans[t];
-        if (p.coded && std::memcmp(p.symbols, symbols, 32) == 0) continue;
-        refuse_capture(stream);
-        // kernels on other streams may still read the codes of the last alphabet
-        if (p.coded && s->owns) STB_CUDA(cudaDeviceSynchronize());
-        p.coded = false;
-        p.packB = p.packW = 0;
-        args.in[todo] = s->d_bytes;
-        args.out[todo] = s->d_codes;
-        args.bytes[todo++] = s->total;
-        if (sets[0] == sets[1]) break;
+        if (al.symbols[c >> 5] & (1u << (c & 31))) al.lut.v[c] = uint8_t(al.sigma++);
+    return al;
+}
+
+// Both sets' codes or packed words for one call: those they keep, or room for what the call makes.
+struct CallForms {
+    void* ptr[2] = {};
+    int todo[2], count = 0;         // the sets whose form is to be made, with one launch on the call's stream
+    StreamScratch fresh[2];
+    bool keep[2] = {};
+
+    CallForms(Form form, const Alphabet& al, st_seqset_s* const sets[2], DistPlan* const plans[2],
+              const size_t bytes[2], cudaStream_t stream, Context& ctx) {
+        for (int t = 0; t < 2; ++t) {
+            if (t == 1 && sets[0] == sets[1]) {
+                ptr[1] = ptr[0];
+                break;
+            }
+            DistPlan& p = *plans[t];
+            int have = 0;
+            for (const Kept& k : p.kept) {
+                have += k.form == form;
+                if (k.form == form && std::memcmp(k.symbols, al.symbols, 32) == 0) ptr[t] = k.ptr;
+            }
+            if (ptr[t]) continue;
+            keep[t] = !p.owns || have < kMaxKept;
+            if (keep[t]) refuse_capture(stream);
+            if (p.owns) {
+                fresh[t].take(ctx.device, std::max<size_t>(bytes[t], 16), stream);
+                ptr[t] = fresh[t].ptr;
+            } else {
+                ptr[t] = p.transient[form].get(bytes[t]);
+            }
+            todo[count++] = t;
+        }
     }
-    if (todo) {
-        dim3 grid = blocks_of(args);
-        grid.y = unsigned(todo);
-        remap_kernel<<<grid, 256, 0, stream>>>(args, lut);
-        STB_CUDA(cudaGetLastError());
-        note_launch(nullptr);
+    // After the launch: what is to be kept is kept only once it is there, as the next call may be on
+    // another stream (a transient set's calls are all on one).
+    void made(Form form, const Alphabet& al, DistPlan* const plans[2], cudaStream_t stream) {
+        if ((keep[0] && plans[0]->owns) || (keep[1] && plans[1]->owns)) STB_CUDA(cudaStreamSynchronize(stream));
+        for (int t = 0; t < 2; ++t) {
+            if (!keep[t]) continue;
+            Kept k{form, {}, ptr[t]};
+            std::memcpy(k.symbols, al.symbols, 32);
+            plans[t]->kept.push_back(k);
+            fresh[t].keep();
+        }
     }
-    DistCodes dc{plans[0], plans[1], sigma, {}, todo > 0};
-    std::memcpy(dc.symbols, symbols, 32);
-    return dc;
+};
+
+// The table in shared memory (every thread of a block of at least 64 calls this).
+__device__ __forceinline__ void load_lut(uint8_t* s, const ByteLut& lut) {
+    if (threadIdx.x < 64)
+        reinterpret_cast<uint32_t*>(s)[threadIdx.x] = reinterpret_cast<const uint32_t*>(lut.v)[threadIdx.x];
+    __syncthreads();
+}
+
+// Dense codes of up to two sets' bytes, a set per blockIdx.y.
+struct RemapArgs {
+    const uint8_t* in[2];
+    uint8_t* out[2];
+    int64_t bytes[2];
+};
+
+__global__ void remap_kernel(const __grid_constant__ RemapArgs a, const __grid_constant__ ByteLut lut) {
+    __shared__ __align__(4) uint8_t code[256];
+    load_lut(code, lut);
+    const uint8_t* in = a.in[blockIdx.y];
+    uint8_t* out = a.out[blockIdx.y];
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < a.bytes[blockIdx.y];
+         i += int64_t(gridDim.x) * blockDim.x)
+        out[i] = code[in[i]];
 }
 
 // ---------------------------------------------------------------------------- Hamming -------
-// Pack each string's codes at B bits per symbol into W words (low symbol in low bits); up to two
+// Pack each string's codes (lut of its bytes) at B bits per symbol into W words (low symbol in low bits); up to two
 // sets in one launch, a set per blockIdx.y.
 struct PackArgs {
-    const uint8_t* codes[2];
+    const uint8_t* bytes[2];
     const int64_t* off[2];
     int64_t count[2];
     uint32_t* packed[2];
 };
 
-__global__ void pack_kernel(const PackArgs a, int L, int B, int W) {
+__global__ void pack_kernel(const __grid_constant__ PackArgs a, const __grid_constant__ ByteLut lut, int L, int B,
+                            int W) {
+    __shared__ __align__(4) uint8_t code[256];
+    load_lut(code, lut);
     const int64_t s = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (s >= a.count[blockIdx.y]) return;
-    const uint8_t* c = a.codes[blockIdx.y] + a.off[blockIdx.y][s];
+    const uint8_t* c = a.bytes[blockIdx.y] + a.off[blockIdx.y][s];
     const int per = 32 / B;
     for (int w = 0; w < W; ++w) {
         uint32_t v = 0;
         for (int t = 0; t < per; ++t) {
             const int j = w * per + t;
-            if (j < L) v |= uint32_t(c[j]) << (t * B);
+            if (j < L) v |= uint32_t(code[c[j]]) << (t * B);
         }
         a.packed[blockIdx.y][s * W + w] = v;
     }
@@ -512,43 +548,31 @@ void hamming_sets(st_seqset_s& a, st_seqset_s& b, int32_t* out_d, cudaStream_t s
                             std::to_string(a.h_len[size_t(bi)]) + " and " +
                             std::to_string(b.h_len[size_t(bk)]) + ")");
     Context& ctx = context();
-    DistCodes dc = compute_codes(a, b, stream, ctx);
-    const int sigma = dc.sigma;
+    st_seqset_s* sets[2] = {&a, &b};
+    DistPlan* plans[2] = {&dist_plan(a, ctx, 0), &dist_plan(b, ctx, 1)};
+    const Alphabet al = joint_alphabet(a, b, plans, stream, ctx);
+    const int sigma = al.sigma;
     const int B = sigma <= 2 ? 1 : sigma <= 4 ? 2 : sigma <= 16 ? 4 : 8;
     const int per = 32 / B;
     const int W = std::max(1, int(ceil_div(L, per)));
-    const st_seqset_s* sets[2] = {&a, &b};
-    DistPlan* plans[2] = {dc.a, dc.b};
-    bool fresh = dc.fresh;
-    PackArgs pa{};
-    int todo = 0;
-    for (int t = 0; t < 2; ++t) {
-        DistPlan& p = *plans[t];
-        if (p.packB == B && p.packW == W) continue;
-        pa.codes[todo] = sets[t]->d_codes;
-        pa.off[todo] = sets[t]->d_off;
-        pa.count[todo] = sets[t]->count;
-        pa.packed[todo++] = sets[t]->d_packed;
-        p.packB = p.packW = 0;
-    }
-    if (todo) {
-        refuse_capture(stream);
-        fresh = true;
+    const size_t bytes[2] = {size_t(N) * size_t(W) * 4, size_t(K) * size_t(W) * 4};
+    CallForms f(kWords, al, sets, plans, bytes, stream, ctx);
+    if (f.count) {
+        PackArgs pa{};
+        for (int i = 0; i < f.count; ++i) {
+            const st_seqset_s& s = *sets[f.todo[i]];
+            pa.bytes[i] = s.d_bytes;
+            pa.off[i] = s.d_off;
+            pa.count[i] = s.count;
+            pa.packed[i] = static_cast<uint32_t*>(f.ptr[f.todo[i]]);
+        }
         const int64_t most = std::max(pa.count[0], pa.count[1]);
-        pack_kernel<<<dim3(unsigned(ceil_div(most, 256)), unsigned(todo)), 256, 0, stream>>>(pa, L, B, W);
+        pack_kernel<<<dim3(unsigned(ceil_div(most, 256)), unsigned(f.count)), 256, 0, stream>>>(pa, al.lut, L, B, W);
         STB_CUDA(cudaGetLastError());
         note_launch(nullptr);
+        f.made(kWords, al, plans, stream);
     }
-    if (fresh) {  // recorded as made only now that they are
-        settle(a, b, stream);
-        dc.made();
-        for (DistPlan* p : plans) {
-            p->packB = B;
-            p->packW = W;
-        }
-    }
-    const uint32_t* qp = a.d_packed;
-    const uint32_t* rp = b.d_packed;
+    const auto *qp = static_cast<const uint32_t*>(f.ptr[0]), *rp = static_cast<const uint32_t*>(f.ptr[1]);
     const char* name;
     switch (B) {
         case 1: name = launch_hamming<1>(qp, rp, N, K, W, out_d, stream, ctx.num_sms); break;
@@ -568,14 +592,9 @@ void levenshtein_sets(st_seqset_s& a, st_seqset_s& b, int32_t* out_d, cudaStream
     const int64_t N = r1 - r0, K = b.count;
     if (N == 0 || K == 0) return;
     Context& ctx = context();
-    DistCodes dc = compute_codes(a, b, stream, ctx);
-    if (dc.fresh) {
-        settle(a, b, stream);
-        dc.made();
-    }
-    const int sigma = std::max(1, dc.sigma);
-    const uint8_t* ac = a.d_codes;
-    const uint8_t* bc = b.d_codes;
+    DistPlan* plans[2] = {&dist_plan(a, ctx, 0), &dist_plan(b, ctx, 1)};
+    const Alphabet al = joint_alphabet(a, b, plans, stream, ctx);
+    const int sigma = std::max(1, al.sigma);
     // rows [r0, r1): their offsets and their block of the result
     const int64_t* aoff = a.d_off + r0;
     out_d += r0 * K;
@@ -590,8 +609,27 @@ void levenshtein_sets(st_seqset_s& a, st_seqset_s& b, int32_t* out_d, cudaStream
         128, std::max<int64_t>(16, N * colblocks / (int64_t(ctx.num_sms) * 8 * 6))));
     const dim3 grid(unsigned(colblocks), unsigned(std::min<int64_t>(ceil_div(N, rows), 65536)));
     if (kern && sigma <= 64 && smem <= size_t(200) * 1024 && grid.y <= 65535) {
+        st_seqset_s* sets[2] = {&a, &b};
+        const size_t bytes[2] = {size_t(a.total), size_t(b.total)};
+        CallForms f(kCodes, al, sets, plans, bytes, stream, ctx);
+        if (f.count) {
+            RemapArgs ra{};
+            for (int i = 0; i < f.count; ++i) {
+                ra.in[i] = sets[f.todo[i]]->d_bytes;
+                ra.out[i] = static_cast<uint8_t*>(f.ptr[f.todo[i]]);
+                ra.bytes[i] = sets[f.todo[i]]->total;
+            }
+            const int64_t most = std::max<int64_t>({ra.bytes[0], ra.bytes[1], 1});
+            remap_kernel<<<dim3(unsigned(std::min<int64_t>(ceil_div(most, 256), ctx.num_sms * 4)), unsigned(f.count)),
+                           256, 0, stream>>>(ra, al.lut);
+            STB_CUDA(cudaGetLastError());
+            note_launch(nullptr);
+            f.made(kCodes, al, plans, stream);
+        }
         ensure_smem_limit(reinterpret_cast<const void*>(kern), smem);
-        kern<<<grid, kLevWarps * 32, smem, stream>>>(ac, aoff, bc, b.d_off, N, K, sigma, rows, out_d);
+        kern<<<grid, kLevWarps * 32, smem, stream>>>(static_cast<const uint8_t*>(f.ptr[0]), aoff,
+                                                     static_cast<const uint8_t*>(f.ptr[1]), b.d_off, N, K, sigma,
+                                                     rows, out_d);
         STB_CUDA(cudaGetLastError());
         note_launch("levenshtein_kernel");
         return;
@@ -605,7 +643,7 @@ void levenshtein_sets(st_seqset_s& a, st_seqset_s& b, int32_t* out_d, cudaStream
     threads = std::max<int64_t>(256, std::min<int64_t>(threads, (int64_t(1) << 29) / per));
     threads = ceil_div(threads, 256) * 256;
     int32_t* scratch = ctx.work_a.as<int32_t>(size_t(threads) * per);
-    levenshtein_dp_kernel<<<unsigned(threads / 256), 256, 0, stream>>>(ac, aoff, bc, b.d_off, N, K,
+    levenshtein_dp_kernel<<<unsigned(threads / 256), 256, 0, stream>>>(a.d_bytes, aoff, b.d_bytes, b.d_off, N, K,
                                                                        scratch, out_d);
     STB_CUDA(cudaGetLastError());
     note_launch("levenshtein_dp_kernel");

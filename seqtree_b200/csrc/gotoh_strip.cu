@@ -383,43 +383,6 @@ StripRefPlan& ref_plan(st_seqset_s& s, Context& ctx, cudaStream_t stream) {
     return p;
 }
 
-// Stream-ordered scratch from a pool of our own: calls on several streams each get theirs, a
-// captured call gets its allocation as graph nodes, and at most kKeep bytes stay cached.
-constexpr uint64_t kKeep = uint64_t(256) << 20;
-
-struct StripScratch {
-    void* ptr = nullptr;
-    cudaStream_t stream;
-    StripScratch(int device, size_t bytes, cudaStream_t st) : stream(st) {
-        if (!bytes) return;
-        static std::mutex mu;
-        static std::map<int, cudaMemPool_t> pools;
-        cudaMemPool_t pool;
-        {
-            std::lock_guard<std::mutex> lk(mu);
-            cudaMemPool_t& slot = pools[device];
-            if (!slot) {
-                cudaMemPoolProps props{};
-                props.allocType = cudaMemAllocationTypePinned;
-                props.location.type = cudaMemLocationTypeDevice;
-                props.location.id = device;
-                cudaMemPool_t fresh = nullptr;
-                STB_CUDA(cudaMemPoolCreate(&fresh, &props));
-                uint64_t keep = kKeep;
-                STB_CUDA(cudaMemPoolSetAttribute(fresh, cudaMemPoolAttrReleaseThreshold, &keep));
-                slot = fresh;
-            }
-            pool = slot;
-        }
-        STB_CUDA(cudaMallocFromPoolAsync(&ptr, bytes, pool, st));
-    }
-    ~StripScratch() {
-        if (ptr) cudaFreeAsync(ptr, stream);
-    }
-    StripScratch(const StripScratch&) = delete;
-    StripScratch& operator=(const StripScratch&) = delete;
-};
-
 // The similarity grid plus the raise, per device and mode, uploaded when it changes.
 struct StripTable {
     std::vector<uint8_t> key;
@@ -531,7 +494,7 @@ void align_strip(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, in
     a.scratch_cols = qs.max_len > most ? ceil_div(rs.max_len, 4) * 4 : 0;
     const bool queued = grid < a.nqp * a.nchunks;
     const size_t columns = size_t(grid) * kStripWarps * size_t(a.scratch_cols) * 32 * sizeof(uint2);
-    StripScratch scratch(ctx.device, columns + (queued ? 256 : 0), stream);
+    StreamScratch scratch(ctx.device, columns + (queued ? 256 : 0), stream);
     a.scratch = static_cast<uint2*>(scratch.ptr);
     if (queued) {
         a.queue = reinterpret_cast<unsigned long long*>(static_cast<uint8_t*>(scratch.ptr) + columns);

@@ -37,3 +37,57 @@ def test_a_refused_capture_leaves_nothing_behind(cuda_ready, warm):
         into(name, a, b, out)
         torch.cuda.synchronize()
         assert np.array_equal(out.cpu().numpy(), getattr(oracle, name + "_matrix")(sa, sb))
+
+
+SYMBOLS = {"acgt": "ACGT", "acgtn": "ACGTN", "aa": "ACDEFGHIKLMNPQRSTVWY", "two": "AC", "lower": "acgt",
+           "digits": "0123456789", "all": "".join(map(chr, range(33, 90)))}
+
+
+def sets_of(rng, count, length=21):
+    from seqtree_b200 import device
+    strings = {n: rand_seqs(rng, count + 7 * i, length, length, s) for i, (n, s) in enumerate(SYMBOLS.items())}
+    return strings, {n: device.SeqSet(s, None) for n, s in strings.items()}
+
+
+@pytest.mark.parametrize("name", ["hamming", "levenshtein"])
+def test_a_captured_call_keeps_its_alphabet(cuda_ready, name):
+    """A captured A x B call replayed after A and B have met sets over other symbols, more of them than a
+    set keeps packed words for; each of those calls is right too, on either side."""
+    import torch
+    strings, sets = sets_of(np.random.default_rng(10), 37)
+    want = getattr(oracle, name + "_matrix")(strings["acgt"], strings["two"])
+    out = torch.full(want.shape, -1, dtype=torch.int32, device="cuda")
+    into(name, sets["acgt"], sets["two"], out)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        into(name, sets["acgt"], sets["two"], out)
+    for _ in range(2):
+        for other in ("acgtn", "aa", "lower", "digits", "all", "acgt"):
+            for a, b in ((other, "acgt"), ("acgt", other), ("two", other)):
+                got = torch.full((len(strings[a]), len(strings[b])), -1, dtype=torch.int32, device="cuda")
+                into(name, sets[a], sets[b], got)
+                torch.cuda.synchronize()
+                assert np.array_equal(got.cpu().numpy(),
+                                      getattr(oracle, name + "_matrix")(strings[a], strings[b])), (a, b)
+            out.fill_(-1)
+            graph.replay()
+            torch.cuda.synchronize()
+            assert np.array_equal(out.cpu().numpy(), want), other
+
+
+@pytest.mark.parametrize("name", ["hamming", "levenshtein"])
+def test_changing_partners_waits_for_no_other_stream(cuda_ready, name):
+    """A set that meets partners over different symbols in turn, while another stream is busy."""
+    import torch
+    strings, sets = sets_of(np.random.default_rng(11), 33)
+    outs = {b: torch.zeros((33, len(strings[b])), dtype=torch.int32, device="cuda") for b in strings}
+    for b in strings:
+        into(name, sets["acgt"], sets[b], outs[b])
+    torch.cuda.synchronize()
+    busy = torch.cuda.Stream()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(1_500_000_000)
+    for b in ("aa", "acgt", "lower", "aa"):
+        into(name, sets["acgt"], sets[b], outs[b])
+    assert not busy.query()
+    torch.cuda.synchronize()
