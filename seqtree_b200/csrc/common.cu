@@ -547,24 +547,15 @@ st_seqset_s* make_seqset(const st_strings* s, int32_t alphabet, cudaStream_t str
     Context& ctx = context();
     std::unique_ptr<st_seqset_s> set = describe(s, alphabet, ctx);
     const size_t padded = size_t(set->total) + 64;
-    // Raw sets have room for the distances' dense codes and packed words behind their bytes, so that
-    // a first distance call allocates nothing.
-    auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
-    const size_t codes_at = up(padded), packed_at = codes_at + up(padded);
-    const size_t bytes = alphabet < 0 ? packed_at + size_t(set->total) + 4 * size_t(s->count) + 64 : padded;
     if (storage) {
         set->owns = false;
-        set->d_bytes = storage[0].as<uint8_t>(bytes);
+        set->d_bytes = storage[0].as<uint8_t>(padded);
         set->d_off = storage[1].as<int64_t>(size_t(s->count + 1));
         set->d_len = storage[2].as<int32_t>(size_t(std::max<int64_t>(s->count, 1)));
     } else {
-        STB_CUDA(cudaMalloc(&set->d_bytes, bytes));
+        STB_CUDA(cudaMalloc(&set->d_bytes, padded));
         STB_CUDA(cudaMalloc(&set->d_off, sizeof(int64_t) * size_t(s->count + 1)));
         STB_CUDA(cudaMalloc(&set->d_len, sizeof(int32_t) * size_t(std::max<int64_t>(s->count, 1))));
-    }
-    if (alphabet < 0) {
-        set->d_codes = set->d_bytes + codes_at;
-        set->d_packed = reinterpret_cast<uint32_t*>(set->d_bytes + packed_at);
     }
     STB_CUDA(cudaMemsetAsync(set->d_bytes, 0, padded, stream));
     STB_CUDA(cudaMemcpyAsync(set->d_off, set->h_off.data(), sizeof(int64_t) * size_t(s->count + 1),

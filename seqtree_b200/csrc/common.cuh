@@ -192,8 +192,6 @@ struct st_seqset_s {
     std::vector<int64_t> h_off; // count + 1
     std::vector<int32_t> h_len; // count
     uint8_t* d_bytes = nullptr; // encoded codes (alphabet >= 0) or raw bytes, +64 B padding
-    uint8_t* d_codes = nullptr;   // raw sets: room for total + 64 dense codes,
-    uint32_t* d_packed = nullptr; // and for total + 4 * count bytes of packed words (in d_bytes' block)
     int64_t* d_off = nullptr;
     int32_t* d_len = nullptr;
     bool owns = true;           // false: storage borrowed from the context (transient set)

@@ -91,3 +91,17 @@ def test_changing_partners_waits_for_no_other_stream(cuda_ready, name):
         into(name, sets["acgt"], sets[b], outs[b])
     assert not busy.query()
     torch.cuda.synchronize()
+
+
+def test_a_raw_set_takes_its_own_bytes(cuda_ready):
+    """Device memory of a set of 256 MiB: its bytes and the allocator's 2 MiB granules, no room for forms
+    that only some calls make."""
+    import torch
+    from seqtree_b200 import device
+    device.SeqSet(["ACGT"], None)
+    strings = ["ACGT" * (1 << 20)] * 64
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    kept = device.SeqSet(strings, None)
+    assert before - torch.cuda.mem_get_info()[0] <= (256 + 16) << 20
+    del kept
