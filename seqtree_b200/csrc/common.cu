@@ -274,6 +274,25 @@ void h2d(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
     STB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream));
 }
 
+const int32_t* kept_table(Context& ctx, const std::vector<int32_t>& v, cudaStream_t stream, StreamScratch& spare) {
+    constexpr size_t kSlots = 64, kWords = 1024;
+    const size_t bytes = v.size() * sizeof(int32_t);
+    if (v.size() > kWords) fail(ST_ECUDA, "seqtree_b200: internal error: table too large to keep");
+    const auto it = ctx.tables.find(v);
+    if (it != ctx.tables.end()) return static_cast<int32_t*>(ctx.table_block.ptr) + size_t(it->second) * kWords;
+    if (ctx.tables.size() == kSlots) {
+        spare.take(ctx.device, bytes, stream);
+        h2d(spare.ptr, v.data(), bytes, stream);
+        return static_cast<int32_t*>(spare.ptr);
+    }
+    const int slot = int(ctx.tables.size());
+    int32_t* d = ctx.table_block.as<int32_t>(kSlots * kWords) + size_t(slot) * kWords;
+    h2d(d, v.data(), bytes, stream);
+    STB_CUDA(cudaStreamSynchronize(stream));  // the next call may be on another stream
+    ctx.tables.emplace(v, slot);
+    return d;
+}
+
 bool same_as_last(std::vector<uint8_t>& slot, const void* data, size_t bytes) {
     if (slot.size() == bytes && (bytes == 0 || std::memcmp(slot.data(), data, bytes) == 0))
         return true;

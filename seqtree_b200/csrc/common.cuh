@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <cstring>
 #include <functional>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <stdexcept>
@@ -125,6 +126,9 @@ struct Context {
     uint8_t* stage_h = nullptr;
     // storage of the transient sets made by the host-buffer entry points
     DevBuf tq[3], tr[3];  // bytes, offsets, lengths
+    // kept_table's tables by content, and their block
+    std::map<std::vector<int32_t>, int> tables;
+    DevBuf table_block;
     // plans reused by transient sets (rebuilt in place for every call)
     std::shared_ptr<void> tmp_query_plan, tmp_ref_plan, tmp_wave_plan[2];
     std::shared_ptr<void> tmp_strip_query_plan, tmp_strip_ref_plan, tmp_dist_plan[2];
@@ -148,6 +152,11 @@ void ensure_smem_limit(const void* kernel, size_t bytes);
 // graph is replayed.  Plans and tables are cached, so a call made once before capturing leaves
 // nothing to upload inside the capture.
 void h2d(void* dst, const void* src, size_t bytes, cudaStream_t stream);
+
+// A small table (at most 1,024 words) on the device, by content.  The first 64 of a device are uploaded once
+// and never rewritten, so calls on any streams and captured graphs may read them at any time; a
+// further one is uploaded into `spare` for its call alone.
+const int32_t* kept_table(Context& ctx, const std::vector<int32_t>& v, cudaStream_t stream, StreamScratch& spare);
 
 // Byte-exact content cache: returns true when `bytes` equals what was uploaded last time
 // under `slot`, so re-uploads of unchanged tables are skipped.

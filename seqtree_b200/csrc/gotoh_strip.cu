@@ -383,36 +383,6 @@ StripRefPlan& ref_plan(st_seqset_s& s, Context& ctx, cudaStream_t stream) {
     return p;
 }
 
-// The similarity grid plus the raise, per device and mode, uploaded when it changes.
-struct StripTable {
-    std::vector<uint8_t> key;
-    DevBuf sim;
-};
-
-const int32_t* strip_table(int device, bool local, const int32_t* similarity, int A, int add,
-                           cudaStream_t stream) {
-    static std::mutex mu;
-    static std::map<std::pair<int, bool>, std::unique_ptr<StripTable>> all;
-    StripTable* t;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        auto& slot = all[std::make_pair(device, local)];
-        if (!slot) slot = std::make_unique<StripTable>();
-        t = slot.get();
-    }
-    std::vector<int32_t> v(size_t(A) * A);
-    for (int i = 0; i < A * A; ++i) v[size_t(i)] = similarity[i] + add;
-    if (!same_as_last(t->key, v.data(), v.size() * 4)) {
-        try {
-            h2d(t->sim.as<int32_t>(v.size()), v.data(), v.size() * 4, stream);
-        } catch (...) {
-            t->key.clear();  // not uploaded: the next call builds it again
-            throw;
-        }
-    }
-    return static_cast<const int32_t*>(t->sim.ptr);
-}
-
 }  // namespace
 
 // Whether the strip kernel takes a call: gap_extend <= gap_open (the raised forms need it), no
@@ -435,8 +405,9 @@ bool strip_eligible(const st_seqset_s& qs, const st_seqset_s& rs, const int32_t*
     return maxabs * (std::min(rows, cols) + 1) + 2 * int64_t(go) + int64_t(ge) * (rows + cols) <= 14000;
 }
 
-// Scores (or, with self scores, distances) of every pair into out_d.
-void align_strip(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int A, int32_t mode,
+// Scores (or, with self scores, distances) of every pair into out_d; raised_d: s(a, b) + gap_extend in local
+// mode, + 2 * gap_extend in global mode, on the device.
+void align_strip(st_seqset_s& qs, st_seqset_s& rs, const int32_t* raised_d, int A, int32_t mode,
                  int32_t go, int32_t ge, int32_t dist, const int64_t* q_self, const int64_t* r_self,
                  int32_t* out_d, unsigned int* ovf, cudaStream_t stream) {
     Context& ctx = context();
@@ -445,7 +416,7 @@ void align_strip(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, in
     StripQueryPlan& qp = query_plan(qs, ctx, stream);
     StripRefPlan& rp = ref_plan(rs, ctx, stream);
     StripArgs a{};
-    a.sim = strip_table(ctx.device, local, similarity, A, add, stream);
+    a.sim = raised_d;
     a.A = A;
     a.add = add;
     a.go = go;

@@ -24,7 +24,7 @@ namespace stb {
 // The strip kernel's path (gotoh_strip.cu).
 bool strip_eligible(const st_seqset_s& qs, const st_seqset_s& rs, const int32_t* sim, int A,
                     int32_t go, int32_t ge);
-void align_strip(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int A, int32_t mode,
+void align_strip(st_seqset_s& qs, st_seqset_s& rs, const int32_t* raised_d, int A, int32_t mode,
                  int32_t go, int32_t ge, int32_t dist, const int64_t* q_self, const int64_t* r_self,
                  int32_t* out_d, unsigned int* ovf, cudaStream_t stream);
 
@@ -350,8 +350,8 @@ struct SelfArgs {
     const uint8_t* codes[2];
     const int64_t* off[2];
     int64_t count[2];
-    const int32_t* sim;
-    int A;
+    const int32_t* sim;  // A x A: s(a, b) + add
+    int A, add;
     uint32_t plain;      // bit c: residue c is plain
     int local;
     int32_t go, ge;
@@ -362,7 +362,7 @@ constexpr int kSelfRows = 16;
 
 __global__ void __launch_bounds__(256) self_score_kernel(const SelfArgs a) {
     extern __shared__ int32_t s_sim[];
-    for (int i = threadIdx.x; i < a.A * a.A; i += blockDim.x) s_sim[i] = a.sim[i];
+    for (int i = threadIdx.x; i < a.A * a.A; i += blockDim.x) s_sim[i] = a.sim[i] - a.add;
     __syncthreads();
     const unsigned full = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
@@ -706,10 +706,7 @@ const void* qpair_kernel(int R, bool local, bool exact) {
 // Rows per lane of the query-pair kernel: the smallest R with 32 * R >= m.
 int qpair_rows_per_lane(int m) { return std::min(16, std::max(1, int((m + 31) / 32))); }
 
-// The A x A s(a, b) + add grid the query-pair kernel builds its profiles from, per device.
 struct WaveState {
-    std::vector<uint8_t> key;
-    DevBuf simadd;
     // Side streams and events that run the row buckets' launches concurrently (fork / join on
     // the caller's stream), so that one bucket's tail of idle SMs is filled by the next bucket.
     static constexpr int kSide = 4;
@@ -764,6 +761,7 @@ WavePlan& wave_plan(st_seqset_s& s, Context& ctx, int slot, cudaStream_t stream)
     // (a pageable-source copy has consumed the host vectors by the time it returns)
     h2d(p.qpairs.as<int32_t>(qpairs.size()), qpairs.data(), qpairs.size() * 4, stream);
     h2d(p.sorted.as<int32_t>(order.size()), order.data(), order.size() * 4, stream);
+    if (s.owns) STB_CUDA(cudaStreamSynchronize(stream));  // the plan may be used from other streams
     p.uid = s.uid;
     return p;
 }
@@ -807,37 +805,11 @@ void launch_qpair(QpArgs qa, int R, bool local, bool exact, cudaStream_t stream)
 }
 
 
-// A similarity grid on the device, uploaded only when it changes (so warmed-up calls capture).
-struct SimTable {
-    std::vector<uint8_t> key;
-    DevBuf sim;
-};
-
-const int32_t* sim_table(Context& ctx, const int32_t* similarity, int A, cudaStream_t stream) {
-    static std::mutex mu;
-    static std::map<int, std::unique_ptr<SimTable>> all;
-    SimTable* t;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        auto& slot = all[ctx.device];
-        if (!slot) slot = std::make_unique<SimTable>();
-        t = slot.get();
-    }
-    int32_t* d_sim = t->sim.as<int32_t>(size_t(A) * A);
-    if (!same_as_last(t->key, similarity, size_t(A) * A * 4)) {
-        try {
-            h2d(d_sim, similarity, size_t(A) * A * 4, stream);
-        } catch (...) {
-            t->key.clear();
-            throw;
-        }
-    }
-    return d_sim;
-}
-
-// Self scores of both sets (N words, then K) into the context's scratch.
-const int64_t* self_scores(const st_seqset_s& qs, const st_seqset_s& rs, const int32_t* similarity, int A,
-                           int32_t mode, int32_t go, int32_t ge, cudaStream_t stream) {
+// Self scores of both sets (N words, then K), for one call: in memory of the call's own, as the kernels
+// that read them may run beside another stream's.  raised_d: the call's similarity + add on the device.
+const int64_t* self_scores(const st_seqset_s& qs, const st_seqset_s& rs, const int32_t* similarity,
+                           const int32_t* raised_d, int add, int A, int32_t mode, int32_t go, int32_t ge,
+                           cudaStream_t stream, StreamScratch& mem) {
     Context& ctx = context();
     SelfArgs a{};
     const st_seqset_s* sets[2] = {&qs, &rs};
@@ -846,8 +818,9 @@ const int64_t* self_scores(const st_seqset_s& qs, const st_seqset_s& rs, const i
         a.off[t] = sets[t]->d_off;
         a.count[t] = sets[t]->count;
     }
-    a.sim = sim_table(ctx, similarity, A, stream);
+    a.sim = raised_d;
     a.A = A;
+    a.add = add;
     for (int c = 0; c < A; ++c) {
         const int32_t own = similarity[c * A + c];
         bool ok = own >= 0;
@@ -858,7 +831,8 @@ const int64_t* self_scores(const st_seqset_s& qs, const st_seqset_s& rs, const i
     a.go = go;
     a.ge = ge;
     const int64_t total = qs.count + rs.count;
-    a.out = ctx.work_b.as<int64_t>(size_t(total));
+    mem.take(ctx.device, size_t(total) * sizeof(int64_t), stream);
+    a.out = static_cast<int64_t*>(mem.ptr);
     const int64_t blocks = std::min<int64_t>(ceil_div(total, 8), int64_t(ctx.num_sms) * 16);
     self_score_kernel<<<unsigned(blocks), 256, size_t(A) * A * 4, stream>>>(a);
     STB_CUDA(cudaGetLastError());
@@ -879,17 +853,11 @@ void align_wave(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
     const int32_t add = (mode != ST_MODE_LOCAL && ge <= go) ? 2 * ge : 0;
     std::vector<int32_t> sa(size_t(A) * A);
     for (int x = 0; x < A * A; ++x) sa[size_t(x)] = similarity[x] + add;
-    if (!same_as_last(ws.key, sa.data(), sa.size() * 4)) {
-        try {
-            h2d(ws.simadd.as<int32_t>(sa.size()), sa.data(), sa.size() * 4, stream);
-        } catch (...) {
-            ws.key.clear();  // not uploaded: the next call builds it again
-            throw;
-        }
-    }
+    StreamScratch sim, self;
+    const int32_t* simadd = kept_table(ctx, sa, stream, sim);
     WavePlan& qp = wave_plan(qs, ctx, 0, stream);
     WavePlan& rp = wave_plan(rs, ctx, 1, stream);
-    const int64_t* q_self = dist ? self_scores(qs, rs, similarity, A, mode, go, ge, stream) : nullptr;
+    const int64_t* q_self = dist ? self_scores(qs, rs, similarity, simadd, add, A, mode, go, ge, stream, self) : nullptr;
     const int64_t* r_self = dist ? q_self + N : nullptr;
     const bool local = mode == ST_MODE_LOCAL;
     const bool exact = ge > go;
@@ -913,7 +881,7 @@ void align_wave(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
         ma.rorder = static_cast<int32_t*>(rp.sorted.ptr);
         ma.K = K;
         ma.chunk = 256;
-        ma.simadd = static_cast<int32_t*>(ws.simadd.ptr);
+        ma.simadd = simadd;
         ma.A = A;
         ma.go = go;
         ma.ge = ge;
@@ -954,9 +922,11 @@ void align_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
     const bool strip_ok = strip_eligible(qs, rs, similarity, A, go, ge);
 
     auto run_thread = [&](st_seqset_s& q) {  // registers only; sequences of at most 32
-        const int64_t* self = dist ? self_scores(q, rs, similarity, A, mode, go, ge, stream) : nullptr;
+        StreamScratch sim, mem;
         ThreadArgs t{};
-        t.sim = sim_table(ctx, similarity, A, stream);
+        t.sim = kept_table(ctx, std::vector<int32_t>(similarity, similarity + A * A), stream, sim);
+        const int64_t* self =
+            dist ? self_scores(q, rs, similarity, t.sim, 0, A, mode, go, ge, stream, mem) : nullptr;
         t.A = A;
         t.go = go;
         t.ge = ge;
@@ -974,8 +944,15 @@ void align_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
         launch_thread(ctx, t, tn, mode == ST_MODE_LOCAL, q.count * K, stream);
     };
     auto run_strip = [&](st_seqset_s& q) {
-        const int64_t* self = dist ? self_scores(q, rs, similarity, A, mode, go, ge, stream) : nullptr;
-        align_strip(q, rs, similarity, A, mode, go, ge, dist, self, dist ? self + q.count : nullptr, out_d,
+        // the strip kernel's states are raised by this a cell (its file's head says why)
+        const int add = mode == ST_MODE_LOCAL ? ge : 2 * ge;
+        std::vector<int32_t> raised(similarity, similarity + A * A);
+        for (int32_t& v : raised) v += add;
+        StreamScratch sim, mem;
+        const int32_t* sim_d = kept_table(ctx, raised, stream, sim);
+        const int64_t* self =
+            dist ? self_scores(q, rs, similarity, sim_d, add, A, mode, go, ge, stream, mem) : nullptr;
+        align_strip(q, rs, sim_d, A, mode, go, ge, dist, self, dist ? self + q.count : nullptr, out_d,
                     ovf, stream);
     };
 
