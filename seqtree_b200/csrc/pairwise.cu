@@ -703,8 +703,14 @@ const void* qpair_kernel(int R, bool local, bool exact) {
     }
 }
 
-// Rows per lane of the query-pair kernel: the smallest R with 32 * R >= m.
-int qpair_rows_per_lane(int m) { return std::min(16, std::max(1, int((m + 31) / 32))); }
+// Rows per lane of the query-pair kernel: the smallest R with 32 * R >= m, in steps of 1 (buckets of 32 rows: a
+// query carries fewer than 32 padded rows) or 2 (64 rows: fewer launches, better filled).  Few queries
+// spread over many lengths want the wide buckets: 200 x 100 proteins 0.93 ms against 1.61, 64 x 500 of 300-510
+// residues with gap_extend > gap_open 4.6 against 8.1 (B200).  The tuner measures both.
+int qpair_rows_per_lane(int m, int step) {
+    const int r = std::max(1, int((m + 31) / 32));
+    return std::min(16, (r + step - 1) / step * step);
+}
 
 struct WaveState {
     // Side streams and events that run the row buckets' launches concurrently (fork / join on
@@ -722,13 +728,13 @@ struct WaveState {
     }
 };
 
-// Per-set launch plan (depends only on the lengths): the sequences of each 32-row bucket sorted by
-// length and paired with their neighbour (the query side), with the (R, offset, count) of each
-// bucket's pairs; and every index sorted by length (the ref side).
+// Per-set launch plan (depends only on the lengths): the sequences of each row bucket sorted by length and
+// paired with their neighbour (the query side), with the (R, offset, count) of each bucket's pairs, for both
+// bucket widths; and every index sorted by length (the ref side).
 struct WavePlan {
     uint64_t uid = 0;
-    std::vector<std::tuple<int, int64_t, int64_t>> pair_groups;
-    OwnedBuf qpairs, sorted;
+    std::vector<std::tuple<int, int64_t, int64_t>> pair_groups[2];
+    OwnedBuf qpairs[2], sorted;
 };
 
 WavePlan& wave_plan(st_seqset_s& s, Context& ctx, int slot, cudaStream_t stream) {
@@ -740,26 +746,25 @@ WavePlan& wave_plan(st_seqset_s& s, Context& ctx, int slot, cudaStream_t stream)
     std::vector<int32_t> order(static_cast<size_t>(s.count));
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), by_len);
-    // Query pairs per bucket of 32 rows.
-    std::vector<int32_t> qpairs;
-    qpairs.reserve(size_t(s.count) + 17);
-    p.pair_groups.clear();
-    std::vector<std::vector<int32_t>> fine(17);
-    for (int64_t i = 0; i < s.count; ++i)
-        fine[size_t(qpair_rows_per_lane(s.h_len[size_t(i)]))].push_back(int32_t(i));
-    for (int R = 1; R <= 16; ++R) {
-        std::vector<int32_t>& g = fine[size_t(R)];
-        if (g.empty()) continue;
-        std::stable_sort(g.begin(), g.end(), by_len);
-        const int64_t first = int64_t(qpairs.size() / 2);
-        for (size_t i = 0; i < g.size(); i += 2) {
-            qpairs.push_back(g[i]);
-            qpairs.push_back(i + 1 < g.size() ? g[i + 1] : g[i]);
+    for (int w = 0; w < 2; ++w) {  // `order` dealt into the buckets keeps each sorted
+        std::vector<int32_t> qpairs;
+        qpairs.reserve(size_t(s.count) + 17);
+        p.pair_groups[w].clear();
+        std::vector<std::vector<int32_t>> bucket(17);
+        for (int32_t i : order) bucket[size_t(qpair_rows_per_lane(s.h_len[size_t(i)], w + 1))].push_back(i);
+        for (int R = 1; R <= 16; ++R) {
+            const std::vector<int32_t>& g = bucket[size_t(R)];
+            if (g.empty()) continue;
+            const int64_t first = int64_t(qpairs.size() / 2);
+            for (size_t i = 0; i < g.size(); i += 2) {
+                qpairs.push_back(g[i]);
+                qpairs.push_back(i + 1 < g.size() ? g[i + 1] : g[i]);
+            }
+            p.pair_groups[w].emplace_back(R, first, int64_t(qpairs.size() / 2) - first);
         }
-        p.pair_groups.emplace_back(R, first, int64_t(qpairs.size() / 2) - first);
+        // (a pageable-source copy has consumed the host vectors by the time it returns)
+        h2d(p.qpairs[w].as<int32_t>(qpairs.size()), qpairs.data(), qpairs.size() * 4, stream);
     }
-    // (a pageable-source copy has consumed the host vectors by the time it returns)
-    h2d(p.qpairs.as<int32_t>(qpairs.size()), qpairs.data(), qpairs.size() * 4, stream);
     h2d(p.sorted.as<int32_t>(order.size()), order.data(), order.size() * 4, stream);
     if (s.owns) STB_CUDA(cudaStreamSynchronize(stream));  // the plan may be used from other streams
     p.uid = s.uid;
@@ -842,10 +847,11 @@ const int64_t* self_scores(const st_seqset_s& qs, const st_seqset_s& rs, const i
 
 }  // namespace
 
-// The warp-wavefront path for every pair (int16x2 cells; the caller checked wave_eligible).
+// The warp-wavefront path for every pair (int16x2 cells; the caller checked wave_eligible), with buckets of 32
+// (bucket 0) or 64 rows (1).
 void align_wave(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int A, int32_t mode,
                 int32_t go, int32_t ge, int32_t dist, int32_t* out_d, unsigned int* ovf,
-                cudaStream_t stream) {
+                cudaStream_t stream, int bucket) {
     Context& ctx = context();
     const int64_t N = qs.count, K = rs.count;
     WaveState& ws = wave_state(ctx.device);
@@ -864,7 +870,7 @@ void align_wave(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
     // The buckets' launches run on side streams forked from (and joined back into) the caller's
     // stream; the longest rows first, so the short buckets fill the long ones' tails.
     ws.ensure_streams();
-    const auto& pgroups = qp.pair_groups;
+    const auto& pgroups = qp.pair_groups[bucket];
     const int nside = std::min<int>(WaveState::kSide, int(pgroups.size()));
     STB_CUDA(cudaEventRecord(ws.fork, stream));
     for (int i = 0; i < nside; ++i) STB_CUDA(cudaStreamWaitEvent(ws.side[i], ws.fork, 0));
@@ -876,7 +882,7 @@ void align_wave(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
         ma.qoff = qs.d_off;
         ma.rc = rs.d_bytes;
         ma.roff = rs.d_off;
-        ma.qpairs = static_cast<int2*>(qp.qpairs.ptr) + off;
+        ma.qpairs = static_cast<int2*>(qp.qpairs[bucket].ptr) + off;
         ma.nqp = cnt;
         ma.rorder = static_cast<int32_t*>(rp.sorted.ptr);
         ma.K = K;
@@ -959,16 +965,20 @@ void align_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
     // The kernels that can take the call; where there are several, the autotuner measures them
     // once per shape.  The strip kernel wins wherever the pairs fill the GPU's warps; a
     // small matrix of long sequences leaves them idle, and there a warp per (query pair, ref) wins.
-    enum Kind { kThread, kWave, kStrip };
+    enum Kind { kThread, kWave32, kWave64, kStrip };
     std::vector<Kind> kinds;
     if (tn > 0) kinds.push_back(kThread);
-    if (wave_ok) kinds.push_back(kWave);
+    if (wave_ok) kinds.insert(kinds.end(), {kWave32, kWave64});
     if (strip_ok) kinds.push_back(kStrip);
     if (!kinds.empty()) {
         auto variant = [&](int c, st_seqset_s& q) {
             switch (kinds[size_t(c)]) {
                 case kThread: run_thread(q); break;
-                case kWave: align_wave(q, rs, similarity, A, mode, go, ge, dist, out_d, ovf, stream); break;
+                case kWave32:
+                case kWave64:
+                    align_wave(q, rs, similarity, A, mode, go, ge, dist, out_d, ovf, stream,
+                               kinds[size_t(c)] == kWave64);
+                    break;
                 case kStrip: run_strip(q); break;
             }
         };
@@ -980,7 +990,7 @@ void align_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
                           "|" + std::to_string(A) + "|" + std::to_string(qs.max_len) + "|" +
                           std::to_string(rs.max_len) + "|" + std::to_string(size_bucket(N)) + "|" +
                           std::to_string(size_bucket(K)) + "|";
-        for (Kind k : kinds) key += "tws"[k];
+        for (Kind k : kinds) key += "twWs"[k];
         // Without a measurement (tuning off, or a stream being captured): the strip kernel when
         // its warps fill the GPU, else the first kind.
         const bool fills = N / 2 * (K / 32) >= int64_t(ctx.num_sms) * 16;
