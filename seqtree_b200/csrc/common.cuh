@@ -158,6 +158,8 @@ void h2d(void* dst, const void* src, size_t bytes, cudaStream_t stream);
 // further one is uploaded into `spare` for its call alone.
 const int32_t* kept_table(Context& ctx, const std::vector<int32_t>& v, cudaStream_t stream, StreamScratch& spare);
 
+inline bool table_kept(const Context& ctx, const std::vector<int32_t>& v) { return ctx.tables.count(v) != 0; }
+
 // Byte-exact content cache: returns true when `bytes` equals what was uploaded last time
 // under `slot`, so re-uploads of unchanged tables are skipped.
 bool same_as_last(std::vector<uint8_t>& slot, const void* data, size_t bytes);
@@ -208,6 +210,7 @@ struct st_seqset_s {
     // plan caches (opaque; transient sets share the context's)
     std::shared_ptr<void> gb_query_plan, gb_ref_plan, wave_plan, strip_query_plan, strip_ref_plan;
     std::shared_ptr<void> dist_plan;
+    int64_t align_calls = 0;    // alignment calls so far (a set is planned for on its second)
     ~st_seqset_s();
 };
 

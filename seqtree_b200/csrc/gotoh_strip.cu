@@ -385,6 +385,23 @@ StripRefPlan& ref_plan(st_seqset_s& s, Context& ctx, cudaStream_t stream) {
 
 }  // namespace
 
+bool strip_planned(const st_seqset_s& s, bool query) {
+    if (!s.owns) return false;
+    if (query) return s.strip_query_plan && static_cast<const StripQueryPlan*>(s.strip_query_plan.get())->uid == s.uid;
+    return s.strip_ref_plan && static_cast<const StripRefPlan*>(s.strip_ref_plan.get())->uid == s.uid;
+}
+
+void strip_forget(st_seqset_s& s, bool query) {
+    Context& ctx = context();
+    if (query) {
+        const auto& p = s.owns ? s.strip_query_plan : ctx.tmp_strip_query_plan;
+        if (p) static_cast<StripQueryPlan*>(p.get())->uid = 0;
+    } else {
+        const auto& p = s.owns ? s.strip_ref_plan : ctx.tmp_strip_ref_plan;
+        if (p) static_cast<StripRefPlan*>(p.get())->uid = 0;
+    }
+}
+
 // Whether the strip kernel takes a call: gap_extend <= gap_open (the raised forms need it), no
 // empty sequence, lengths up to 512, and every raised state of every real or padded cell within
 // +-14000, so that int16 halves hold it (local mode adds kBias: 30384 < 32767).  Padding adds at

@@ -27,6 +27,9 @@ bool strip_eligible(const st_seqset_s& qs, const st_seqset_s& rs, const int32_t*
 void align_strip(st_seqset_s& qs, st_seqset_s& rs, const int32_t* raised_d, int A, int32_t mode,
                  int32_t go, int32_t ge, int32_t dist, const int64_t* q_self, const int64_t* r_self,
                  int32_t* out_d, unsigned int* ovf, cudaStream_t stream);
+// Whether a set's strip plan of that side is made; a plan not to be kept.
+bool strip_planned(const st_seqset_s& s, bool query);
+void strip_forget(st_seqset_s& s, bool query);
 
 namespace {
 
@@ -771,6 +774,16 @@ WavePlan& wave_plan(st_seqset_s& s, Context& ctx, int slot, cudaStream_t stream)
     return p;
 }
 
+bool wave_planned(const st_seqset_s& s) {
+    const auto* p = s.owns ? static_cast<const WavePlan*>(s.wave_plan.get()) : nullptr;
+    return p && p->uid == s.uid;
+}
+
+void wave_forget(st_seqset_s& s, Context& ctx, int slot) {
+    std::shared_ptr<void>& holder = s.owns ? s.wave_plan : ctx.tmp_wave_plan[slot];
+    if (holder) static_cast<WavePlan*>(holder.get())->uid = 0;
+}
+
 WaveState& wave_state(int device) {
     static std::mutex mu;
     static std::map<int, std::unique_ptr<WaveState>> all;
@@ -809,6 +822,17 @@ void launch_qpair(QpArgs qa, int R, bool local, bool exact, cudaStream_t stream)
     note_launch("gotoh_qpair_kernel");
 }
 
+
+std::vector<int32_t> raised(const int32_t* similarity, int A, int32_t add) {
+    std::vector<int32_t> v(similarity, similarity + A * A);
+    for (int32_t& x : v) x += add;
+    return v;
+}
+
+// What a kernel's states are raised by a cell, which its similarity grid carries (the heads of this file and of
+// gotoh_strip.cu say why).
+int32_t wave_raise(int32_t mode, int32_t go, int32_t ge) { return mode != ST_MODE_LOCAL && ge <= go ? 2 * ge : 0; }
+int32_t strip_raise(int32_t mode, int32_t ge) { return mode == ST_MODE_LOCAL ? ge : 2 * ge; }
 
 // Self scores of both sets (N words, then K), for one call: in memory of the call's own, as the kernels
 // that read them may run beside another stream's.  raised_d: the call's similarity + add on the device.
@@ -855,12 +879,9 @@ void align_wave(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
     Context& ctx = context();
     const int64_t N = qs.count, K = rs.count;
     WaveState& ws = wave_state(ctx.device);
-    // s(a, b), plus 2 * gap_extend in the raised form (global, gap_extend <= gap_open)
-    const int32_t add = (mode != ST_MODE_LOCAL && ge <= go) ? 2 * ge : 0;
-    std::vector<int32_t> sa(size_t(A) * A);
-    for (int x = 0; x < A * A; ++x) sa[size_t(x)] = similarity[x] + add;
+    const int32_t add = wave_raise(mode, go, ge);
     StreamScratch sim, self;
-    const int32_t* simadd = kept_table(ctx, sa, stream, sim);
+    const int32_t* simadd = kept_table(ctx, raised(similarity, A, add), stream, sim);
     WavePlan& qp = wave_plan(qs, ctx, 0, stream);
     WavePlan& rp = wave_plan(rs, ctx, 1, stream);
     const int64_t* q_self = dist ? self_scores(qs, rs, similarity, simadd, add, A, mode, go, ge, stream, self) : nullptr;
@@ -930,7 +951,7 @@ void align_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
     auto run_thread = [&](st_seqset_s& q) {  // registers only; sequences of at most 32
         StreamScratch sim, mem;
         ThreadArgs t{};
-        t.sim = kept_table(ctx, std::vector<int32_t>(similarity, similarity + A * A), stream, sim);
+        t.sim = kept_table(ctx, raised(similarity, A, 0), stream, sim);
         const int64_t* self =
             dist ? self_scores(q, rs, similarity, t.sim, 0, A, mode, go, ge, stream, mem) : nullptr;
         t.A = A;
@@ -950,12 +971,9 @@ void align_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
         launch_thread(ctx, t, tn, mode == ST_MODE_LOCAL, q.count * K, stream);
     };
     auto run_strip = [&](st_seqset_s& q) {
-        // the strip kernel's states are raised by this a cell (its file's head says why)
-        const int add = mode == ST_MODE_LOCAL ? ge : 2 * ge;
-        std::vector<int32_t> raised(similarity, similarity + A * A);
-        for (int32_t& v : raised) v += add;
+        const int32_t add = strip_raise(mode, ge);
         StreamScratch sim, mem;
-        const int32_t* sim_d = kept_table(ctx, raised, stream, sim);
+        const int32_t* sim_d = kept_table(ctx, raised(similarity, A, add), stream, sim);
         const int64_t* self =
             dist ? self_scores(q, rs, similarity, sim_d, add, A, mode, go, ge, stream, mem) : nullptr;
         align_strip(q, rs, sim_d, A, mode, go, ge, dist, self, dist ? self + q.count : nullptr, out_d,
@@ -986,27 +1004,71 @@ void align_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
             variant(0, qs);
             return;
         }
+        // A call on sets without plans is its own case: the thread kernel needs none, the wavefront's and
+        // the strips' take 20 to 40 us of host work and uploads.  So what is measured for a set's first
+        // call, and for the transient sets of a call on lists, makes the plans in every run (64 x 500
+        // junctions on lists: 171 us with the kernel that is faster once there are plans, 152 with the
+        // thread kernel).  From its second call on a set is taken to be used again.
+        st_seqset_s* sets[2] = {&qs, &rs};
+        bool fresh[2];
+        for (int t = 0; t < 2; ++t) {
+            const bool planned = wave_planned(*sets[t]) || (sets[t]->owns && strip_planned(*sets[t], t == 0));
+            fresh[t] = !sets[t]->owns || (!planned && sets[t]->align_calls == 0);
+        }
         std::string key = (tn > 0 ? "align|" : "wave|") + std::to_string(mode) + "|" + std::to_string(dist) +
                           "|" + std::to_string(A) + "|" + std::to_string(qs.max_len) + "|" +
                           std::to_string(rs.max_len) + "|" + std::to_string(size_bucket(N)) + "|" +
                           std::to_string(size_bucket(K)) + "|";
         for (Kind k : kinds) key += "twWs"[k];
+        if (fresh[0] || fresh[1]) key += std::string("|new") + (fresh[0] ? "q" : "") + (fresh[1] ? "r" : "");
         // Without a measurement (tuning off, or a stream being captured): the strip kernel when
         // its warps fill the GPU, else the first kind.
         const bool fills = N / 2 * (K / 32) >= int64_t(ctx.num_sms) * 16;
         const int fallback = strip_ok && (fills || !wave_ok) ? int(kinds.size()) - 1 : 0;
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        STB_CUDA(cudaStreamIsCapturing(stream, &cs));
+        if (cs != cudaStreamCaptureStatusNone) {
+            // a captured call cannot make plans or upload tables: the choice if it has its own, else a
+            // kernel that has (one of them after a call with these sets and arguments)
+            auto ready = [&](int c) {
+                const Kind k = kinds[size_t(c)];
+                if (k != kThread && !(k == kStrip ? strip_planned(qs, true) && strip_planned(rs, false)
+                                                  : wave_planned(qs) && wave_planned(rs)))
+                    return false;
+                return table_kept(ctx, raised(similarity, A,
+                                              k == kThread  ? 0
+                                              : k == kStrip ? strip_raise(mode, ge)
+                                                            : wave_raise(mode, go, ge)));
+            };
+            int c = tuned_lookup(key);
+            if (c < 0) c = fallback;
+            for (int k = int(kinds.size()) - 1; !ready(c) && k >= 0; --k)
+                if (ready(k)) c = k;
+            variant(c, qs);
+            return;
+        }
+        auto timed = [&](int c, st_seqset_s& q) {
+            if (fresh[0]) {
+                wave_forget(q, ctx, 0);
+                strip_forget(q, true);
+            }
+            if (fresh[1]) {
+                wave_forget(rs, ctx, 1);
+                strip_forget(rs, false);
+            }
+            variant(c, q);
+        };
         // A shape seen for the first time is tuned on its first query rows only (about
         // kAlignTunePairs pairs, written into their own rows of the result); the choice then
         // computes the whole matrix.
         const int64_t slice = std::min<int64_t>(
             N, std::max<int64_t>(64, kAlignTunePairs / std::max<int64_t>(K, 1)));
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        STB_CUDA(cudaStreamIsCapturing(stream, &cs));
-        if (slice < N && tuning_enabled() && cs == cudaStreamCaptureStatusNone && tuned_lookup(key) < 0) {
+        if (slice < N && tuning_enabled() && tuned_lookup(key) < 0) {
             std::unique_ptr<st_seqset_s> view = row_view(qs, slice);
-            tuned_run(key, int(kinds.size()), fallback, [&](int c) { variant(c, *view); }, stream);
+            tuned_run(key, int(kinds.size()), fallback, [&](int c) { timed(c, *view); }, stream);
         }
-        tuned_run(key, int(kinds.size()), fallback, [&](int c) { variant(c, qs); }, stream);
+        tuned_run(key, int(kinds.size()), fallback, [&](int c) { timed(c, qs); }, stream);
+        for (st_seqset_s* t : sets) ++t->align_calls;
         return;
     }
 
