@@ -264,13 +264,56 @@ void StreamScratch::take(int device, size_t bytes, cudaStream_t st) {
     stream = st;
 }
 
-void h2d(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
-    if (bytes == 0) return;
+namespace {
+void refuse_capture(cudaStream_t stream) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     STB_CUDA(cudaStreamIsCapturing(stream, &st));
     if (st != cudaStreamCaptureStatusNone)
         fail(ST_EINVAL, "seqtree_b200: this call has tables or plans to upload; make the same call "
                         "once before capturing it into a CUDA graph");
+}
+}  // namespace
+
+void* OwnedBuf::get(size_t bytes, cudaStream_t stream) {
+    if (bytes <= cap && ptr) return ptr;
+    refuse_capture(stream);  // (the memory would belong to the graph)
+    if (ptr) {
+        STB_CUDA(cudaDeviceSynchronize());  // kernels of any stream may read the old one
+        cudaFree(ptr);
+        ptr = nullptr;
+        cap = 0;
+    }
+    const size_t want = (std::max<size_t>(bytes + bytes / 8, 256) + 255) & ~size_t(255);
+    StreamScratch fresh(context().device, want, stream);
+    ptr = fresh.keep();
+    cap = want;
+    return ptr;
+}
+
+void Made::on(cudaStream_t stream) {
+    if (!event) STB_CUDA(cudaEventCreateWithFlags(&event, cudaEventDisableTiming));
+    STB_CUDA(cudaStreamGetId(stream, &stream_id));
+    STB_CUDA(cudaEventRecord(event, stream));
+}
+
+void Made::need(cudaStream_t stream) {
+    if (!event) return;
+    unsigned long long id = 0;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    STB_CUDA(cudaStreamIsCapturing(stream, &st));
+    if (st != cudaStreamCaptureStatusNone) {  // a node that waits in every replay, whichever stream that is on
+        STB_CUDA(cudaStreamWaitEvent(stream, event, cudaEventWaitExternal));
+        return;
+    }
+    STB_CUDA(cudaStreamGetId(stream, &id));
+    if (id == stream_id) return;  // behind it already
+    STB_CUDA(cudaStreamWaitEvent(stream, event, 0));
+    stream_id = id;
+}
+
+void h2d(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
+    if (bytes == 0) return;
+    refuse_capture(stream);
     STB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream));
 }
 

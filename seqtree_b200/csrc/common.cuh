@@ -67,15 +67,6 @@ struct DevBuf {
     ~DevBuf();
 };
 
-// A DevBuf that frees its memory with its owner: the buffers of a set's plans (the set's destructor
-// frees device memory, which waits for the kernels that still read it).
-struct OwnedBuf : DevBuf {
-    OwnedBuf() = default;
-    OwnedBuf(const OwnedBuf&) = delete;
-    OwnedBuf& operator=(const OwnedBuf&) = delete;
-    ~OwnedBuf() { release(); }
-};
-
 // Stream-ordered memory from a pool of the library's own: calls on several streams each get theirs, a
 // captured call gets its allocation as graph nodes, and a bounded amount stays cached for the next.  Freed
 // on the stream it was taken for, unless keep() hands it to an owner.
@@ -95,6 +86,41 @@ struct StreamScratch {
     }
     StreamScratch(const StreamScratch&) = delete;
     StreamScratch& operator=(const StreamScratch&) = delete;
+};
+
+// The buffers of a set's plans: they grow, and go with their owner (whose destructor frees device memory of its
+// own first, which waits for the kernels that still read them).  From the library's pool, as plans come
+// and go with their sets: cudaMalloc after such a free had to map memory again, 1 to 2 ms in a first
+// call on new sets (B200).
+struct OwnedBuf {
+    void* ptr = nullptr;
+    size_t cap = 0;
+    void* get(size_t bytes, cudaStream_t stream);
+    template <class T>
+    T* as(size_t count, cudaStream_t stream) { return static_cast<T*>(get(count * sizeof(T), stream)); }
+    OwnedBuf() = default;
+    OwnedBuf(const OwnedBuf&) = delete;
+    OwnedBuf& operator=(const OwnedBuf&) = delete;
+    ~OwnedBuf() {
+        if (ptr) cudaFree(ptr);
+    }
+};
+
+// Something made on one stream (a plan) that calls on any stream then read: other streams wait for it on the
+// device, nothing on the host does.  (Transient sets' calls are all on the context's stream.)
+struct Made {
+    void on(cudaStream_t stream);    // everything enqueued on `stream` so far
+    void need(cudaStream_t stream);  // what follows on `stream` may read it
+    Made() = default;
+    Made(const Made&) = delete;
+    Made& operator=(const Made&) = delete;
+    ~Made() {
+        if (event) cudaEventDestroy(event);
+    }
+
+private:
+    cudaEvent_t event = nullptr;
+    unsigned long long stream_id = 0;  // the last stream known to be behind it
 };
 
 struct Context {

@@ -65,6 +65,7 @@ struct Kept {
     Form form;
     uint32_t symbols[8];
     void* ptr;
+    std::shared_ptr<Made> made;
 };
 
 struct DistPlan {
@@ -85,8 +86,7 @@ struct Alphabet {
     int sigma;
 };
 
-// What a set keeps is made before a capture, not as part of it (a capture would only record the
-// launches, and the wait for them would end it).
+// What a set keeps is made before a capture, not as part of it (a capture would only record the launches).
 void refuse_capture(cudaStream_t stream) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     STB_CUDA(cudaStreamIsCapturing(stream, &st));
@@ -158,7 +158,9 @@ struct CallForms {
             int have = 0;
             for (const Kept& k : p.kept) {
                 have += k.form == form;
-                if (k.form == form && std::memcmp(k.symbols, al.symbols, 32) == 0) ptr[t] = k.ptr;
+                if (k.form != form || std::memcmp(k.symbols, al.symbols, 32) != 0) continue;
+                ptr[t] = k.ptr;
+                k.made->need(stream);
             }
             if (ptr[t]) continue;
             keep[t] = !p.owns || have < kMaxKept;
@@ -172,15 +174,14 @@ struct CallForms {
             todo[count++] = t;
         }
     }
-    // After the launch: what is to be kept is kept only once it is there, as the next call may be on
-    // another stream (a transient set's calls are all on one).
+    // After the launch (nothing is kept of a call that fails before).
     void made(Form form, const Alphabet& al, DistPlan* const plans[2], cudaStream_t stream) {
-        if ((keep[0] && plans[0]->owns) || (keep[1] && plans[1]->owns)) STB_CUDA(cudaStreamSynchronize(stream));
         for (int t = 0; t < 2; ++t) {
             if (!keep[t]) continue;
-            Kept k{form, {}, ptr[t]};
+            Kept k{form, {}, ptr[t], std::make_shared<Made>()};
             std::memcpy(k.symbols, al.symbols, 32);
-            plans[t]->kept.push_back(k);
+            if (plans[t]->owns) k.made->on(stream);
+            plans[t]->kept.push_back(std::move(k));
             fresh[t].keep();
         }
     }

@@ -82,6 +82,7 @@ struct QueryPlan {
     OwnedBuf d_plan;                     // quads, then slices
     std::vector<uint8_t> prof_key;       // (A, word width, penalty grid) the profile was built for
     OwnedBuf d_prof;                     // [row][quad][32] uint32 (twice the words when WIDE)
+    Made made;
 };
 
 struct RefPlan {
@@ -99,6 +100,7 @@ struct RefPlan {
     OwnedBuf d_plan;                     // chunks, then tasks
     OwnedBuf d_meta;                     // per slot: column in the chunk | length << 16
     OwnedBuf d_slab;                     // per task: longest rows of 32 bytes (4*code per lane)
+    Made made;
 };
 
 // Queries (rows [r0, r1) of the set; r1 = -1 for all) sorted by length (stable); each length's
@@ -134,7 +136,7 @@ void build_query_plan(QueryPlan& plan, const st_seqset_s& q, cudaStream_t stream
     if (plan.prof_rows > INT32_MAX) fail(ST_EINVAL, "seqtree_b200: query set too large for one call");
     std::vector<int4> up(plan.quads);
     up.insert(up.end(), plan.slices.begin(), plan.slices.end());
-    h2d(plan.d_plan.as<int4>(up.size()), up.data(), sizeof(int4) * up.size(), stream);
+    h2d(plan.d_plan.as<int4>(up.size(), stream), up.data(), sizeof(int4) * up.size(), stream);
     plan.prof_key.clear();
     plan.uid = q.uid;
     plan.r0 = r0;
@@ -1070,10 +1072,10 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
                 if (rp.rc != best_rc) build_ref_plan(rp, rs, best_rc);
                 std::vector<int4> up(rp.chunks);
                 up.insert(up.end(), rp.tasks.begin(), rp.tasks.end());
-                int4* d_plan = rp.d_plan.as<int4>(up.size());
+                int4* d_plan = rp.d_plan.as<int4>(up.size(), stream);
                 h2d(d_plan, up.data(), sizeof(int4) * up.size(), stream);
-                uint32_t* meta = rp.d_meta.as<uint32_t>(size_t(K));
-                uint8_t* slab = rp.d_slab.as<uint8_t>(size_t(rp.slab_bytes) + 16);
+                uint32_t* meta = rp.d_meta.as<uint32_t>(size_t(K), stream);
+                uint8_t* slab = rp.d_slab.as<uint8_t>(size_t(rp.slab_bytes) + 16, stream);
                 const int4* tasks = d_plan + rp.nchunks;
                 const bool few = rp.nchunks <= 4;  // beyond, a block per task fills more of the GPU
                 (few ? chunk_order_kernel<true> : chunk_order_kernel<false>)<<<unsigned(rp.nchunks), 256, 0, stream>>>(
@@ -1085,6 +1087,7 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
                     STB_CUDA(cudaGetLastError());
                 }
                 note_launch(nullptr, few ? 1 : 2);
+                if (rs.owns) rp.made.on(stream);
                 rp.uid = rs.uid;
             }
         }
@@ -1134,7 +1137,7 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
         if (!same_as_last(qp.prof_key, key.data(), key.size())) {
             qp.prof_key.clear();  // set again once the profile kernel is enqueued
             const size_t words = size_t(qp.prof_rows) * kQuads * kRow * (wide ? 2 : 1);
-            uint32_t* prof = qp.d_prof.as<uint32_t>(words);
+            uint32_t* prof = qp.d_prof.as<uint32_t>(words, stream);
             const int4* quads = static_cast<const int4*>(qp.d_plan.ptr);
             const int4* slices = quads + qp.quads.size();
             auto fill = wide ? profile_kernel<true> : profile_kernel<false>;
@@ -1143,9 +1146,12 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
                 uint32_t(maxpen), prof);
             STB_CUDA(cudaGetLastError());
             note_launch(nullptr);
+            if (qs.owns) qp.made.on(stream);
             qp.prof_key = key;
         }
     }
+    rp.made.need(stream);
+    qp.made.need(stream);
 
     auto* err = reinterpret_cast<unsigned long long*>(ctx.flags_d + 8);
     if (qs.owns || rs.owns) STB_CUDA(cudaMemsetAsync(err, 0, 8, stream));  // host calls cleared it

@@ -317,19 +317,23 @@ struct StripQueryPlan {
     uint64_t uid = 0;
     int64_t nqp = 0;
     OwnedBuf pairs;
+    Made made;
 };
 
 struct StripRefPlan {
     uint64_t uid = 0;
     int ngroups = 0;
-    OwnedBuf meta, groups, slab;
+    OwnedBuf buf;                    // meta, groups, slab
+    const int2 *meta = nullptr, *groups = nullptr;
+    const uint32_t* slab = nullptr;
+    Made made;
 };
 
 std::vector<int32_t> longest_first(const st_seqset_s& s) {
-    std::vector<int32_t> order(static_cast<size_t>(s.count));
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int32_t x, int32_t y) { return s.h_len[size_t(x)] > s.h_len[size_t(y)]; });
+    std::vector<int32_t> order(static_cast<size_t>(s.count)), at(size_t(s.max_len) + 2, 0);
+    for (int32_t l : s.h_len) ++at[size_t(s.max_len - l) + 1];
+    for (size_t l = 1; l < at.size(); ++l) at[l] += at[l - 1];
+    for (int64_t i = 0; i < s.count; ++i) order[size_t(at[size_t(s.max_len - s.h_len[size_t(i)])]++)] = int32_t(i);
     return order;
 }
 
@@ -342,44 +346,50 @@ Plan& strip_slot(std::shared_ptr<void>& own, std::shared_ptr<void>& shared, bool
 
 StripQueryPlan& query_plan(st_seqset_s& s, Context& ctx, cudaStream_t stream) {
     auto& p = strip_slot<StripQueryPlan>(s.strip_query_plan, ctx.tmp_strip_query_plan, s.owns);
-    if (p.uid == s.uid) return p;
-    std::vector<int32_t> order = longest_first(s);
-    if (order.size() & 1) order.push_back(order.back());
-    p.uid = 0;
-    h2d(p.pairs.as<int32_t>(order.size()), order.data(), order.size() * 4, stream);
-    STB_CUDA(cudaStreamSynchronize(stream));  // the plan may be used from other streams
-    p.nqp = int64_t(order.size() / 2);
-    p.uid = s.uid;
+    if (p.uid != s.uid) {
+        std::vector<int32_t> order = longest_first(s);
+        if (order.size() & 1) order.push_back(order.back());
+        p.uid = 0;
+        h2d(p.pairs.as<int32_t>(order.size(), stream), order.data(), order.size() * 4, stream);
+        if (s.owns) p.made.on(stream);
+        p.nqp = int64_t(order.size() / 2);
+        p.uid = s.uid;
+    }
+    p.made.need(stream);
     return p;
 }
 
 StripRefPlan& ref_plan(st_seqset_s& s, Context& ctx, cudaStream_t stream) {
     auto& p = strip_slot<StripRefPlan>(s.strip_ref_plan, ctx.tmp_strip_ref_plan, s.owns);
-    if (p.uid == s.uid) return p;
-    const std::vector<int32_t> order = longest_first(s);
-    std::vector<int2> groups(size_t(ceil_div(s.count, 32)));
-    int64_t rows = 0;
-    for (size_t g = 0; g < groups.size(); ++g) {
-        const int longest = s.h_len[size_t(order[g * 32])];
-        const bool one_length = g * 32 + 32 <= order.size() &&
-                                s.h_len[size_t(order[g * 32 + 31])] == longest;
-        groups[g] = make_int2(int(rows), longest | (one_length ? 1 << 16 : 0));
-        rows += (longest + 3) / 4;
+    if (p.uid != s.uid) {
+        const std::vector<int32_t> order = longest_first(s);
+        const size_t ngroups = size_t(ceil_div(s.count, 32));
+        std::vector<int2> up(order.size() + ngroups);  // meta, then groups
+        for (size_t t = 0; t < order.size(); ++t) up[t] = make_int2(order[t], s.h_len[size_t(order[t])]);
+        int64_t rows = 0;
+        for (size_t g = 0; g < ngroups; ++g) {
+            const int longest = up[g * 32].y;
+            const bool one_length = g * 32 + 32 <= order.size() && up[g * 32 + 31].y == longest;
+            up[order.size() + g] = make_int2(int(rows), longest | (one_length ? 1 << 16 : 0));
+            rows += (longest + 3) / 4;
+        }
+        if (rows > INT32_MAX) fail(ST_EINVAL, "seqtree_b200: reference set too large for one call");
+        p.uid = 0;
+        const size_t slab_at = (up.size() * sizeof(int2) + 255) & ~size_t(255);
+        uint8_t* d = p.buf.as<uint8_t>(slab_at + size_t(rows) * 128, stream);
+        p.meta = reinterpret_cast<int2*>(d);
+        p.groups = p.meta + order.size();
+        auto* slab = reinterpret_cast<uint32_t*>(d + slab_at);
+        p.slab = slab;
+        h2d(d, up.data(), up.size() * sizeof(int2), stream);
+        strip_slab_kernel<<<unsigned(ngroups), 256, 0, stream>>>(s.d_bytes, s.d_off, p.meta, s.count, p.groups, slab);
+        STB_CUDA(cudaGetLastError());
+        note_launch(nullptr);
+        if (s.owns) p.made.on(stream);
+        p.ngroups = int(ngroups);
+        p.uid = s.uid;
     }
-    if (rows > INT32_MAX) fail(ST_EINVAL, "seqtree_b200: reference set too large for one call");
-    p.uid = 0;
-    std::vector<int2> meta(order.size());
-    for (size_t t = 0; t < order.size(); ++t) meta[t] = make_int2(order[t], s.h_len[size_t(order[t])]);
-    h2d(p.meta.as<int2>(meta.size()), meta.data(), meta.size() * sizeof(int2), stream);
-    h2d(p.groups.as<int2>(groups.size()), groups.data(), groups.size() * sizeof(int2), stream);
-    strip_slab_kernel<<<unsigned(groups.size()), 256, 0, stream>>>(
-        s.d_bytes, s.d_off, static_cast<int2*>(p.meta.ptr), s.count,
-        static_cast<int2*>(p.groups.ptr), p.slab.as<uint32_t>(size_t(rows) * 32));
-    STB_CUDA(cudaGetLastError());
-    note_launch(nullptr);
-    STB_CUDA(cudaStreamSynchronize(stream));  // the plan may be used from other streams
-    p.ngroups = int(groups.size());
-    p.uid = s.uid;
+    p.made.need(stream);
     return p;
 }
 
@@ -443,9 +453,9 @@ void align_strip(st_seqset_s& qs, st_seqset_s& rs, const int32_t* raised_d, int 
     a.qoff = qs.d_off;
     a.qpairs = static_cast<const int2*>(qp.pairs.ptr);
     a.nqp = qp.nqp;
-    a.slab = static_cast<const uint32_t*>(rp.slab.ptr);
-    a.groups = static_cast<const int2*>(rp.groups.ptr);
-    a.rmeta = static_cast<const int2*>(rp.meta.ptr);
+    a.slab = rp.slab;
+    a.groups = rp.groups;
+    a.rmeta = rp.meta;
     a.K = rs.count;
     a.ngroups = rp.ngroups;
     a.dist = dist;

@@ -737,40 +737,51 @@ struct WaveState {
 struct WavePlan {
     uint64_t uid = 0;
     std::vector<std::tuple<int, int64_t, int64_t>> pair_groups[2];
-    OwnedBuf qpairs[2], sorted;
+    OwnedBuf buf;
+    const int2* qpairs[2] = {};
+    const int32_t* sorted = nullptr;
+    Made made;
 };
 
 WavePlan& wave_plan(st_seqset_s& s, Context& ctx, int slot, cudaStream_t stream) {
     std::shared_ptr<void>& holder = s.owns ? s.wave_plan : ctx.tmp_wave_plan[slot];
     if (!holder) holder = std::make_shared<WavePlan>();
     WavePlan& p = *static_cast<WavePlan*>(holder.get());
-    if (p.uid == s.uid) return p;
-    auto by_len = [&](int32_t x, int32_t y) { return s.h_len[size_t(x)] < s.h_len[size_t(y)]; };
-    std::vector<int32_t> order(static_cast<size_t>(s.count));
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), by_len);
-    for (int w = 0; w < 2; ++w) {  // `order` dealt into the buckets keeps each sorted
-        std::vector<int32_t> qpairs;
-        qpairs.reserve(size_t(s.count) + 17);
-        p.pair_groups[w].clear();
-        std::vector<std::vector<int32_t>> bucket(17);
-        for (int32_t i : order) bucket[size_t(qpair_rows_per_lane(s.h_len[size_t(i)], w + 1))].push_back(i);
-        for (int R = 1; R <= 16; ++R) {
-            const std::vector<int32_t>& g = bucket[size_t(R)];
-            if (g.empty()) continue;
-            const int64_t first = int64_t(qpairs.size() / 2);
-            for (size_t i = 0; i < g.size(); i += 2) {
-                qpairs.push_back(g[i]);
-                qpairs.push_back(i + 1 < g.size() ? g[i + 1] : g[i]);
+    if (p.uid != s.uid) {
+        std::vector<int32_t> order(static_cast<size_t>(s.count)), at(size_t(s.max_len) + 2, 0);  // by length
+        for (int32_t l : s.h_len) ++at[size_t(l) + 1];
+        for (size_t l = 1; l < at.size(); ++l) at[l] += at[l - 1];
+        for (int64_t i = 0; i < s.count; ++i) order[size_t(at[size_t(s.h_len[size_t(i)])]++)] = int32_t(i);
+        std::vector<int32_t> up;  // the pairs of both widths, then the order
+        up.reserve(size_t(3 * s.count) + 34);
+        size_t first_of[2];
+        for (int w = 0; w < 2; ++w) {  // `order` dealt into the buckets keeps each sorted
+            first_of[w] = up.size();
+            p.pair_groups[w].clear();
+            std::vector<std::vector<int32_t>> bucket(17);
+            for (int32_t i : order) bucket[size_t(qpair_rows_per_lane(s.h_len[size_t(i)], w + 1))].push_back(i);
+            for (int R = 1; R <= 16; ++R) {
+                const std::vector<int32_t>& g = bucket[size_t(R)];
+                if (g.empty()) continue;
+                const int64_t first = int64_t((up.size() - first_of[w]) / 2);
+                for (size_t i = 0; i < g.size(); i += 2) {
+                    up.push_back(g[i]);
+                    up.push_back(i + 1 < g.size() ? g[i + 1] : g[i]);
+                }
+                p.pair_groups[w].emplace_back(R, first, int64_t((up.size() - first_of[w]) / 2) - first);
             }
-            p.pair_groups[w].emplace_back(R, first, int64_t(qpairs.size() / 2) - first);
         }
-        // (a pageable-source copy has consumed the host vectors by the time it returns)
-        h2d(p.qpairs[w].as<int32_t>(qpairs.size()), qpairs.data(), qpairs.size() * 4, stream);
+        const size_t sorted_at = up.size();
+        up.insert(up.end(), order.begin(), order.end());
+        p.uid = 0;
+        int32_t* d = p.buf.as<int32_t>(up.size(), stream);
+        h2d(d, up.data(), up.size() * 4, stream);
+        for (int w = 0; w < 2; ++w) p.qpairs[w] = reinterpret_cast<int2*>(d + first_of[w]);
+        p.sorted = d + sorted_at;
+        if (s.owns) p.made.on(stream);
+        p.uid = s.uid;
     }
-    h2d(p.sorted.as<int32_t>(order.size()), order.data(), order.size() * 4, stream);
-    if (s.owns) STB_CUDA(cudaStreamSynchronize(stream));  // the plan may be used from other streams
-    p.uid = s.uid;
+    p.made.need(stream);
     return p;
 }
 
@@ -903,9 +914,9 @@ void align_wave(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
         ma.qoff = qs.d_off;
         ma.rc = rs.d_bytes;
         ma.roff = rs.d_off;
-        ma.qpairs = static_cast<int2*>(qp.qpairs[bucket].ptr) + off;
+        ma.qpairs = qp.qpairs[bucket] + off;
         ma.nqp = cnt;
-        ma.rorder = static_cast<int32_t*>(rp.sorted.ptr);
+        ma.rorder = rp.sorted;
         ma.K = K;
         ma.chunk = 256;
         ma.simadd = simadd;
