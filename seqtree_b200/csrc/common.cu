@@ -85,13 +85,9 @@ int tuned_lookup(const std::string& key) {
 int tuned_run(const std::string& key, int n, int fallback, const std::function<void(int)>& run,
               cudaStream_t stream) {
     const std::string k = dev_key(key);
-    {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_tune.find(k);
-        if (it != g_tune.end()) {
-            run(it->second);
-            return it->second;
-        }
+    if (const int known = tuned_lookup(key); known >= 0) {
+        run(known);  // (not under the lock: a run looks choices up too)
+        return known;
     }
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     STB_CUDA(cudaStreamIsCapturing(stream, &cs));
@@ -264,15 +260,13 @@ void StreamScratch::take(int device, size_t bytes, cudaStream_t st) {
     stream = st;
 }
 
-namespace {
 void refuse_capture(cudaStream_t stream) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     STB_CUDA(cudaStreamIsCapturing(stream, &st));
     if (st != cudaStreamCaptureStatusNone)
-        fail(ST_EINVAL, "seqtree_b200: this call has tables or plans to upload; make the same call "
+        fail(ST_EINVAL, "seqtree_b200: this call has tables or plans to make; make the same call "
                         "once before capturing it into a CUDA graph");
 }
-}  // namespace
 
 void* OwnedBuf::get(size_t bytes, cudaStream_t stream) {
     if (bytes <= cap && ptr) return ptr;
@@ -296,19 +290,22 @@ void Made::on(cudaStream_t stream) {
     STB_CUDA(cudaEventRecord(event, stream));
 }
 
-void Made::need(cudaStream_t stream) {
-    if (!event) return;
-    unsigned long long id = 0;
+StreamNow::StreamNow(cudaStream_t s) : stream(s) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    STB_CUDA(cudaStreamIsCapturing(stream, &st));
-    if (st != cudaStreamCaptureStatusNone) {  // a node that waits in every replay, whichever stream that is on
-        STB_CUDA(cudaStreamWaitEvent(stream, event, cudaEventWaitExternal));
+    STB_CUDA(cudaStreamIsCapturing(s, &st));
+    capturing = st != cudaStreamCaptureStatusNone;
+    if (!capturing) STB_CUDA(cudaStreamGetId(s, &id));
+}
+
+void Made::need(const StreamNow& now) {
+    if (!event) return;
+    if (now.capturing) {  // a node that waits in every replay, whichever stream that is on
+        STB_CUDA(cudaStreamWaitEvent(now.stream, event, cudaEventWaitExternal));
         return;
     }
-    STB_CUDA(cudaStreamGetId(stream, &id));
-    if (id == stream_id) return;  // behind it already
-    STB_CUDA(cudaStreamWaitEvent(stream, event, 0));
-    stream_id = id;
+    if (now.id == stream_id) return;  // behind it already
+    STB_CUDA(cudaStreamWaitEvent(now.stream, event, 0));
+    stream_id = now.id;
 }
 
 void h2d(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
@@ -318,21 +315,23 @@ void h2d(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
 }
 
 const int32_t* kept_table(Context& ctx, const std::vector<int32_t>& v, cudaStream_t stream, StreamScratch& spare) {
-    constexpr size_t kSlots = 64, kWords = 1024;
+    constexpr size_t kBlock = 64, kWords = 1024;  // tables per block
     const size_t bytes = v.size() * sizeof(int32_t);
     if (v.size() > kWords) fail(ST_ECUDA, "seqtree_b200: internal error: table too large to keep");
     const auto it = ctx.tables.find(v);
-    if (it != ctx.tables.end()) return static_cast<int32_t*>(ctx.table_block.ptr) + size_t(it->second) * kWords;
-    if (ctx.tables.size() == kSlots) {
+    if (it != ctx.tables.end()) return it->second;
+    constexpr size_t kBlocks = sizeof ctx.table_blocks / sizeof ctx.table_blocks[0];
+    const size_t slot = ctx.tables.size();
+    if (slot == kBlock * kBlocks) {
         spare.take(ctx.device, bytes, stream);
         h2d(spare.ptr, v.data(), bytes, stream);
         return static_cast<int32_t*>(spare.ptr);
     }
-    const int slot = int(ctx.tables.size());
-    int32_t* d = ctx.table_block.as<int32_t>(kSlots * kWords) + size_t(slot) * kWords;
+    refuse_capture(stream);
+    int32_t* d = ctx.table_blocks[slot / kBlock].as<int32_t>(kBlock * kWords) + slot % kBlock * kWords;
     h2d(d, v.data(), bytes, stream);
     STB_CUDA(cudaStreamSynchronize(stream));  // the next call may be on another stream
-    ctx.tables.emplace(v, slot);
+    ctx.tables.emplace(v, d);
     return d;
 }
 

@@ -108,9 +108,19 @@ struct OwnedBuf {
 
 // Something made on one stream (a plan) that calls on any stream then read: other streams wait for it on the
 // device, nothing on the host does.  (Transient sets' calls are all on the context's stream.)
+struct StreamNow {  // a call's stream, looked at once
+    cudaStream_t stream;
+    unsigned long long id = 0;
+    bool capturing = false;
+    explicit StreamNow(cudaStream_t s);
+};
+
 struct Made {
-    void on(cudaStream_t stream);    // everything enqueued on `stream` so far
-    void need(cudaStream_t stream);  // what follows on `stream` may read it
+    void on(cudaStream_t stream);      // everything enqueued on `stream` so far
+    void need(const StreamNow& now);   // what follows on the stream may read it
+    void need(cudaStream_t stream) {
+        if (event) need(StreamNow(stream));
+    }
     Made() = default;
     Made(const Made&) = delete;
     Made& operator=(const Made&) = delete;
@@ -152,11 +162,13 @@ struct Context {
     uint8_t* stage_h = nullptr;
     // storage of the transient sets made by the host-buffer entry points
     DevBuf tq[3], tr[3];  // bytes, offsets, lengths
-    // kept_table's tables by content, and their block
-    std::map<std::vector<int32_t>, int> tables;
-    DevBuf table_block;
+    // kept_table's tables by content, and their blocks
+    std::map<std::vector<int32_t>, int32_t*> tables;
+    DevBuf table_blocks[16];
     // plans reused by transient sets (rebuilt in place for every call)
     std::shared_ptr<void> tmp_query_plan, tmp_ref_plan, tmp_wave_plan[2];
+    // ref plan of the tuner's trials on a resident set (each trial is waited for)
+    std::shared_ptr<void> trial_ref_plan;
     std::shared_ptr<void> tmp_strip_query_plan, tmp_strip_ref_plan, tmp_dist_plan[2];
     // query plan of a row block (sparse calls whose hits are taken in several blocks)
     std::shared_ptr<void> tmp_block_plan;
@@ -173,13 +185,16 @@ Context& context();
 // devices needs the call on each of them.
 void ensure_smem_limit(const void* kernel, size_t bytes);
 
+// Fails while `stream` is being captured: for what a call makes and keeps, which a capture would only record.
+void refuse_capture(cudaStream_t stream);
+
 // Host -> device copy of per-call tables or plans.  Refuses to run while `stream` is being
 // captured into a CUDA graph: the captured copy would read host memory that is gone when the
 // graph is replayed.  Plans and tables are cached, so a call made once before capturing leaves
 // nothing to upload inside the capture.
 void h2d(void* dst, const void* src, size_t bytes, cudaStream_t stream);
 
-// A small table (at most 1,024 words) on the device, by content.  The first 64 of a device are uploaded once
+// A small table (at most 1,024 words) on the device, by content.  The first 1,024 of a device are uploaded once
 // and never rewritten, so calls on any streams and captured graphs may read them at any time; a
 // further one is uploaded into `spare` for its call alone.
 const int32_t* kept_table(Context& ctx, const std::vector<int32_t>& v, cudaStream_t stream, StreamScratch& spare);

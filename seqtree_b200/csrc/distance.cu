@@ -57,7 +57,7 @@ __global__ void presence_kernel(const TwoSets t, unsigned int* __restrict__ pres
 // sets' bytes.  Nothing here is ever written again once it is made, so calls on several streams and
 // captured graphs may read it for as long as the set lives, whatever partners the set meets in
 // between; an alphabet past the last place is coded for its call alone.
-constexpr int kMaxKept = 4;  // of either kind
+constexpr int kMaxKept = 8;  // of either kind
 
 enum Form { kCodes, kWords };
 
@@ -85,15 +85,6 @@ struct Alphabet {
     ByteLut lut;   // byte -> 0 .. sigma - 1
     int sigma;
 };
-
-// What a set keeps is made before a capture, not as part of it (a capture would only record the launches).
-void refuse_capture(cudaStream_t stream) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    STB_CUDA(cudaStreamIsCapturing(stream, &st));
-    if (st != cudaStreamCaptureStatusNone)
-        fail(ST_EINVAL, "seqtree_b200: this call has codes or packed words of a set to make; make the same "
-                        "call once before capturing it into a CUDA graph");
-}
 
 DistPlan& dist_plan(st_seqset_s& s, Context& ctx, int slot) {
     std::shared_ptr<void>& holder = s.owns ? s.dist_plan : ctx.tmp_dist_plan[slot];

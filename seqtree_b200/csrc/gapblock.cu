@@ -72,7 +72,17 @@ static_assert(kWarps == 2 * kQuads, "the dense write-out gives each result word 
 // ---------------------------------------------------------------------------- plans ---------
 // Plans depend only on the lengths (and codes) of a set, so a device-resident set builds them
 // once; transient sets (host-buffer calls) rebuild them in place inside the context's plan
-// objects, whose device buffers only grow.
+// objects, whose device buffers only grow.  What a resident set keeps -- its plans, a ref plan for each
+// chunk width it is called with, a profile for each of the first four penalty grids -- is never written
+// again, so calls on any streams and captured graphs may read it as long as the set lives.  Further grids
+// share a fifth profile: it changes only when the device is idle, and captured calls are refused it.
+struct Profile {
+    std::vector<uint8_t> key;            // (A, word width, penalty grid) it was built for
+    OwnedBuf buf;                        // [row][quad][32] uint32 (twice the words when WIDE)
+    Made made;
+};
+constexpr size_t kMaxProfiles = 5;  // the last one changes hands
+
 struct QueryPlan {
     uint64_t uid = 0;                    // set the plan was built for
     int64_t r0 = 0, r1 = -1;             // its rows [r0, r1) (r1 = -1: the whole set)
@@ -80,9 +90,8 @@ struct QueryPlan {
     std::vector<int4> slices;            // (first quad, quads, length, profile row offset)
     int64_t prof_rows = 0;               // profile rows of all slices
     OwnedBuf d_plan;                     // quads, then slices
-    std::vector<uint8_t> prof_key;       // (A, word width, penalty grid) the profile was built for
-    OwnedBuf d_prof;                     // [row][quad][32] uint32 (twice the words when WIDE)
     Made made;
+    std::vector<std::unique_ptr<Profile>> profiles;
 };
 
 struct RefPlan {
@@ -137,7 +146,8 @@ void build_query_plan(QueryPlan& plan, const st_seqset_s& q, cudaStream_t stream
     std::vector<int4> up(plan.quads);
     up.insert(up.end(), plan.slices.begin(), plan.slices.end());
     h2d(plan.d_plan.as<int4>(up.size(), stream), up.data(), sizeof(int4) * up.size(), stream);
-    plan.prof_key.clear();
+    for (auto& p : plan.profiles) p->key.clear();
+    if (q.owns && r1 < 0) plan.made.on(stream);
     plan.uid = q.uid;
     plan.r0 = r0;
     plan.r1 = r1;
@@ -198,6 +208,11 @@ void build_ref_plan(RefPlan& plan, const st_seqset_s& r, int rc) {
     plan.ntasks = int64_t(plan.tasks.size());
     plan.slab_bytes = slab;
 }
+
+// A resident ref set's plans, one per chunk width.
+struct RefPlans {
+    std::vector<std::unique_ptr<RefPlan>> of;
+};
 
 template <class Plan>
 Plan& plan_slot(std::shared_ptr<void>& own, std::shared_ptr<void>& shared, bool owns) {
@@ -834,23 +849,26 @@ FastKernel fast_kernel(bool prior, bool wide) {
 // 16-byte aligned and the last aligned group of four stays inside the row.
 int prior_stride(int W1) { return (W1 + 3 + 4 + 3) & ~3; }
 
-// Device-side tables of the fast path and the arguments they were built from.
+// Device-side tables of the fast path and the arguments they were built from.  The first 64 argument sets
+// of a device (each of at most 1.2 MB, 0.1 with sequences up to 25) are kept and never written again, so
+// calls on other streams and captured graphs may read them.  Further ones share one more, as with
+// the profiles.
 struct GbTables {
     std::vector<uint8_t> key;
-    DevBuf buf;
+    OwnedBuf buf;
+    Made made;
     const uint32_t* prior2 = nullptr;
     const int32_t *pen = nullptr, *ftab = nullptr;
     int32_t least_term = 0;  // of ftab: below 0 where a prior's minimum outweighs the gap cost
     int32_t most_term = 0;
 };
+constexpr size_t kMaxTables = 65;  // the last one changes hands
 
-GbTables& gb_tables(int device) {
+std::vector<std::unique_ptr<GbTables>>& gb_tables(int device) {
     static std::mutex mu;
-    static std::map<int, std::unique_ptr<GbTables>> all;
+    static std::map<int, std::vector<std::unique_ptr<GbTables>>> all;
     std::lock_guard<std::mutex> lk(mu);
-    auto& p = all[device];
-    if (!p) p = std::make_unique<GbTables>();
-    return *p;
+    return all[device];
 }
 
 // Penalty grid; per-(M,d) prior rows shifted by their minimum (added back through ftab) and
@@ -900,7 +918,7 @@ void build_tables(GbTables& tb, const std::vector<int32_t>& pen, int32_t go, int
     const size_t pen_at = up.size(), ftab_at = pen_at + pen.size();
     up.insert(up.end(), pen.begin(), pen.end());
     up.insert(up.end(), ftab.begin(), ftab.end());
-    uint32_t* d = tb.buf.as<uint32_t>(up.size());
+    uint32_t* d = tb.buf.as<uint32_t>(up.size(), stream);
     h2d(d, up.data(), up.size() * 4, stream);
     tb.prior2 = d;
     tb.pen = reinterpret_cast<int32_t*>(d + pen_at);
@@ -926,7 +944,8 @@ constexpr int kNumRc = int(sizeof(kRcCandidates) / sizeof(kRcCandidates[0]));
 static_assert(kRcCandidates[0] <= kMaxRounds * 32, "chunk_order_kernel's buckets");
 // Pairs a dense call's first-time tuning runs each variant on (its first query rows).
 constexpr int64_t kTuneSlicePairs = int64_t(100) * 1000 * 1000;
-thread_local int t_force_rc = 0;  // set while the autotuner times one chunk width
+thread_local int t_force_rc = 0;      // the chunk width of a run: the tuner's choice, or one it times
+thread_local bool t_trial_rc = false;  // (a trial)
 
 // The conditions under which gapblock_run takes the fast kernel (non-negative penalties, every
 // length <= 64, halves that cannot carry), the form whose sparse output is ordered.
@@ -994,9 +1013,11 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
 
     const int W = longest, W1 = W + 1;
     const bool wide = maxpen > 255;  // the penalties of four queries do not fit one word
-    // Tables for this (matrix, gaps, prior, lengths): rebuilt only when they change, so repeated
-    // calls with the same arguments enqueue nothing but the kernel.
-    GbTables& tb = gb_tables(ctx.device);
+    // Tables for this (matrix, gaps, prior, lengths): kept, so repeated calls with the same arguments
+    // enqueue nothing but the kernel.
+    const StreamNow now(stream);
+    static const GbTables no_tables;  // (the general kernel reads none)
+    const GbTables* tbp = &no_tables;
     if (fast) {
         const int64_t hdr[8] = {A, go, ge, W, int64_t(prior_width), has_prior, 0, 0};
         const struct {
@@ -1005,21 +1026,46 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
         } parts[3] = {{hdr, sizeof hdr}, {pen.data(), pen.size() * 4},
                       {prior, has_prior ? size_t(prior_len) * 4 : 0}};
         Phase ph("tables");
-        bool same = tb.key.size() == parts[0].n + parts[1].n + parts[2].n;
-        size_t at = 0;
-        for (const auto& part : parts) {
-            same = same && (part.n == 0 || std::memcmp(tb.key.data() + at, part.p, part.n) == 0);
-            at += part.n;
-        }
-        if (!same) {
-            tb.key.clear();  // set again once everything is uploaded
-            build_tables(tb, pen, go, ge, W, has_prior ? prior : nullptr, W1p, stream);
+        auto same = [&](const GbTables& t) {
+            if (t.key.size() != parts[0].n + parts[1].n + parts[2].n) return false;
+            size_t at = 0;
+            for (const auto& part : parts) {
+                if (part.n && std::memcmp(t.key.data() + at, part.p, part.n) != 0) return false;
+                at += part.n;
+            }
+            return true;
+        };
+        auto& kept = gb_tables(ctx.device);
+        static thread_local size_t recent = 0;  // most calls repeat the last one's arguments
+        auto it = kept.begin() + int64_t(std::min(recent, kept.size()));
+        if (it == kept.end() || !same(**it))
+            it = std::find_if(kept.begin(), kept.end(), [&](const auto& t) { return same(*t); });
+        recent = size_t(it - kept.begin());
+        const bool last = it != kept.end() ? it + 1 == kept.end() && kept.size() == kMaxTables
+                                           : kept.size() + 1 >= kMaxTables;
+        if (last) refuse_capture(stream);
+        if (it != kept.end()) {
+            (*it)->made.need(now);
+            tbp = it->get();
+        } else {
+            auto fresh = std::make_unique<GbTables>();
+            if (kept.size() == kMaxTables) {
+                STB_CUDA(cudaDeviceSynchronize());  // any stream's kernels may read them
+                fresh = std::move(kept.back());
+                kept.pop_back();
+                fresh->key.clear();
+            }
+            build_tables(*fresh, pen, go, ge, W, has_prior ? prior : nullptr, W1p, stream);
             for (const auto& part : parts) {
                 const auto* bytes = static_cast<const uint8_t*>(part.p);
-                if (part.n) tb.key.insert(tb.key.end(), bytes, bytes + part.n);
+                if (part.n) fresh->key.insert(fresh->key.end(), bytes, bytes + part.n);
             }
+            fresh->made.on(stream);
+            kept.push_back(std::move(fresh));  // (nothing is kept of a call that fails before)
+            tbp = kept.back().get();
         }
     }
+    const GbTables& tb = *tbp;
     // A sparse tile keeps a hit's sum without its term, at most threshold - term; sums stay below
     // 2^15, so two bytes always hold one.  Where sum + term can pass the end of int32 any sum is kept.
     const bool wraps = sink && tb.most_term > INT32_MAX - kMaxHalf;
@@ -1039,8 +1085,20 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
                          rp.max_tasks, sink ? (score16 ? 2 : 1) : 0);
     };
     if (fast) {
-        RefPlan& rp = plan_slot<RefPlan>(rs.gb_ref_plan, ctx.tmp_ref_plan, rs.owns);
         const int want_rc = t_force_rc ? t_force_rc : (tuned_choice >= 0 ? kRcCandidates[tuned_choice] : 0);
+        // A resident set keeps a plan per width it is called with; the tuner's trials share one.
+        RefPlans* own = rs.owns ? &plan_slot<RefPlans>(rs.gb_ref_plan, rs.gb_ref_plan, true) : nullptr;
+        if (own)
+            for (auto& p : own->of)
+                if (!want_rc || p->rc == want_rc) rpp = p.get();
+        std::unique_ptr<RefPlan> added;
+        if (!rpp && own && !t_trial_rc) {
+            added = std::make_unique<RefPlan>();
+            rpp = added.get();
+        }
+        if (!rpp) rpp = &plan_slot<RefPlan>(own ? ctx.trial_ref_plan : ctx.tmp_ref_plan,
+                                            own ? ctx.trial_ref_plan : ctx.tmp_ref_plan, false);
+        RefPlan& rp = *rpp;
         if (rp.uid != rs.uid || (want_rc && rp.rc != want_rc)) {
             Phase ph("ref_plan");
             // Chunk width: the autotuner's measured choice when there is one; otherwise the
@@ -1087,13 +1145,13 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
                     STB_CUDA(cudaGetLastError());
                 }
                 note_launch(nullptr, few ? 1 : 2);
-                if (rs.owns) rp.made.on(stream);
+                if (added) rp.made.on(stream);
                 rp.uid = rs.uid;
             }
         }
         sm = layout(rp);
         fast = rp.uid == rs.uid && sm.total <= ctx.max_smem_optin;
-        rpp = &rp;
+        if (added && fast) own->of.push_back(std::move(added));
     }
 
     if (!sink && !out_d) fail(ST_EINVAL, "seqtree_b200: null output buffer");
@@ -1129,35 +1187,56 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
         Phase ph("query_plan");
         build_query_plan(qp, qs, stream, r0, row_block ? r1 : -1);
     }
+    const uint32_t* prof = nullptr;
     {
         std::vector<uint8_t> key(sizeof(int) * 2 + pen.size() * 4);
         const int hdr[2] = {A, int(wide)};
         std::memcpy(key.data(), hdr, sizeof hdr);
         std::memcpy(key.data() + sizeof hdr, pen.data(), pen.size() * 4);
-        if (!same_as_last(qp.prof_key, key.data(), key.size())) {
-            qp.prof_key.clear();  // set again once the profile kernel is enqueued
+        // a resident set keeps the profiles of its first grids; a transient set's and a row block's plan has one
+        const bool kept = qs.owns && !row_block;
+        Profile* found = nullptr;
+        for (auto& p : qp.profiles)
+            if (!kept || p->key == key) found = p.get();
+        if (kept && (found ? found == qp.profiles.back().get() && qp.profiles.size() == kMaxProfiles
+                           : qp.profiles.size() + 1 >= kMaxProfiles))
+            refuse_capture(stream);
+        if (!found || found->key != key) {
             const size_t words = size_t(qp.prof_rows) * kQuads * kRow * (wide ? 2 : 1);
-            uint32_t* prof = qp.d_prof.as<uint32_t>(words, stream);
+            std::unique_ptr<Profile> added;
+            if (!found && qp.profiles.size() < kMaxProfiles) {
+                added = std::make_unique<Profile>();
+                found = added.get();
+            } else if (!found) {
+                STB_CUDA(cudaDeviceSynchronize());  // any stream's kernels may read it
+                found = qp.profiles.back().get();
+            }
+            found->key.clear();  // set again once the profile kernel is enqueued
+            uint32_t* p = found->buf.as<uint32_t>(words, stream);
+            qp.made.need(now);
             const int4* quads = static_cast<const int4*>(qp.d_plan.ptr);
             const int4* slices = quads + qp.quads.size();
             auto fill = wide ? profile_kernel<true> : profile_kernel<false>;
             fill<<<unsigned(qp.slices.size()), 256, 0, stream>>>(
                 qs.d_bytes, qs.d_off, quads, slices, tb.pen, A,
-                uint32_t(maxpen), prof);
+                uint32_t(maxpen), p);
             STB_CUDA(cudaGetLastError());
             note_launch(nullptr);
-            if (qs.owns) qp.made.on(stream);
-            qp.prof_key = key;
+            if (kept) found->made.on(stream);
+            found->key = key;
+            if (added) qp.profiles.push_back(std::move(added));
         }
+        found->made.need(now);
+        prof = static_cast<const uint32_t*>(found->buf.ptr);
     }
-    rp.made.need(stream);
-    qp.made.need(stream);
+    rp.made.need(now);
+    qp.made.need(now);
 
     auto* err = reinterpret_cast<unsigned long long*>(ctx.flags_d + 8);
     if (qs.owns || rs.owns) STB_CUDA(cudaMemsetAsync(err, 0, 8, stream));  // host calls cleared it
 
     FastArgs fa{};
-    fa.prof = static_cast<uint32_t*>(qp.d_prof.ptr);
+    fa.prof = prof;
     fa.slab = static_cast<uint8_t*>(rp.d_slab.ptr);
     fa.rlen = rs.d_len;
     fa.K = K;
@@ -1223,8 +1302,9 @@ void gapblock_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int
     const bool has_prior = prior && prior_len > 0;
     const std::string key = gb_shape_key(qs, rs, has_prior);
     // Candidates: every chunk width.
-    auto variant = [&](int c, int64_t rows) {
+    auto variant = [&](int c, int64_t rows, bool trial) {
         t_force_rc = c >= 0 ? kRcCandidates[c] : 0;  // -1: the static choice
+        t_trial_rc = trial;
         try {
             if (rows < 0)
                 run();
@@ -1233,10 +1313,16 @@ void gapblock_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int
                              out_d, nullptr, stream, 0, rows);
         } catch (...) {
             t_force_rc = 0;
+            t_trial_rc = false;
             throw;
         }
         t_force_rc = 0;
+        t_trial_rc = false;
     };
+    if (const int known = tuned_lookup(key); known >= 0) {
+        variant(known, -1, false);
+        return;
+    }
     // A shape seen for the first time is tuned on its first query rows only (about
     // kTuneSlicePairs pairs, written into their own rows of the result), so the first call costs
     // the variants' runs on that slice rather than on the whole matrix; the chosen variant then
@@ -1245,10 +1331,13 @@ void gapblock_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int
         qs.count, std::max<int64_t>(2 * kSliceQ, kTuneSlicePairs / std::max<int64_t>(rs.count, 1)));
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     STB_CUDA(cudaStreamIsCapturing(stream, &cs));
-    if (slice < qs.count && tuning_enabled() && cs == cudaStreamCaptureStatusNone &&
-        tuned_lookup(key) < 0)
-        tuned_run(key, kNumRc, -1, [&](int c) { variant(c, slice); }, stream);
-    tuned_run(key, kNumRc, -1, [&](int c) { variant(c, -1); }, stream);
+    const bool tunes = tuning_enabled() && cs == cudaStreamCaptureStatusNone;
+    if (slice < qs.count && tunes) {
+        const int c = tuned_run(key, kNumRc, -1, [&](int v) { variant(v, slice, true); }, stream);
+        variant(c, -1, false);
+        return;
+    }
+    tuned_run(key, kNumRc, -1, [&](int c) { variant(c, -1, tunes); }, stream);
 }
 
 // Scores of listed pairs (device index arrays) into out_d; the general int32 kernel's
@@ -1499,15 +1588,18 @@ void gapblock_sparse_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penal
             }
             tuned_run(skey, kNumRc, -1, [&](int c) {
                 t_force_rc = c >= 0 ? kRcCandidates[c] : 0;
+                t_trial_rc = true;
                 try {
                     STB_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned long long), stream));
                     gapblock_run(qs, rs, penalty, matrix_size, go, ge, prior, prior_len,
                                  prior_width, nullptr, &ts, stream, 0, tr1 == N ? -1 : tr1);
                 } catch (...) {
                     t_force_rc = 0;
+                    t_trial_rc = false;
                     throw;
                 }
                 t_force_rc = 0;
+                t_trial_rc = false;
             }, stream);
         }
     }

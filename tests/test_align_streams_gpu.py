@@ -60,10 +60,10 @@ def test_more_matrices_than_are_kept(cuda_ready):
     rng = np.random.default_rng(2)
     q, r = rand_seqs(rng, 5, 8, 40, "ACGT"), rand_seqs(rng, 40, 8, 40, "ACGT")
     grids = []
-    for _ in range(70):
+    for _ in range(1030):
         g = rng.integers(-4, 6, size=(4, 4))
         grids.append((g + g.T) // 2)
-    for g in grids + grids[:2] + grids[-2:]:
+    for g in grids + grids[:2] + grids[-8:]:
         m = SubstitutionMatrix.from_similarity(g)
         got = np.asarray(pairwise.dist_matrix(q, r, m, gap_open=5, gap_extend=2, alphabet="nt"))
         want = oracle.align_matrix(q, r, m.similarity_grid, mode="global", gap_open=5, gap_extend=2, dist=True,

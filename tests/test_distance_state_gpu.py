@@ -40,7 +40,8 @@ def test_a_refused_capture_leaves_nothing_behind(cuda_ready, warm):
 
 
 SYMBOLS = {"acgt": "ACGT", "acgtn": "ACGTN", "aa": "ACDEFGHIKLMNPQRSTVWY", "two": "AC", "lower": "acgt",
-           "digits": "0123456789", "all": "".join(map(chr, range(33, 90)))}
+           "digits": "0123456789", "all": "".join(map(chr, range(33, 90))), "gap": "ACGT-", "rna": "ACGU",
+           "soft": "ACGTacgt", "iupac": "ACGTRYSWKMBDHVN", "binary": "01"}
 
 
 def sets_of(rng, count, length=21):
@@ -62,7 +63,7 @@ def test_a_captured_call_keeps_its_alphabet(cuda_ready, name):
     with torch.cuda.graph(graph):
         into(name, sets["acgt"], sets["two"], out)
     for _ in range(2):
-        for other in ("acgtn", "aa", "lower", "digits", "all", "acgt"):
+        for other in SYMBOLS:
             for a, b in ((other, "acgt"), ("acgt", other), ("two", other)):
                 got = torch.full((len(strings[a]), len(strings[b])), -1, dtype=torch.int32, device="cuda")
                 into(name, sets[a], sets[b], got)
