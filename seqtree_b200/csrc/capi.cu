@@ -470,6 +470,7 @@ int32_t st_align_pair(const char* query, int64_t query_len, const char* ref, int
         if (bad >= 0) fail(ST_EINVAL, std::string("invalid symbol '") + bc + "' in sequence");
         const int64_t slot = std::max<int64_t>(query_len + ref_len, 1);
         // device scratch: pair indices, score, start, three string slots
+        ScratchTurn turn(ctx, ctx.stream);
         auto* base = static_cast<uint8_t*>(ctx.work_b.get(size_t(64 + 3 * slot)));
         auto* idx = reinterpret_cast<int32_t*>(base);
         auto* sc = reinterpret_cast<int64_t*>(base + 16);
@@ -560,6 +561,7 @@ int32_t st_penalty_align_pairs(const st_strings* queries, const st_strings* refs
         const int64_t slot = std::max<int64_t>(mq + mr, 1);
         // device: pair indices, scores, starts, op slots
         const size_t idx_b = size_t(n) * 8, sc_b = size_t(n) * 4, st_b = size_t(n) * 4;
+        ScratchTurn turn(ctx, ctx.stream);
         auto* base = static_cast<uint8_t*>(ctx.work_b.get(idx_b + sc_b + st_b + size_t(n * slot) + 64));
         auto* qi_d = reinterpret_cast<int32_t*>(base);
         auto* ri_d = qi_d + n;

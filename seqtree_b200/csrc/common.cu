@@ -234,29 +234,32 @@ DevBuf::~DevBuf() {
     // Contexts live until process exit; the driver reclaims device memory then.
 }
 
-void StreamScratch::take(int device, size_t bytes, cudaStream_t st) {
-    if (!bytes) return;
-    constexpr uint64_t kKeep = uint64_t(256) << 20;  // bytes that stay cached in the pool
+namespace {
+// The device's pool, made with its context (a captured call may take memory but not make the pool).
+cudaMemPool_t scratch_pool(int device) {
+    constexpr uint64_t kKeep = uint64_t(256) << 20;  // bytes that stay cached in it
     static std::mutex mu;
     static std::map<int, cudaMemPool_t> pools;
-    cudaMemPool_t pool;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        cudaMemPool_t& slot = pools[device];
-        if (!slot) {
-            cudaMemPoolProps props{};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = device;
-            cudaMemPool_t fresh = nullptr;
-            STB_CUDA(cudaMemPoolCreate(&fresh, &props));
-            uint64_t keep_bytes = kKeep;
-            STB_CUDA(cudaMemPoolSetAttribute(fresh, cudaMemPoolAttrReleaseThreshold, &keep_bytes));
-            slot = fresh;
-        }
-        pool = slot;
+    std::lock_guard<std::mutex> lk(mu);
+    cudaMemPool_t& slot = pools[device];
+    if (!slot) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t fresh = nullptr;
+        STB_CUDA(cudaMemPoolCreate(&fresh, &props));
+        uint64_t keep_bytes = kKeep;
+        STB_CUDA(cudaMemPoolSetAttribute(fresh, cudaMemPoolAttrReleaseThreshold, &keep_bytes));
+        slot = fresh;
     }
-    STB_CUDA(cudaMallocFromPoolAsync(&ptr, bytes, pool, st));
+    return slot;
+}
+}  // namespace
+
+void StreamScratch::take(int device, size_t bytes, cudaStream_t st) {
+    if (!bytes) return;
+    STB_CUDA(cudaMallocFromPoolAsync(&ptr, bytes, scratch_pool(device), st));
     stream = st;
 }
 
@@ -288,6 +291,19 @@ void Made::on(cudaStream_t stream) {
     if (!event) STB_CUDA(cudaEventCreateWithFlags(&event, cudaEventDisableTiming));
     STB_CUDA(cudaStreamGetId(stream, &stream_id));
     STB_CUDA(cudaEventRecord(event, stream));
+}
+
+ScratchTurn::ScratchTurn(Context& c, cudaStream_t s) : ctx(c), now(s) {
+    if (!now.capturing) ctx.scratch.need(now);
+}
+
+ScratchTurn::~ScratchTurn() {
+    if (now.capturing) return;
+    try {
+        ctx.scratch.on(now.stream);
+    } catch (...) {
+        cudaGetLastError();  // (a failed stream: the call's own error says so)
+    }
 }
 
 StreamNow::StreamNow(cudaStream_t s) : stream(s) {
@@ -369,6 +385,7 @@ Context& context() {
                                     dev));
     STB_CUDA(cudaMalloc(&c->flags_d, 64 * sizeof(int64_t)));
     STB_CUDA(cudaHostAlloc(&c->flags_h, 64 * sizeof(int64_t), cudaHostAllocDefault));
+    scratch_pool(dev);
     Context& ref = *c;
     g_ctx.emplace(dev, std::move(c));
     return ref;
@@ -633,6 +650,7 @@ st_seqset_s* make_seqset(const st_strings* s, int32_t alphabet, cudaStream_t str
             STB_CUDA(cudaMemcpyAsync(set->d_bytes, src, size_t(set->total), cudaMemcpyHostToDevice,
                                      stream));
         } else {
+            ScratchTurn turn(ctx, stream);
             DevBuf& raw = ctx.work_c;
             uint8_t* d_raw = raw.as<uint8_t>(padded);
             STB_CUDA(cudaMemsetAsync(d_raw + set->total, 0, 64, stream));

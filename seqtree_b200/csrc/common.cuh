@@ -148,6 +148,8 @@ struct Context {
     // second stream and events of the host calls that overlap the result copy with the kernels
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t block_ev[8] = {};
+    // the last use of the scratch and tables below by a call on a caller's stream (ScratchTurn)
+    Made scratch;
     // named scratch, grow-only
     DevBuf out_buf, q_codes, r_codes, table_buf, prior_buf, ftab_buf, work_a, work_b, work_c;
     // sparse output: unsorted hit keys and scores, sorted keys, radix-sort scratch
@@ -179,6 +181,24 @@ struct Context {
 // Context of the current CUDA device (created on first use).  Fails with ST_ENODEV when no
 // device is usable.
 Context& context();
+
+// A call's turn with the context's scratch and tables: what it enqueues while this lives comes after the
+// last such call's kernels, whatever stream they are on.  Nothing orders a graph's replays with later
+// calls, so a captured call takes memory of its own instead (`own`, which becomes the graph's).
+struct ScratchTurn {
+    Context& ctx;
+    const StreamNow now;
+    ScratchTurn(Context& c, cudaStream_t s);
+    ~ScratchTurn();
+    ScratchTurn(const ScratchTurn&) = delete;
+    ScratchTurn& operator=(const ScratchTurn&) = delete;
+    template <class T>
+    T* as(DevBuf& shared, size_t count, StreamScratch& own) {
+        if (!now.capturing) return shared.as<T>(count);
+        own.take(ctx.device, count * sizeof(T), now.stream);
+        return static_cast<T*>(own.ptr);
+    }
+};
 
 // Raises `kernel`'s dynamic shared-memory limit to `bytes` on the current device, once per
 // (device, kernel, size).  The attribute belongs to a device, so a process that uses several

@@ -634,7 +634,9 @@ void levenshtein_sets(st_seqset_s& a, st_seqset_s& b, int32_t* out_d, cudaStream
     const int64_t per = int64_t(shorter_max) + 1;
     threads = std::max<int64_t>(256, std::min<int64_t>(threads, (int64_t(1) << 29) / per));
     threads = ceil_div(threads, 256) * 256;
-    int32_t* scratch = ctx.work_a.as<int32_t>(size_t(threads) * per);
+    ScratchTurn turn(ctx, stream);
+    StreamScratch own;
+    int32_t* scratch = turn.as<int32_t>(ctx.work_a, size_t(threads) * per, own);
     levenshtein_dp_kernel<<<unsigned(threads / 256), 256, 0, stream>>>(a.d_bytes, aoff, b.d_bytes, b.d_off, N, K,
                                                                        scratch, out_d);
     STB_CUDA(cudaGetLastError());

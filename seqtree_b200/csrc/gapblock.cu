@@ -1158,6 +1158,7 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
     if (!fast && sink && sink->ordered)
         fail(ST_ECUDA, "seqtree_b200: internal error: the ordered sparse form needs the fast kernel");
     if (!fast) {
+        ScratchTurn turn(ctx, stream);
         int32_t* d_pen = ctx.table_buf.as<int32_t>(pen.size());
         h2d(d_pen, pen.data(), pen.size() * 4, stream);
         int32_t* d_prior = nullptr;
@@ -1365,37 +1366,48 @@ void gapblock_pairs_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* qi_d, 
     std::vector<int32_t> pen(size_t(A) * A);
     for (int x = 0; x < A; ++x)
         for (int y = 0; y < A; ++y) pen[size_t(x) * A + y] = penalty ? penalty[x * A + y] : int32_t(x != y);
-    // Tables cached per device by content, so repeated calls upload nothing (and can be
-    // captured in a CUDA graph once warmed up).
-    struct PairTables {
-        std::vector<uint8_t> key;
-        DevBuf pen, prior;
+    // Tables kept per device by content, so repeated calls upload nothing (and can be captured in a CUDA graph
+    // once warmed up); prior cubes as the matrix tables: 16 are never rewritten, one more changes hands.
+    struct PairPrior {
+        std::vector<int32_t> cube;
+        OwnedBuf buf;
+        Made made;
     };
+    constexpr size_t kMaxPriors = 17;
     static std::mutex mu;
-    static std::map<int, std::unique_ptr<PairTables>> all;
-    PairTables* pt;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        auto& slot = all[ctx.device];
-        if (!slot) slot = std::make_unique<PairTables>();
-        pt = slot.get();
-    }
-    {
-        std::vector<uint8_t> key(pen.size() * 4 + (has_prior ? size_t(prior_len) * 4 : 0) + 8);
-        const int64_t hdr = has_prior ? prior_len : -1;
-        std::memcpy(key.data(), &hdr, 8);
-        std::memcpy(key.data() + 8, pen.data(), pen.size() * 4);
-        if (has_prior) std::memcpy(key.data() + 8 + pen.size() * 4, prior, size_t(prior_len) * 4);
-        if (!same_as_last(pt->key, key.data(), key.size())) {
-            pt->key.clear();
-            h2d(pt->pen.as<int32_t>(pen.size()), pen.data(), pen.size() * 4, stream);
-            if (has_prior)
-                h2d(pt->prior.as<int32_t>(size_t(prior_len)), prior, size_t(prior_len) * 4, stream);
-            pt->key = key;
+    static std::map<int, std::vector<std::unique_ptr<PairPrior>>> all;
+    StreamScratch pen_mem;
+    const int32_t* d_pen = kept_table(ctx, pen, stream, pen_mem);
+    const int32_t* d_prior = nullptr;
+    if (has_prior) {
+        std::vector<std::unique_ptr<PairPrior>>* kept;
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            kept = &all[ctx.device];
         }
+        auto it = std::find_if(kept->begin(), kept->end(), [&](const auto& p) {
+            return int64_t(p->cube.size()) == prior_len &&
+                   std::memcmp(p->cube.data(), prior, size_t(prior_len) * 4) == 0;
+        });
+        const bool found = it != kept->end();
+        if (found ? it + 1 == kept->end() && kept->size() == kMaxPriors : kept->size() + 1 >= kMaxPriors)
+            refuse_capture(stream);
+        if (!found) {
+            auto fresh = std::make_unique<PairPrior>();
+            if (kept->size() == kMaxPriors) {
+                STB_CUDA(cudaDeviceSynchronize());  // any stream's kernels may read it
+                fresh = std::move(kept->back());
+                kept->pop_back();
+            }
+            h2d(fresh->buf.as<int32_t>(size_t(prior_len), stream), prior, size_t(prior_len) * 4, stream);
+            fresh->cube.assign(prior, prior + prior_len);
+            fresh->made.on(stream);
+            kept->push_back(std::move(fresh));
+            it = kept->end() - 1;
+        }
+        (*it)->made.need(stream);
+        d_prior = static_cast<const int32_t*>((*it)->buf.ptr);
     }
-    const int32_t* d_pen = static_cast<const int32_t*>(pt->pen.ptr);
-    const int32_t* d_prior = has_prior ? static_cast<const int32_t*>(pt->prior.ptr) : nullptr;
     const int64_t blocks = std::min<int64_t>(ceil_div(n, 256), int64_t(ctx.num_sms) * 16);
     gapblock_pairs_kernel<<<unsigned(blocks), 256, size_t(A) * A * 4, stream>>>(
         qs.d_bytes, qs.d_off, rs.d_bytes, rs.d_off, qi_d, ri_d, n, d_pen, A, go, ge, d_prior, W1p,
@@ -1542,6 +1554,7 @@ void gapblock_sparse_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penal
         STB_CUDA(cudaMemsetAsync(indptr, 0, sizeof(int64_t) * size_t(N + 1), stream));
         return;
     }
+    ScratchTurn turn(ctx, stream);
     const int shift = bits_for(K);
     if (shift + bits_for(N) > 63) fail(ST_EINVAL, "seqtree_b200: matrix too large for sparse keys");
     const int end_bit = shift + bits_for(N);

@@ -397,9 +397,10 @@ bool vec_ok(const PackSrc& s, int K) {
 }
 
 // op[i][k] = trans ? s[k][i] : s[i][k]
-const uint8_t* pack(const PackSrc& s, bool trans, int rows, int K, DevBuf& buf, cudaStream_t st) {
+size_t pack_bytes(int rows, int K) { return size_t(ceil_div(rows, kGT)) * size_t(ceil_div(K, kGK)) * kBlockB; }
+
+const uint8_t* pack(const PackSrc& s, bool trans, int rows, int K, uint8_t* op, cudaStream_t st) {
     const int tiles = int(ceil_div(rows, kGT)), kchunks = int(ceil_div(K, kGK));
-    uint8_t* op = buf.as<uint8_t>(size_t(tiles) * kchunks * kBlockB);
     const int64_t units = int64_t(tiles) * kchunks * kGT * 8;
     if (trans)
         pack_cols_kernel<<<unsigned(tiles * kchunks), 256, 0, st>>>(s, rows, K, kchunks, op);
@@ -513,6 +514,7 @@ void gemm_bf16(bool ta, bool tb, int M, int N, int K, const float* A, int lda, c
         return;
     }
     Context& ctx = context();
+    ScratchTurn turn(ctx, st);
     PackSrc a{}, b{};
     a.x = A;
     a.ld = lda;
@@ -520,8 +522,9 @@ void gemm_bf16(bool ta, bool tb, int M, int N, int K, const float* A, int lda, c
     b.ld = ldb;
     GemmBf16Args g{};
     // op(A)[i][k] = ta ? A[k][i] : A[i][k];  op(B)^T[n][k] = tb ? B[n][k] : B[k][n]
-    g.a = pack(a, ta, M, K, ctx.gemm_a, st);
-    g.b = pack(b, !tb, N, K, ctx.gemm_b, st);
+    StreamScratch own_a, own_b;
+    g.a = pack(a, ta, M, K, turn.as<uint8_t>(ctx.gemm_a, pack_bytes(M, K), own_a), st);
+    g.b = pack(b, !tb, N, K, turn.as<uint8_t>(ctx.gemm_b, pack_bytes(N, K), own_b), st);
     g.kchunks = int(ceil_div(K, kGK));
     g.C = C;
     g.ldc = ldc;

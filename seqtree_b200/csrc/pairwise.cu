@@ -1083,6 +1083,7 @@ void align_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
         return;
     }
 
+    ScratchTurn turn(ctx, stream);
     int32_t* d_sim = ctx.table_buf.as<int32_t>(size_t(A) * A);
     h2d(d_sim, similarity, size_t(A) * A * 4, stream);
     ExactArgs a{};

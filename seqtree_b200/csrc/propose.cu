@@ -812,7 +812,9 @@ void propose_topk(const void* qemb, int64_t nq, const void* remb, int64_t nr, in
     a.nr = nr;
     a.k = k;
     a.ranges = ranges;
-    a.cand = ctx.topk_cand.as<unsigned long long>(size_t(grid) * kQT * kCap);
+    ScratchTurn turn(ctx, stream);
+    StreamScratch own;
+    a.cand = turn.as<unsigned long long>(ctx.topk_cand, size_t(grid) * kQT * kCap, own);
     a.out_ids = ids;
     a.out_scores = scores;
     a.err = reinterpret_cast<unsigned long long*>(ctx.flags_d + 8);
@@ -839,6 +841,7 @@ int64_t propose_range(const void* qemb, int64_t nq, const uint8_t* qlens, const 
         fail(ST_EINVAL, "seqtree_b200: embeddings must be 16-byte aligned");
     Context& ctx = context();
     constexpr size_t kThrBytes = sizeof(float) * kLenSlots * kLenSlots;
+    ScratchTurn turn(ctx, stream);
     float* d_thr = ctx.prop_thr.as<float>(kLenSlots * kLenSlots);
     if (!same_as_last(ctx.prop_thr_key, thr, kThrBytes)) h2d(d_thr, thr, kThrBytes, stream);
     ensure_smem_limit(reinterpret_cast<const void*>(propose_range_kernel), kSmemBytes);

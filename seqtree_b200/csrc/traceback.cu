@@ -375,6 +375,7 @@ void align_pairs_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* qi_d, con
         fail(ST_EINVAL, "seqtree_b200: output slots shorter than the longest query + ref");
     if (n == 0) return;
     Context& ctx = context();
+    ScratchTurn turn(ctx, stream);
     int32_t* d_sim = ctx.table_buf.as<int32_t>(size_t(A) * A);
     h2d(d_sim, similarity, size_t(A) * A * 4, stream);
     TraceArgs a{};
@@ -426,6 +427,7 @@ void penalty_align_pairs_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* q
         fail(ST_EINVAL, "seqtree_b200: output slots shorter than the longest query + ref");
     if (n == 0) return;
     Context& ctx = context();
+    ScratchTurn turn(ctx, stream);
     int32_t* d_pen = nullptr;
     if (penalty) {
         d_pen = ctx.table_buf.as<int32_t>(size_t(A) * A);
