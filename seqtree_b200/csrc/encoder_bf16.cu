@@ -1040,6 +1040,9 @@ __global__ void __launch_bounds__(kOutWarps * 32, 1) out_bf16_kernel(const float
 struct Bf16State {
     int64_t version = -1;
     DevBuf w2, wl[2], bl[2], wout, lens, h1, ha, hb, pooled;
+    ~Bf16State() {  // (with the encoder: 0.84 GB)
+        for (DevBuf* b : {&w2, &wl[0], &wl[1], &bl[0], &bl[1], &wout, &lens, &h1, &ha, &hb, &pooled}) b->release();
+    }
 };
 
 void launch_conv2(const GemmArgs& g, int sms, cudaStream_t st) {
