@@ -434,7 +434,8 @@ void run_gemm(GemmBf16Args g, bool tn, bool accumulate, cudaStream_t st, int sms
     splits = int(ceil_div(g.kchunks, g.chunks_per_split));
     g.mode = splits > 1 ? 2 : (accumulate ? 1 : 0);
     if (splits > 1 && !accumulate)
-        STB_CUDA(cudaMemsetAsync(g.C, 0, sizeof(float) * size_t(g.M) * size_t(g.ldc), st));
+        STB_CUDA(cudaMemset2DAsync(g.C, sizeof(float) * size_t(g.ldc), 0, sizeof(float) * size_t(g.N), size_t(g.M),
+                                   st));  // (columns past N are not C's)
     g.err = reinterpret_cast<unsigned long long*>(ctx.flags_d + 8);
     auto kernel = tn ? gemm_bf16_kernel<true> : gemm_bf16_kernel<false>;
     ensure_smem_limit(reinterpret_cast<const void*>(kernel), kGSmem);
