@@ -696,6 +696,7 @@ struct Encoder {
     int64_t step = 0;            // Adam steps taken: also the version of the parameters
     int precision = 1;           // training products: 1 bf16 tensor cores, 0 fp32 SIMT
     std::shared_ptr<void> bf16;  // weights and workspace of the bf16 inference path
+    Made last;                   // the last embedding call: it reads the parameters and works in these buffers
     int S_cap = 0;  // sequences the workspace holds
     // forward activations (rows = 32 * S)
     DevBuf codes, lens, scores, pre1, h1, x2, pre2, hA, hB, hC, qkv0, qkv1, a0, a1, o0, o1, y, pool,
@@ -947,6 +948,7 @@ void upload_batch(Encoder& m, const uint8_t* codes, const int32_t* lens, const i
             fail(ST_EINVAL, "seqtree_b200: encoder inputs must have 1..32 residues");
     for (int64_t i = 0; i < int64_t(S) * kP; ++i)
         if (codes[i] >= kA) fail(ST_EINVAL, "seqtree_b200: encoder codes must be < 24");
+    m.last.need(st);
     m.reserve(S, m.precision == 1);
     h2d(m.codes.ptr, codes, size_t(S) * kP, st);
     h2d(m.lens.ptr, lens, sizeof(int32_t) * size_t(S), st);
@@ -1048,8 +1050,11 @@ void encoder_embed(Encoder& m, const st_seqset_s& set, void* out, int layout, cu
         fail(ST_EINVAL, "seqtree_b200: the encoder takes amino-acid sets");
     for (int32_t L : set.h_len)
         if (L < 1 || L > kP) fail(ST_EINVAL, "seqtree_b200: encoder inputs must have 1..32 residues");
+    const StreamNow now(st);
+    m.last.need(now);
     if (layout == 1) {
         encoder_embed_bf16(P(m), m.step, m.bf16, set, static_cast<__nv_bfloat16*>(out), st);
+        if (!now.capturing) m.last.on(st);
         return;
     }
     Context& ctx = context();
@@ -1066,6 +1071,7 @@ void encoder_embed(Encoder& m, const st_seqset_s& set, void* out, int layout, cu
         STB_CUDA(cudaGetLastError());
         note_launch(nullptr, 2);
     }
+    if (!now.capturing) m.last.on(st);
 }
 
 }  // namespace stb
