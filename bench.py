@@ -9,8 +9,9 @@ central_prior(21); int32 output bit-identical to seqtree's C++.
     python bench.py [--gpus N] [--steps K] [--warmup W] [--workload NAME] [--impl ours|reference]
                     [--no-suite]
 
-At N = 1 the headline line also carries, under ``workloads``, one complete line for each other
-named configuration (unless ``--no-suite``): ``hamming`` / ``levenshtein`` (20,000 x 20,000 ACGT),
+At N = 1 each other named configuration is measured too (unless ``--no-suite``): its value, end-to-end value
+and parity stand under the headline line's ``workloads``, its complete line, like the measured
+instruction peaks, on standard error (a line of 24 KB had been cut off where the output is kept). They are ``hamming`` / ``levenshtein`` (20,000 x 20,000 ACGT),
 ``nw`` / ``sw`` (4,096 x 4,096 proteins, distance matrix), ``sparse`` / ``sparse_structural``
 (100,000 x 1,000,000 CDR3-like, thresholded at max_penalty 24 into CSR rows; the dense matrix would
 be 400 GB) and ``learned`` (1,000,000 x 1,000,000, learned proposal + exact rescore).
@@ -461,6 +462,38 @@ def parity(w, rows, ref, got, kind) -> dict:
             "checker": checker}
 
 
+def short(v):
+    """Numbers to six digits, throughout."""
+    if isinstance(v, dict):
+        return {k: short(x) for k, x in v.items()}
+    if isinstance(v, (list, tuple)):
+        return [short(x) for x in v]
+    return float(f"{v:.6g}") if isinstance(v, float) else v
+
+
+def emit(line: dict) -> None:
+    """The one line on standard output; complete lines of the nested configurations, the peaks and the
+    soak on standard error."""
+    line = dict(line)
+    nested = line.pop("workloads", {})
+    more = {k: line.pop(k) for k in ("int_peaks", "soak", "tuning", "clocks_timed_region") if k in line}
+    for name, sub in nested.items():
+        print(json.dumps({"workload": name, **sub}), file=sys.stderr, flush=True)
+    if more:
+        print(json.dumps(more), file=sys.stderr, flush=True)
+    if nested:
+        brief = {}
+        for name, sub in nested.items():
+            if "error" in sub:
+                brief[name] = {"error": str(sub["error"])[:80]}
+                continue
+            par = (sub.get("cpu_baseline") or {}).get("parity") or {}
+            brief[name] = {"value": sub.get("value"), "e2e": (sub.get("e2e") or {}).get("value"),
+                           **{k: par[k] for k in ("exact", "hits_exact", "recall") if k in par}}
+        line["workloads"] = brief
+    print(json.dumps(short(line)), flush=True)
+
+
 def main_reference(args):
     world, rank, _ = dist_env()
     if rank != 0:
@@ -475,7 +508,7 @@ def main_reference(args):
                                                          steps=min(args.steps, 5), warmup=1)
             except Exception as e:  # report and carry on with the next configuration
                 line["workloads"][name] = {"impl": "reference", "error": str(e)}
-    print(json.dumps(line), flush=True)
+    emit(line)
     return 0
 
 
@@ -554,7 +587,7 @@ def main_ours(args):
                                   "all_sms_per_sm_clk": v["all_sms"]["per_sm_clk"],
                                   "one_sm_per_clk": v["one_sm"]["per_sm_clk"]}
                              for op, v in int_peaks.items()}
-        print(json.dumps(line), flush=True)
+        emit(line)
     if world > 1:
         import torch.distributed as dist
         dist.destroy_process_group()
