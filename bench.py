@@ -28,7 +28,7 @@ be 400 GB) and ``learned`` (1,000,000 x 1,000,000, learned proposal + exact resc
 * ``kernel_roofline``: the dominant kernel against its own bound, with the instruction peaks
   measured in this process (``int_peaks``).
 * ``--impl reference``: times that CPU implementation alone, on the same workloads; it imports
-  nothing that loads this library.
+  nothing that loads this library.  Where the reference was not built it says so and times nothing.
 """
 from __future__ import annotations
 
@@ -497,6 +497,11 @@ def emit(line: dict) -> None:
 def main_reference(args):
     world, rank, _ = dist_env()
     if rank != 0:
+        return 0
+    import oracle
+    if not oracle.ref_available():
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "the reference's sources are not present, so its build was not made"}))
         return 0
     line = reference_line(args, args.workload, world, float(
         os.environ.get("SEQTREE_B200_REF_STEP_S", "5")))

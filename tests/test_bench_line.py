@@ -25,3 +25,12 @@ def test_one_short_line(capsys):
     whole = [json.loads(t) for t in err.splitlines()]
     assert [t.get("workload") for t in whole] == bench.SUITE + [None]
     assert whole[0]["config"] == sub["config"] and "int_peaks" in whole[-1]
+
+
+def test_the_reference_arm_times_only_the_reference(capsys, monkeypatch):
+    import bench
+    import oracle
+    monkeypatch.setattr(oracle, "ref_available", lambda: False)
+    assert bench.main(["--impl", "reference"]) == 0
+    got = json.loads(capsys.readouterr().out)
+    assert got["impl"] == "reference" and got["unavailable"]
