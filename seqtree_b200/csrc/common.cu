@@ -82,8 +82,13 @@ int tuned_lookup(const std::string& key) {
     return it == g_tune.end() ? -1 : it->second;
 }
 
+void tuned_keep(const std::string& key, int choice) {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    g_tune.emplace(dev_key(key), choice);
+}
+
 int tuned_run(const std::string& key, int n, int fallback, const std::function<void(int)>& run,
-              cudaStream_t stream) {
+              cudaStream_t stream, float* best_ms) {
     const std::string k = dev_key(key);
     if (const int known = tuned_lookup(key); known >= 0) {
         run(known);  // (not under the lock: a run looks choices up too)
@@ -142,6 +147,7 @@ int tuned_run(const std::string& key, int n, int fallback, const std::function<v
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune[k] = pick;
     g_tune_log[k] = log;
+    if (best_ms) *best_ms = best;
     return pick;
 }
 
@@ -361,7 +367,7 @@ bool same_as_last(std::vector<uint8_t>& slot, const void* data, size_t bytes) {
 // ----------------------------------------------------------------------------- context ------
 namespace {
 std::mutex g_ctx_mu;
-std::map<int, std::unique_ptr<Context>> g_ctx;
+std::map<int, std::unique_ptr<Context>>& g_ctx = *new std::map<int, std::unique_ptr<Context>>;  // until exit
 }  // namespace
 
 Context& context() {

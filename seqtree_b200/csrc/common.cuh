@@ -234,8 +234,11 @@ bool same_as_last(std::vector<uint8_t>& slot, const void* data, size_t bytes);
 // choice directly.  Tuning is off with SEQTREE_B200_TUNE=0; then, and while `stream` is being
 // captured before the key was tuned, `run(fallback)` runs (`fallback` may be -1, the caller's
 // static choice).
+// `best_ms`, when given, gets the choice's time if this call measured it.
 int tuned_run(const std::string& key, int n, int fallback, const std::function<void(int)>& run,
-              cudaStream_t stream);
+              cudaStream_t stream, float* best_ms = nullptr);
+// Records a choice for `key` unless it has one.
+void tuned_keep(const std::string& key, int choice);
 // The cached choice for `key` on the current device, or -1.
 int tuned_lookup(const std::string& key);
 // False when SEQTREE_B200_TUNE=0 switched measured tuning off.

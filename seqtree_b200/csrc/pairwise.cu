@@ -1031,6 +1031,7 @@ void align_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
                           std::to_string(rs.max_len) + "|" + std::to_string(size_bucket(N)) + "|" +
                           std::to_string(size_bucket(K)) + "|";
         for (Kind k : kinds) key += "twWs"[k];
+        const std::string shape = key;
         if (fresh[0] || fresh[1]) key += std::string("|new") + (fresh[0] ? "q" : "") + (fresh[1] ? "r" : "");
         // Without a measurement (tuning off, or a stream being captured): the strip kernel when
         // its warps fill the GPU, else the first kind.
@@ -1074,11 +1075,15 @@ void align_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* similarity, int
         // computes the whole matrix.
         const int64_t slice = std::min<int64_t>(
             N, std::max<int64_t>(64, kAlignTunePairs / std::max<int64_t>(K, 1)));
+        float best_ms = 0.f;
         if (slice < N && tuning_enabled() && tuned_lookup(key) < 0) {
             std::unique_ptr<st_seqset_s> view = row_view(qs, slice);
-            tuned_run(key, int(kinds.size()), fallback, [&](int c) { timed(c, *view); }, stream);
+            tuned_run(key, int(kinds.size()), fallback, [&](int c) { timed(c, *view); }, stream, &best_ms);
         }
-        tuned_run(key, int(kinds.size()), fallback, [&](int c) { timed(c, qs); }, stream);
+        const int choice = tuned_run(key, int(kinds.size()), fallback, [&](int c) { timed(c, qs); }, stream, &best_ms);
+        // beside a millisecond the plans' cost changes no choice: one measurement serves every key of the shape
+        if (best_ms >= 1.f)
+            for (const char* suffix : {"", "|newq", "|newr", "|newqr"}) tuned_keep(shape + suffix, choice);
         for (st_seqset_s* t : sets) ++t->align_calls;
         return;
     }

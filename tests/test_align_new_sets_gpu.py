@@ -66,3 +66,21 @@ def test_one_call_is_enough_before_a_capture(cuda_ready, lo, hi, nq, nr):
             out.zero_()
             graph.replay()
             check(out, q, r, m, dist=dist)
+
+
+def test_large_shapes_are_measured_once(cuda_ready):
+    """Beside a kernel of a millisecond the plans do not count: the first call's choice serves all later ones."""
+    import torch
+    from seqtree_b200 import _lib, device
+    m, _ = matrices()
+    rng = np.random.default_rng(5)
+    a, b = device.SeqSet(rand_seqs(rng, 130, 150, 210)), device.SeqSet(rand_seqs(rng, 1500, 150, 211))
+    out = torch.zeros((130, 1500), dtype=torch.int32, device="cuda")
+    tables = []
+    for _ in range(3):
+        device.align_into(a, b, out.data_ptr(), torch.cuda.current_stream().cuda_stream, matrix=m)
+        torch.cuda.synchronize()
+        tables.append([t for t in _lib.tuning_table().splitlines() if "|0|0|24|" in t and "|7|10|" in t and "ms" in t])
+    assert tables[0] == tables[1] == tables[2]
+    if os.environ.get("SEQTREE_B200_TUNE") != "0":
+        assert len(tables[0]) == 1
