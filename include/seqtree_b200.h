@@ -17,7 +17,9 @@
  *   - `threads` is accepted for signature parity with the reference and ignored: the work
  *     runs on the current CUDA device.
  *   - There is no CPU fallback.  Without a usable CUDA device the calls return ST_ENODEV.
- *   - Calls are thread-safe; calls on the same device are serialised internally.
+ *   - Calls are thread-safe; calls on the same device are serialised internally.  Calls on resident
+ *     sets (st_*_sets) may run on several streams at once, over the same sets and with different
+ *     arguments.  (Not so st_levenshtein_matrix_noalloc: see there.)
  */
 #ifndef SEQTREE_B200_H
 #define SEQTREE_B200_H

@@ -866,7 +866,7 @@ constexpr size_t kMaxTables = 65;  // the last one changes hands
 
 std::vector<std::unique_ptr<GbTables>>& gb_tables(int device) {
     static std::mutex mu;
-    static std::map<int, std::vector<std::unique_ptr<GbTables>>> all;
+    static auto& all = *new std::map<int, std::vector<std::unique_ptr<GbTables>>>;  // (until the process exits)
     std::lock_guard<std::mutex> lk(mu);
     return all[device];
 }
@@ -1375,7 +1375,7 @@ void gapblock_pairs_sets(st_seqset_s& qs, st_seqset_s& rs, const int32_t* qi_d, 
     };
     constexpr size_t kMaxPriors = 17;
     static std::mutex mu;
-    static std::map<int, std::vector<std::unique_ptr<PairPrior>>> all;
+    static auto& all = *new std::map<int, std::vector<std::unique_ptr<PairPrior>>>;  // (until the process exits)
     StreamScratch pen_mem;
     const int32_t* d_pen = kept_table(ctx, pen, stream, pen_mem);
     const int32_t* d_prior = nullptr;

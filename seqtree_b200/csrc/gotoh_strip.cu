@@ -2,8 +2,8 @@
 //
 // A warp scores two queries (neighbours in length order, packed int16x2) against 32 refs
 // (neighbours in length order), one ref per lane.  The query's rows are cut into strips of R rows
-// (R <= 48, even up to 24 and a multiple of 4 beyond, so at most 3 rows per strip are padding); a lane keeps H
-// and Y of the strip's rows in registers and walks the columns of its ref, so there are no
+// (R <= 48, even up to 24 and a multiple of 4 beyond, so fewer than 4 rows a strip are padding: 49 rows are two
+// strips of 28); a lane keeps H and Y of the strip's rows in registers and walks the columns of its ref, so there are no
 // shuffles, no ramp and no idle lanes, which is where the query-pair wavefront (pairwise.cu) loses
 // its time: 31 of n + 31 steps, up to 31 padded rows and the per-step exchange.  Between strips the
 // bottom row's (H, next X) pair of each column goes through a per-warp slice of global scratch
@@ -27,10 +27,10 @@
 // in local mode a padded cell never exceeds the best cell before it.
 //
 // Measured, B200 at 1965 MHz, whole calls: 4,096 x 4,096 proteins (median 180 residues) global
-// distance 128 -> 94.6 ms (query-pair wavefront -> this), local scores of 1,501 x 4,003 of them
-// 66.4 -> 41.2 ms, 4,096 x 4,096 junctions (10-20) global distance 7.98 -> 0.73 ms (one int32
+// distance 128 -> 96 ms (query-pair wavefront -> this), local scores of 1,501 x 4,003 of them
+// 66.7 -> 39.9 ms, 4,096 x 4,096 junctions (10-20) global distance 7.98 -> 0.71 ms (one int32
 // thread per pair -> this).  ncu counts 4.26 ALU instructions per cell pair in global mode (4.7
-// local) at 76 % ALU pipe activity before the units were dealt from a queue.
+// local; 4.75 on junctions, at 82 % ALU pipe activity).
 #include <algorithm>
 #include <climits>
 #include <map>
