@@ -106,8 +106,6 @@ struct OwnedBuf {
     }
 };
 
-// Something made on one stream (a plan) that calls on any stream then read: other streams wait for it on the
-// device, nothing on the host does.  (Transient sets' calls are all on the context's stream.)
 struct StreamNow {  // a call's stream, looked at once
     cudaStream_t stream;
     unsigned long long id = 0;
@@ -115,6 +113,8 @@ struct StreamNow {  // a call's stream, looked at once
     explicit StreamNow(cudaStream_t s);
 };
 
+// Something made on one stream (a plan) that calls on any stream then read: other streams wait for it on the
+// device, nothing on the host does.  (Transient sets' calls are all on the context's stream.)
 struct Made {
     void on(cudaStream_t stream);      // everything enqueued on `stream` so far
     void need(const StreamNow& now);   // what follows on the stream may read it
