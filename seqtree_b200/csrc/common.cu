@@ -241,32 +241,86 @@ DevBuf::~DevBuf() {
 }
 
 namespace {
-// The device's pool, made with its context (a captured call may take memory but not make the pool).
-cudaMemPool_t scratch_pool(int device) {
-    constexpr uint64_t kKeep = uint64_t(256) << 20;  // bytes that stay cached in it
-    static std::mutex mu;
-    static std::map<int, cudaMemPool_t> pools;
-    std::lock_guard<std::mutex> lk(mu);
-    cudaMemPool_t& slot = pools[device];
-    if (!slot) {
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        cudaMemPool_t fresh = nullptr;
-        STB_CUDA(cudaMemPoolCreate(&fresh, &props));
-        uint64_t keep_bytes = kKeep;
-        STB_CUDA(cudaMemPoolSetAttribute(fresh, cudaMemPoolAttrReleaseThreshold, &keep_bytes));
-        slot = fresh;
-    }
-    return slot;
+// A device's two pools, made with its context (a captured call may take memory but not make a pool): the scratch
+// of calls, and what sets keep.  They cache 256 and 128 MB that nothing uses, and what else of a block of the
+// driver's (32 MB and more) is in use.  They are two because the
+// driver's threshold counts used memory too: beside 30 MB of plans the strips' scratch (232 MB) would be
+// unmapped at every synchronisation (local scores of 1,501 x 4,003 proteins 40 -> 67 ms).
+constexpr uint64_t kCached = uint64_t(256) << 20, kKeptCached = uint64_t(128) << 20;
+
+struct Pools {
+    cudaMemPool_t scratch = nullptr, kept = nullptr;
+    cudaStream_t frees = nullptr;  // kept memory goes back on it
+    uint64_t kept_threshold = kKeptCached;
+};
+
+std::mutex g_pool_mu;
+std::map<int, Pools>& g_pools = *new std::map<int, Pools>;  // until exit
+
+cudaMemPool_t make_pool(int device, uint64_t keep) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t pool = nullptr;
+    STB_CUDA(cudaMemPoolCreate(&pool, &props));
+    STB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    return pool;
+}
+
+Pools& pools_of(int device) {  // (under g_pool_mu)
+    Pools& p = g_pools[device];
+    if (!p.scratch) p.scratch = make_pool(device, kCached);
+    if (!p.kept) p.kept = make_pool(device, kKeptCached);
+    if (!p.frees) STB_CUDA(cudaStreamCreateWithFlags(&p.frees, cudaStreamNonBlocking));
+    return p;
+}
+
+// Moves the threshold of the kept memory with what is used of it, in steps of 64 MB; past kKeptCached unused bytes
+// the rest goes back at once.  (A few microseconds: looked at for pieces of at least kLarge.)
+constexpr size_t kLarge = size_t(1) << 20;
+void adjust_kept(Pools& p) {
+    uint64_t used = 0, reserved = 0;
+    if (cudaMemPoolGetAttribute(p.kept, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) return;
+    uint64_t want = (used + kKeptCached) >> 26 << 26;
+    if (want != p.kept_threshold &&
+        cudaMemPoolSetAttribute(p.kept, cudaMemPoolAttrReleaseThreshold, &want) == cudaSuccess)
+        p.kept_threshold = want;
+    if (cudaMemPoolGetAttribute(p.kept, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        reserved > used + kKeptCached)
+        cudaMemPoolTrimTo(p.kept, size_t(used + kKeptCached));
 }
 }  // namespace
 
-void StreamScratch::take(int device, size_t bytes, cudaStream_t st) {
+void StreamScratch::take(int device, size_t bytes, cudaStream_t st, bool to_keep) {
     if (!bytes) return;
-    STB_CUDA(cudaMallocFromPoolAsync(&ptr, bytes, scratch_pool(device), st));
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    Pools& p = pools_of(device);
+    STB_CUDA(cudaMallocFromPoolAsync(&ptr, bytes, to_keep ? p.kept : p.scratch, st));
     stream = st;
+    if (to_keep && bytes >= kLarge) adjust_kept(p);
+}
+
+// Nothing reads the memory any more.  (cudaFree would take it too, but the pool then counts it as used and gives
+// none of it back.)
+void kept_free(void* ptr, size_t bytes) {
+    if (!ptr) return;
+    cudaPointerAttributes at{};
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    const bool known = cudaPointerGetAttributes(&at, ptr) == cudaSuccess;
+    const auto it = known ? g_pools.find(at.device) : g_pools.end();
+    if (it == g_pools.end() || !it->second.frees) {
+        cudaGetLastError();
+        cudaFree(ptr);
+        return;
+    }
+    int prev = -1;
+    cudaGetDevice(&prev);
+    if (prev != at.device) cudaSetDevice(at.device);
+    if (cudaFreeAsync(ptr, it->second.frees) == cudaSuccess && bytes >= kLarge &&
+        cudaStreamSynchronize(it->second.frees) == cudaSuccess)
+        adjust_kept(it->second);
+    if (prev >= 0 && prev != at.device) cudaSetDevice(prev);
 }
 
 void refuse_capture(cudaStream_t stream) {
@@ -282,12 +336,13 @@ void* OwnedBuf::get(size_t bytes, cudaStream_t stream) {
     refuse_capture(stream);  // (the memory would belong to the graph)
     if (ptr) {
         STB_CUDA(cudaDeviceSynchronize());  // kernels of any stream may read the old one
-        cudaFree(ptr);
+        kept_free(ptr, cap);
         ptr = nullptr;
         cap = 0;
     }
     const size_t want = (std::max<size_t>(bytes + bytes / 8, 256) + 255) & ~size_t(255);
-    StreamScratch fresh(context().device, want, stream);
+    StreamScratch fresh;
+    fresh.take(context().device, want, stream, true);
     ptr = fresh.keep();
     cap = want;
     return ptr;
@@ -391,7 +446,10 @@ Context& context() {
                                     dev));
     STB_CUDA(cudaMalloc(&c->flags_d, 64 * sizeof(int64_t)));
     STB_CUDA(cudaHostAlloc(&c->flags_h, 64 * sizeof(int64_t), cudaHostAllocDefault));
-    scratch_pool(dev);
+    {
+        std::lock_guard<std::mutex> pools(g_pool_mu);
+        pools_of(dev);
+    }
     Context& ref = *c;
     g_ctx.emplace(dev, std::move(c));
     return ref;

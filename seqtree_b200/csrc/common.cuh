@@ -67,15 +67,18 @@ struct DevBuf {
     ~DevBuf();
 };
 
-// Stream-ordered memory from a pool of the library's own: calls on several streams each get theirs, a
+// Stream-ordered memory from pools of the library's own: calls on several streams each get theirs, a
 // captured call gets its allocation as graph nodes, and a bounded amount stays cached for the next.  Freed
-// on the stream it was taken for, unless keep() hands it to an owner.
+// on the stream it was taken for, unless keep() hands it (taken to_keep) to an owner, which gives it to
+// kept_free() once nothing reads it.
+void kept_free(void* ptr, size_t bytes);
+
 struct StreamScratch {
     void* ptr = nullptr;
     cudaStream_t stream = nullptr;
     StreamScratch() = default;
     StreamScratch(int device, size_t bytes, cudaStream_t st) { take(device, bytes, st); }
-    void take(int device, size_t bytes, cudaStream_t st);
+    void take(int device, size_t bytes, cudaStream_t st, bool to_keep = false);
     void* keep() {
         void* p = ptr;
         ptr = nullptr;
@@ -89,7 +92,7 @@ struct StreamScratch {
 };
 
 // The buffers of a set's plans: they grow, and go with their owner (whose destructor frees device memory of its
-// own first, which waits for the kernels that still read them).  From the library's pool, as plans come
+// own first, which waits for the kernels that still read them).  From the library's pools, as plans come
 // and go with their sets: cudaMalloc after such a free had to map memory again, 1 to 2 ms in a first
 // call on new sets (B200).
 struct OwnedBuf {
@@ -101,9 +104,7 @@ struct OwnedBuf {
     OwnedBuf() = default;
     OwnedBuf(const OwnedBuf&) = delete;
     OwnedBuf& operator=(const OwnedBuf&) = delete;
-    ~OwnedBuf() {
-        if (ptr) cudaFree(ptr);
-    }
+    ~OwnedBuf() { kept_free(ptr, cap); }
 };
 
 struct StreamNow {  // a call's stream, looked at once

@@ -65,6 +65,7 @@ struct Kept {
     Form form;
     uint32_t symbols[8];
     void* ptr;
+    size_t bytes;
     std::shared_ptr<Made> made;
 };
 
@@ -76,7 +77,7 @@ struct DistPlan {
     DevBuf transient[2];            // by form
     ~DistPlan() {  // (with the set, after its bytes: freeing those waits for the kernels that read either)
         for (const Kept& k : kept)
-            if (owns) cudaFree(k.ptr);
+            if (owns) kept_free(k.ptr, k.bytes);
     }
 };
 
@@ -136,10 +137,12 @@ struct CallForms {
     void* ptr[2] = {};
     int todo[2], count = 0;         // the sets whose form is to be made, with one launch on the call's stream
     StreamScratch fresh[2];
+    size_t size[2];
     bool keep[2] = {};
 
     CallForms(Form form, const Alphabet& al, st_seqset_s* const sets[2], DistPlan* const plans[2],
-              const size_t bytes[2], cudaStream_t stream, Context& ctx) {
+              const size_t (&bytes)[2], cudaStream_t stream, Context& ctx)
+        : size{bytes[0], bytes[1]} {
         for (int t = 0; t < 2; ++t) {
             if (t == 1 && sets[0] == sets[1]) {
                 ptr[1] = ptr[0];
@@ -157,7 +160,7 @@ struct CallForms {
             keep[t] = !p.owns || have < kMaxKept;
             if (keep[t]) refuse_capture(stream);
             if (p.owns) {
-                fresh[t].take(ctx.device, std::max<size_t>(bytes[t], 16), stream);
+                fresh[t].take(ctx.device, std::max<size_t>(bytes[t], 16), stream, keep[t]);
                 ptr[t] = fresh[t].ptr;
             } else {
                 ptr[t] = p.transient[form].get(bytes[t]);
@@ -169,7 +172,7 @@ struct CallForms {
     void made(Form form, const Alphabet& al, DistPlan* const plans[2], cudaStream_t stream) {
         for (int t = 0; t < 2; ++t) {
             if (!keep[t]) continue;
-            Kept k{form, {}, ptr[t], std::make_shared<Made>()};
+            Kept k{form, {}, ptr[t], size[t], std::make_shared<Made>()};
             std::memcpy(k.symbols, al.symbols, 32);
             if (plans[t]->owns) k.made->on(stream);
             plans[t]->kept.push_back(std::move(k));
