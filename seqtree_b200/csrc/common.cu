@@ -354,7 +354,7 @@ void Made::on(cudaStream_t stream) {
     STB_CUDA(cudaEventRecord(event, stream));
 }
 
-ScratchTurn::ScratchTurn(Context& c, cudaStream_t s) : ctx(c), now(s) {
+ScratchTurn::ScratchTurn(Context& c, cudaStream_t s) : ctx(c), now(c, s) {
     if (!now.capturing) ctx.scratch.need(now);
 }
 
@@ -373,6 +373,9 @@ StreamNow::StreamNow(cudaStream_t s) : stream(s) {
     capturing = st != cudaStreamCaptureStatusNone;
     if (!capturing) STB_CUDA(cudaStreamGetId(s, &id));
 }
+
+StreamNow::StreamNow(const Context& ctx, cudaStream_t s)
+    : StreamNow(s == ctx.stream ? StreamNow(s, ctx.stream_id) : StreamNow(s)) {}
 
 void Made::need(const StreamNow& now) {
     if (!event) return;
@@ -441,6 +444,7 @@ Context& context() {
     auto c = std::make_unique<Context>();
     c->device = dev;
     STB_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+    STB_CUDA(cudaStreamGetId(c->stream, &c->stream_id));
     STB_CUDA(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, dev));
     STB_CUDA(cudaDeviceGetAttribute(&c->max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin,
                                     dev));

@@ -67,6 +67,8 @@ struct DevBuf {
     ~DevBuf();
 };
 
+struct Context;
+
 // Stream-ordered memory from pools of the library's own: calls on several streams each get theirs, a
 // captured call gets its allocation as graph nodes, and a bounded amount stays cached for the next.  Freed
 // on the stream it was taken for, unless keep() hands it (taken to_keep) to an owner, which gives it to
@@ -112,6 +114,10 @@ struct StreamNow {  // a call's stream, looked at once
     unsigned long long id = 0;
     bool capturing = false;
     explicit StreamNow(cudaStream_t s);
+    StreamNow(const Context& ctx, cudaStream_t s);  // (nothing to look at for the context's own stream)
+
+private:
+    StreamNow(cudaStream_t s, unsigned long long known) : stream(s), id(known) {}
 };
 
 // Something made on one stream (a plan) that calls on any stream then read: other streams wait for it on the
@@ -138,6 +144,7 @@ struct Context {
     int device = 0;
     std::mutex mu;              // serialises calls on this device
     cudaStream_t stream = nullptr;
+    unsigned long long stream_id = 0;
     int num_sms = 148;
     int max_smem_optin = 0;
     // Small device word area for error reporting, with a pinned host mirror.  Word 0: first

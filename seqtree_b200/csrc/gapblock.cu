@@ -1015,7 +1015,7 @@ void gapblock_run(st_seqset_s& qs, st_seqset_s& rs, const int32_t* penalty, int3
     const bool wide = maxpen > 255;  // the penalties of four queries do not fit one word
     // Tables for this (matrix, gaps, prior, lengths): kept, so repeated calls with the same arguments
     // enqueue nothing but the kernel.
-    const StreamNow now(stream);
+    const StreamNow now(ctx, stream);
     static const GbTables no_tables;  // (the general kernel reads none)
     const GbTables* tbp = &no_tables;
     if (fast) {
