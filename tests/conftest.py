@@ -81,7 +81,7 @@ def as_np(sm) -> np.ndarray:
 
 @pytest.hookimpl(wrapper=True)
 def pytest_runtest_call(item):
-    """A test whose checker is the reference's own build is skipped where that build cannot be made (the
+    """A test whose oracle is the reference's own build is skipped where that build cannot be made (the
     reference's sources are absent)."""
     try:
         return (yield)
